@@ -11,7 +11,7 @@ namespace kache_b200
 // Inserts one key with its value, known absent (every key of a table is distinct), into `T`. Returns INSERTED or
 // OV_FULL. No other thread inserts the same key, so none waits for the value: no fence before publishing.
 template <bool set_>
-__device__ __forceinline__ uint32_t place_key(const Dev_Table& T, const uint64_t key, const uint64_t h, const unsigned long long val)
+__device__ __forceinline__ uint32_t place_key(const Dev_Table& T, const uint64_t key, const uint32_t h, const unsigned long long val)
 {
     Landing L{};
     const uint32_t r = upsert_chain<set_>(T, key, h, checksum_of(key), L);
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) split_kernel(const Dev_Table from, const 
     for(uint64_t b = uint64_t(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5); b < from.cap; b += warps)
     {
         const uint64_t s = b * B + lane;
-        const uint8_t c = from.cs[s];
+        const uint8_t c = *cs_of(from, static_cast<uint32_t>(b), lane);
         unsigned long long key_st = 0, val = 0;
         uint32_t dest = 0xFFFFFFFFu;
         if(c)
@@ -109,9 +109,9 @@ __global__ void __launch_bounds__(256) split_kernel(const Dev_Table from, const 
             key_st = from.slots[s * slot_words<set_>()];
             if constexpr(!set_)
                 val = from.slots[s * 2 + 1];
-            const uint64_t h = minimizer_hash<k, l>(~key_st);
+            const uint32_t h = minimizer_hash<k, l>(~key_st);
             if(bucket_of(h, from.cap) == b)
-                dest = static_cast<uint32_t>(bucket_of(h, to.cap) - (b << d));
+                dest = bucket_of(h, to.cap) - static_cast<uint32_t>(b << d);
         }
         const uint32_t other = __ballot_sync(0xFFFFFFFFu, c != 0 && dest == 0xFFFFFFFFu);
         if(lane == 0 && other)
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(256) split_kernel(const Dev_Table from, const 
             to.slots[ns * slot_words<set_>()] = lane < n ? k_j : 0ull;
             if constexpr(!set_)
                 to.slots[ns * 2 + 1] = lane < n ? v_j : 0ull;
-            to.cs[ns] = lane < n ? static_cast<uint8_t>(c_j) : 0;
+            *cs_of(to, static_cast<uint32_t>(nb), lane) = lane < n ? static_cast<uint8_t>(c_j) : 0;
             if(lane < 8)
                 to.spill[nb * 8 + lane] = 0;
         }
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256) collect_kernel(const Dev_Table T, const u
         if(s < n_main)
         {
             const uint64_t slot = b_b * B + s;
-            if(T.cs[slot])
+            if(*cs_of(T, static_cast<uint32_t>(slot / B), slot % B))
             {
                 have = true;
                 key_st = T.slots[slot * slot_words<set_>()];
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) collect_kernel(const Dev_Table T, const u
         if(have)
         {
             const uint64_t o = base + __popc(m & ((1u << lane) - 1));
-            keys[o] = ~key_st;
+            keys[o] = encoding_of(~key_st);
             if(vals)
                 vals[o] = val;
         }
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const Dev_Table T, const ui
         unsigned long long raw = 0;
         if(s < n_main)
         {
-            have = T.cs[s] != 0;
+            have = *cs_of(T, static_cast<uint32_t>(s / B), s % B) != 0;
             if constexpr(!set_)
                 if(have)
                     raw = T.slots[s * 2 + 1];
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256) distribution_kernel(const Dev_Table T, un
     unsigned long long p = 0, s2 = 0;
     for(uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < n_main; s += uint64_t(gridDim.x) * blockDim.x)
     {
-        if(!T.cs[s])
+        if(!*cs_of(T, static_cast<uint32_t>(s / B), s % B))
             continue;
         const uint64_t key = ~T.slots[s * slot_words<set_>()];
         if(bucket_of(minimizer_hash<k, l>(key), T.cap) == s / B)
@@ -311,73 +311,87 @@ static __global__ void batch_counts_kernel(const uint64_t* off, const uint64_t n
 
 // The counting and summing of a small device batch's staging in one block of 1024 threads: each thread takes a run
 // of sequences; pos_off[0..n] and seg_off[0..n] get the exclusive sums of positions and segments, and out[0..2] the
-// positions, the segments and whether a sequence has more segments than a list entry indexes. In place of a counting
-// kernel, two scans and their copies; segs_kernel then lists the segments.
+// positions, the segments and the segment length, fitted to the batch (fitted_seg_len, then eight times longer while
+// the longest sequence would have more segments than a list entry indexes). In place of a counting kernel, two scans
+// and their copies; segs_kernel then lists the segments.
 constexpr uint32_t small_stage_max = 4096;  // Sequences of a batch summed by one block (at most 4 per thread).
 
-static __global__ void __launch_bounds__(1024) stage_small_kernel(const uint64_t* off, const uint64_t n, const int k, const uint32_t seg_len,
-                                                                 uint64_t* pos_off, uint64_t* seg_off, unsigned long long* out)
+// The inclusive sum of x over the block's threads in order; `warps` is 32 words of shared memory.
+__device__ __forceinline__ unsigned long long block_sum(unsigned long long x, unsigned long long* warps)
 {
-    __shared__ unsigned long long wp[32], ws[32];
-    __shared__ unsigned int long_seq;
-    const uint32_t t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    if(t == 0)
-        long_seq = 0;
-    const uint64_t per = (n + 1023) / 1024, q0 = min(n, uint64_t(t) * per), q1 = min(n, q0 + per);
-    unsigned long long P = 0, S = 0;
-    bool too_long = false;
-    for(uint64_t q = q0; q < q1; ++q)
-    {
-        const uint64_t len = off[q + 1] - off[q];
-        const uint64_t np = len >= uint64_t(k) ? len - k + 1 : 0, ns = (np + seg_len - 1) / seg_len;
-        P += np, S += ns;
-        too_long |= ns > max_seg_index + 1;
-    }
-    // Exclusive prefix sums over the block: within warps by shuffles, then over the warps' totals.
-    unsigned long long ip = P, is = S;
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for(int o = 1; o < 32; o <<= 1)
     {
-        const unsigned long long a = __shfl_up_sync(0xFFFFFFFFu, ip, o), b = __shfl_up_sync(0xFFFFFFFFu, is, o);
+        const unsigned long long a = __shfl_up_sync(0xFFFFFFFFu, x, o);
         if(lane >= static_cast<uint32_t>(o))
-            ip += a, is += b;
+            x += a;
     }
     if(lane == 31)
-        wp[wid] = ip, ws[wid] = is;
+        warps[wid] = x;
     __syncthreads();
-    if(too_long)
-        atomicOr(&long_seq, 1u);
     if(wid == 0)
     {
-        unsigned long long a = wp[lane], b = ws[lane];
+        unsigned long long a = warps[lane];
 #pragma unroll
         for(int o = 1; o < 32; o <<= 1)
         {
-            const unsigned long long x = __shfl_up_sync(0xFFFFFFFFu, a, o), y = __shfl_up_sync(0xFFFFFFFFu, b, o);
+            const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, a, o);
             if(lane >= static_cast<uint32_t>(o))
-                a += x, b += y;
+                a += y;
         }
-        wp[lane] = a, ws[lane] = b;
+        warps[lane] = a;
     }
     __syncthreads();
-    unsigned long long bp = ip - P + (wid ? wp[wid - 1] : 0), bs = is - S + (wid ? ws[wid - 1] : 0);
-    for(uint64_t q = q0; q < q1; ++q)
+    return x + (wid ? warps[wid - 1] : 0);
+}
+
+static __global__ void __launch_bounds__(1024) stage_small_kernel(const uint64_t* off, const uint64_t n, const int k, const uint32_t sms,
+                                                                 uint64_t* pos_off, uint64_t* seg_off, unsigned long long* out)
+{
+    __shared__ unsigned long long wp[32], ws[32], longest;
+    const uint32_t t = threadIdx.x;
+    if(t == 0)
+        longest = 0;
+    const uint64_t per = (n + 1023) / 1024, q0 = min(n, uint64_t(t) * per), q1 = min(n, q0 + per);
+    const auto npos = [&](const uint64_t q) -> uint64_t
     {
         const uint64_t len = off[q + 1] - off[q];
-        const uint64_t np = len >= uint64_t(k) ? len - k + 1 : 0, ns = (np + seg_len - 1) / seg_len;
+        return len >= uint64_t(k) ? len - k + 1 : 0;
+    };
+    unsigned long long P = 0, S = 0, top = 0;
+    for(uint64_t q = q0; q < q1; ++q)
+    {
+        const unsigned long long np = npos(q);
+        P += np, top = max(top, np);
+    }
+    unsigned long long bp = block_sum(P, wp) - P;
+    atomicMax(&longest, top);
+    __syncthreads();
+    uint64_t seg_len = fitted_seg_len(wp[31], sms);
+    while((longest + seg_len - 1) / seg_len > max_seg_index + 1)
+        seg_len *= 8;
+    for(uint64_t q = q0; q < q1; ++q)
+        S += (npos(q) + seg_len - 1) / seg_len;
+    unsigned long long bs = block_sum(S, ws) - S;
+    for(uint64_t q = q0; q < q1; ++q)
+    {
+        const uint64_t np = npos(q);
         pos_off[q] = bp, seg_off[q] = bs;
-        bp += np, bs += ns;
+        bp += np, bs += (np + seg_len - 1) / seg_len;
     }
     if(t == 1023)
     {
         pos_off[n] = wp[31], seg_off[n] = ws[31];
-        out[0] = wp[31], out[1] = ws[31], out[2] = long_seq;
+        out[0] = wp[31], out[1] = ws[31], out[2] = seg_len;
     }
 }
 
 // Lists the segments, one thread per segment: its sequence by binary search in seg_off[0..n] (exclusive sums of
-// segments per sequence), so that long sequences' many segments are listed in parallel.
-static __global__ void segs_kernel(const uint64_t* seg_off, const uint64_t n, const uint64_t nsegs, uint64_t* segs)
+// segments per sequence), so that long sequences' many segments are listed in parallel. Sequence q's bases are at offset
+// off[q], or with `addr` at the address addr[q].
+static __global__ void segs_kernel(const uint64_t* seg_off, const uint64_t* pos_off, const uint64_t* off, const uint64_t* addr, const uint64_t n, const uint64_t nsegs,
+                                   const uint32_t seg_len, Segment* segs)
 {
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
     for(uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nsegs; i += stride)
@@ -391,11 +405,10 @@ static __global__ void segs_kernel(const uint64_t* seg_off, const uint64_t n, co
             else
                 hi = mid;
         }
-        segs[i] = (lo << 24) | (i - seg_off[lo]);
+        const uint64_t p0 = (i - seg_off[lo]) * seg_len, first = pos_off[lo] + p0;
+        segs[i] = Segment{(addr ? addr[lo] : off[lo]) + p0, first, lo, static_cast<uint32_t>(min(pos_off[lo + 1] - first, static_cast<uint64_t>(seg_len))), 0};
     }
 }
-
-
 
 // Several device batches run as one call. desc holds 8 words per batch -- bases, offsets, sequences, first merged
 // sequence, out0, out1, out2, 0 -- in batch order. For merged sequence q: its batch, its length (the merged offsets are

@@ -2,15 +2,25 @@
 // row, and hands each row's k-mers to a visitor (upsert, update, lookup, count, ...), one k-mer per lane.
 //
 // What it computes per position is the reference describers' description (include/Kmer_Batch.hpp:191-250,
-// include/Kmer_Lanes.hpp:164-244): the canonical key, its orientation, its checksum and its l-minimizer hash. How:
-//   - each row of 32 bases is loaded coalesced (lane j reads base j), turned into 2-bit codes and an ACGT bit, and
-//     packed by warp OR-reductions into a forward word W (first base most significant) and a complemented word R
-//     (first base least significant), once per row rather than once per k-mer;
-//   - lane j's k-mer is a 2k-bit funnel window of (W_r, W_r+1) and its reverse complement one of (R_r, R_r+1);
-//   - each lane hashes the l-mer at its position; the minima of neighbouring pairs of those hashes go to a per-warp
-//     ring in shared memory, and a k-mer's minimizer hash, the least of the w = k - l + 1 hashes from its own position
-//     on, is the least of ceil(w / 2) pair minima;
+// include/Kmer_Lanes.hpp:164-244) with this library's placement hash (device_common.cuh): the canonical key, its
+// orientation, its checksum and its minimizer hash. How:
+//   - each row of 32 bases is loaded coalesced (lane j reads base j); three ballots per row hold its ACGT flags and its
+//     codes' high and low bits, base j at bit j;
+//   - lane j's k-mer is a window of k bits of each plane, one funnel shift of two consecutive rows. First base lowest,
+//     its complement is the reverse complement's plane; bit-reversed, it is the forward plane;
+//   - the l-mer at a k-mer's start is a shift of its forward planes and a mask of its reverse ones. Each lane hashes
+//     that one; the minima of neighbouring pairs of hashes go to a per-warp ring in shared memory, and a k-mer's
+//     minimizer hash, the least of the w = k - l + 1 hashes from its own position on, is the least of ceil(w / 2) pair
+//     minima;
 //   - non-ACGT characters split sequences (DNA_Utility.hpp:199-224): a window with one is not a k-mer.
+// Every operation runs so, also those without per-position outputs: consecutive k-mers share minimizers, so a row of 32
+// touches about seven buckets where 32 lanes on 32 different reads would touch 32 (a lane per segment, rolling its k-mers,
+// took 9.19 ms for 130M upserts into a 6.7 GB map, rows 3.1 ms; 7.1 against 4.0 ms for 190M updates).
+//
+// What bounds it is instructions (about 290 per row in a lookup, the integer pipe two thirds busy) and, next, the latency
+// of three dependent loads; so more resident warps pay even at the price of some spills: six blocks of 256 threads per SM
+// (40 registers) against five, four and three, lookup of 120M positions 1.81 against 1.82, 1.80 (a variant that overlapped
+// two rows) and 2.29 ms, upsert of 40M 1.08 against 1.11, 1.15 and 1.46 ms.
 // Sequences are cut into segments of up to `seg_positions` positions; each segment re-reads the k - 1 bases it
 // shares with the next, so segments, like the reference's lanes (include/Streaming_Kmer_Hash_Table.hpp:1751-1781),
 // need no state from one another.
@@ -21,173 +31,182 @@
 namespace kache_b200
 {
 
-// A batch on the device: sequence q is bases[off[q], off[q+1]); segs lists (q << 24 | s) for the s'th segment, of
-// seg_len positions, of each sequence of at least k bases; pos_off[q] counts the positions of the sequences before q.
-// With seq_addr set (several batches run as one), off only lays the lengths end to end and sequence q's
-// off[q+1] - off[q] bases are read at the device address seq_addr[q], where its own batch holds them.
+// A segment: up to seg_len consecutive k-mer positions of one sequence, with all that a warp needs to start on it in one
+// 32-byte entry.
+struct alignas(16) Segment
+{
+    uint64_t base;      // Its first base, as an offset from the batch's bases.
+    uint64_t pos;       // Its first position, counted over the batch's sequences.
+    uint64_t q;         // Its sequence.
+    uint32_t npos;      // Its positions.
+    uint32_t unused;
+};
+
+// A batch on the device: its segments in sequence order. Several batches run as one have no bases in common (null): their
+// segments' offsets are addresses.
 struct Dev_Batch
 {
     const uint8_t* bases;
-    const uint64_t* off;
-    const uint64_t* segs;
-    const uint64_t* pos_off;
-    uint64_t n;
-    uint64_t nsegs;
-    uint32_t seg_len;   // A multiple of 32.
-    const uint64_t* seq_addr = nullptr;
-
-    __device__ __forceinline__ const uint8_t* seq(const uint64_t q, const uint64_t b0) const
-    {
-        return seq_addr ? reinterpret_cast<const uint8_t*>(seq_addr[q]) : bases + b0;
-    }
+    const Segment* segs;
 };
 
 constexpr int stream_warps = 8;
 
-// One row of 32 bases, packed.
+// One row of 32 bases: base j's flag (one of A, C, G, T) and code bits at bit j.
 struct Row
 {
-    uint64_t W, R;
-    uint32_t valid;
+    uint32_t hi, lo, valid;
 };
 
-// The row at offset o of a segment, through this lane's base pointer sp (the segment's first base + lane) and its
-// bound rem (the sequence's bases from sp on, capped at 2^30): 32-bit arithmetic per row.
-__device__ __forceinline__ Row load_row(const uint8_t* sp, const int32_t rem, const uint32_t o, const uint32_t lane)
+constexpr int base_table_bytes = 256;
+
+// Fills a block's table of base_bits by character, in shared memory (one load per base in place of the tests).
+__device__ __forceinline__ void fill_base_table(uint8_t* tab)
 {
-    constexpr uint32_t all = 0xFFFFFFFFu;
-    const uint32_t ch = static_cast<int32_t>(o) < rem ? sp[o] : 0u;
-    const uint32_t x = (ch | 0x20u) - 'a';
-    const bool ok = x < 20u && ((0x80045u >> x) & 1u);     // a, c, g, t
-    const uint32_t code = ((ch >> 2) ^ (ch >> 1)) & 3u;
-    const bool first = lane < 16;
-    const uint32_t s = 2 * (lane & 15);
-    const uint32_t f = code << (30 - s), z = code << s;
-    Row r;
-    r.valid = __ballot_sync(all, ok);
-    // Base j at bits 63 - 2j .. 62 - 2j of W, and at bits 2j .. 2j + 1 of ~R.
-    const uint32_t w_hi = __reduce_or_sync(all, first ? f : 0u), w_lo = __reduce_or_sync(all, first ? 0u : f);
-    const uint32_t z_lo = __reduce_or_sync(all, first ? z : 0u), z_hi = __reduce_or_sync(all, first ? 0u : z);
-    r.W = (uint64_t(w_hi) << 32) | w_lo;
-    r.R = ~((uint64_t(z_hi) << 32) | z_lo);
-    return r;
+    for(uint32_t ch = threadIdx.x; ch < base_table_bytes; ch += blockDim.x)
+        tab[ch] = base_bits(ch);
+    __syncthreads();
 }
 
-// The forward and reverse-complement n-mers (n <= 32) starting at base j of row a, spilling into row b: 64-bit
-// windows of the 128-bit pairs (a.W, b.W) and (b.R, a.R) at bit offset 2j, as two 32-bit funnel shifts each; which
-// words feed them depends on the lane only (j >= 16).
-template <int n>
-__device__ __forceinline__ void window(const Row& a, const Row& b, const uint32_t j, uint64_t& f, uint64_t& r)
+// A row of characters, one per lane.
+__device__ __forceinline__ Row pack_row(const uint32_t ch, const uint8_t* tab)
 {
-    const bool big = j >= 16;
-    const uint32_t sh = (2 * j) & 31;
-    const uint32_t a1 = static_cast<uint32_t>(a.W >> 32), a0 = static_cast<uint32_t>(a.W);
-    const uint32_t b1 = static_cast<uint32_t>(b.W >> 32), b0 = static_cast<uint32_t>(b.W);
-    const uint32_t x3 = big ? a0 : a1, x2 = big ? b1 : a0, x1 = big ? b0 : b1;
-    const uint64_t top = (uint64_t(__funnelshift_l(x2, x3, sh)) << 32) | __funnelshift_l(x1, x2, sh);
-    f = top >> (64 - 2 * n);
-    const uint32_t r0 = static_cast<uint32_t>(a.R), r1 = static_cast<uint32_t>(a.R >> 32);
-    const uint32_t r2 = static_cast<uint32_t>(b.R), r3 = static_cast<uint32_t>(b.R >> 32);
-    const uint32_t y0 = big ? r1 : r0, y1 = big ? r2 : r1, y2 = big ? r3 : r2;
-    const uint64_t low = (uint64_t(__funnelshift_r(y1, y2, sh)) << 32) | __funnelshift_r(y0, y1, sh);
-    r = low & kmer_mask(n);
+    constexpr uint32_t all = 0xFFFFFFFFu;
+    const uint32_t t = tab[ch];
+    Row r;
+    r.valid = __ballot_sync(all, t & 1u);
+    r.lo = __ballot_sync(all, t & 2u);
+    r.hi = __ballot_sync(all, t & 4u);
+    return r;
 }
 
 // A k-mer as the visitors get it.
 struct Kmer_Desc
 {
-    uint64_t key, h;
-    uint64_t q, pos;    // Sequence and position in it.
-    uint64_t out;       // Index of the position in the batch's outputs (set by the lane kernel; 0 in the warp kernel).
-    uint8_t c;
+    uint64_t key;       // Its canonical form's planes.
+    uint32_t pos;       // Position in the segment.
+    uint32_t h;         // Minimizer hash.
     bool fwd;           // Occurs as its canonical form.
     bool valid;         // All k characters are ACGT.
     bool in;            // The position exists (is in the segment).
-    bool last;          // Unused; false.
 };
 
+constexpr int ring_words = 96;  // A warp's ring: two rows of 32, then a copy of the first row (entries up to w <= 32).
+
+// A row's k-mers as a row ahead of the visits holds them: the canonical key and two flags.
+struct Row_Kmers
+{
+    uint64_t key;
+    bool fwd, acgt;
+};
+
+// This lane's k-mer in the window that starts in row a, and the hash of the l-mer that it starts with.
+template <int k, int l>
+__device__ __forceinline__ Row_Kmers window(const Row& a, const Row& b, const uint32_t lane, uint32_t& lmer)
+{
+    constexpr uint32_t km = (k == 32 ? ~0u : (1u << k) - 1), lm = (1u << l) - 1;
+    const uint32_t hi = __funnelshift_r(a.hi, b.hi, lane), lo = __funnelshift_r(a.lo, b.lo, lane);
+    const Planes f{__brev(hi) >> (32 - k), __brev(lo) >> (32 - k)}, r{~hi & km, ~lo & km};
+    const bool gt = planes_greater(f, r);
+    Row_Kmers x;
+    x.key = gt ? key_of(r) : key_of(f);
+    x.fwd = !gt;
+    x.acgt = (__funnelshift_r(a.valid, b.valid, lane) & km) == km;
+    lmer = lmer_hash(Planes{f.hi >> (k - l), f.lo >> (k - l)}, Planes{r.hi & lm, r.lo & lm});
+    return x;
+}
+
+// Describes a segment of npos positions, whose bases start at seq, to the visitor, by a whole warp.
 template <int k, int l, typename Visitor>
-__global__ void __launch_bounds__(32 * stream_warps) stream_kernel(const Dev_Batch batch, const uint64_t seg_b, const uint64_t seg_e, Visitor vis)
+__device__ __forceinline__ void describe_segment(const uint8_t* const seq, const uint32_t npos, uint32_t* const ring, const uint8_t* const tab,
+                                                 const uint32_t lane, Visitor& vis)
 {
     constexpr int w = k - l + 1;
     static_assert(k <= 32 && l < k && w <= 32, "k-mers in a machine word, minimizers of at least two l-mers");
     constexpr uint32_t all = 0xFFFFFFFFu;
-    // Pair minima: entry 32 (r & 1) + j is min(H[i - 1], H[i]) for position i = 32 r + j of the segment, where H are
-    // the l-mer hashes; rows r and r + 1 are held.
-    __shared__ uint64_t ring_all[stream_warps][64];
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint64_t* ring = ring_all[wid];
-    vis.begin();
+    const uint32_t bases = npos + k - 1;
+    // Characters are asked for a row ahead of their use: L1 returns loads in order, so one waited for at once would wait
+    // for the table's sectors that other warps miss in front of it.
+    const auto load = [&](const uint32_t o) -> uint32_t { return o + lane < bases ? __ldg(seq + o + lane) : 0u; };
+    const uint32_t ch0 = load(0), ch1 = load(32);
+    uint32_t ch = load(64);
 
-    const uint64_t warps = uint64_t(gridDim.x) * stream_warps;
-    for(uint64_t g = seg_b + uint64_t(blockIdx.x) * stream_warps + wid; g < seg_e; g += warps)
+    // Ring entry 32 (r & 1) + j is min(H[i - 1], H[i]) for position i = 32 r + j of the segment, where H are the l-mer
+    // hashes; rows r and r + 1 are held. An even row's first entries are also at 64 + j, so that a window of an odd row
+    // reads past its end.
+    const Row r0 = pack_row(ch0, tab);
+    Row r1 = pack_row(ch1, tab);
+    uint32_t hash;      // Of this lane's l-mer in the newest row described.
+    Row_Kmers x = window<k, l>(r0, r1, lane, hash);
+    const uint32_t left = __shfl_up_sync(all, hash, 1);
+    ring[lane] = min(left, hash);   // Entry 0 is never read.
+
+    // The k-mers of the row at offset o, whose windows were taken when the row before was described; takes the next
+    // row's windows, whose first hashes this row's minimizers need.
+    const auto describe = [&](const uint32_t o)
     {
-        const uint64_t packed = batch.segs[g];
-        const uint64_t q = packed >> 24, s = packed & 0xFFFFFF;
-        const uint64_t b0 = batch.off[q], len = batch.off[q + 1] - b0;
-        const uint8_t* seq = batch.seq(q, b0);
-        const uint64_t npos = len - k + 1;
-        const uint64_t p0 = s * batch.seg_len;
-        const uint64_t p1 = min(npos, p0 + batch.seg_len);
-        const uint32_t rows = static_cast<uint32_t>((p1 - p0 + 31) / 32);
-        const uint32_t in_seg = static_cast<uint32_t>(p1 - p0);
-        const uint8_t* sp = seq + p0 + lane;
-        const int32_t rem = static_cast<int32_t>(min(len - p0, uint64_t(1) << 30)) - static_cast<int32_t>(lane);
+        const uint32_t half = o & 32;
+        __syncwarp();       // The previous row's reads of the ring are done.
+        const Row r2 = pack_row(ch, tab);
+        ch = load(o + 96);
+        const uint32_t last = __shfl_sync(all, hash, 31);
+        const Row_Kmers y = window<k, l>(r1, r2, lane, hash);
+        const uint32_t up = __shfl_up_sync(all, hash, 1), pair = min(lane ? up : last, hash);
+        ring[(half ^ 32) + lane] = pair;
+        if(half && lane < w)
+            ring[64 + lane] = pair;
+        __syncwarp();
 
-        Row r0 = load_row(sp, rem, 0, lane);
-        Row r1 = load_row(sp, rem, 32, lane);
-        uint64_t hprev;     // This lane's l-mer hash in the newest row hashed.
-        {
-            uint64_t f, rc;
-            window<l>(r0, r1, lane, f, rc);
-            hprev = wang_u64(f < rc ? f : rc);
-            const uint64_t left = __shfl_up_sync(all, hprev, 1);
-            ring[lane] = lane ? min64(left, hprev) : hprev;  // Entry 0 is never read.
-        }
-
-        vis.begin_segment(q);
-        for(uint32_t r = 0; r < rows; ++r)
-        {
-            const Row r2 = load_row(sp, rem, 32 * (r + 2), lane);
-            {
-                uint64_t f, rc;
-                window<l>(r1, r2, lane, f, rc);
-                const uint64_t hc = wang_u64(f < rc ? f : rc);
-                const uint64_t up = __shfl_up_sync(all, hc, 1), last = __shfl_sync(all, hprev, 31);
-                ring[((r + 1) & 1) * 32 + lane] = min64(lane ? up : last, hc);
-                hprev = hc;
-            }
-            __syncwarp();
-
-            Kmer_Desc d;
-            uint64_t f, rc;
-            window<k>(r0, r1, lane, f, rc);
-            // ACGT flags of the 32 bases from this lane's position on (k <= 32 of them make its k-mer).
-            const uint32_t vbits = __funnelshift_r(r0.valid, r1.valid, lane);
-            constexpr uint32_t km = (k == 32 ? 0xFFFFFFFFu : (1u << k) - 1);
-            d.pos = p0 + 32 * r + lane;
-            d.out = 0, d.last = false;
-            d.q = q;
-            d.in = 32 * r + lane < in_seg;
-            d.valid = d.in && (vbits & km) == km;
-            d.key = f < rc ? f : rc;
-            d.fwd = f <= rc;
-            d.c = checksum_of(d.key);
-            // Pairs (i - 1, i) at i = j + 1, j + 3, ...: w / 2 of them cover [j, j + w - 1] for even w; for odd w the
-            // pair at j + w - 1 adds the last hash.
-            uint64_t h = ~0ull;
-            const uint32_t base = (r & 1) * 32 + lane;
+        Kmer_Desc d;
+        d.pos = o + lane;
+        d.in = d.pos < npos;
+        d.valid = d.in && x.acgt;
+        d.key = x.key;
+        d.fwd = x.fwd;
+        // Pairs (i - 1, i) at i = j + 1, j + 3, ...: w / 2 of them cover [j, j + w - 1] for even w; for odd w the
+        // pair at j + w - 1 adds the last hash.
+        const uint32_t* at = ring + half + lane;
+        d.h = at[1];
 #pragma unroll
-            for(int o = 1; o < w; o += 2)
-                h = min64(h, ring[(base + o) & 63]);
-            if constexpr(w % 2 == 1)
-                h = min64(h, ring[(base + w - 1) & 63]);
-            d.h = h;
+        for(int i = 3; i < w; i += 2)
+            d.h = min(d.h, at[i]);
+        if constexpr(w % 2 == 1)
+            d.h = min(d.h, at[w - 1]);
+        r1 = r2, x = y;
+        return d;
+    };
 
-            vis.visit(d, lane);
-            __syncwarp();
-            r0 = r1, r1 = r2;
-        }
+#pragma unroll 1
+    for(uint32_t o = 0; o < npos; o += 32)
+        vis.visit(describe(o), lane);
+    __syncwarp();
+}
+
+template <int k, int l, typename Visitor>
+__global__ void __launch_bounds__(32 * stream_warps, Visitor::min_blocks) stream_kernel(const Dev_Batch batch, const uint64_t seg_b, const uint64_t seg_e, Visitor vis)
+{
+    __shared__ uint32_t ring_all[stream_warps][ring_words];
+    __shared__ uint8_t tab[base_table_bytes];
+    fill_base_table(tab);
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    vis.begin();
+    const uint64_t warps = uint64_t(gridDim.x) * stream_warps;
+    // A segment's entry is asked for a segment ahead, a word per lane.
+    const auto ask = [&](const uint64_t g) -> uint32_t
+    {
+        return g < seg_e && lane < sizeof(Segment) / 4 ? __ldg(reinterpret_cast<const uint32_t*>(batch.segs + g) + lane) : 0u;
+    };
+    uint64_t g = seg_b + uint64_t(blockIdx.x) * stream_warps + wid;
+    for(uint32_t entry = ask(g); g < seg_e; )
+    {
+        const auto word = [&](const int i) { return __shfl_sync(0xFFFFFFFFu, entry, i); };
+        const auto wide = [&](const int i) { return uint64_t(word(i + 1)) << 32 | word(i); };
+        const uint64_t base = wide(0), pos = wide(2), q = wide(4);
+        const uint32_t npos = word(6);
+        g += warps;
+        entry = ask(g);
+        vis.begin_segment(q, pos);
+        describe_segment<k, l>(batch.bases + base, npos, ring_all[wid], tab, lane, vis);
         vis.end_segment(q, lane);
     }
     vis.end(lane);
@@ -202,52 +221,105 @@ __device__ __forceinline__ void warp_flush(unsigned long long* ctr, const unsign
         atomicAdd(ctr, c);
 }
 
+// Finds a row's k-mers, for visitors that insert nothing: `hit` where the key is present, its value then in `val` (with
+// val_), its value word (the key word of a set) in `at`. What few lanes need, candidates past the second and what lies
+// beyond a full bucket, is behind a branch of the whole warp.
+template <bool set_, bool val_>
+struct Found
+{
+    bool hit;
+    unsigned long long* at;
+    unsigned long long val;
+
+    __device__ __forceinline__ Found(const Dev_Table& T, const Kmer_Desc& d)
+    {
+        const Probe p = probe_primary<set_, false, val_>(T, d.valid, d.key, d.h);
+        const uint32_t b = bucket_of(d.h, T.cap);
+        hit = p.slot < B;
+        at = key_word<set_>(T, b, p.slot) + (set_ ? 0 : 1);
+        val = p.val;
+        const bool on = !hit && (p.rest != 0 || p.full);
+        if(__any_sync(0xFFFFFFFFu, on))
+        {
+            if(on)
+            {
+                at = find_on<set_, false>(T, b, p.rest, p.full, ~d.key, d.h, checksum_of(d.key), val);
+                hit = at != nullptr;
+            }
+            __syncwarp();
+        }
+    }
+};
+
 // Upsert / insert / upsert_oriented (include/Streaming_Kmer_Hash_Table.hpp:2219-2514): returns the keys inserted;
 // k-mers that found the overflow table full set their bit in `retry_out` and change nothing. In retry mode, only
 // the positions whose bit is set in `retry_in` run.
 template <bool set_, typename V, typename Fn>
 struct Upsert_Visitor
 {
+    static constexpr int min_blocks = 6;
     Dev_Table T;
     Fn fn;
-    const uint64_t* pos_off;
     unsigned long long* inserted;
     unsigned int* retry_out;
     const unsigned int* retry_in;
     unsigned int* retried;      // Set to 1 if any bit of retry_out was set.
-    unsigned long long ins;
-    unsigned long long* per_seq;    // If set, keys inserted per sequence are added at per_seq[q] (lane kernel only).
-    uint32_t lane_ins;
-    static constexpr int stage_bytes = 0;
+    unsigned long long* per_seq;    // If set, keys inserted per sequence are added at per_seq[q].
+    unsigned long long ins = 0;     // By this warp, before its current segment.
+    uint32_t seg_ins = 0;           // In the current segment,
+    uint64_t seg_pos = 0;           // whose first position this is.
 
-    // No checksum cache for inserts: other lanes insert into the same buckets meanwhile, and a stale copy's missed
-    // candidates cost a re-read; measured slower than reading the sector each time (config-1 upsert 1.91 vs 1.74 ms).
-    __device__ __forceinline__ void lane_cache(uint4*, uint4*) {}
-
-    __device__ __forceinline__ void begin() { ins = 0; }
-    __device__ __forceinline__ void begin(uint8_t*) { ins = 0; }
-    __device__ __forceinline__ void begin_segment(uint64_t) {}
-    __device__ __forceinline__ void end_segment(uint64_t, uint32_t) {}
-    __device__ __forceinline__ void lane_begin(uint64_t, bool) { lane_ins = 0; }
-    __device__ __forceinline__ void lane_end(const uint64_t q, const bool has)
+    __device__ __forceinline__ void begin() {}
+    __device__ __forceinline__ void begin_segment(uint64_t, const uint64_t pos) { seg_ins = 0, seg_pos = pos; }
+    __device__ __forceinline__ void end_segment(const uint64_t q, const uint32_t lane)
     {
-        if(per_seq && has && lane_ins)
-            atomicAdd(per_seq + q, static_cast<unsigned long long>(lane_ins));
+        ins += seg_ins;
+        if(per_seq && lane == 0 && seg_ins)
+            atomicAdd(per_seq + q, static_cast<unsigned long long>(seg_ins));
     }
 
     __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t lane)
     {
+        constexpr uint32_t all = 0xFFFFFFFFu;
         bool active = d.valid;
         if(retry_in && active)
         {
-            const uint64_t gpos = d.out;
+            const uint64_t gpos = seg_pos + d.pos;
             active = (retry_in[gpos >> 5] >> (gpos & 31)) & 1;
         }
 
-        Landing L{};
-        uint32_t r = NONE;
-        if(active)
-            r = upsert_chain<set_>(T, d.key, d.h, d.c, L);
+        const unsigned long long key_st = ~d.key;
+        const uint32_t c = checksum_of(d.key);
+        uint32_t j = probe_primary<set_, true, false>(T, active, d.key, d.h).slot;
+        uint32_t r = j < B ? FOUND : NONE, at = active ? bucket_of(d.h, T.cap) : no_bucket;
+        uint64_t ov_i = 0;
+        const uint32_t need_m = __ballot_sync(all, active && r == NONE);
+        if(need_m)
+        {
+            // The bucket is read again: its checksums would take registers that other warps need.
+            if((need_m >> lane) & 1)
+                r = bucket_probe<set_>(T, at, key_st, c, j);
+            const bool need = active && r == NONE;
+            // Of lanes with one key, the first upserts it; the others then update it where it is.
+            uint32_t lead = lane;
+            const uint32_t lead_m = __ballot_sync(all, need);
+            if(need)
+                lead = __ffs(__match_any_sync(lead_m, key_st)) - 1;
+            warp_claim<set_>(T, key_st, d.h, c, lane, need && lead == lane, at, j, r, ov_i);
+            if(__any_sync(all, lead != lane))
+            {
+                const uint32_t r_l = __shfl_sync(all, r, lead), at_l = __shfl_sync(all, at, lead), j_l = __shfl_sync(all, j, lead);
+                const uint64_t ov_l = __shfl_sync(all, ov_i, lead);
+                if(lead != lane)
+                    r = r_l == OV_FULL ? OV_FULL : FOUND_PENDING, at = at_l, j = j_l, ov_i = ov_l;
+            }
+        }
+
+        Landing L;
+        if(at != no_bucket)
+            L = Landing{set_ ? nullptr : key_word<set_>(T, at, j) + 1, cs_of(T, at, j), nullptr, c};
+        else
+            L = Landing{T.ov + 4 * ov_i + 1, nullptr, T.ov + 4 * ov_i + 2, c};
         const bool comm = fn.commutes();
         if(r == INSERTED)
         {
@@ -262,13 +334,11 @@ struct Upsert_Visitor
         }
         else if(r == OV_FULL)
         {
-            const uint64_t gpos = d.out;
+            const uint64_t gpos = seg_pos + d.pos;
             atomicOr(retry_out + (gpos >> 5), 1u << (gpos & 31));
             *retried = 1;
         }
-        ins += __popc(__ballot_sync(0xFFFFFFFFu, r == INSERTED));
-        lane_ins += (r == INSERTED);
-        __syncwarp();
+        seg_ins += __popc(__ballot_sync(all, r == INSERTED));
 
         if constexpr(!set_)
             if((r == FOUND || r == FOUND_PENDING) && !fn.is_noop())
@@ -285,40 +355,33 @@ struct Upsert_Visitor
 };
 
 // Present-only update (include/Streaming_Kmer_Hash_Table.hpp:2650-2691): returns the k-mers present, repeats counted.
+// Nothing is inserted meanwhile, so checksums and keys are read through L1; only values change, atomically.
 template <typename V, typename Fn>
 struct Update_Visitor
 {
+    static constexpr int min_blocks = 6;
     Dev_Table T;
     Fn fn;
     unsigned long long* present;
-    unsigned long long cnt;
-    Bucket_Cache bc;            // Bound by the lane kernel (exact: an update inserts nothing); unbound elsewhere.
-    unsigned long long* per_seq = nullptr;  // If set, k-mers present per sequence are added at per_seq[q] (lane kernel).
-    uint32_t lane_cnt = 0;
-    static constexpr int stage_bytes = 0;
+    unsigned long long* per_seq;    // If set, k-mers present per sequence are added at per_seq[q].
+    unsigned long long cnt = 0;     // By this warp, before its current segment.
+    uint32_t seg_cnt = 0;           // In the current segment.
 
-    __device__ __forceinline__ void lane_cache(uint4* lo, uint4* hi) { bc.lo = lo, bc.hi = hi, bc.b = ~0ull; }
-
-    __device__ __forceinline__ void begin() { cnt = 0; }
-    __device__ __forceinline__ void begin(uint8_t*) { cnt = 0; }
-    __device__ __forceinline__ void begin_segment(uint64_t) {}
-    __device__ __forceinline__ void end_segment(uint64_t, uint32_t) {}
-    __device__ __forceinline__ void lane_begin(uint64_t, bool) { lane_cnt = 0; }
-    __device__ __forceinline__ void lane_end(const uint64_t q, const bool has)
+    __device__ __forceinline__ void begin() {}
+    __device__ __forceinline__ void begin_segment(uint64_t, uint64_t) { seg_cnt = 0; }
+    __device__ __forceinline__ void end_segment(const uint64_t q, const uint32_t lane)
     {
-        if(per_seq && has && lane_cnt)
-            atomicAdd(per_seq + q, static_cast<unsigned long long>(lane_cnt));
+        cnt += seg_cnt;
+        if(per_seq && lane == 0 && seg_cnt)
+            atomicAdd(per_seq + q, static_cast<unsigned long long>(seg_cnt));
     }
 
     __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t)
     {
-        unsigned long long* v = nullptr;
-        if(d.valid)
-            v = find_chain<false, true>(T, d.key, d.h, d.c, bc.lo ? &bc : nullptr);
-        if(v)
-            fn.apply(v, d.fwd);
-        cnt += __popc(__ballot_sync(0xFFFFFFFFu, v != nullptr));
-        lane_cnt += (v != nullptr);
+        const Found<false, false> f(T, d);
+        if(f.hit)
+            fn.apply(f.at, d.fwd);
+        seg_cnt += __popc(__ballot_sync(0xFFFFFFFFu, f.hit));
     }
 
     __device__ __forceinline__ void end(const uint32_t lane) { warp_flush(present, cnt, lane); }
@@ -329,34 +392,28 @@ struct Update_Visitor
 template <bool set_, typename V>
 struct Lookup_Visitor
 {
+    static constexpr int min_blocks = 6;
     Dev_Table T;
-    const uint64_t* pos_off;
     uint8_t* found;
     V* values;
     uint8_t* fwd;
-    uint64_t obase;
+    uint64_t obase = 0;     // The current segment's first position in them.
 
     __device__ __forceinline__ void begin() {}
-    __device__ __forceinline__ void begin_segment(const uint64_t q) { obase = pos_off[q]; }
+    __device__ __forceinline__ void begin_segment(uint64_t, const uint64_t pos) { obase = pos; }
     __device__ __forceinline__ void end_segment(uint64_t, uint32_t) {}
-    __device__ __forceinline__ void lane_begin(const uint64_t q, const bool has) { obase = has ? pos_off[q] : 0; }
-    __device__ __forceinline__ void lane_end(uint64_t, bool) {}
     __device__ __forceinline__ void end(uint32_t) {}
-    __device__ __forceinline__ void lane_cache(uint4*, uint4*) {}
 
     __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t)
     {
-        const unsigned long long* v = nullptr;
-        unsigned long long w = 0;
-        if(d.valid)
-            v = find_chain<set_, false>(T, d.key, d.h, d.c, w);
+        const Found<set_, !set_> f(T, d);
         if(!d.in)
             return;
         const uint64_t o = obase + d.pos;
-        found[o] = d.valid ? (v ? 1 : 0) : 2;
+        found[o] = d.valid ? (f.hit ? 1 : 0) : 2;
         if constexpr(!set_)
             if(values)
-                values[o] = v ? value_of<V>(w) : V(0);
+                values[o] = f.hit ? value_of<V>(f.val) : V(0);
         if(fwd)
             fwd[o] = d.valid && d.fwd;
     }
@@ -367,23 +424,18 @@ struct Lookup_Visitor
 template <bool set_, typename V>
 struct Lookup_Batches_Visitor : Lookup_Visitor<set_, V>
 {
+    static constexpr int min_blocks = 6;
     const uint32_t* batch_of;   // Sequence -> batch.
     const uint64_t* outs;       // Per batch, 8 words: found, values, fwd at words 4-6 (device addresses, or 0).
     const uint64_t* pos_base;   // Per batch: the merged position of its first k-mer.
 
-    __device__ __forceinline__ void bind(const uint64_t q)
+    __device__ __forceinline__ void begin_segment(const uint64_t q, const uint64_t pos)
     {
         const uint32_t b = batch_of[q];
         this->found = reinterpret_cast<uint8_t*>(outs[8 * uint64_t(b) + 4]);
         this->values = reinterpret_cast<V*>(outs[8 * uint64_t(b) + 5]);
         this->fwd = reinterpret_cast<uint8_t*>(outs[8 * uint64_t(b) + 6]);
-        this->obase = this->pos_off[q] - pos_base[b];
-    }
-    __device__ __forceinline__ void begin_segment(const uint64_t q) { bind(q); }
-    __device__ __forceinline__ void lane_begin(const uint64_t q, const bool has)
-    {
-        if(has)
-            bind(q);
+        this->obase = pos - pos_base[b];
     }
 };
 
@@ -392,32 +444,26 @@ struct Lookup_Batches_Visitor : Lookup_Visitor<set_, V>
 template <bool set_, typename V, int mode_>
 struct Seq_Reduce_Visitor
 {
+    static constexpr int min_blocks = 6;
     Dev_Table T;
     unsigned long long* out;
     V m_fwd, m_rev;
     unsigned long long acc;
     unsigned long long total;
-    Bucket_Cache bc;
-    static constexpr int stage_bytes = 0;
-
-    __device__ __forceinline__ void lane_cache(uint4* lo, uint4* hi) { bc.lo = lo, bc.hi = hi, bc.b = ~0ull; }
 
     __device__ __forceinline__ void begin() { total = 0; }
-    __device__ __forceinline__ void begin(uint8_t*) { total = 0; }
-    __device__ __forceinline__ void begin_segment(uint64_t) { acc = 0; }
+    __device__ __forceinline__ void begin_segment(uint64_t, uint64_t) { acc = 0; }
     __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t)
     {
-        if(!d.valid)
-            return;
-        unsigned long long w = 0;
-        if(!find_chain<set_, false>(T, d.key, d.h, d.c, w, bc.lo ? &bc : nullptr))
+        const Found<set_, !set_ && mode_ != 0> f(T, d);
+        if(!f.hit)
             return;
         if constexpr(mode_ == 0)
             acc += 1;
         else if constexpr(mode_ == 1)
-            acc += (value_of<V>(w) & (d.fwd ? m_fwd : m_rev)) != 0;
+            acc += (value_of<V>(f.val) & (d.fwd ? m_fwd : m_rev)) != 0;
         else
-            acc += static_cast<unsigned long long>(value_of<V>(w));
+            acc += static_cast<unsigned long long>(value_of<V>(f.val));
     }
     __device__ __forceinline__ void end_segment(const uint64_t q, const uint32_t lane)
     {
@@ -429,42 +475,32 @@ struct Seq_Reduce_Visitor
             atomicAdd(out + q, a);
         total += a;
     }
-    // One lane, one sequence's segment: its own total.
-    __device__ __forceinline__ void lane_begin(uint64_t, bool) { acc = 0; }
-    __device__ __forceinline__ void lane_end(const uint64_t q, const bool has)
-    {
-        if(has && acc)
-            atomicAdd(out + q, acc);
-    }
     __device__ __forceinline__ void end(uint32_t) {}
 };
 
-// The descriptions themselves, for checking the describer.
+// The descriptions that callers can see, for checking the describer: the key's 2-bit encoding, and the reference's
+// checksum and minimizer hash of it.
+template <int k, int l>
 struct Describe_Visitor
 {
-    const uint64_t* pos_off;
+    static constexpr int min_blocks = 4;
     uint64_t* key;
     uint64_t* h;
     uint8_t* cs;
     uint8_t* fwd;
     uint8_t* valid;
-    bool by_out;    // Outputs at d.out (the lane kernel) rather than pos_off[q] + pos.
-    static constexpr int stage_bytes = 0;
+    uint64_t obase = 0;
 
     __device__ __forceinline__ void begin() {}
-    __device__ __forceinline__ void begin(uint8_t*) {}
-    __device__ __forceinline__ void begin_segment(uint64_t) {}
+    __device__ __forceinline__ void begin_segment(uint64_t, const uint64_t pos) { obase = pos; }
     __device__ __forceinline__ void end_segment(uint64_t, uint32_t) {}
-    __device__ __forceinline__ void lane_begin(uint64_t, bool) {}
-    __device__ __forceinline__ void lane_end(uint64_t, bool) {}
-    __device__ __forceinline__ void lane_cache(uint4*, uint4*) {}
     __device__ __forceinline__ void end(uint32_t) {}
     __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t)
     {
         if(!d.in)
             return;
-        const uint64_t o = by_out ? d.out : pos_off[d.q] + d.pos;
-        key[o] = d.valid ? d.key : 0, h[o] = d.valid ? d.h : 0, cs[o] = d.valid ? d.c : 0;
+        const uint64_t o = obase + d.pos, e = encoding_of(d.key);
+        key[o] = d.valid ? e : 0, h[o] = d.valid ? described_minimizer<k, l>(e) : 0, cs[o] = d.valid ? described_checksum(e) : 0;
         fwd[o] = d.valid && d.fwd, valid[o] = d.valid;
     }
 };

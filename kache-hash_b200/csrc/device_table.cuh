@@ -1,12 +1,13 @@
 // The table in HBM and its lock-free per-k-mer operations.
 //
 // Layout (structure of arrays, one entry per bucket of B = 32 slots):
-//   cs[cap][32]     u8   checksums; 0 = empty. One 32-byte sector per bucket, so one load tests all 32 slots.
+//   cs[cap][32]     u8   checksums; 0 = empty. One 32-byte sector per bucket, so two 16-byte loads of it test all 32
+//                        slots (slot j's is byte cs_byte(j)).
 //   spill[cap][8]   u32  the 255-bit spill filter of minimizers whose keys left the (full) bucket
 //                        (include/Streaming_Kmer_Hash_Table.hpp:91-97,1064-1093). Bit 0 is unused.
 //   slots[cap][32]       maps: {u64 ~key, u64 value} (16 B; a key and its value share one sector);
-//                        sets: {u64 ~key} (8 B). The key is stored complemented, so zeroed memory is empty: no
-//                        canonical k-mer is all T's, whose complement would be 0.
+//                        sets: {u64 ~key} (8 B). The key (its planes, device_common.cuh) is stored complemented, so
+//                        zeroed memory is empty: no canonical k-mer is all T's, whose complement would be 0.
 //   ov[ov_cap]           the overflow table: {u64 ~key, u64 value, u64 ready, u64 pad}, linear probing.
 //
 // Concurrency without locks, in place of the reference's bucket spin locks (include/Streaming_Kmer_Hash_Table.hpp:
@@ -44,6 +45,7 @@ struct Dev_Table
 
 constexpr uint32_t default_wait_polls = 1u << 22;
 
+constexpr uint32_t no_bucket = ~0u;     // No bucket's index: there are at most 2^32 - 1.
 constexpr uint32_t ERR_WAIT = 1;    // A wait for a racing insert's publication ran out.
 
 template <bool set_> __host__ __device__ constexpr int slot_words() { return set_ ? 1 : 2; }
@@ -52,6 +54,16 @@ template <bool set_> __host__ __device__ constexpr int slot_words() { return set
 __device__ __forceinline__ unsigned long long ld_cg(const unsigned long long* p) { return __ldcg(p); }
 __device__ __forceinline__ uint4 ld_cg4(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ uint8_t ld_volatile_u8(const uint8_t* p) { return *reinterpret_cast<const volatile uint8_t*>(p); }
+
+// Atomics on the table's words that return nothing, as reductions: no lane waits for their results.
+__device__ __forceinline__ void red_add(unsigned long long* p, const unsigned long long x) { asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" :: "l"(__cvta_generic_to_global(p)), "l"(x) : "memory"); }
+__device__ __forceinline__ void red_add(unsigned int* p, const unsigned int x) { asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" :: "l"(__cvta_generic_to_global(p)), "r"(x) : "memory"); }
+__device__ __forceinline__ void red_or(unsigned long long* p, const unsigned long long x) { asm volatile("red.relaxed.gpu.global.or.b64 [%0], %1;" :: "l"(__cvta_generic_to_global(p)), "l"(x) : "memory"); }
+__device__ __forceinline__ void red_or(unsigned int* p, const unsigned int x) { asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" :: "l"(__cvta_generic_to_global(p)), "r"(x) : "memory"); }
+__device__ __forceinline__ void red_max(unsigned long long* p, const unsigned long long x) { asm volatile("red.relaxed.gpu.global.max.u64 [%0], %1;" :: "l"(__cvta_generic_to_global(p)), "l"(x) : "memory"); }
+__device__ __forceinline__ void red_max(unsigned int* p, const unsigned int x) { asm volatile("red.relaxed.gpu.global.max.u32 [%0], %1;" :: "l"(__cvta_generic_to_global(p)), "r"(x) : "memory"); }
+__device__ __forceinline__ void red_min(unsigned long long* p, const unsigned long long x) { asm volatile("red.relaxed.gpu.global.min.u64 [%0], %1;" :: "l"(__cvta_generic_to_global(p)), "l"(x) : "memory"); }
+__device__ __forceinline__ void red_min(unsigned int* p, const unsigned int x) { asm volatile("red.relaxed.gpu.global.min.u32 [%0], %1;" :: "l"(__cvta_generic_to_global(p)), "r"(x) : "memory"); }
 
 // Reads a stored value as V.
 template <typename V>
@@ -170,10 +182,10 @@ struct Op_Fn
                     atomicExch(w, static_cast<unsigned long long>(mx));
                 return;
             case OP_ASSIGN: atomicExch(w, static_cast<unsigned long long>(x)); return;
-            case OP_OR: atomicOr(w, static_cast<unsigned long long>(x)); return;
-            case OP_MIN: atomicMin(w, static_cast<unsigned long long>(x)); return;
-            case OP_MAX: atomicMax(w, static_cast<unsigned long long>(x)); return;
-            case OP_ADD_WRAP: atomicAdd(w, static_cast<unsigned long long>(x)); return;
+            case OP_OR: red_or(w, static_cast<unsigned long long>(x)); return;
+            case OP_MIN: red_min(w, static_cast<unsigned long long>(x)); return;
+            case OP_MAX: red_max(w, static_cast<unsigned long long>(x)); return;
+            case OP_ADD_WRAP: red_add(w, static_cast<unsigned long long>(x)); return;
             default: break;
             }
         }
@@ -187,11 +199,11 @@ struct Op_Fn
                     atomicExch(p, static_cast<unsigned int>(mx));
                 return;
             case OP_ASSIGN: atomicExch(p, static_cast<unsigned int>(x)); return;
-            case OP_OR: atomicOr(p, static_cast<unsigned int>(x)); return;
-            case OP_MIN: atomicMin(p, static_cast<unsigned int>(x)); return;
-            case OP_MAX: atomicMax(p, static_cast<unsigned int>(x)); return;
+            case OP_OR: red_or(p, static_cast<unsigned int>(x)); return;
+            case OP_MIN: red_min(p, static_cast<unsigned int>(x)); return;
+            case OP_MAX: red_max(p, static_cast<unsigned int>(x)); return;
             case OP_ADD_WRAP:
-                if constexpr(sizeof(V) == 4) { atomicAdd(p, static_cast<unsigned int>(x)); return; }
+                if constexpr(sizeof(V) == 4) { red_add(p, static_cast<unsigned int>(x)); return; }
                 break;
             default: break;
             }
@@ -261,80 +273,65 @@ __device__ __forceinline__ unsigned long long* key_word(const Dev_Table& T, cons
     return T.slots + (b * B + j) * slot_words<set_>();
 }
 
-// A lane's copy, in shared memory, of the checksums of the last primary bucket it probed: consecutive k-mers of a
-// read mostly share their minimizer, so their primary bucket, and the copy saves re-reading its sector. The copy may
-// miss checksums published since by other lanes. Every probe stays correct with such a copy, only slower: a missed
-// candidate of an upsert is met by the claim scan's failed compare-and-swap, whose result is the claimer's key, and
-// finds and updates run in kernels without inserts, where nothing changes.
-struct Bucket_Cache
+// A bucket's checksums: words 0..3 and 4..7.
+struct Checksums
 {
-    uint4* lo;      // Checksums of slots 0..15 and 16..31.
-    uint4* hi;
-    uint64_t b;     // The bucket copied; ~0 for none.
+    uint4 lo, hi;
+
+    __device__ __forceinline__ bool full() const { return (hi.w >> 24) != 0; }  // Keys fill a bucket's slots in order.
+    // The first slot whose checksum is empty, or B.
+    __device__ __forceinline__ uint32_t first_empty() const
+    {
+        const uint32_t m = candidates32<true>(lo, hi, 0);
+        return m ? __ffs(m) - 1 : B;
+    }
 };
 
-// The checksums of bucket b, from the cache where it holds them, else loaded (and cached).
 template <bool cg_>
-__device__ __forceinline__ void bucket_cs(const Dev_Table& T, const uint64_t b, Bucket_Cache* bc, uint4& c0, uint4& c1)
+__device__ __forceinline__ Checksums bucket_cs(const Dev_Table& T, const uint32_t b)
 {
-    if(bc && bc->b == b)
-    {
-        c0 = *bc->lo, c1 = *bc->hi;
-        return;
-    }
-    const uint8_t* csb = T.cs + b * B;
-    c0 = cg_ ? ld_cg4(csb) : *reinterpret_cast<const uint4*>(csb);
-    c1 = cg_ ? ld_cg4(csb + 16) : *reinterpret_cast<const uint4*>(csb + 16);
-    if(bc)
-        *bc->lo = c0, *bc->hi = c1, bc->b = b;
+    const uint8_t* p = T.cs + uint64_t(b) * B;
+    if constexpr(cg_)
+        return Checksums{ld_cg4(p), ld_cg4(p + 16)};
+    else
+        return Checksums{*reinterpret_cast<const uint4*>(p), *reinterpret_cast<const uint4*>(p + 16)};
 }
 
-// Tries the bucket b for the key: its published candidates, then the claim scan. Returns FOUND, FOUND_PENDING or
-// INSERTED with the slot at `j`, or NONE if the bucket is full without the key. With a cache holding b, the cached
-// candidates are tried first; if none is the key, the checksums are read afresh (other lanes may have published it
-// since), cached, and the probe goes on from them. A slot this lane claims is entered in the cache.
+__device__ __forceinline__ uint8_t* cs_of(const Dev_Table& T, const uint32_t b, const uint32_t j) { return T.cs + uint64_t(b) * B + cs_byte(j); }
+
+// Looks for the key among the published slots of bucket b. Returns FOUND with its slot at `j`, or NONE with the first
+// slot whose checksum is empty at `j` (B if there is none).
 template <bool set_>
-__device__ __forceinline__ uint32_t bucket_upsert(const Dev_Table& T, const uint64_t b, const unsigned long long key_st, const uint8_t c, uint32_t& j_out, Bucket_Cache* bc = nullptr)
+__device__ __forceinline__ uint32_t bucket_probe(const Dev_Table& T, const uint32_t b, const unsigned long long key_st, const uint32_t c, uint32_t& j)
 {
-    const uint8_t* csb = T.cs + b * B;
-    uint4 c0, c1;
-    if(bc && bc->b == b)
+    const Checksums s = bucket_cs<true>(T, b);
+    for(uint32_t cand = candidates32<true>(s.lo, s.hi, c); cand; cand &= cand - 1)
     {
-        c0 = *bc->lo, c1 = *bc->hi;
-        for(uint32_t cand = candidates32<true>(c0, c1, c); cand; cand &= cand - 1)
-        {
-            const uint32_t j = candidate_slot(__ffs(cand) - 1);
-            if(ld_cg(key_word<set_>(T, b, j)) == key_st)
-                return j_out = j, FOUND;
-        }
-    }
-    c0 = ld_cg4(csb), c1 = ld_cg4(csb + 16);
-    if(bc)
-        *bc->lo = c0, *bc->hi = c1, bc->b = b;
-    uint32_t cand = candidates32<true>(c0, c1, c);
-    while(cand)
-    {
-        const uint32_t j = candidate_slot(__ffs(cand) - 1);
-        cand &= cand - 1;
+        j = __ffs(cand) - 1;
         if(ld_cg(key_word<set_>(T, b, j)) == key_st)
-            return j_out = j, FOUND;
+            return FOUND;
     }
-    const uint32_t empty = match32(c0, c1, 0);
+    j = s.first_empty();
+    return NONE;
+}
+
+// Tries the bucket b for the key, one lane by itself: its published candidates, then the claim scan. Returns FOUND,
+// FOUND_PENDING or INSERTED with the slot at `j`, or NONE if the bucket is full without the key.
+template <bool set_>
+__device__ __forceinline__ uint32_t bucket_upsert(const Dev_Table& T, const uint32_t b, const unsigned long long key_st, const uint32_t c, uint32_t& j)
+{
+    if(bucket_probe<set_>(T, b, key_st, c, j) == FOUND)
+        return FOUND;
 
     // The claim scan: a compare-and-swap straight away (a slot with an empty checksum is most likely unclaimed), whose
     // result, if it fails, is the racing claimer's key.
-    for(uint32_t j = empty ? __ffs(empty) - 1 : B; j < B; ++j)
+    for(; j < B; ++j)
     {
-        unsigned long long* kw = key_word<set_>(T, b, j);
-        const unsigned long long cur = atomicCAS(kw, 0ull, key_st);
+        const unsigned long long cur = atomicCAS(key_word<set_>(T, b, j), 0ull, key_st);
         if(cur == 0)
-        {
-            if(bc)
-                reinterpret_cast<uint8_t*>(j < 16 ? bc->lo : bc->hi)[j & 15] = c;
-            return j_out = j, INSERTED;
-        }
+            return INSERTED;
         if(cur == key_st)
-            return j_out = j, (ld_volatile_u8(csb + j) != 0 ? FOUND : FOUND_PENDING);
+            return ld_volatile_u8(cs_of(T, b, j)) != 0 ? FOUND : FOUND_PENDING;
     }
 
     return NONE;
@@ -367,39 +364,37 @@ struct Landing
     unsigned long long* val;
     uint8_t* cs;            // Non-null in the main table.
     unsigned long long* ready;  // Non-null in the overflow table.
-    uint8_t c;
+    uint32_t c;
 };
 
 // The upsert chain of one k-mer (include/Streaming_Kmer_Hash_Table.hpp:2431-2490, lock-free): primary bucket; if
 // full, mark its spill filter, then the secondary buckets in order; then the overflow table.
 template <bool set_>
-__device__ __forceinline__ uint32_t upsert_chain(const Dev_Table& T, const uint64_t key, const uint64_t h, const uint8_t c, Landing& L, Bucket_Cache* bc = nullptr)
+__device__ __forceinline__ uint32_t upsert_chain(const Dev_Table& T, const uint64_t key, const uint32_t h, const uint32_t c, Landing& L)
 {
     const unsigned long long key_st = ~key;
     uint32_t j;
-    const uint64_t b = bucket_of(h, T.cap);
-    uint32_t r = bucket_upsert<set_>(T, b, key_st, c, j, bc);
-    uint64_t at = b;
+    const uint32_t b = bucket_of(h, T.cap);
+    uint32_t r = bucket_upsert<set_>(T, b, key_st, c, j);
+    uint32_t at = b;
     if(r == NONE)
     {
         const uint32_t fp = filter_pos(h);
-        uint32_t* sw = T.spill + b * 8 + (fp >> 5);
+        uint32_t* sw = T.spill + uint64_t(b) * 8 + (fp >> 5);
         const uint32_t bit = 1u << (fp & 31);
         if(!(__ldcg(sw) & bit))
             atomicOr(sw, bit);
 
-        uint64_t p, q;
-        secondaries(h, T.cap, p, q);
-        r = bucket_upsert<set_>(T, p, key_st, c, j);
-        at = p;
+        at = second_bucket(h, T.cap);
+        r = bucket_upsert<set_>(T, at, key_st, c, j);
         if(r == NONE)
-            r = bucket_upsert<set_>(T, q, key_st, c, j), at = q;
+            at = third_bucket(h, T.cap), r = bucket_upsert<set_>(T, at, key_st, c, j);
     }
 
     if(r != NONE)
     {
         unsigned long long* kw = key_word<set_>(T, at, j);
-        L.val = set_ ? nullptr : kw + 1, L.cs = T.cs + at * B + j, L.ready = nullptr, L.c = c;
+        L.val = set_ ? nullptr : kw + 1, L.cs = cs_of(T, at, j), L.ready = nullptr, L.c = c;
         return r;
     }
 
@@ -409,13 +404,114 @@ __device__ __forceinline__ uint32_t upsert_chain(const Dev_Table& T, const uint6
     return r;
 }
 
+// The upsert chain past the first probe, for the lanes of a whole warp that `want` it (no two with the same key). On
+// entry such a lane's `at` is its primary bucket, `j` that bucket's first empty slot as probed (B if full) and `r`
+// NONE; every other lane's `at` is its k-mer's primary bucket, or no_bucket. On return r is as upsert_chain's, with the
+// slot at (at, j), or with at = no_bucket at overflow slot `ov_i`.
+//
+// The lanes hold consecutive k-mers, so the new ones come in runs of neighbours that share a minimizer, hence a bucket.
+// A run claims together: its lane of rank i tries slot j + i at once with the others, where lanes trying the same slot
+// one after another would take as many rounds of compare-and-swaps as the run has keys. What keeps one copy of each key
+// is that a run as a whole tries every slot from the first empty one on, as a single inserter would: a lane whose key a
+// failed swap of its run shows in a lower slot takes that slot, and leaves a slot that it has itself claimed higher up
+// as a hole: unpublished for good (its checksum stays 0, so nothing iterates it), its key replaced by one that no k-mer
+// has (so no lookup takes it for a candidate, and inserters pass it by as another key's claim). The lowest slot that
+// holds a key is the one that everybody settles on, since an inserter either finds it published when it first probes the
+// bucket, or its run tries that slot. A hole is never the last slot, which marks a bucket full: only a lane of rank 0,
+// whose claim is the lowest tried, takes that one.
+constexpr unsigned long long hole_key = 1;  // ~key of T...TG, whose reverse complement CA...A is the lesser.
+
+template <bool set_>
+__device__ __forceinline__ void warp_claim(const Dev_Table& T, const unsigned long long key_st, const uint32_t h, const uint32_t c, const uint32_t lane,
+                                           const bool want, uint32_t& at, uint32_t& j, uint32_t& r, uint64_t& ov_i)
+{
+    constexpr uint32_t all = 0xFFFFFFFFu;
+    const uint32_t le = all >> (31 - lane), lt = le >> 1;
+    for(uint32_t stage = 0; ; ++stage)
+    {
+        for(;;)
+        {
+            const bool in = want && r == NONE && j < B;
+            const uint32_t in_m = __ballot_sync(all, in);
+            if(in_m == 0)
+                break;
+            // This lane's run: the lanes from the last change of bucket on, up to the next.
+            const uint32_t left = __shfl_up_sync(all, at, 1);
+            const uint32_t heads = __ballot_sync(all, lane == 0 || at != left);
+            const uint32_t from = all << (31 - __clz(heads & le)), next = heads & ~le;
+            const uint32_t run = next ? from & ((next & (0u - next)) - 1) : from;
+            // Lanes of a run whose probes saw different first empty slots do not claim together: those unlike the
+            // first probe afresh.
+            const uint32_t first = __shfl_sync(all, j, in ? __ffs(in_m & run) - 1 : lane);
+            const bool ok = in && j == first;
+            const uint32_t ok_run = __ballot_sync(all, ok) & run;
+            const uint32_t rank = __popc(ok_run & lt), slot = j + rank;
+            const bool tries = ok && (rank == 0 || slot < B - 1);
+            unsigned long long cur = 0;
+            uint32_t got = slot;
+            if(tries)
+            {
+                cur = atomicCAS(key_word<set_>(T, at, slot), 0ull, key_st);
+                if(cur == 0)
+                    r = INSERTED;
+                else if(cur == key_st)
+                    r = FOUND_PENDING;
+            }
+            const uint32_t tried = __popc(__ballot_sync(all, tries) & run);
+            for(uint32_t lost = __ballot_sync(all, tries && r == NONE); lost; lost &= lost - 1)
+            {
+                const uint32_t s = __ffs(lost) - 1;
+                const unsigned long long k_s = __shfl_sync(all, cur, s);
+                const uint32_t slot_s = __shfl_sync(all, slot, s);
+                if(ok && ((run >> s) & 1) && k_s == key_st && (r == NONE || slot_s < got))
+                {
+                    if(r == INSERTED)
+                        *reinterpret_cast<volatile unsigned long long*>(key_word<set_>(T, at, got)) = hole_key;
+                    r = FOUND_PENDING, got = slot_s;
+                }
+            }
+            if(ok)
+                j = r == NONE ? j + tried : got;
+            else if(in)
+                r = bucket_probe<set_>(T, at, key_st, c, j);
+        }
+
+        const bool full = want && r == NONE;
+        if(!__any_sync(all, full))
+            return;
+        if(full)
+        {
+            if(stage == 2)
+            {
+                at = no_bucket;
+                r = overflow_upsert(T, key_st, ov_i);
+            }
+            else
+            {
+                if(stage == 0)
+                {
+                    const uint32_t fp = filter_pos(h);
+                    uint32_t* sw = T.spill + uint64_t(at) * 8 + (fp >> 5);
+                    const uint32_t bit = 1u << (fp & 31);
+                    if(!(__ldcg(sw) & bit))
+                        atomicOr(sw, bit);
+                }
+                at = stage == 0 ? second_bucket(h, T.cap) : third_bucket(h, T.cap);
+                r = bucket_probe<set_>(T, at, key_st, c, j);
+            }
+        }
+        if(stage == 2)
+            return;
+    }
+}
+
 // Publishes a claimed slot after its value is written.
 __device__ __forceinline__ void publish(const Landing& L, const bool fence)
 {
     if(fence)
         __threadfence();
     if(L.cs)
-        *reinterpret_cast<volatile uint8_t*>(L.cs) = L.c;
+        *reinterpret_cast<volatile uint8_t*>(L.cs) = static_cast<uint8_t>(L.c);
     else
         *reinterpret_cast<volatile unsigned long long*>(L.ready) = 1ull;
 }
@@ -436,60 +532,64 @@ __device__ __forceinline__ bool await_published(const Landing& L, const uint32_t
     return false;
 }
 
-// Compares the key of the slot at kw (16-byte aligned for a map) with key_st (a stored, complemented key), keeping its
-// value in `val`.
+// The key and value of a map's slot at kw (16-byte aligned), in one load.
+template <bool cg_>
+__device__ __forceinline__ void load_slot(const unsigned long long* kw, unsigned long long& k, unsigned long long& v)
+{
+    const ulonglong2 s = cg_ ? __ldcg(reinterpret_cast<const ulonglong2*>(kw)) : *reinterpret_cast<const ulonglong2*>(kw);
+    k = s.x, v = s.y;
+}
+
+// Compares the key of the slot at kw with key_st (a stored, complemented key), keeping a map's value in `val`.
 template <bool set_, bool cg_>
 __device__ __forceinline__ bool slot_is(const unsigned long long* kw, const unsigned long long key_st, unsigned long long& val)
 {
+    unsigned long long k;
     if constexpr(set_)
-        return (cg_ ? ld_cg(kw) : *kw) == key_st;
+        k = cg_ ? ld_cg(kw) : *kw;
     else
-    {
-        const ulonglong2 s = cg_ ? __ldcg(reinterpret_cast<const ulonglong2*>(kw)) : *reinterpret_cast<const ulonglong2*>(kw);
-        val = s.y;
-        return s.x == key_st;
-    }
+        load_slot<cg_>(kw, k, val);
+    return k == key_st;
 }
 
-// The candidates of bucket b in `cand` (candidates32's bits), tried in order: the found key's value word (its key word
-// in a set), or null.
+// Looks for the key, which the first probe of its primary bucket b did not find, among the candidates `cand` left there
+// and then, if b is full, past it: absent unless b's spill filter marks the minimizer; else the secondary buckets; then
+// the overflow table iff both are full (include/Streaming_Kmer_Hash_Table.hpp:2548-2574). Returns the value word (the
+// key word of a set), or null if absent; a map's value also goes to `val`.
 template <bool set_, bool cg_>
-__device__ __forceinline__ unsigned long long* try_candidates(const Dev_Table& T, const uint64_t b, uint32_t cand, const unsigned long long key_st, unsigned long long& val)
+__device__ __forceinline__ unsigned long long* find_on(const Dev_Table& T, const uint32_t b, uint32_t cand, const bool full, const unsigned long long key_st,
+                                                       const uint32_t h, const uint32_t c, unsigned long long& val)
 {
-    while(cand)
+    bool both_full = full;
+    for(int t = 0; ; ++t)
     {
-        const uint32_t j = candidate_slot(__ffs(cand) - 1);
-        cand &= cand - 1;
-        unsigned long long* kw = key_word<set_>(T, b, j);
-        if(slot_is<set_, cg_>(kw, key_st, val))
-            return set_ ? kw : kw + 1;
+        // t = 0: the primary bucket; 1 and 2: the secondary ones.
+        const uint32_t at = t == 0 ? b : t == 1 ? second_bucket(h, T.cap) : third_bucket(h, T.cap);
+        if(t > 0)
+        {
+            const Checksums s = bucket_cs<cg_>(T, at);
+            cand = candidates32<false>(s.lo, s.hi, c);
+            both_full = both_full && s.full();
+        }
+        for(; cand; cand &= cand - 1)
+        {
+            unsigned long long* kw = key_word<set_>(T, at, __ffs(cand) - 1);
+            if(slot_is<set_, cg_>(kw, key_st, val))
+                return set_ ? kw : kw + 1;
+        }
+        if(t == 0)
+        {
+            if(!full)
+                return nullptr;
+            const uint32_t fp = filter_pos(h);
+            const uint32_t* sw = T.spill + uint64_t(b) * 8 + (fp >> 5);
+            if(!(((cg_ ? __ldcg(sw) : *sw) >> (fp & 31)) & 1))
+                return nullptr;
+        }
+        if(t == 2)
+            break;
     }
-    return nullptr;
-}
-
-// A find past a full primary bucket b (include/Streaming_Kmer_Hash_Table.hpp:2555-2574): absent unless b's spill
-// filter marks the minimizer; else the secondary buckets; then the overflow table iff both are full.
-template <bool set_, bool cg_>
-__device__ __forceinline__ unsigned long long* find_past_primary(const Dev_Table& T, const uint64_t b, const unsigned long long key_st, const uint64_t h, const uint8_t c, unsigned long long& val)
-{
-    const uint32_t fp = filter_pos(h);
-    const uint32_t sw = cg_ ? __ldcg(T.spill + b * 8 + (fp >> 5)) : T.spill[b * 8 + (fp >> 5)];
-    if(!((sw >> (fp & 31)) & 1))
-        return nullptr;
-
-    uint64_t p, q;
-    secondaries(h, T.cap, p, q);
-    bool full_p = false, full_q = false;
-    for(int t = 0; t < 2; ++t)
-    {
-        const uint64_t s = t ? q : p;
-        uint4 c0, c1;
-        bucket_cs<cg_>(T, s, nullptr, c0, c1);
-        if(auto* r = try_candidates<set_, cg_>(T, s, candidates32<false>(c0, c1, c), key_st, val))
-            return r;
-        (t ? full_q : full_p) = (c1.w >> 24) != 0;
-    }
-    if(!(full_p && full_q))
+    if(!both_full)
         return nullptr;
 
     uint64_t i = ov_hash(key_st) & T.ov_mask;
@@ -505,29 +605,68 @@ __device__ __forceinline__ unsigned long long* find_past_primary(const Dev_Table
     return nullptr;
 }
 
-// Finds a key: primary bucket; absent if it is not full, or if its spill filter does not mark the minimizer; else the
-// secondary buckets; then the overflow table iff both are full (include/Streaming_Kmer_Hash_Table.hpp:2548-2574).
-// Returns the value word (the key word for a set), or null if absent; a map's value word, read together with its key
-// in one 16-byte load, also goes to `val`.
+// Finds a key, one lane by itself: its value word (the key word of a set), or null.
 template <bool set_, bool cg_>
-__device__ __forceinline__ unsigned long long* find_chain(const Dev_Table& T, const uint64_t key, const uint64_t h, const uint8_t c, unsigned long long& val, Bucket_Cache* bc = nullptr)
+__device__ __forceinline__ unsigned long long* find_chain(const Dev_Table& T, const uint64_t key, const uint32_t h, const uint32_t c)
 {
-    const unsigned long long key_st = ~key;
-    const uint64_t b = bucket_of(h, T.cap);
-    uint4 c0, c1;
-    bucket_cs<cg_>(T, b, bc, c0, c1);
-    if(auto* r = try_candidates<set_, cg_>(T, b, candidates32<false>(c0, c1, c), key_st, val))
-        return r;
-    if((c1.w >> 24) == 0)   // Keys fill a bucket's slots in order: full iff its last checksum is set.
-        return nullptr;
-    return find_past_primary<set_, cg_>(T, b, key_st, h, c, val);
+    const uint32_t b = bucket_of(h, T.cap);
+    const Checksums s = bucket_cs<cg_>(T, b);
+    unsigned long long val;
+    return find_on<set_, cg_>(T, b, candidates32<false>(s.lo, s.hi, c), s.full(), ~key, h, c, val);
 }
 
-template <bool set_, bool cg_>
-__device__ __forceinline__ unsigned long long* find_chain(const Dev_Table& T, const uint64_t key, const uint64_t h, const uint8_t c, Bucket_Cache* bc = nullptr)
+// The first probe of a lane's k-mer, in its primary bucket.
+struct Probe
 {
-    unsigned long long val;
-    return find_chain<set_, cg_>(T, key, h, c, val, bc);
+    uint32_t slot;      // The key's slot there, B if it was not found.
+    uint32_t rest;      // Candidate slots not tried.
+    bool full;          // Whether the bucket is full.
+    unsigned long long val;     // With val_, the value in a map of the key found.
+};
+
+// Probes the primary bucket of the k-mer `key` of minimizer hash h where `valid`. The first two candidates are read
+// together: one lane in fourteen or so has a candidate besides its key, so most warps have some, and a warp waits for a
+// second read as long as for the first.
+template <bool set_, bool cg_, bool val_>
+__device__ __forceinline__ Probe probe_primary(const Dev_Table& T, const bool valid, const uint64_t key, const uint32_t h)
+{
+    const unsigned long long key_st = ~key;
+    const uint32_t b = bucket_of(h, T.cap);
+    uint32_t cand = 0;
+    Probe p{B, 0, false, 0};
+    if(valid)
+    {
+        const Checksums s = bucket_cs<cg_>(T, b);
+        // Exactly where inserts run (cg_): a slot claimed but not yet published is no candidate.
+        cand = candidates32<cg_>(s.lo, s.hi, checksum_of(key));
+        p.full = s.full();
+    }
+    const uint32_t j1 = top_bit(cand), more = cand & ~(1u << (j1 & 31)), j2 = top_bit(more);
+    unsigned long long k1, v1, k2, v2;
+    const auto read = [&](const uint32_t j, unsigned long long& k, unsigned long long& v)
+    {
+        const unsigned long long* kw = key_word<set_>(T, b, j);
+        if constexpr(val_ && !set_)
+            load_slot<cg_>(kw, k, v);
+        else
+            k = cg_ ? ld_cg(kw) : *kw;
+    };
+    if(cand)
+        read(j1, k1, v1);
+    if(more)
+        read(j2, k2, v2);
+    if(cand && k1 == key_st)
+        p.slot = j1;
+    if constexpr(val_ && !set_)
+        p.val = v1;
+    if(more && k2 == key_st)
+    {
+        p.slot = j2;
+        if constexpr(val_ && !set_)
+            p.val = v2;
+    }
+    p.rest = more & ~(1u << (j2 & 31));
+    return p;
 }
 
 // For failure-injection tests: claims a slot of the key's primary bucket for it, as a racing inserter would, and
@@ -537,12 +676,11 @@ template <int k, int l, bool set_>
 __global__ void plant_claim_kernel(const Dev_Table T, const uint64_t key, unsigned long long* ok)
 {
     const uint64_t b = bucket_of(minimizer_hash<k, l>(key), T.cap);
-    const uint4 c0 = *reinterpret_cast<const uint4*>(T.cs + b * B), c1 = *reinterpret_cast<const uint4*>(T.cs + b * B + 16);
-    const uint32_t empty = match32(c0, c1, 0);
+    const uint32_t j = bucket_cs<false>(T, static_cast<uint32_t>(b)).first_empty();
     *ok = 0;
-    if(!empty)
+    if(j == B)
         return;
-    unsigned long long* kw = key_word<set_>(T, b, __ffs(empty) - 1);
+    unsigned long long* kw = key_word<set_>(T, b, j);
     *ok = atomicCAS(kw, 0ull, ~key) == 0ull;
 }
 

@@ -10,9 +10,7 @@
 #pragma once
 
 #include "device_misc.cuh"
-#include "device_lanes.cuh"
 #include "host_copy.hpp"
-#include "seg_tuner.hpp"
 #include "kache_b200.h"
 
 #include <cub/device/device_scan.cuh>
@@ -309,18 +307,15 @@ inline bool host_acgt(const char c)
     return x == 'a' || x == 'c' || x == 'g' || x == 't';
 }
 
-// ---- The lane kernel's autotuner: seg_tuner.hpp ------------------------------------------------------------------
-
 }
 
-// A batch shape staged once: its offsets, each sequence's first position, and the list of its 512-position segments,
-// all in device memory owned here, for lookups that launch without staging (kache_b200_lookup_prepared).
+// A batch shape staged once: the list of its segments in device memory owned here, for lookups that launch without
+// staging (kache_b200_lookup_prepared).
 struct kache_prepared
 {
     const kache_table* t = nullptr;     // The table that staged it.
-    kache_b200::Dev_Buf off, pos_off, segs;
+    kache_b200::Dev_Buf segs;
     uint64_t n = 0, nsegs = 0, total_pos = 0;
-    uint32_t seg_len = 0;
 };
 
 namespace kache_b200
@@ -395,13 +390,6 @@ class Engine final : public kache_table
     bool prof_ = false;
     struct Ev { cudaEvent_t a, b; uint32_t kind; };
     std::vector<Ev> ev_;
-    // The autotuner, and the current call's choice and lane-kernel event pairs.
-    Seg_Tuner tuner_;
-    int tune_kind_ = -1, tune_cand_ = -1;
-    uint32_t last_seg_len_[3] = {lane_seg_positions, lane_seg_positions, lane_seg_positions};   // Per tuned kind.
-    uint64_t tune_pos_ = 0;
-    std::vector<std::pair<cudaEvent_t, cudaEvent_t>> tune_ev_;
-    size_t tune_used_ = 0;
     double prof_ms_[K_KINDS] = {};
     uint64_t prof_n_[K_KINDS] = {};
 
@@ -411,14 +399,16 @@ class Engine final : public kache_table
     struct Batch_Info
     {
         Dev_Batch b{};
-        uint64_t total_pos = 0;
+        uint64_t n = 0, nsegs = 0, total_pos = 0;
+        // Device arrays over the sequences: offsets of their bases, and the positions before each (n + 1 each).
+        const uint64_t *off = nullptr, *pos_off = nullptr;
         // Listed on the device in sequence order: seg_off[q] (device) counts the segments of the sequences before q,
         // so a range of sequences is a range of segments and of output positions. Null where listed otherwise.
         const uint64_t* seg_off = nullptr;
         // Set where the bases are still in page-locked host memory here, laid end to end (staged with defer_bases).
         const char* host_bases = nullptr;
         // Set where the bases cross in two halves of sequences (ev_in_[0], ev_in_[1]): the table's stream waits for
-        // the first before any launch, lane launches over segments from half_seg on wait for the second.
+        // the first before any launch, launches over segments from half_seg on wait for the second.
         bool in_halves = false;
         uint64_t half_seg = 0;
     };
@@ -586,63 +576,16 @@ class Engine final : public kache_table
     }
 
     bool dretry_dirty_ = true;
-    std::vector<uint64_t> seg_hist_;
 
     // ---- Batches ----
 
-    // Stages a host batch: offsets, positions and segments computed here, bases gathered into pinned memory and copied
-    // in pieces, each piece's H2D copy running while the next one is gathered.
-    // Positions per segment: 512 for the warp kernel (16 rows per warp); for the lane kernel 64, or down to 16 in a
-    // batch too small to give each of the GPU's threads 64 positions, so that small batches still spread over every
-    // SM; eight times longer while a sequence would have more segments than a list entry indexes.
-    uint32_t builtin_seg_len(const uint64_t total_pos) const
+    // Positions per segment: 512 (16 rows of a warp), halved down to one row while a batch of `total` positions would
+    // give each SM fewer than 32 warps; eight times longer while the longest sequence, of `longest` positions, would
+    // have more segments than a list entry indexes.
+    uint32_t seg_len_for(const uint64_t longest, const uint64_t total) const
     {
-        const uint64_t threads = uint64_t(sm_count_) * 2048;
-        uint32_t s = lane_seg_positions;
-        while(s > 16 && total_pos < uint64_t(s) * threads)
-            s /= 2;
-        return s;
-    }
-
-    // The lane segment length for this call: the autotuner's pick for the call's kind, once the batch's positions are
-    // known (total_pos = ~0 while they are not).
-    uint32_t first_seg_len(const bool lanes, const uint64_t total_pos)
-    {
-        if(!lanes)
-            return seg_positions;
-        if(tune_kind_ < 0)
-            return builtin_seg_len(total_pos);
-        if(total_pos == ~0ull)
-            return last_seg_len_[tune_kind_];     // Before counting: likely the length this kind's last call used.
-        tune_cand_ = tuner_.pick(tune_kind_, total_pos, builtin_seg_len(total_pos));
-        tune_pos_ = total_pos;
-        return last_seg_len_[tune_kind_] = Seg_Tuner::seg_len_of(tune_cand_);
-    }
-
-    // Starts a tuned call of `kind` (0 upsert, 1 update, 2 per-sequence reduction); finish_tune() records it.
-    void begin_tune(const int kind) { tune_kind_ = kind, tune_cand_ = -1, tune_pos_ = 0, tune_used_ = 0; }
-
-    // After the call's last sync: its lane kernels' time goes to the tuner.
-    void finish_tune()
-    {
-        double ms = 0;
-        for(size_t i = 0; i < tune_used_; ++i)
-        {
-            float t = 0;
-            if(cudaEventElapsedTime(&t, tune_ev_[i].first, tune_ev_[i].second) == cudaSuccess)
-                ms += t;
-            else
-                (void)cudaGetLastError();
-        }
-        if(tune_used_ > 0)
-            tuner_.record(tune_kind_, tune_pos_, tune_cand_, ms);
-        tune_kind_ = -1, tune_cand_ = -1, tune_used_ = 0;
-    }
-
-    uint32_t seg_len_for(const bool lanes, const uint64_t max_pos, const uint64_t total_pos)
-    {
-        uint64_t s = first_seg_len(lanes, total_pos);
-        while((max_pos + s - 1) / s > max_seg_index + 1)
+        uint64_t s = fitted_seg_len(total, static_cast<uint32_t>(sm_count_));
+        while((longest + s - 1) / s > max_seg_index + 1)
             s *= 8;
         return static_cast<uint32_t>(s);
     }
@@ -684,7 +627,7 @@ class Engine final : public kache_table
         return t;
     }
 
-    Batch_Info stage_host(const char* const* seqs, const size_t* lens, const size_t n, const bool lanes, const bool defer_bases = false,
+    Batch_Info stage_host(const char* const* seqs, const size_t* lens, const size_t n, const bool defer_bases = false,
                           const Host_Scan* scanned = nullptr)
     {
         const Host_Scan hs = scanned ? *scanned : scan_host(seqs, lens, n);
@@ -713,9 +656,8 @@ class Engine final : public kache_table
             // The bases cross next, on the input stream, while the segments are listed here (host-to-device copies
             // share a copy engine, so they follow the offsets); the table's stream waits for them before its next
             // launch.
-            // A large batch for the lane kernel crosses in two halves of sequences, so that its first launch need not
-            // wait for the second half (two at most: a half of a 150 bp read set still fills the GPU's lanes).
-            const bool halves = !defer_bases && lanes && n > small_stage_max && bytes >= (size_t(32) << 20);
+            // A large batch crosses in two halves of sequences, so that its first launch need not wait for the second.
+            const bool halves = !defer_bases && n > small_stage_max && bytes >= (size_t(32) << 20);
             const uint64_t q_half = n / 2, b_half = halves ? off[q_half] : bytes;
             if(!defer_bases)
             {
@@ -729,7 +671,7 @@ class Engine final : public kache_table
                     check(cudaMemcpyAsync(d + b_half, base + b_half, bytes - b_half, cudaMemcpyHostToDevice, in_stream_), "H2D batch");
                 check(cudaEventRecord(ev_bases_, in_stream_), "event record");
             }
-            Batch_Info bi = stage_dev(reinterpret_cast<const uint8_t*>(d), reinterpret_cast<const uint64_t*>(d + o_off), n, lanes);
+            Batch_Info bi = stage_dev(reinterpret_cast<const uint8_t*>(d), reinterpret_cast<const uint64_t*>(d + o_off), n);
             if(defer_bases)
             {
                 bi.host_bases = base;
@@ -741,55 +683,37 @@ class Engine final : public kache_table
                 check(cudaMemcpyAsync(h, bi.seg_off + q_half, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
                 sync();
                 bi.half_seg = *h;
-                bi.in_halves = bi.half_seg > 0 && bi.half_seg < bi.b.nsegs;
+                bi.in_halves = bi.half_seg > 0 && bi.half_seg < bi.nsegs;
             }
             check(cudaStreamWaitEvent(stream_, bi.in_halves ? ev_in_[0] : ev_bases_, 0), "event wait");
             return bi;
         }
         if(n >= host_list_max)
-            return stage_gathered(seqs, lens, n, bytes, lanes);
-        const uint32_t seg_len = seg_len_for(lanes, max_pos, all_pos);
+            return stage_gathered(seqs, lens, n, bytes);
+        const uint32_t seg_len = seg_len_for(max_pos, all_pos);
         uint64_t nsegs = 0;
         for(size_t i = 0; i < n; ++i)
         {
             const uint64_t p = lens[i] >= size_t(k) ? lens[i] - k + 1 : 0;
             nsegs += (p + seg_len - 1) / seg_len;
         }
-        const size_t o_off = 0, o_pos = o_off + (n + 1) * 8, o_seg = o_pos + (n + 1) * 8, o_bases = o_seg + nsegs * 8;
+        const size_t o_off = 0, o_pos = o_off + (n + 1) * 8, o_seg = (o_pos + (n + 1) * 8 + 15) / 16 * 16, o_bases = o_seg + nsegs * sizeof(Segment);
         const size_t total = o_bases + bytes + 64;
         pin_.ensure(total);
         auto* off = pin_.as<uint64_t>(o_off);
         auto* pos_off = pin_.as<uint64_t>(o_pos);
-        auto* segs = pin_.as<uint64_t>(o_seg);
+        auto* segs = pin_.as<Segment>(o_seg);
         char* bases = pin_.as<char>(o_bases);
-        // Segments listed longest first (a counting sort by length), so that the 32 lanes of a warp, which step as
-        // long as their longest segment, get segments of similar lengths.
-        seg_hist_.assign(seg_len + 1, 0);
-        uint64_t b = 0, p = 0;
+        uint64_t b = 0, p = 0, at = 0;
         for(size_t i = 0; i < n; ++i)
         {
             off[i] = b, pos_off[i] = p;
             const uint64_t np = lens[i] >= size_t(k) ? lens[i] - k + 1 : 0;
-            if(np)
-                seg_hist_[seg_len] += np / seg_len, seg_hist_[np % seg_len]++;
+            for(uint64_t p0 = 0; p0 < np; p0 += seg_len)
+                segs[at++] = Segment{b + p0, p + p0, i, static_cast<uint32_t>(std::min<uint64_t>(np - p0, seg_len)), 0};
             b += lens[i], p += np;
         }
         off[n] = b, pos_off[n] = p;
-        seg_hist_[0] = 0;
-        for(uint64_t len = seg_len, at = 0; len > 0; --len)
-        {
-            const uint64_t c = seg_hist_[len];
-            seg_hist_[len] = at, at += c;
-        }
-        for(size_t i = 0; i < n; ++i)
-        {
-            const uint64_t np = lens[i] >= size_t(k) ? lens[i] - k + 1 : 0;
-            for(uint64_t s = 0; s * seg_len < np; ++s)
-            {
-                const uint64_t len = std::min<uint64_t>(np - s * seg_len, seg_len);
-                segs[seg_hist_[len]++] = (uint64_t(i) << 24) | s;
-            }
-        }
         dbatch_.ensure(total);
         char* d = dbatch_.as<char>();
         check(cudaMemcpyAsync(d, pin_.p, o_bases, cudaMemcpyHostToDevice, stream_), "H2D batch");
@@ -810,8 +734,8 @@ class Engine final : public kache_table
             i0 = i1;
         }
         Batch_Info bi;
-        bi.b = Dev_Batch{reinterpret_cast<const uint8_t*>(d + o_bases), reinterpret_cast<const uint64_t*>(d + o_off),
-                         reinterpret_cast<const uint64_t*>(d + o_seg), reinterpret_cast<const uint64_t*>(d + o_pos), n, nsegs, seg_len};
+        bi.b = Dev_Batch{reinterpret_cast<const uint8_t*>(d + o_bases), reinterpret_cast<const Segment*>(d + o_seg)};
+        bi.n = n, bi.nsegs = nsegs, bi.off = reinterpret_cast<const uint64_t*>(d + o_off), bi.pos_off = reinterpret_cast<const uint64_t*>(d + o_pos);
         bi.total_pos = p;
         return bi;
     }
@@ -821,7 +745,7 @@ class Engine final : public kache_table
     // million reads on the host (three passes and a counting sort) would take longer than the kernel that follows.
     static constexpr size_t host_list_max = 16384;
 
-    Batch_Info stage_gathered(const char* const* seqs, const size_t* lens, const size_t n, const uint64_t bytes, const bool lanes)
+    Batch_Info stage_gathered(const char* const* seqs, const size_t* lens, const size_t n, const uint64_t bytes)
     {
         const size_t o_hb = (n + 1) * 8;
         pin_.ensure(o_hb + bytes + 64);
@@ -853,58 +777,44 @@ class Engine final : public kache_table
             i0 = i1;
         }
         check(cudaMemsetAsync(d + bytes, 0, 64, stream_), "memset");
-        return stage_dev(reinterpret_cast<const uint8_t*>(d), reinterpret_cast<const uint64_t*>(d + o_off), n, lanes);
+        return stage_dev(reinterpret_cast<const uint8_t*>(d), reinterpret_cast<const uint64_t*>(d + o_off), n);
     }
 
-    // stage_dev for a batch of at most small_stage_max sequences: one block counts and sums, one kernel lists.
-    Batch_Info stage_dev_small(const uint8_t* bases, const uint64_t* off, const uint64_t n, const bool lanes)
+    // stage_dev for a batch of at most small_stage_max sequences: one block counts, fits the segment length and sums, one
+    // kernel lists.
+    Batch_Info stage_dev_small(const uint8_t* bases, const uint64_t* off, const uint64_t n, const uint64_t* addr)
     {
         dtmp_.ensure(2 * (n + 1) * 8);
         uint64_t* pos_off = dtmp_.as<uint64_t>();
         uint64_t* seg_off = pos_off + (n + 1);
-        unsigned long long* out = ctr() + 3;    // Three words: positions, segments, too long.
+        unsigned long long* out = ctr() + 3;    // Three words: positions, segments, segment length.
         uint64_t* h = pin_ctr_.as<uint64_t>(32);
-        uint32_t seg_len = first_seg_len(lanes, ~0ull);
-        bool sized = false;
-        for(;;)
-        {
-            launch(K_OTHER, [&](){ stage_small_kernel<<<1, 1024, 0, stream_>>>(off, n, k, seg_len, pos_off, seg_off, out); });
-            check(cudaMemcpyAsync(h, out, 24, cudaMemcpyDeviceToHost, stream_), "D2H");
-            sync();
-            if(h[2])
-            {
-                seg_len *= 8;   // A sequence has more segments than a list entry indexes.
-                sized = true;
-                continue;
-            }
-            if(!sized && lanes)
-            {
-                sized = true;
-                const uint32_t want = first_seg_len(lanes, h[0]);
-                if(want != seg_len)
-                {
-                    seg_len = want;
-                    continue;
-                }
-            }
-            break;
-        }
-        const uint64_t nsegs = h[1];
-        dbatch_.ensure(nsegs * 8 + 8);
+        launch(K_OTHER, [&](){ stage_small_kernel<<<1, 1024, 0, stream_>>>(off, n, k, static_cast<uint32_t>(sm_count_), pos_off, seg_off, out); });
+        check(cudaMemcpyAsync(h, out, 24, cudaMemcpyDeviceToHost, stream_), "D2H");
+        sync();
+        return list_dev(bases, off, addr, n, pos_off, seg_off, h[0], h[1], static_cast<uint32_t>(h[2]));
+    }
+
+    // Lists the segments of a batch whose positions and segments are counted.
+    Batch_Info list_dev(const uint8_t* bases, const uint64_t* off, const uint64_t* addr, const uint64_t n, const uint64_t* pos_off, const uint64_t* seg_off,
+                        const uint64_t total_pos, const uint64_t nsegs, const uint32_t seg_len)
+    {
+        dbatch_.ensure((nsegs + 1) * sizeof(Segment));
         if(nsegs > 0)
-            launch(K_OTHER, [&](){ segs_kernel<<<grid_for((nsegs + 31) / 32, 8), 256, 0, stream_>>>(seg_off, n, nsegs, dbatch_.as<uint64_t>()); });
+            launch(K_OTHER, [&](){ segs_kernel<<<grid_for((nsegs + 31) / 32, 8), 256, 0, stream_>>>(seg_off, pos_off, off, addr, n, nsegs, seg_len, dbatch_.as<Segment>()); });
         Batch_Info bi;
-        bi.b = Dev_Batch{bases, off, dbatch_.as<uint64_t>(), pos_off, n, nsegs, seg_len};
-        bi.total_pos = h[0];
-        bi.seg_off = seg_off;
+        bi.b = Dev_Batch{bases, dbatch_.as<Segment>()};
+        bi.n = n, bi.nsegs = nsegs, bi.total_pos = total_pos;
+        bi.off = off, bi.pos_off = pos_off, bi.seg_off = seg_off;
         return bi;
     }
 
-    // Prepares a batch already in device memory: positions and segments computed on the device.
-    Batch_Info stage_dev(const uint8_t* bases, const uint64_t* off, const uint64_t n, const bool lanes)
+    // Prepares a batch already in device memory: positions and segments computed on the device. With `addr`, sequence q's
+    // bases are at the device address addr[q] and off only lays the lengths end to end.
+    Batch_Info stage_dev(const uint8_t* bases, const uint64_t* off, const uint64_t n, const uint64_t* addr = nullptr)
     {
         if(n > 0 && n <= small_stage_max)
-            return stage_dev_small(bases, off, n, lanes);
+            return stage_dev_small(bases, off, n, addr);
         const size_t o_npos = 0, o_nseg = o_npos + (n + 1) * 8, o_pos = o_nseg + (n + 1) * 8, o_sego = o_pos + (n + 1) * 8;
         const size_t head = o_sego + (n + 1) * 8;
         dtmp_.ensure(head);
@@ -915,8 +825,7 @@ class Engine final : public kache_table
         auto* seg_off = reinterpret_cast<uint64_t*>(d + o_sego);
         unsigned int* too_long = reinterpret_cast<unsigned int*>(ctr() + 3);
         uint64_t* h = pin_ctr_.as<uint64_t>(32);
-        uint32_t seg_len = first_seg_len(lanes, ~0ull);
-        bool sized = false;     // Whether the lane segments were fitted to the batch's positions.
+        uint32_t seg_len = seg_positions;   // A batch of this many sequences has a warp's segment for each.
         for(;;)
         {
             check(cudaMemsetAsync(too_long, 0, 4, stream_), "memset");
@@ -936,40 +845,15 @@ class Engine final : public kache_table
             check(cudaMemcpyAsync(h + 1, seg_off + n, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
             check(cudaMemcpyAsync(h + 2, too_long, 4, cudaMemcpyDeviceToHost, stream_), "D2H");
             sync();
-            if(static_cast<uint32_t>(h[2]))
-            {
-                seg_len *= 8;   // A sequence has more segments than a list entry indexes.
-                sized = true;
-                continue;
-            }
-            if(!sized && lanes)
-            {
-                sized = true;
-                const uint32_t want = first_seg_len(lanes, h[0]);
-                if(want != seg_len)
-                {
-                    seg_len = want;     // Count again with the segment length chosen for this batch's size.
-                    continue;
-                }
-            }
-            break;
+            if(static_cast<uint32_t>(h[2]) == 0)
+                break;
+            seg_len *= 8;   // A sequence has more segments than a list entry indexes.
         }
-        const uint64_t total_pos = h[0], nsegs = h[1];
-        dbatch_.ensure(nsegs * 8 + 8);
-        if(nsegs > 0)
-            launch(K_OTHER, [&](){ segs_kernel<<<grid_for((nsegs + 31) / 32, 8), 256, 0, stream_>>>(seg_off, n, nsegs, dbatch_.as<uint64_t>()); });
-        Batch_Info bi;
-        bi.b = Dev_Batch{bases, off, dbatch_.as<uint64_t>(), pos_off, n, nsegs, seg_len};
-        bi.total_pos = total_pos;
-        bi.seg_off = seg_off;
-        return bi;
+        return list_dev(bases, off, addr, n, pos_off, seg_off, h[0], h[1], seg_len);
     }
 
-    // Operations without per-position output (upsert, update, per-sequence reductions) run one lane per segment
-    // (device_lanes.cuh): rolling descriptions, and lanes of a warp on different reads. Lookups and descriptions, whose
-    // outputs are per position, run one warp per segment (device_stream.cuh), so that a row's 32 outputs are written
-    // as one coalesced store.
-    template <typename Vis> void stream_launch(const uint32_t kind, const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Vis& vis, const bool per_position = false)
+    // Runs the visitor over segments [sb, se) of a batch, a warp per segment (device_stream.cuh).
+    template <typename Vis> void stream_launch(const uint32_t kind, const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Vis& vis)
     {
         if(se <= sb)
             return;
@@ -977,44 +861,18 @@ class Engine final : public kache_table
         {
             // Segments before half_seg read the first half of the bases, which has crossed; the rest wait for the
             // second.
-            if(per_position || sb >= bi.half_seg)
-                check(cudaStreamWaitEvent(stream_, ev_bases_, 0), "event wait");
-            else
-            {
-                lane_launch(kind, bi, sb, bi.half_seg, vis);
-                check(cudaStreamWaitEvent(stream_, ev_bases_, 0), "event wait");
-                lane_launch(kind, bi, bi.half_seg, se, vis);
-                return;
-            }
-        }
-        if(per_position)
-        {
-            launch(kind, [&](){ stream_kernel<k, l, Vis><<<grid_for(se - sb, stream_warps), 32 * stream_warps, 0, stream_>>>(bi.b, sb, se, vis); });
+            if(sb < bi.half_seg)
+                segs_launch(kind, bi, sb, bi.half_seg, vis);
+            check(cudaStreamWaitEvent(stream_, ev_bases_, 0), "event wait");
+            segs_launch(kind, bi, std::max(sb, bi.half_seg), se, vis);
             return;
         }
-        lane_launch(kind, bi, sb, se, vis);
+        segs_launch(kind, bi, sb, se, vis);
     }
 
-    template <typename Vis> void lane_launch(const uint32_t kind, const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Vis& vis)
+    template <typename Vis> void segs_launch(const uint32_t kind, const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Vis& vis)
     {
-        const bool timed = tune_kind_ >= 0 && tune_cand_ >= 0;
-        const uint64_t per_sm = timed ? Seg_Tuner::blocks_of(tune_cand_) : Seg_Tuner::blocks[0];
-        const uint64_t blocks = std::min<uint64_t>((se - sb + lane_block - 1) / lane_block, uint64_t(sm_count_) * per_sm);
-        unsigned long long* next = ctr() + 7;     // The lane kernel's work counter.
-        check(cudaMemsetAsync(next, 0, sizeof(unsigned long long), stream_), "memset");
-        if(timed)
-        {
-            if(tune_used_ == tune_ev_.size())
-            {
-                std::pair<cudaEvent_t, cudaEvent_t> e{};
-                check(cudaEventCreate(&e.first), "event"), check(cudaEventCreate(&e.second), "event");
-                tune_ev_.push_back(e);
-            }
-            check(cudaEventRecord(tune_ev_[tune_used_].first, stream_), "record");
-        }
-        launch(kind, [&](){ lane_kernel<k, l, Vis><<<static_cast<unsigned>(blocks), lane_block, 0, stream_>>>(bi.b, sb, se, next, vis); });
-        if(timed)
-            check(cudaEventRecord(tune_ev_[tune_used_++].second, stream_), "record");
+        launch(kind, [&](){ stream_kernel<k, l, Vis><<<grid_for(se - sb, stream_warps), 32 * stream_warps, 0, stream_>>>(bi.b, sb, se, vis); });
     }
 
     // The reference's per-user flush accounting over one call (include/Streaming_Kmer_Hash_Table.hpp:2248-2286,
@@ -1140,7 +998,7 @@ class Engine final : public kache_table
     // Upserts a staged batch with the value functor `fn`, chunk by chunk (see the top of this file).
     template <typename Fn> uint64_t run_upsert(const uint32_t user, const Batch_Info& bi, const Fn& fn, unsigned long long* per_seq = nullptr)
     {
-        const uint64_t nsegs = bi.b.nsegs;
+        const uint64_t nsegs = bi.nsegs;
         const double pos_per_seg = nsegs ? static_cast<double>(bi.total_pos) / nsegs : 1.0;
         uint64_t total_ins = 0;
         // Keys inserted per position: as the previous call measured (1/2 before the first), then as the last chunk
@@ -1169,7 +1027,7 @@ class Engine final : public kache_table
             const double rate = assume_all_new ? 1.0 : std::max(1.25 * novelty, 0.25);
             const double want_pos = room / rate;
             uint64_t se = sb + std::max<uint64_t>(1, static_cast<uint64_t>(want_pos / pos_per_seg));
-            // No small last chunk (it would run with too few lanes to fill the GPU), if the rest fits at the rate.
+            // No small last chunk (it would run with too few warps to fill the GPU), if the rest fits at the rate.
             if(se + (se - sb) / 2 >= nsegs && static_cast<double>(nsegs - sb) * pos_per_seg * rate <= 1.25 * room)
                 se = nsegs;
             se = std::min(se, nsegs);
@@ -1177,7 +1035,7 @@ class Engine final : public kache_table
 
             check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
             check(cudaMemsetAsync(retried, 0, 4, stream_), "memset");
-            Upsert_Visitor<set_, VT, Fn> vis{T_, fn, bi.b.pos_off, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, 0, per_seq};
+            Upsert_Visitor<set_, VT, Fn> vis{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per_seq};
             stream_launch(K_UPSERT, bi, sb, se, vis);
             const unsigned long long* c = read_ctr(3);
             uint64_t ins = c[0];
@@ -1188,7 +1046,7 @@ class Engine final : public kache_table
                 check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
                 check(cudaMemsetAsync(retried, 0, 4, stream_), "memset");
                 check(cudaMemsetAsync(dretry_b_.p, 0, bits, stream_), "memset");
-                Upsert_Visitor<set_, VT, Fn> rv{T_, fn, bi.b.pos_off, ctr(), dretry_b_.as<unsigned int>(), dretry_a_.as<unsigned int>(), retried, 0, per_seq};
+                Upsert_Visitor<set_, VT, Fn> rv{T_, fn, ctr(), dretry_b_.as<unsigned int>(), dretry_a_.as<unsigned int>(), retried, per_seq};
                 stream_launch(K_UPSERT, bi, sb, se, rv);
                 check(cudaMemsetAsync(dretry_a_.p, 0, bits, stream_), "memset");
                 std::swap(dretry_a_.p, dretry_b_.p), std::swap(dretry_a_.bytes, dretry_b_.bytes);
@@ -1215,26 +1073,26 @@ class Engine final : public kache_table
     template <typename Fn> uint64_t run_update(const Batch_Info& bi, const Fn& fn)
     {
         check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
-        Update_Visitor<VT, Fn> vis{T_, fn, ctr(), 0};
-        stream_launch(K_UPDATE, bi, 0, bi.b.nsegs, vis);
+        Update_Visitor<VT, Fn> vis{T_, fn, ctr(), nullptr};
+        stream_launch(K_UPDATE, bi, 0, bi.nsegs, vis);
         return read_ctr(3)[0];
     }
 
     void run_lookup(const Batch_Info& bi, uint8_t* found, VT* values, uint8_t* fwd)
     {
-        Lookup_Visitor<set_, VT> vis{T_, bi.b.pos_off, found, values, fwd, 0};
-        stream_launch(K_LOOKUP, bi, 0, bi.b.nsegs, vis, true);
+        Lookup_Visitor<set_, VT> vis{T_, found, values, fwd};
+        stream_launch(K_LOOKUP, bi, 0, bi.nsegs, vis);
     }
 
     void run_seq_reduce(const Batch_Info& bi, const int mode, const uint64_t mf, const uint64_t mr, unsigned long long* out)
     {
-        check(cudaMemsetAsync(out, 0, bi.b.n * 8, stream_), "memset");
+        check(cudaMemsetAsync(out, 0, bi.n * 8, stream_), "memset");
         if(mode == 0)
-            stream_launch(K_REDUCE, bi, 0, bi.b.nsegs, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(mf), VT(mr), 0, 0});
+            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(mf), VT(mr), 0, 0});
         else if(mode == 1)
-            stream_launch(K_REDUCE, bi, 0, bi.b.nsegs, Seq_Reduce_Visitor<set_, VT, 1>{T_, out, VT(mf), VT(mr), 0, 0});
+            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 1>{T_, out, VT(mf), VT(mr), 0, 0});
         else
-            stream_launch(K_REDUCE, bi, 0, bi.b.nsegs, Seq_Reduce_Visitor<set_, VT, 2>{T_, out, VT(mf), VT(mr), 0, 0});
+            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 2>{T_, out, VT(mf), VT(mr), 0, 0});
     }
 
     // Whether host memory at p is page-locked (the caller's cudaHostAlloc'd or registered memory): copies then use it
@@ -1274,21 +1132,21 @@ class Engine final : public kache_table
         side_streams();
         piece_events();
         // Piece boundaries at sequences c * n / pieces: their first output position, first segment and first base.
-        const uint64_t n = bi.b.n;
+        const uint64_t n = bi.n;
         pin_piece_.ensure(3 * (out_pieces + 1) * 8);
         auto* h = pin_piece_.as<uint64_t>();
         for(int c = 0; c <= out_pieces; ++c)
         {
             const uint64_t q = n * c / out_pieces;
-            check(cudaMemcpyAsync(h + c, bi.b.pos_off + q, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
+            check(cudaMemcpyAsync(h + c, bi.pos_off + q, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
             check(cudaMemcpyAsync(h + out_pieces + 1 + c, bi.seg_off + q, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
             if(bi.host_bases)
-                check(cudaMemcpyAsync(h + 2 * (out_pieces + 1) + c, bi.b.off + q, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
+                check(cudaMemcpyAsync(h + 2 * (out_pieces + 1) + c, bi.off + q, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
         }
         sync();
         if(bi.host_bases)   // The input stream's copies come after this stream's earlier work.
             check(cudaEventRecord(ev_stage_, stream_), "event record"), check(cudaStreamWaitEvent(in_stream_, ev_stage_, 0), "event wait");
-        Lookup_Visitor<set_, VT> vis{T_, bi.b.pos_off, d_found, d_val, d_fwd, 0};
+        Lookup_Visitor<set_, VT> vis{T_, d_found, d_val, d_fwd};
         for(int c = 0; c < out_pieces; ++c)
         {
             const uint64_t p0 = h[c], p1 = h[c + 1], g0 = h[out_pieces + 1 + c], g1 = h[out_pieces + 2 + c];
@@ -1301,7 +1159,7 @@ class Engine final : public kache_table
                 check(cudaEventRecord(ev_in_[c], in_stream_), "event record");
                 check(cudaStreamWaitEvent(stream_, ev_in_[c], 0), "event wait");
             }
-            stream_launch(K_LOOKUP, bi, g0, g1, vis, true);
+            stream_launch(K_LOOKUP, bi, g0, g1, vis);
             check(cudaEventRecord(ev_piece_[c], stream_), "event record");
             check(cudaStreamWaitEvent(copy_stream_, ev_piece_[c], 0), "event wait");
             if(p1 > p0)
@@ -1393,8 +1251,6 @@ public:
         for(auto& e : ev_out_)
             if(e)
                 cudaEventDestroy(e);
-        for(auto& e : tune_ev_)
-            cudaEventDestroy(e.first), cudaEventDestroy(e.second);
         for(int c = 0; c < out_pieces; ++c)
         {
             if(ev_piece_[c])
@@ -1422,23 +1278,19 @@ public:
     uint64_t upsert(uint32_t user, const char* const* seqs, const size_t* lens, size_t n, uint32_t op, uint64_t x, uint64_t init) override
     {
         std::lock_guard<std::mutex> g(work);
-        begin_tune(0);
-        const auto bi = stage_host(seqs, lens, n, true);
+        const auto bi = stage_host(seqs, lens, n);
         const uint64_t r = run_upsert(user, bi, op_fn(op, x, init));
-        finish_tune();
         return r;
     }
 
     uint64_t upsert_split(uint32_t user, const char* const* seqs, const size_t* lens, size_t n, uint32_t op, uint64_t x, uint64_t init, uint64_t* per_seq) override
     {
         std::lock_guard<std::mutex> g(work);
-        begin_tune(0);
-        const auto bi = stage_host(seqs, lens, n, true);
+        const auto bi = stage_host(seqs, lens, n);
         dout_.ensure(n * 8 + 8);
         check(cudaMemsetAsync(dout_.p, 0, n * 8, stream_), "memset");
         const uint64_t r = run_upsert(user, bi, op_fn(op, x, init), dout_.as<unsigned long long>());
         d2h(per_seq, dout_.p, n * 8);
-        finish_tune();
         return r;
     }
 
@@ -1449,10 +1301,8 @@ public:
         else
         {
             std::lock_guard<std::mutex> g(work);
-            begin_tune(0);
-            const auto bi = stage_host(seqs, lens, n, true);
+            const auto bi = stage_host(seqs, lens, n);
             const uint64_t r = run_upsert(user, bi, Oriented_Op_Fn<VT>{op, static_cast<VT>(xf), static_cast<VT>(xr)});
-            finish_tune();
             return r;
         }
     }
@@ -1464,10 +1314,8 @@ public:
         else
         {
             std::lock_guard<std::mutex> g(work);
-            begin_tune(1);
-            const auto bi = stage_host(seqs, lens, n, true);
+            const auto bi = stage_host(seqs, lens, n);
             const uint64_t r = run_update(bi, op_fn(op, x, 0));
-            finish_tune();
             return r;
         }
     }
@@ -1483,7 +1331,7 @@ public:
         const bool out_pinned = P_est > 0 && pinned_range(found, P_est) && (!vb_est || pinned_range(values, P_est * vb_est)) &&
                                 (!fwd || pinned_range(fwd, P_est));
         const bool pieces = out_pinned && n >= 2 * out_pieces && P_est >= (uint64_t(1) << 22);
-        const auto bi = stage_host(seqs, lens, n, false, pieces, &hs);
+        const auto bi = stage_host(seqs, lens, n, pieces, &hs);
         const uint64_t P = bi.total_pos;
         const size_t vb = (!set_ && values) ? sizeof(VT) : 0;
         const size_t a_found = (P + 15) / 16 * 16, a_val = (P * vb + 15) / 16 * 16;
@@ -1501,7 +1349,7 @@ public:
             return;
         }
         if(bi.host_bases)   // Staged for pieces but not run in them: the bases cross whole first.
-            check(cudaMemcpyAsync(const_cast<uint8_t*>(bi.b.bases), bi.host_bases, bi.b.off ? host_bytes(lens, n) : 0, cudaMemcpyHostToDevice, stream_), "H2D batch");
+            check(cudaMemcpyAsync(const_cast<uint8_t*>(bi.b.bases), bi.host_bases, bi.off ? host_bytes(lens, n) : 0, cudaMemcpyHostToDevice, stream_), "H2D batch");
         run_lookup(bi, d_found, d_val, d_fwd);
         d2h(found, d_found, P);
         if(vb)
@@ -1513,34 +1361,30 @@ public:
     void seq_reduce(const char* const* seqs, const size_t* lens, size_t n, int mode, uint64_t m_fwd, uint64_t m_rev, uint64_t* out) override
     {
         std::lock_guard<std::mutex> g(work);
-        begin_tune(2);
-        const auto bi = stage_host(seqs, lens, n, true);
+        const auto bi = stage_host(seqs, lens, n);
         dout_.ensure(n * 8 + 8);
         run_seq_reduce(bi, mode, m_fwd, m_rev, dout_.as<unsigned long long>());
         d2h(out, dout_.p, n * 8);
-        finish_tune();
     }
 
     void describe(const char* const* seqs, const size_t* lens, size_t n, uint64_t* key, uint64_t* h, uint8_t* cs, uint8_t* fwd, uint8_t* valid) override
     {
         std::lock_guard<std::mutex> g(work);
-        const auto bi = stage_host(seqs, lens, n, false);
+        const auto bi = stage_host(seqs, lens, n);
         const uint64_t P = bi.total_pos;
         dout_.ensure(P * 19 + 64);
         auto* dk = dout_.as<uint64_t>();
         auto* dh = dk + P;
         auto* dc = reinterpret_cast<uint8_t*>(dh + P);
-        stream_launch(K_OTHER, bi, 0, bi.b.nsegs, Describe_Visitor{bi.b.pos_off, dk, dh, dc, dc + P, dc + 2 * P, false}, true);
+        stream_launch(K_OTHER, bi, 0, bi.nsegs, Describe_Visitor<k, l>{dk, dh, dc, dc + P, dc + 2 * P});
         d2h(key, dk, P * 8), d2h(h, dh, P * 8), d2h(cs, dc, P), d2h(fwd, dc + P, P), d2h(valid, dc + 2 * P, P);
     }
 
     uint64_t upsert_dev(uint32_t user, const uint8_t* b, const uint64_t* off, uint64_t n, uint32_t op, uint64_t x, uint64_t init) override
     {
         std::lock_guard<std::mutex> g(work);
-        begin_tune(0);
-        const auto bi = stage_dev(b, off, n, true);
+        const auto bi = stage_dev(b, off, n);
         const uint64_t r = run_upsert(user, bi, op_fn(op, x, init));
-        finish_tune();
         return r;
     }
 
@@ -1551,10 +1395,8 @@ public:
         else
         {
             std::lock_guard<std::mutex> g(work);
-            begin_tune(0);
-            const auto bi = stage_dev(b, off, n, true);
+            const auto bi = stage_dev(b, off, n);
             const uint64_t r = run_upsert(user, bi, Oriented_Op_Fn<VT>{op, static_cast<VT>(xf), static_cast<VT>(xr)});
-            finish_tune();
             return r;
         }
     }
@@ -1566,10 +1408,8 @@ public:
         else
         {
             std::lock_guard<std::mutex> g(work);
-            begin_tune(1);
-            const auto bi = stage_dev(b, off, n, true);
+            const auto bi = stage_dev(b, off, n);
             const uint64_t r = run_update(bi, op_fn(op, x, 0));
-            finish_tune();
             return r;
         }
     }
@@ -1577,7 +1417,7 @@ public:
     void lookup_dev(const uint8_t* b, const uint64_t* off, uint64_t n, uint8_t* found, void* values, uint8_t* fwd) override
     {
         std::lock_guard<std::mutex> g(work);
-        const auto bi = stage_dev(b, off, n, false);
+        const auto bi = stage_dev(b, off, n);
         run_lookup(bi, found, set_ ? nullptr : static_cast<VT*>(values), fwd);
         sync();
     }
@@ -1587,19 +1427,14 @@ public:
     kache_prepared* prepare_dev(const uint64_t* off, const uint64_t n) override
     {
         std::lock_guard<std::mutex> g(work);
-        const auto bi = stage_dev(nullptr, off, n, false);
+        const auto bi = stage_dev(nullptr, off, n);
         auto* p = new kache_prepared;
         try
         {
-            p->t = this, p->n = n, p->nsegs = bi.b.nsegs, p->total_pos = bi.total_pos, p->seg_len = bi.b.seg_len;
-            p->off.ensure((n + 1) * 8), p->pos_off.ensure((n + 1) * 8), p->segs.ensure(bi.b.nsegs * 8 + 8);
-            if(n > 0)
-            {
-                check(cudaMemcpyAsync(p->off.p, off, (n + 1) * 8, cudaMemcpyDeviceToDevice, stream_), "copy");
-                check(cudaMemcpyAsync(p->pos_off.p, bi.b.pos_off, (n + 1) * 8, cudaMemcpyDeviceToDevice, stream_), "copy");
-            }
-            if(bi.b.nsegs)
-                check(cudaMemcpyAsync(p->segs.p, bi.b.segs, bi.b.nsegs * 8, cudaMemcpyDeviceToDevice, stream_), "copy");
+            p->t = this, p->n = n, p->nsegs = bi.nsegs, p->total_pos = bi.total_pos;
+            p->segs.ensure((bi.nsegs + 1) * sizeof(Segment));
+            if(bi.nsegs)
+                check(cudaMemcpyAsync(p->segs.p, bi.b.segs, bi.nsegs * sizeof(Segment), cudaMemcpyDeviceToDevice, stream_), "copy");
             sync();
         }
         catch(...)
@@ -1616,8 +1451,8 @@ public:
     {
         std::lock_guard<std::mutex> g(work);
         Batch_Info bi;
-        bi.b = Dev_Batch{b, p.off.as<uint64_t>(), p.segs.as<uint64_t>(), p.pos_off.as<uint64_t>(), p.n, p.nsegs, p.seg_len};
-        bi.total_pos = p.total_pos;
+        bi.b = Dev_Batch{b, p.segs.as<Segment>()};
+        bi.n = p.n, bi.nsegs = p.nsegs, bi.total_pos = p.total_pos;
         run_lookup(bi, found, set_ ? nullptr : static_cast<VT*>(values), fwd);
     }
 
@@ -1627,12 +1462,12 @@ public:
     {
         std::lock_guard<std::mutex> g(work);
         Batch_Info bi;
-        bi.b = Dev_Batch{b, p.off.as<uint64_t>(), p.segs.as<uint64_t>(), p.pos_off.as<uint64_t>(), p.n, p.nsegs, p.seg_len};
-        bi.total_pos = p.total_pos;
+        bi.b = Dev_Batch{b, p.segs.as<Segment>()};
+        bi.n = p.n, bi.nsegs = p.nsegs, bi.total_pos = p.total_pos;
         auto* out = reinterpret_cast<unsigned long long*>(counts);
         if(p.n)
             check(cudaMemsetAsync(out, 0, p.n * 8, stream_), "memset");
-        stream_launch(K_REDUCE, bi, 0, bi.b.nsegs, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(0), VT(0), 0, 0}, true);
+        stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(0), VT(0), 0, 0});
     }
 
     // A number that stays the same while the table's device arrays do (a graph captured with a prepared lookup stays
@@ -1650,15 +1485,13 @@ public:
     void count_dev(const uint8_t* b, const uint64_t* off, uint64_t n, uint64_t* counts) override
     {
         std::lock_guard<std::mutex> g(work);
-        begin_tune(2);
-        const auto bi = stage_dev(b, off, n, true);
+        const auto bi = stage_dev(b, off, n);
         run_seq_reduce(bi, 0, 0, 0, reinterpret_cast<unsigned long long*>(counts));
         sync();
-        finish_tune();
     }
 
     // Several batches in device memory as one call: their sequences are listed as one batch whose lengths lie end to
-    // end and whose sequences are read where they lie (Dev_Batch::seq_addr), so all share one segment list, one
+    // end and whose sequences are read where they lie, so all share one segment list, one
     // launch and one pass of the resize schedule; results go back to each batch.
     void run_dev_batches(const uint32_t user, const uint32_t kind, const uint32_t op, const uint64_t x, const uint64_t y,
                          kache_dev_batch* const bs, const size_t count) override
@@ -1700,15 +1533,7 @@ public:
         dscan_.ensure(tmp);
         check(cub::DeviceScan::InclusiveSum(dscan_.p, tmp, lens, voff + 1, static_cast<int64_t>(N), stream_), "scan");
 
-        const bool lanes = kind != KACHE_B200_RUN_LOOKUP;
-        if(kind == KACHE_B200_RUN_UPSERT || kind == KACHE_B200_RUN_UPSERT_ORIENTED)
-            begin_tune(0);
-        else if(kind == KACHE_B200_RUN_UPDATE)
-            begin_tune(1);
-        else if(kind == KACHE_B200_RUN_COUNT)
-            begin_tune(2);
-        auto bi = stage_dev(nullptr, voff, N, lanes);
-        bi.b.seq_addr = addr;
+        const auto bi = stage_dev(nullptr, voff, N, addr);
         dout_.ensure(N * 8 + 8);
         auto* per_seq = dout_.as<unsigned long long>();
         check(cudaMemsetAsync(per_seq, 0, N * 8, stream_), "memset");
@@ -1724,9 +1549,8 @@ public:
             if constexpr(!set_)
             {
                 check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
-                Update_Visitor<VT, Op_Fn<VT>> vis{T_, op_fn(op, x, 0), ctr(), 0};
-                vis.per_seq = per_seq;
-                stream_launch(K_UPDATE, bi, 0, bi.b.nsegs, vis);
+                Update_Visitor<VT, Op_Fn<VT>> vis{T_, op_fn(op, x, 0), ctr(), per_seq};
+                stream_launch(K_UPDATE, bi, 0, bi.nsegs, vis);
             }
         }
         else if(kind == KACHE_B200_RUN_COUNT)
@@ -1736,10 +1560,10 @@ public:
         }
         else
         {
-            launch(K_OTHER, [&](){ batches_pos_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, stream_>>>(desc, count, bi.b.pos_off, pos_base); });
-            Lookup_Batches_Visitor<set_, VT> vis{{T_, bi.b.pos_off, nullptr, nullptr, nullptr, 0}, batch_of, desc, pos_base};
-            stream_launch(K_LOOKUP, bi, 0, bi.b.nsegs, vis, true);
-            launch(K_OTHER, [&](){ batches_hits_kernel<<<grid_for(N, 8), 256, 0, stream_>>>(desc, batch_of, bi.b.pos_off, pos_base, N, per_seq); });
+            launch(K_OTHER, [&](){ batches_pos_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, stream_>>>(desc, count, bi.pos_off, pos_base); });
+            Lookup_Batches_Visitor<set_, VT> vis{{T_, nullptr, nullptr, nullptr}, batch_of, desc, pos_base};
+            stream_launch(K_LOOKUP, bi, 0, bi.nsegs, vis);
+            launch(K_OTHER, [&](){ batches_hits_kernel<<<grid_for(N, 8), 256, 0, stream_>>>(desc, batch_of, bi.pos_off, pos_base, N, per_seq); });
         }
         // Per-batch results: the per-sequence counters (keys inserted, k-mers present, positions found, counts)
         // summed per batch.
@@ -1750,8 +1574,6 @@ public:
         sync();
         for(size_t b = 0; b < count; ++b)
             bs[b].result = hr[b];
-        if(lanes)
-            finish_tune();
     }
 
     bool get(const char* kmer, uint64_t& value) override
@@ -1770,7 +1592,7 @@ public:
         const uint64_t key = f < r ? f : r;
         std::lock_guard<std::mutex> g(work);
         auto* h = pin_ctr_.as<uint64_t>(0);
-        h[0] = key;
+        h[0] = key_of_encoding(key);
         unsigned long long* d = ctr() + 4;
         check(cudaMemcpyAsync(d, h, 8, cudaMemcpyHostToDevice, stream_), "H2D");
         launch(K_OTHER, [&](){ get_kernel<k, l, set_, VT><<<1, 32, 0, stream_>>>(T_, reinterpret_cast<const uint64_t*>(d), 1, d + 1); });
@@ -1871,20 +1693,16 @@ public:
     template <typename Fn> uint64_t upsert_with(const uint32_t user, const char* const* seqs, const size_t* lens, const size_t n, const Fn& fn)
     {
         std::lock_guard<std::mutex> g(work);
-        begin_tune(0);
-        const auto bi = stage_host(seqs, lens, n, true);
+        const auto bi = stage_host(seqs, lens, n);
         const uint64_t r = run_upsert(user, bi, fn);
-        finish_tune();
         return r;
     }
 
     template <typename Fn> uint64_t update_with(const char* const* seqs, const size_t* lens, const size_t n, const Fn& fn)
     {
         std::lock_guard<std::mutex> g(work);
-        begin_tune(1);
-        const auto bi = stage_host(seqs, lens, n, true);
+        const auto bi = stage_host(seqs, lens, n);
         const uint64_t r = run_update(bi, fn);
-        finish_tune();
         return r;
     }
 
@@ -1899,7 +1717,7 @@ public:
     {
         std::lock_guard<std::mutex> g(work);
         unsigned long long* d = ctr() + 4;
-        launch(K_OTHER, [&](){ plant_claim_kernel<k, l, set_><<<1, 1, 0, stream_>>>(T_, key, d); });
+        launch(K_OTHER, [&](){ plant_claim_kernel<k, l, set_><<<1, 1, 0, stream_>>>(T_, key_of_encoding(key), d); });
         auto* h = pin_ctr_.as<uint64_t>(0);
         check(cudaMemcpyAsync(h, d, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
         sync();

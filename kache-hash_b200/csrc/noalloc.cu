@@ -75,10 +75,10 @@ __global__ void noalloc_segments_kernel(const uint64_t* off, const uint64_t n, c
 template <int k, int l, bool set_>
 __global__ void __launch_bounds__(32 * stream_warps) noalloc_count_kernel(const Dev_Table T, const uint8_t* bases, const uint64_t* off, const Scratch s, unsigned long long* counts)
 {
-    constexpr int w = k - l + 1;
-    __shared__ uint64_t ring_all[stream_warps][64];
+    __shared__ uint32_t ring_all[stream_warps][ring_words];
+    __shared__ uint8_t tab[base_table_bytes];
+    fill_base_table(tab);
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint64_t* ring = ring_all[wid];
     if(*s.overflow)
         return;
     Seq_Reduce_Visitor<set_, uint8_t, 0> vis{T, counts, 0, 0, 0, 0};
@@ -88,59 +88,11 @@ __global__ void __launch_bounds__(32 * stream_warps) noalloc_count_kernel(const 
     const uint64_t warps = uint64_t(gridDim.x) * stream_warps;
     for(uint64_t g = uint64_t(blockIdx.x) * stream_warps + wid; g < nsegs; g += warps)
     {
-        const uint64_t packed = s.segs[g];
-        const uint64_t q = packed >> 24, sg = packed & 0xFFFFFF;
+        const uint64_t packed = s.segs[g], q = packed >> 24;
         const uint64_t b0 = off[q], len = off[q + 1] - b0;
-        const uint8_t* seq = bases + b0;
-        const uint64_t npos = len - k + 1;
-        const uint64_t p0 = sg * seg_positions;
-        const uint64_t p1 = min(npos, p0 + seg_positions);
-        const uint32_t rows = static_cast<uint32_t>((p1 - p0 + 31) / 32);
-        const uint8_t* sp = seq + p0 + lane;
-        const int32_t rem = static_cast<int32_t>(min(len - p0, uint64_t(1) << 30)) - static_cast<int32_t>(lane);
-
-        Row r0 = load_row(sp, rem, 0, lane);
-        Row r1 = load_row(sp, rem, 32, lane);
-        {
-            uint64_t f, rc;
-            window<l>(r0, r1, lane, f, rc);
-            ring[lane] = wang_u64(f < rc ? f : rc);
-        }
-        vis.begin_segment(q);
-        for(uint32_t r = 0; r < rows; ++r)
-        {
-            const Row r2 = load_row(sp, rem, 32 * (r + 2), lane);
-            {
-                uint64_t f, rc;
-                window<l>(r1, r2, lane, f, rc);
-                ring[((r + 1) & 1) * 32 + lane] = wang_u64(f < rc ? f : rc);
-            }
-            __syncwarp();
-            Kmer_Desc d;
-            uint64_t f, rc;
-            window<k>(r0, r1, lane, f, rc);
-            const uint64_t vbits = ((uint64_t(r1.valid) << 32) | r0.valid) >> lane;
-            const uint64_t km = (k == 32 ? 0xFFFFFFFFull : (1ull << k) - 1);
-            d.pos = p0 + 32 * r + lane;
-            d.q = q;
-            d.in = d.pos < p1;
-            d.valid = d.in && (vbits & km) == km;
-            d.key = f < rc ? f : rc;
-            d.fwd = f <= rc;
-            d.c = checksum_of(d.key);
-            uint64_t h = ~0ull;
-            const uint32_t base = (r & 1) * 32 + lane;
-#pragma unroll
-            for(int x = 0; x < w; ++x)
-            {
-                const uint64_t v = ring[(base + x) & 63];
-                h = v < h ? v : h;
-            }
-            d.h = h;
-            vis.visit(d, lane);
-            __syncwarp();
-            r0 = r1, r1 = r2;
-        }
+        const uint64_t p0 = (packed & 0xFFFFFF) * seg_positions;
+        vis.begin_segment(q, 0);
+        describe_segment<k, l>(bases + b0 + p0, static_cast<uint32_t>(min(len - k + 1 - p0, static_cast<uint64_t>(seg_positions))), ring_all[wid], tab, lane, vis);
         vis.end_segment(q, lane);
     }
 }
