@@ -205,42 +205,39 @@ __global__ void __launch_bounds__(256) collect_kernel(const Dev_Table T, const u
     }
 }
 
-// Reductions of the C interface over all keys (capi/Kmer_Table.hpp:203-230): 0 keys with v & m nonzero (all keys
-// in a set), 1 popcount of v & m, 2 sum of v & m; and 3, the histogram of values in [1, max] (counter/
-// Kmer_Set_Counter.cpp:96-119), into `hist`.
-template <bool set_, typename V>
-__global__ void __launch_bounds__(256) reduce_kernel(const Dev_Table T, const uint32_t what, const uint64_t mask, unsigned long long* out, const uint64_t hmax, unsigned long long* hist)
+// The value of slot s of the table, its main slots first and then the overflow table's, if it holds a key.
+template <bool set_>
+__device__ __forceinline__ bool slot_value(const Dev_Table& T, const uint64_t s, unsigned long long& raw)
 {
-    const uint64_t n_main = T.cap * B, total = n_main + T.ov_mask + 1;
+    const uint64_t n_main = T.cap * B;
+    if(s < n_main)
+    {
+        if(*cs_of(T, static_cast<uint32_t>(s / B), s % B) == 0)
+            return false;
+        if constexpr(!set_)
+            raw = T.slots[s * 2 + 1];
+        return true;
+    }
+    const uint64_t i = s - n_main;
+    if(T.ov[4 * i] == 0)
+        return false;
+    raw = T.ov[4 * i + 1];
+    return true;
+}
+
+// Reductions of the C interface over all keys (capi/Kmer_Table.hpp:203-230): 0 keys with v & m nonzero (all keys
+// in a set), 1 popcount of v & m, 2 sum of v & m.
+template <bool set_, typename V>
+__global__ void __launch_bounds__(256) reduce_kernel(const Dev_Table T, const uint32_t what, const uint64_t mask, unsigned long long* out)
+{
+    const uint64_t total = T.cap * B + T.ov_mask + 1;
     unsigned long long acc = 0;
     for(uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < total; s += uint64_t(gridDim.x) * blockDim.x)
     {
-        bool have;
         unsigned long long raw = 0;
-        if(s < n_main)
-        {
-            have = *cs_of(T, static_cast<uint32_t>(s / B), s % B) != 0;
-            if constexpr(!set_)
-                if(have)
-                    raw = T.slots[s * 2 + 1];
-        }
-        else
-        {
-            const uint64_t i = s - n_main;
-            have = T.ov[4 * i] != 0;
-            if(have)
-                raw = T.ov[4 * i + 1];
-        }
-        if(!have)
+        if(!slot_value<set_>(T, s, raw))
             continue;
-        const uint64_t v = static_cast<uint64_t>(static_cast<V>(raw));
-        if(what == 3)
-        {
-            if(v >= 1 && v <= hmax)
-                atomicAdd(hist + v, 1ull);
-            continue;
-        }
-        const uint64_t x = v & mask;
+        const uint64_t x = static_cast<uint64_t>(static_cast<V>(raw)) & mask;
         if(set_)
             acc += 1;
         else if(what == 0)
@@ -255,6 +252,38 @@ __global__ void __launch_bounds__(256) reduce_kernel(const Dev_Table T, const ui
         acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
     if((threadIdx.x & 31) == 0 && acc)
         atomicAdd(out, acc);
+}
+
+// The histogram of the values in [1, hmax] (counter/Kmer_Set_Counter.cpp:96-119), added to hist[0..hmax]. Counts of k-mers
+// crowd on a few values, so a block counts those up to hist_bins in shared memory and adds its bins up at the end; one
+// global atomic per key on those few words took 41.8 ms over 100M keys, against 0.62 with the blocks' bins (reading the 2.1 GB table takes 0.33).
+constexpr uint32_t hist_bins = 8192;    // 32 KB: six blocks per SM.
+
+template <typename V>
+__global__ void __launch_bounds__(256) histogram_kernel(const Dev_Table T, const uint64_t hmax, unsigned long long* hist)
+{
+    __shared__ uint32_t bins[hist_bins];
+    const uint32_t held = static_cast<uint32_t>(min(hmax + 1, static_cast<uint64_t>(hist_bins)));
+    for(uint32_t i = threadIdx.x; i < held; i += blockDim.x)
+        bins[i] = 0;
+    __syncthreads();
+    const uint64_t total = T.cap * B + T.ov_mask + 1;
+    // A block's share of the slots stays below 2^32, so its bins cannot overflow.
+    for(uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < total; s += uint64_t(gridDim.x) * blockDim.x)
+    {
+        unsigned long long raw = 0;
+        if(!slot_value<false>(T, s, raw))
+            continue;
+        const uint64_t v = static_cast<uint64_t>(static_cast<V>(raw));
+        if(v < held)
+            atomicAdd(bins + v, 1u);
+        else if(v <= hmax)
+            atomicAdd(hist + v, 1ull);
+    }
+    __syncthreads();
+    for(uint32_t i = threadIdx.x; i < held; i += blockDim.x)
+        if(i > 0 && bins[i])
+            atomicAdd(hist + i, static_cast<unsigned long long>(bins[i]));
 }
 
 // Placement statistics (include/Streaming_Kmer_Hash_Table.hpp:1108-1120,2729-2752): keys in their primary bucket

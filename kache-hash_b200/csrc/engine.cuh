@@ -571,7 +571,7 @@ class Engine final : public kache_table
         unsigned long long* out = ctr() + 3;
         check(cudaMemsetAsync(out, 0, 8, stream_), "memset");
         U.ov_mask = slots - 1;
-        launch(K_OTHER, [&](){ reduce_kernel<true, uint8_t><<<grid_for(slots / 32 + 1, 8), 256, 0, stream_>>>(U, 0, 0, out, 0, nullptr); });
+        launch(K_OTHER, [&](){ reduce_kernel<true, uint8_t><<<grid_for(slots / 32 + 1, 8), 256, 0, stream_>>>(U, 0, 0, out); });
         check(cudaMemcpyAsync(ctr() + 1, out, 8, cudaMemcpyDeviceToDevice, stream_), "copy");
     }
 
@@ -1611,7 +1611,7 @@ public:
         unsigned long long* out = ctr() + 3;
         check(cudaMemsetAsync(out, 0, 8, stream_), "memset");
         const uint64_t total = T_.cap * B + ov_slots_;
-        launch(K_OTHER, [&](){ reduce_kernel<set_, VT><<<grid_for(total / 32 + 1, 8), 256, 0, stream_>>>(T_, what, mask, out, 0, nullptr); });
+        launch(K_OTHER, [&](){ reduce_kernel<set_, VT><<<grid_for(total / 32 + 1, 8), 256, 0, stream_>>>(T_, what, mask, out); });
         return read_ctr(4)[3];
     }
 
@@ -1621,7 +1621,9 @@ public:
         dout_.ensure((max + 1) * 8);
         check(cudaMemsetAsync(dout_.p, 0, (max + 1) * 8, stream_), "memset");
         const uint64_t total = T_.cap * B + ov_slots_;
-        launch(K_OTHER, [&](){ reduce_kernel<set_, VT><<<grid_for(total / 32 + 1, 8), 256, 0, stream_>>>(T_, 3, 0, ctr() + 3, max, dout_.as<unsigned long long>()); });
+        const unsigned blocks = std::min<unsigned>(grid_for(total / 32 + 1, 8), static_cast<unsigned>(sm_count_) * 6);
+        if constexpr(!set_)
+            launch(K_OTHER, [&](){ histogram_kernel<VT><<<blocks, 256, 0, stream_>>>(T_, max, dout_.as<unsigned long long>()); });
         d2h(h, dout_.p, (max + 1) * 8);
         h[0] = 0;
     }
