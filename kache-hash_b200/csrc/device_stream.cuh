@@ -289,13 +289,13 @@ struct Upsert_Visitor
         }
 
         const unsigned long long key_st = ~d.key;
-        const uint32_t c = checksum_of(d.key);
-        uint32_t j = probe_primary<set_, true, false>(T, active, d.key, d.h).slot;
-        uint32_t r = j < B ? FOUND : NONE, at = active ? bucket_of(d.h, T.cap) : no_bucket;
+        const Probe p = probe_primary<set_, true, false>(T, active, d.key, d.h);
+        uint32_t j = p.slot, r = j < B ? FOUND : NONE, at = active ? bucket_of(d.h, T.cap) : no_bucket;
         uint64_t ov_i = 0;
         const uint32_t need_m = __ballot_sync(all, active && r == NONE);
         if(need_m)
         {
+            const uint32_t c = checksum_of(d.key);
             // The bucket is read again: its checksums would take registers that other warps need.
             if((need_m >> lane) & 1)
                 r = bucket_probe<set_>(T, at, key_st, c, j);
@@ -315,22 +315,24 @@ struct Upsert_Visitor
             }
         }
 
-        Landing L;
-        if(at != no_bucket)
-            L = Landing{set_ ? nullptr : key_word<set_>(T, at, j) + 1, cs_of(T, at, j), nullptr, c};
-        else
-            L = Landing{T.ov + 4 * ov_i + 1, nullptr, T.ov + 4 * ov_i + 2, c};
-        const bool comm = fn.commutes();
+        const bool comm = fn.commutes(), main = at != no_bucket;
+        unsigned long long* const val = main ? key_word<set_>(T, at, j) + 1 : T.ov + 4 * ov_i + 1;
         if(r == INSERTED)
         {
             if constexpr(!set_)
             {
                 if(comm)
-                    fn.apply_init(L.val, d.fwd);
+                    fn.apply_init(val, d.fwd);
                 else
-                    write_val<V>(L.val, fn.initial(d.fwd));
+                    write_val<V>(val, fn.initial(d.fwd)), __threadfence();
             }
-            publish(L, !set_ && !comm);
+            if(main)
+                *reinterpret_cast<volatile uint8_t*>(cs_of(T, at, j)) = static_cast<uint8_t>(checksum_of(d.key));
+            else
+            {
+                *reinterpret_cast<volatile unsigned long long*>(val + 1) = 1ull;
+                atomicAdd(T.ov_count, 1ull);
+            }
         }
         else if(r == OV_FULL)
         {
@@ -343,12 +345,11 @@ struct Upsert_Visitor
         if constexpr(!set_)
             if((r == FOUND || r == FOUND_PENDING) && !fn.is_noop())
             {
-                if(r == FOUND_PENDING && !comm && !await_published(L, T.wait_polls))
+                if(r == FOUND_PENDING && !comm &&
+                   !await_published(Landing{val, main ? cs_of(T, at, j) : nullptr, main ? nullptr : val + 1, 0}, T.wait_polls))
                     atomicOr(T.err, ERR_WAIT);
-                fn.apply(L.val, d.fwd);
+                fn.apply(val, d.fwd);
             }
-        if(r == INSERTED && !L.cs)
-            atomicAdd(T.ov_count, 1ull);
     }
 
     __device__ __forceinline__ void end(const uint32_t lane) { warp_flush(inserted, ins, lane); }

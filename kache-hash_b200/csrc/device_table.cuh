@@ -279,10 +279,11 @@ struct Checksums
     uint4 lo, hi;
 
     __device__ __forceinline__ bool full() const { return (hi.w >> 24) != 0; }  // Keys fill a bucket's slots in order.
-    // The first slot whose checksum is empty, or B.
+    // The first slot whose checksum is empty, or B. (The inexact test can flag a byte above an empty one of its word,
+    // which is a higher slot.)
     __device__ __forceinline__ uint32_t first_empty() const
     {
-        const uint32_t m = candidates32<true>(lo, hi, 0);
+        const uint32_t m = candidates32<false>(lo, hi, 0);
         return m ? __ffs(m) - 1 : B;
     }
 };
@@ -458,18 +459,22 @@ __device__ __forceinline__ void warp_claim(const Dev_Table& T, const unsigned lo
                     r = FOUND_PENDING;
             }
             const uint32_t tried = __popc(__ballot_sync(all, tries) & run);
-            for(uint32_t lost = __ballot_sync(all, tries && r == NONE); lost; lost &= lost - 1)
-            {
-                const uint32_t s = __ffs(lost) - 1;
-                const unsigned long long k_s = __shfl_sync(all, cur, s);
-                const uint32_t slot_s = __shfl_sync(all, slot, s);
-                if(ok && ((run >> s) & 1) && k_s == key_st && (r == NONE || slot_s < got))
+            // Where a swap lost, its run's lanes compare their keys with what it showed: every run at once, lane by lane
+            // from its first.
+            const uint32_t lost = __ballot_sync(all, tries && r == NONE);
+            if(lost)
+                for(uint32_t left_m = run & lost; __any_sync(all, left_m); left_m &= left_m - 1)
                 {
-                    if(r == INSERTED)
-                        *reinterpret_cast<volatile unsigned long long*>(key_word<set_>(T, at, got)) = hole_key;
-                    r = FOUND_PENDING, got = slot_s;
+                    const uint32_t s = left_m ? __ffs(left_m) - 1 : lane;
+                    const unsigned long long k_s = __shfl_sync(all, cur, s);
+                    const uint32_t slot_s = __shfl_sync(all, slot, s);
+                    if(ok && left_m && k_s == key_st && (r == NONE || slot_s < got))
+                    {
+                        if(r == INSERTED)
+                            *reinterpret_cast<volatile unsigned long long*>(key_word<set_>(T, at, got)) = hole_key;
+                        r = FOUND_PENDING, got = slot_s;
+                    }
                 }
-            }
             if(ok)
                 j = r == NONE ? j + tried : got;
             else if(in)
