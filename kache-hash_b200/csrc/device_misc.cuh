@@ -418,9 +418,9 @@ static __global__ void __launch_bounds__(1024) stage_small_kernel(const uint64_t
 
 // Lists the segments, one thread per segment: its sequence by binary search in seg_off[0..n] (exclusive sums of
 // segments per sequence), so that long sequences' many segments are listed in parallel. Sequence q's bases are at offset
-// off[q], or with `addr` at the address addr[q].
-static __global__ void segs_kernel(const uint64_t* seg_off, const uint64_t* pos_off, const uint64_t* off, const uint64_t* addr, const uint64_t n, const uint64_t nsegs,
-                                   const uint32_t seg_len, Segment* segs)
+// off[q], or with `addr` at the address addr[q], where it is of batch batch_of[q].
+static __global__ void segs_kernel(const uint64_t* seg_off, const uint64_t* pos_off, const uint64_t* off, const uint64_t* addr, const uint32_t* batch_of, const uint64_t n,
+                                   const uint64_t nsegs, const uint32_t seg_len, Segment* segs)
 {
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
     for(uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nsegs; i += stride)
@@ -435,15 +435,15 @@ static __global__ void segs_kernel(const uint64_t* seg_off, const uint64_t* pos_
                 hi = mid;
         }
         const uint64_t p0 = (i - seg_off[lo]) * seg_len, first = pos_off[lo] + p0;
-        segs[i] = Segment{(addr ? addr[lo] : off[lo]) + p0, first, lo, static_cast<uint32_t>(min(pos_off[lo + 1] - first, static_cast<uint64_t>(seg_len))), 0};
+        segs[i] = Segment{(addr ? addr[lo] : off[lo]) + p0, first, lo, static_cast<uint32_t>(min(pos_off[lo + 1] - first, static_cast<uint64_t>(seg_len))), batch_of ? batch_of[lo] : 0};
     }
 }
 
 // Several device batches run as one call. desc holds 8 words per batch -- bases, offsets, sequences, first merged
 // sequence, out0, out1, out2, 0 -- in batch order. For merged sequence q: its batch, its length (the merged offsets are
-// the lengths' sums) and the device address of its first base.
+// the lengths' sums) and the device address of its first base; with `zero`, its word of the batch's out0 is zeroed.
 static __global__ void batches_list_kernel(const uint64_t* desc, const uint64_t count, const uint64_t N, uint64_t* lens,
-                                           uint64_t* addr, uint32_t* batch_of)
+                                           uint64_t* addr, uint32_t* batch_of, const bool zero)
 {
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
     for(uint64_t q = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < N; q += stride)
@@ -462,6 +462,8 @@ static __global__ void batches_list_kernel(const uint64_t* desc, const uint64_t 
         lens[q] = off[j + 1] - a;
         addr[q] = desc[8 * lo] + a;
         batch_of[q] = static_cast<uint32_t>(lo);
+        if(zero)
+            reinterpret_cast<uint64_t*>(desc[8 * lo + 4])[j] = 0;
     }
 }
 
@@ -471,69 +473,6 @@ static __global__ void batches_pos_kernel(const uint64_t* desc, const uint64_t c
     const uint64_t b = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if(b < count)
         pos_base[b] = pos_off[desc[8 * b + 3]];
-}
-
-// Per-batch sums of per-sequence counts: each thread adds a run of consecutive sequences, flushing at batch changes.
-static __global__ void batches_sum_kernel(const unsigned long long* per_seq, const uint32_t* batch_of, const uint64_t N,
-                                          unsigned long long* per_batch)
-{
-    const uint64_t threads = uint64_t(gridDim.x) * blockDim.x, t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const uint64_t per = (N + threads - 1) / threads, q0 = min(N, t * per), q1 = min(N, q0 + per);
-    unsigned long long acc = 0;
-    uint32_t cur = 0;
-    for(uint64_t q = q0; q < q1; ++q)
-    {
-        const uint32_t b = batch_of[q];
-        if(b != cur && acc)
-            atomicAdd(per_batch + cur, acc), acc = 0;
-        cur = b, acc += per_seq[q];
-    }
-    if(acc)
-        atomicAdd(per_batch + cur, acc);
-}
-
-// Per-sequence results of the merged batch copied to each batch's own array (desc word 4).
-static __global__ void batches_scatter_kernel(const uint64_t* desc, const unsigned long long* per_seq, const uint32_t* batch_of,
-                                              const uint64_t N)
-{
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for(uint64_t q = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < N; q += stride)
-    {
-        const uint64_t b = batch_of[q];
-        reinterpret_cast<unsigned long long*>(desc[8 * b + 4])[q - desc[8 * b + 3]] = per_seq[q];
-    }
-}
-
-// Per-sequence positions found (found flag 1) of a lookup of several batches, read back from each batch's found array
-// (desc word 4): a warp per sequence, 4-byte words where aligned, bytes equal to 1 counted by a zero-byte test of the
-// word XOR 0x01010101.
-static __global__ void batches_hits_kernel(const uint64_t* desc, const uint32_t* batch_of, const uint64_t* pos_off,
-                                           const uint64_t* pos_base, const uint64_t N, unsigned long long* per_seq)
-{
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x / 32);
-    for(uint64_t q = uint64_t(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5); q < N; q += warps)
-    {
-        const uint32_t b = batch_of[q];
-        const uint8_t* f = reinterpret_cast<const uint8_t*>(desc[8 * uint64_t(b) + 4]) + (pos_off[q] - pos_base[b]);
-        const uint64_t m = pos_off[q + 1] - pos_off[q];
-        const uint64_t lead = (4 - (reinterpret_cast<uintptr_t>(f) & 3)) & 3, head = m < lead ? m : lead;
-        const uint64_t nw = (m - head) / 4, tail = head + 4 * nw;
-        const uint32_t* w = reinterpret_cast<const uint32_t*>(f + head);
-        unsigned long long c = 0;
-        if(lane < head)
-            c += f[lane] == 1;
-#pragma unroll 4
-        for(uint64_t i = lane; i < nw; i += 32)
-            c += __popc(zero_bytes(w[i] ^ 0x01010101u));
-        if(tail + lane < m)
-            c += f[tail + lane] == 1;
-#pragma unroll
-        for(int o = 16; o > 0; o >>= 1)
-            c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-        if(lane == 0)
-            per_seq[q] = c;
-    }
 }
 
 }

@@ -39,7 +39,14 @@ struct alignas(16) Segment
     uint64_t pos;       // Its first position, counted over the batch's sequences.
     uint64_t q;         // Its sequence.
     uint32_t npos;      // Its positions.
-    uint32_t unused;
+    uint32_t batch;     // Its batch, of several run as one.
+};
+
+// What visitors get of a segment.
+struct Seg_Of
+{
+    uint64_t q, pos;
+    uint32_t batch;
 };
 
 // A batch on the device: its segments in sequence order. Several batches run as one have no bases in common (null): their
@@ -201,13 +208,14 @@ __global__ void __launch_bounds__(32 * stream_warps, Visitor::min_blocks) stream
     {
         const auto word = [&](const int i) { return __shfl_sync(0xFFFFFFFFu, entry, i); };
         const auto wide = [&](const int i) { return uint64_t(word(i + 1)) << 32 | word(i); };
-        const uint64_t base = wide(0), pos = wide(2), q = wide(4);
+        const uint64_t base = wide(0);
+        const Seg_Of s{wide(4), wide(2), word(7)};
         const uint32_t npos = word(6);
         g += warps;
         entry = ask(g);
-        vis.begin_segment(q, pos);
+        vis.begin_segment(s);
         describe_segment<k, l>(batch.bases + base, npos, ring_all[wid], tab, lane, vis);
-        vis.end_segment(q, lane);
+        vis.end_segment(s, lane);
     }
     vis.end(lane);
 }
@@ -222,30 +230,26 @@ __device__ __forceinline__ void warp_flush(unsigned long long* ctr, const unsign
 }
 
 // Finds a row's k-mers, for visitors that insert nothing: `hit` where the key is present, its value then in `val` (with
-// val_), its value word (the key word of a set) in `at`. What few lanes need, candidates past the second and what lies
-// beyond a full bucket, is behind a branch of the whole warp.
+// val_), its place in (at, slot) (value_word). What few lanes need, candidates past the second and what lies beyond a full
+// bucket, is behind a branch of the whole warp.
 template <bool set_, bool val_>
 struct Found
 {
     bool hit;
-    unsigned long long* at;
+    uint32_t at;
+    uint64_t slot;
     unsigned long long val;
 
     __device__ __forceinline__ Found(const Dev_Table& T, const Kmer_Desc& d)
     {
         const Probe p = probe_primary<set_, false, val_>(T, d.valid, d.key, d.h);
-        const uint32_t b = bucket_of(d.h, T.cap);
+        at = bucket_of(d.h, T.cap), slot = p.slot, val = p.val;
         hit = p.slot < B;
-        at = key_word<set_>(T, b, p.slot) + (set_ ? 0 : 1);
-        val = p.val;
         const bool on = !hit && (p.rest != 0 || p.full);
         if(__any_sync(0xFFFFFFFFu, on))
         {
             if(on)
-            {
-                at = find_on<set_, false>(T, b, p.rest, p.full, ~d.key, d.h, checksum_of(d.key), val);
-                hit = at != nullptr;
-            }
+                hit = find_on<set_, false, val_>(T, at, slot, p.rest, p.full, ~d.key, d.h, val);
             __syncwarp();
         }
     }
@@ -264,18 +268,19 @@ struct Upsert_Visitor
     unsigned int* retry_out;
     const unsigned int* retry_in;
     unsigned int* retried;      // Set to 1 if any bit of retry_out was set.
-    unsigned long long* per_seq;    // If set, keys inserted per sequence are added at per_seq[q].
+    unsigned long long* per;        // If set, the keys inserted are added there per sequence, or
+    bool by_batch;                  // per batch.
     unsigned long long ins = 0;     // By this warp, before its current segment.
     uint32_t seg_ins = 0;           // In the current segment,
     uint64_t seg_pos = 0;           // whose first position this is.
 
     __device__ __forceinline__ void begin() {}
-    __device__ __forceinline__ void begin_segment(uint64_t, const uint64_t pos) { seg_ins = 0, seg_pos = pos; }
-    __device__ __forceinline__ void end_segment(const uint64_t q, const uint32_t lane)
+    __device__ __forceinline__ void begin_segment(const Seg_Of& s) { seg_ins = 0, seg_pos = s.pos; }
+    __device__ __forceinline__ void end_segment(const Seg_Of& s, const uint32_t lane)
     {
         ins += seg_ins;
-        if(per_seq && lane == 0 && seg_ins)
-            atomicAdd(per_seq + q, static_cast<unsigned long long>(seg_ins));
+        if(per && lane == 0 && seg_ins)
+            atomicAdd(per + (by_batch ? s.batch : s.q), static_cast<unsigned long long>(seg_ins));
     }
 
     __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t lane)
@@ -364,24 +369,24 @@ struct Update_Visitor
     Dev_Table T;
     Fn fn;
     unsigned long long* present;
-    unsigned long long* per_seq;    // If set, k-mers present per sequence are added at per_seq[q].
+    unsigned long long* per_batch;  // If set, the k-mers present are added there per batch.
     unsigned long long cnt = 0;     // By this warp, before its current segment.
     uint32_t seg_cnt = 0;           // In the current segment.
 
     __device__ __forceinline__ void begin() {}
-    __device__ __forceinline__ void begin_segment(uint64_t, uint64_t) { seg_cnt = 0; }
-    __device__ __forceinline__ void end_segment(const uint64_t q, const uint32_t lane)
+    __device__ __forceinline__ void begin_segment(const Seg_Of&) { seg_cnt = 0; }
+    __device__ __forceinline__ void end_segment(const Seg_Of& s, const uint32_t lane)
     {
         cnt += seg_cnt;
-        if(per_seq && lane == 0 && seg_cnt)
-            atomicAdd(per_seq + q, static_cast<unsigned long long>(seg_cnt));
+        if(per_batch && lane == 0 && seg_cnt)
+            atomicAdd(per_batch + s.batch, static_cast<unsigned long long>(seg_cnt));
     }
 
     __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t)
     {
         const Found<false, false> f(T, d);
         if(f.hit)
-            fn.apply(f.at, d.fwd);
+            fn.apply(value_word<false>(T, f.at, f.slot), d.fwd);
         seg_cnt += __popc(__ballot_sync(0xFFFFFFFFu, f.hit));
     }
 
@@ -401,15 +406,17 @@ struct Lookup_Visitor
     uint64_t obase = 0;     // The current segment's first position in them.
 
     __device__ __forceinline__ void begin() {}
-    __device__ __forceinline__ void begin_segment(uint64_t, const uint64_t pos) { obase = pos; }
-    __device__ __forceinline__ void end_segment(uint64_t, uint32_t) {}
+    __device__ __forceinline__ void begin_segment(const Seg_Of& s) { obase = s.pos; }
+    __device__ __forceinline__ void end_segment(const Seg_Of&, uint32_t) {}
     __device__ __forceinline__ void end(uint32_t) {}
 
-    __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t)
+    __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t) { look(d); }
+    // Looks the k-mer up and writes its outputs; whether it is present.
+    __device__ __forceinline__ bool look(const Kmer_Desc& d)
     {
         const Found<set_, !set_> f(T, d);
         if(!d.in)
-            return;
+            return false;
         const uint64_t o = obase + d.pos;
         found[o] = d.valid ? (f.hit ? 1 : 0) : 2;
         if constexpr(!set_)
@@ -417,26 +424,38 @@ struct Lookup_Visitor
                 values[o] = f.hit ? value_of<V>(f.val) : V(0);
         if(fwd)
             fwd[o] = d.valid && d.fwd;
+        return f.hit;
     }
 };
 
-// Lookups of several batches run as one: each sequence's outputs go to its own batch's arrays, at its positions
-// within that batch.
+// Lookups of several batches run as one: each segment's outputs go to its own batch's arrays, at its positions within
+// that batch, and the positions found are added at per_batch.
 template <bool set_, typename V>
 struct Lookup_Batches_Visitor : Lookup_Visitor<set_, V>
 {
-    static constexpr int min_blocks = 6;
-    const uint32_t* batch_of;   // Sequence -> batch.
     const uint64_t* outs;       // Per batch, 8 words: found, values, fwd at words 4-6 (device addresses, or 0).
     const uint64_t* pos_base;   // Per batch: the merged position of its first k-mer.
+    unsigned long long* per_batch;
+    uint32_t hits = 0;          // In the current segment.
 
-    __device__ __forceinline__ void begin_segment(const uint64_t q, const uint64_t pos)
+    __device__ __forceinline__ void begin_segment(const Seg_Of& s)
     {
-        const uint32_t b = batch_of[q];
-        this->found = reinterpret_cast<uint8_t*>(outs[8 * uint64_t(b) + 4]);
-        this->values = reinterpret_cast<V*>(outs[8 * uint64_t(b) + 5]);
-        this->fwd = reinterpret_cast<uint8_t*>(outs[8 * uint64_t(b) + 6]);
-        this->obase = pos - pos_base[b];
+        const uint64_t* o = outs + 8 * uint64_t(s.batch);
+        this->found = reinterpret_cast<uint8_t*>(o[4]);
+        this->values = reinterpret_cast<V*>(o[5]);
+        this->fwd = reinterpret_cast<uint8_t*>(o[6]);
+        this->obase = s.pos - pos_base[s.batch];
+        hits = 0;
+    }
+    __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t)
+    {
+        const bool hit = this->look(d);
+        hits += __popc(__ballot_sync(0xFFFFFFFFu, hit));
+    }
+    __device__ __forceinline__ void end_segment(const Seg_Of& s, const uint32_t lane)
+    {
+        if(lane == 0 && hits)
+            atomicAdd(per_batch + s.batch, static_cast<unsigned long long>(hits));
     }
 };
 
@@ -449,11 +468,10 @@ struct Seq_Reduce_Visitor
     Dev_Table T;
     unsigned long long* out;
     V m_fwd, m_rev;
-    unsigned long long acc;
-    unsigned long long total;
+    unsigned long long acc = 0;
 
-    __device__ __forceinline__ void begin() { total = 0; }
-    __device__ __forceinline__ void begin_segment(uint64_t, uint64_t) { acc = 0; }
+    __device__ __forceinline__ void begin() {}
+    __device__ __forceinline__ void begin_segment(const Seg_Of&) { acc = 0; }
     __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t)
     {
         const Found<set_, !set_ && mode_ != 0> f(T, d);
@@ -466,17 +484,40 @@ struct Seq_Reduce_Visitor
         else
             acc += static_cast<unsigned long long>(value_of<V>(f.val));
     }
-    __device__ __forceinline__ void end_segment(const uint64_t q, const uint32_t lane)
+    __device__ __forceinline__ unsigned long long seg_total() const
     {
         unsigned long long a = acc;
 #pragma unroll
         for(int o = 16; o > 0; o >>= 1)
             a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+        return a;
+    }
+    __device__ __forceinline__ void end_segment(const Seg_Of& s, const uint32_t lane)
+    {
+        const unsigned long long a = seg_total();
         if(lane == 0 && a)
-            atomicAdd(out + q, a);
-        total += a;
+            atomicAdd(out + s.q, a);
     }
     __device__ __forceinline__ void end(uint32_t) {}
+};
+
+// Counts of several batches run as one: per sequence in its own batch's array, and per batch at per_batch.
+template <bool set_, typename V>
+struct Count_Batches_Visitor : Seq_Reduce_Visitor<set_, V, 0>
+{
+    const uint64_t* outs;       // Per batch, 8 words: its first merged sequence at word 3, its counts' address at word 4.
+    unsigned long long* per_batch;
+
+    __device__ __forceinline__ void end_segment(const Seg_Of& s, const uint32_t lane)
+    {
+        const unsigned long long a = this->seg_total();
+        if(lane == 0 && a)
+        {
+            const uint64_t* o = outs + 8 * uint64_t(s.batch);
+            atomicAdd(reinterpret_cast<unsigned long long*>(o[4]) + (s.q - o[3]), a);
+            atomicAdd(per_batch + s.batch, a);
+        }
+    }
 };
 
 // The descriptions that callers can see, for checking the describer: the key's 2-bit encoding, and the reference's
@@ -493,8 +534,8 @@ struct Describe_Visitor
     uint64_t obase = 0;
 
     __device__ __forceinline__ void begin() {}
-    __device__ __forceinline__ void begin_segment(uint64_t, const uint64_t pos) { obase = pos; }
-    __device__ __forceinline__ void end_segment(uint64_t, uint32_t) {}
+    __device__ __forceinline__ void begin_segment(const Seg_Of& s) { obase = s.pos; }
+    __device__ __forceinline__ void end_segment(const Seg_Of&, uint32_t) {}
     __device__ __forceinline__ void end(uint32_t) {}
     __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t)
     {

@@ -306,43 +306,42 @@ template <bool set_>
 __device__ __forceinline__ uint32_t bucket_probe(const Dev_Table& T, const uint32_t b, const unsigned long long key_st, const uint32_t c, uint32_t& j)
 {
     const Checksums s = bucket_cs<true>(T, b);
-    for(uint32_t cand = candidates32<true>(s.lo, s.hi, c); cand; cand &= cand - 1)
-    {
-        j = __ffs(cand) - 1;
-        if(ld_cg(key_word<set_>(T, b, j)) == key_st)
-            return FOUND;
-    }
+    uint32_t r = NONE;
     j = s.first_empty();
-    return NONE;
+    for(uint32_t cand = candidates32<true>(s.lo, s.hi, c); cand != 0 && r == NONE; cand &= cand - 1)
+        if(ld_cg(key_word<set_>(T, b, __ffs(cand) - 1)) == key_st)
+            r = FOUND, j = __ffs(cand) - 1;
+    return r;
 }
 
 // Tries the bucket b for the key, one lane by itself: its published candidates, then the claim scan. Returns FOUND,
-// FOUND_PENDING or INSERTED with the slot at `j`, or NONE if the bucket is full without the key.
+// FOUND_PENDING (claimed by another lane, published or not) or INSERTED with the slot at `j`, or NONE if the bucket is full
+// without the key.
 template <bool set_>
 __device__ __forceinline__ uint32_t bucket_upsert(const Dev_Table& T, const uint32_t b, const unsigned long long key_st, const uint32_t c, uint32_t& j)
 {
-    if(bucket_probe<set_>(T, b, key_st, c, j) == FOUND)
-        return FOUND;
-
+    uint32_t r = bucket_probe<set_>(T, b, key_st, c, j);
     // The claim scan: a compare-and-swap straight away (a slot with an empty checksum is most likely unclaimed), whose
     // result, if it fails, is the racing claimer's key.
-    for(; j < B; ++j)
+    while(r == NONE && j < B)
     {
         const unsigned long long cur = atomicCAS(key_word<set_>(T, b, j), 0ull, key_st);
         if(cur == 0)
-            return INSERTED;
-        if(cur == key_st)
-            return ld_volatile_u8(cs_of(T, b, j)) != 0 ? FOUND : FOUND_PENDING;
+            r = INSERTED;
+        else if(cur == key_st)
+            r = FOUND_PENDING;
+        else
+            ++j;
     }
-
-    return NONE;
+    return r;
 }
 
-// Tries the overflow table. Returns FOUND, FOUND_PENDING or INSERTED with the slot index at `i_out`, or OV_FULL.
+// Tries the overflow table. Returns FOUND_PENDING or INSERTED with the slot index at `i_out`, or OV_FULL.
 __device__ __forceinline__ uint32_t overflow_upsert(const Dev_Table& T, const unsigned long long key_st, uint64_t& i_out)
 {
     uint64_t i = ov_hash(key_st) & T.ov_mask;
-    for(uint32_t t = 0; t < T.ov_probe; ++t, i = (i + 1) & T.ov_mask)
+    uint32_t r = OV_FULL;
+    for(uint32_t t = 0; r == OV_FULL && t < T.ov_probe; ++t, i = (i + 1) & T.ov_mask)
     {
         unsigned long long* kw = T.ov + 4 * i;
         unsigned long long cur = ld_cg(kw);
@@ -350,12 +349,12 @@ __device__ __forceinline__ uint32_t overflow_upsert(const Dev_Table& T, const un
         {
             cur = atomicCAS(kw, 0ull, key_st);
             if(cur == 0)
-                return i_out = i, INSERTED;
+                r = INSERTED, i_out = i;
         }
         if(cur == key_st)
-            return i_out = i, (ld_cg(kw + 2) != 0 ? FOUND : FOUND_PENDING);
+            r = FOUND_PENDING, i_out = i;
     }
-    return OV_FULL;
+    return r;
 }
 
 // Where an upsert chain ended: a value word and the flag that publishes it (a checksum byte, or an overflow slot's
@@ -524,17 +523,15 @@ __device__ __forceinline__ void publish(const Landing& L, const bool fence)
 // Waits, boundedly (`polls` polls), for a racing insert of the same key to publish. Returns false if the wait ran out.
 __device__ __forceinline__ bool await_published(const Landing& L, const uint32_t polls)
 {
-    for(uint32_t t = 0; t < polls; ++t)
+    bool done = false;
+    for(uint32_t t = 0; !done && t < polls; ++t)
     {
-        if(L.cs ? ld_volatile_u8(L.cs) != 0 : *reinterpret_cast<const volatile unsigned long long*>(L.ready) != 0)
-        {
-            __threadfence();
-            return true;
-        }
-        if(t > 64)
+        done = L.cs ? ld_volatile_u8(L.cs) != 0 : *reinterpret_cast<const volatile unsigned long long*>(L.ready) != 0;
+        if(!done && t > 64)
             __nanosleep(64);
     }
-    return false;
+    __threadfence();
+    return done;
 }
 
 // The key and value of a map's slot at kw (16-byte aligned), in one load.
@@ -557,67 +554,82 @@ __device__ __forceinline__ bool slot_is(const unsigned long long* kw, const unsi
     return k == key_st;
 }
 
-// Looks for the key, which the first probe of its primary bucket b did not find, among the candidates `cand` left there
-// and then, if b is full, past it: absent unless b's spill filter marks the minimizer; else the secondary buckets; then
-// the overflow table iff both are full (include/Streaming_Kmer_Hash_Table.hpp:2548-2574). Returns the value word (the
-// key word of a set), or null if absent; a map's value also goes to `val`.
-template <bool set_, bool cg_>
-__device__ __forceinline__ unsigned long long* find_on(const Dev_Table& T, const uint32_t b, uint32_t cand, const bool full, const unsigned long long key_st,
-                                                       const uint32_t h, const uint32_t c, unsigned long long& val)
+// Looks for the key, which the first probe of its primary bucket did not find, among the candidates `cand` left there and
+// then, if that bucket is full, past it: absent unless its spill filter marks the minimizer; else the secondary buckets;
+// then the overflow table iff both are full (include/Streaming_Kmer_Hash_Table.hpp:2548-2574). On entry `at` is the primary
+// bucket; if the key is found, its slot is `slot` of bucket `at`, or with at = no_bucket of the overflow table, and with
+// val_ a map's value goes to `val`. (This and the other chains here leave their loops in one place each: with returns out
+// of nested loops, lanes of a warp went on apart past the end of the chain, and the votes behind it missed them.)
+template <bool set_, bool cg_, bool val_>
+__device__ __forceinline__ bool find_on(const Dev_Table& T, uint32_t& at, uint64_t& slot, uint32_t cand, const bool full, const unsigned long long key_st,
+                                        const uint32_t h, unsigned long long& val)
 {
-    bool both_full = full;
-    for(int t = 0; ; ++t)
+    const uint32_t c = checksum_of(~key_st);
+    bool hit = false, both_full = true, on;
+    uint32_t t = 0;     // 0: the primary bucket; 1 and 2: the secondary ones.
+    do
     {
-        // t = 0: the primary bucket; 1 and 2: the secondary ones.
-        const uint32_t at = t == 0 ? b : t == 1 ? second_bucket(h, T.cap) : third_bucket(h, T.cap);
-        if(t > 0)
+        while(cand != 0 && !hit)
         {
+            slot = __ffs(cand) - 1;
+            cand &= cand - 1;
+            const unsigned long long* kw = key_word<set_>(T, at, static_cast<uint32_t>(slot));
+            if constexpr(val_ && !set_)
+                hit = slot_is<set_, cg_>(kw, key_st, val);
+            else
+                hit = (cg_ ? ld_cg(kw) : *kw) == key_st;
+        }
+        on = !hit && full && t < 2;
+        if(on && t == 0)
+        {
+            const uint32_t fp = filter_pos(h);
+            const uint32_t* sw = T.spill + uint64_t(at) * 8 + (fp >> 5);
+            on = ((cg_ ? __ldcg(sw) : *sw) >> (fp & 31)) & 1;
+        }
+        if(on)
+        {
+            at = ++t == 1 ? second_bucket(h, T.cap) : third_bucket(h, T.cap);
             const Checksums s = bucket_cs<cg_>(T, at);
             cand = candidates32<false>(s.lo, s.hi, c);
             both_full = both_full && s.full();
         }
-        for(; cand; cand &= cand - 1)
-        {
-            unsigned long long* kw = key_word<set_>(T, at, __ffs(cand) - 1);
-            if(slot_is<set_, cg_>(kw, key_st, val))
-                return set_ ? kw : kw + 1;
-        }
-        if(t == 0)
-        {
-            if(!full)
-                return nullptr;
-            const uint32_t fp = filter_pos(h);
-            const uint32_t* sw = T.spill + uint64_t(b) * 8 + (fp >> 5);
-            if(!(((cg_ ? __ldcg(sw) : *sw) >> (fp & 31)) & 1))
-                return nullptr;
-        }
-        if(t == 2)
-            break;
-    }
-    if(!both_full)
-        return nullptr;
-
-    uint64_t i = ov_hash(key_st) & T.ov_mask;
-    for(uint32_t t = 0; t < T.ov_probe; ++t, i = (i + 1) & T.ov_mask)
+    } while(on);
+    on = !hit && t == 2 && both_full;
+    if(on)
     {
-        unsigned long long* kw = T.ov + 4 * i;
-        const ulonglong2 s = cg_ ? __ldcg(reinterpret_cast<const ulonglong2*>(kw)) : *reinterpret_cast<const ulonglong2*>(kw);
-        if(s.x == key_st)
-            return val = s.y, kw + 1;
-        if(s.x == 0)
-            return nullptr;
+        at = no_bucket;
+        slot = ov_hash(key_st) & T.ov_mask;
+        for(uint32_t n = 0; on && n < T.ov_probe; ++n)
+        {
+            unsigned long long k, v;
+            load_slot<cg_>(T.ov + 4 * slot, k, v);
+            hit = k == key_st;
+            on = !hit && k != 0;
+            if constexpr(val_)
+                val = v;
+            slot = on ? (slot + 1) & T.ov_mask : slot;
+        }
     }
-    return nullptr;
+    return hit;
+}
+
+// The value word (the key word of a set) of slot j of bucket `at`, or with at = no_bucket of the overflow table.
+template <bool set_>
+__device__ __forceinline__ unsigned long long* value_word(const Dev_Table& T, const uint32_t at, const uint64_t j)
+{
+    return at == no_bucket ? T.ov + 4 * j + 1 : key_word<set_>(T, at, static_cast<uint32_t>(j)) + (set_ ? 0 : 1);
 }
 
 // Finds a key, one lane by itself: its value word (the key word of a set), or null.
 template <bool set_, bool cg_>
 __device__ __forceinline__ unsigned long long* find_chain(const Dev_Table& T, const uint64_t key, const uint32_t h, const uint32_t c)
 {
-    const uint32_t b = bucket_of(h, T.cap);
-    const Checksums s = bucket_cs<cg_>(T, b);
+    uint32_t at = bucket_of(h, T.cap);
+    uint64_t j = 0;
+    const Checksums s = bucket_cs<cg_>(T, at);
     unsigned long long val;
-    return find_on<set_, cg_>(T, b, candidates32<false>(s.lo, s.hi, c), s.full(), ~key, h, c, val);
+    const bool hit = find_on<set_, cg_, false>(T, at, j, candidates32<false>(s.lo, s.hi, c), s.full(), ~key, h, val);
+    return hit ? value_word<set_>(T, at, j) : nullptr;
 }
 
 // The first probe of a lane's k-mer, in its primary bucket.

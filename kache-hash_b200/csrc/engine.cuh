@@ -782,7 +782,7 @@ class Engine final : public kache_table
 
     // stage_dev for a batch of at most small_stage_max sequences: one block counts, fits the segment length and sums, one
     // kernel lists.
-    Batch_Info stage_dev_small(const uint8_t* bases, const uint64_t* off, const uint64_t n, const uint64_t* addr)
+    Batch_Info stage_dev_small(const uint8_t* bases, const uint64_t* off, const uint64_t n, const uint64_t* addr, const uint32_t* batch_of)
     {
         dtmp_.ensure(2 * (n + 1) * 8);
         uint64_t* pos_off = dtmp_.as<uint64_t>();
@@ -792,16 +792,16 @@ class Engine final : public kache_table
         launch(K_OTHER, [&](){ stage_small_kernel<<<1, 1024, 0, stream_>>>(off, n, k, static_cast<uint32_t>(sm_count_), pos_off, seg_off, out); });
         check(cudaMemcpyAsync(h, out, 24, cudaMemcpyDeviceToHost, stream_), "D2H");
         sync();
-        return list_dev(bases, off, addr, n, pos_off, seg_off, h[0], h[1], static_cast<uint32_t>(h[2]));
+        return list_dev(bases, off, addr, batch_of, n, pos_off, seg_off, h[0], h[1], static_cast<uint32_t>(h[2]));
     }
 
     // Lists the segments of a batch whose positions and segments are counted.
-    Batch_Info list_dev(const uint8_t* bases, const uint64_t* off, const uint64_t* addr, const uint64_t n, const uint64_t* pos_off, const uint64_t* seg_off,
-                        const uint64_t total_pos, const uint64_t nsegs, const uint32_t seg_len)
+    Batch_Info list_dev(const uint8_t* bases, const uint64_t* off, const uint64_t* addr, const uint32_t* batch_of, const uint64_t n, const uint64_t* pos_off,
+                        const uint64_t* seg_off, const uint64_t total_pos, const uint64_t nsegs, const uint32_t seg_len)
     {
         dbatch_.ensure((nsegs + 1) * sizeof(Segment));
         if(nsegs > 0)
-            launch(K_OTHER, [&](){ segs_kernel<<<grid_for((nsegs + 31) / 32, 8), 256, 0, stream_>>>(seg_off, pos_off, off, addr, n, nsegs, seg_len, dbatch_.as<Segment>()); });
+            launch(K_OTHER, [&](){ segs_kernel<<<grid_for((nsegs + 31) / 32, 8), 256, 0, stream_>>>(seg_off, pos_off, off, addr, batch_of, n, nsegs, seg_len, dbatch_.as<Segment>()); });
         Batch_Info bi;
         bi.b = Dev_Batch{bases, dbatch_.as<Segment>()};
         bi.n = n, bi.nsegs = nsegs, bi.total_pos = total_pos;
@@ -810,11 +810,12 @@ class Engine final : public kache_table
     }
 
     // Prepares a batch already in device memory: positions and segments computed on the device. With `addr`, sequence q's
-    // bases are at the device address addr[q] and off only lays the lengths end to end.
-    Batch_Info stage_dev(const uint8_t* bases, const uint64_t* off, const uint64_t n, const uint64_t* addr = nullptr)
+    // bases are at the device address addr[q], of batch batch_of[q], and off only lays the lengths end to end.
+    Batch_Info stage_dev(const uint8_t* bases, const uint64_t* off, const uint64_t n, const uint64_t* addr = nullptr,
+                         const uint32_t* batch_of = nullptr)
     {
         if(n > 0 && n <= small_stage_max)
-            return stage_dev_small(bases, off, n, addr);
+            return stage_dev_small(bases, off, n, addr, batch_of);
         const size_t o_npos = 0, o_nseg = o_npos + (n + 1) * 8, o_pos = o_nseg + (n + 1) * 8, o_sego = o_pos + (n + 1) * 8;
         const size_t head = o_sego + (n + 1) * 8;
         dtmp_.ensure(head);
@@ -849,7 +850,7 @@ class Engine final : public kache_table
                 break;
             seg_len *= 8;   // A sequence has more segments than a list entry indexes.
         }
-        return list_dev(bases, off, addr, n, pos_off, seg_off, h[0], h[1], seg_len);
+        return list_dev(bases, off, addr, batch_of, n, pos_off, seg_off, h[0], h[1], seg_len);
     }
 
     // Runs the visitor over segments [sb, se) of a batch, a warp per segment (device_stream.cuh).
@@ -996,7 +997,7 @@ class Engine final : public kache_table
     }
 
     // Upserts a staged batch with the value functor `fn`, chunk by chunk (see the top of this file).
-    template <typename Fn> uint64_t run_upsert(const uint32_t user, const Batch_Info& bi, const Fn& fn, unsigned long long* per_seq = nullptr)
+    template <typename Fn> uint64_t run_upsert(const uint32_t user, const Batch_Info& bi, const Fn& fn, unsigned long long* per = nullptr, const bool by_batch = false)
     {
         const uint64_t nsegs = bi.nsegs;
         const double pos_per_seg = nsegs ? static_cast<double>(bi.total_pos) / nsegs : 1.0;
@@ -1035,7 +1036,7 @@ class Engine final : public kache_table
 
             check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
             check(cudaMemsetAsync(retried, 0, 4, stream_), "memset");
-            Upsert_Visitor<set_, VT, Fn> vis{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per_seq};
+            Upsert_Visitor<set_, VT, Fn> vis{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per, by_batch};
             stream_launch(K_UPSERT, bi, sb, se, vis);
             const unsigned long long* c = read_ctr(3);
             uint64_t ins = c[0];
@@ -1046,7 +1047,7 @@ class Engine final : public kache_table
                 check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
                 check(cudaMemsetAsync(retried, 0, 4, stream_), "memset");
                 check(cudaMemsetAsync(dretry_b_.p, 0, bits, stream_), "memset");
-                Upsert_Visitor<set_, VT, Fn> rv{T_, fn, ctr(), dretry_b_.as<unsigned int>(), dretry_a_.as<unsigned int>(), retried, per_seq};
+                Upsert_Visitor<set_, VT, Fn> rv{T_, fn, ctr(), dretry_b_.as<unsigned int>(), dretry_a_.as<unsigned int>(), retried, per, by_batch};
                 stream_launch(K_UPSERT, bi, sb, se, rv);
                 check(cudaMemsetAsync(dretry_a_.p, 0, bits, stream_), "memset");
                 std::swap(dretry_a_.p, dretry_b_.p), std::swap(dretry_a_.bytes, dretry_b_.bytes);
@@ -1088,11 +1089,11 @@ class Engine final : public kache_table
     {
         check(cudaMemsetAsync(out, 0, bi.n * 8, stream_), "memset");
         if(mode == 0)
-            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(mf), VT(mr), 0, 0});
+            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(mf), VT(mr)});
         else if(mode == 1)
-            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 1>{T_, out, VT(mf), VT(mr), 0, 0});
+            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 1>{T_, out, VT(mf), VT(mr)});
         else
-            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 2>{T_, out, VT(mf), VT(mr), 0, 0});
+            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 2>{T_, out, VT(mf), VT(mr)});
     }
 
     // Whether host memory at p is page-locked (the caller's cudaHostAlloc'd or registered memory): copies then use it
@@ -1467,7 +1468,7 @@ public:
         auto* out = reinterpret_cast<unsigned long long*>(counts);
         if(p.n)
             check(cudaMemsetAsync(out, 0, p.n * 8, stream_), "memset");
-        stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(0), VT(0), 0, 0});
+        stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(0), VT(0)});
     }
 
     // A number that stays the same while the table's device arrays do (a graph captured with a prepared lookup stays
@@ -1526,49 +1527,38 @@ public:
         auto* res = reinterpret_cast<unsigned long long*>(d + o_res);
         auto* batch_of = reinterpret_cast<uint32_t*>(d + o_bof);
         check(cudaMemcpyAsync(desc, hd, count * 64, cudaMemcpyHostToDevice, stream_), "H2D descriptors");
-        launch(K_OTHER, [&](){ batches_list_kernel<<<grid_for((N + 31) / 32, 8), 256, 0, stream_>>>(desc, count, N, lens, addr, batch_of); });
+        launch(K_OTHER, [&](){ batches_list_kernel<<<grid_for((N + 31) / 32, 8), 256, 0, stream_>>>(desc, count, N, lens, addr, batch_of, kind == KACHE_B200_RUN_COUNT); });
         check(cudaMemsetAsync(voff, 0, 8, stream_), "memset");
         size_t tmp = 0;
         check(cub::DeviceScan::InclusiveSum(nullptr, tmp, lens, voff + 1, static_cast<int64_t>(N), stream_), "scan");
         dscan_.ensure(tmp);
         check(cub::DeviceScan::InclusiveSum(dscan_.p, tmp, lens, voff + 1, static_cast<int64_t>(N), stream_), "scan");
 
-        const auto bi = stage_dev(nullptr, voff, N, addr);
-        dout_.ensure(N * 8 + 8);
-        auto* per_seq = dout_.as<unsigned long long>();
-        check(cudaMemsetAsync(per_seq, 0, N * 8, stream_), "memset");
+        const auto bi = stage_dev(nullptr, voff, N, addr, batch_of);
+        // Per-batch results, added up by the visitors: keys inserted, k-mers present, positions found or counts.
+        check(cudaMemsetAsync(res, 0, count * 8, stream_), "memset");
         if(kind == KACHE_B200_RUN_UPSERT)
-            run_upsert(user, bi, op_fn(op, x, y), per_seq);
+            run_upsert(user, bi, op_fn(op, x, y), res, true);
         else if(kind == KACHE_B200_RUN_UPSERT_ORIENTED)
         {
             if constexpr(!set_)
-                run_upsert(user, bi, Oriented_Op_Fn<VT>{op, static_cast<VT>(x), static_cast<VT>(y)}, per_seq);
+                run_upsert(user, bi, Oriented_Op_Fn<VT>{op, static_cast<VT>(x), static_cast<VT>(y)}, res, true);
         }
         else if(kind == KACHE_B200_RUN_UPDATE)
         {
             if constexpr(!set_)
             {
                 check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
-                Update_Visitor<VT, Op_Fn<VT>> vis{T_, op_fn(op, x, 0), ctr(), per_seq};
-                stream_launch(K_UPDATE, bi, 0, bi.nsegs, vis);
+                stream_launch(K_UPDATE, bi, 0, bi.nsegs, Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), res});
             }
         }
         else if(kind == KACHE_B200_RUN_COUNT)
-        {
-            run_seq_reduce(bi, 0, 0, 0, per_seq);
-            launch(K_OTHER, [&](){ batches_scatter_kernel<<<grid_for((N + 31) / 32, 8), 256, 0, stream_>>>(desc, per_seq, batch_of, N); });
-        }
+            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Count_Batches_Visitor<set_, VT>{{T_, nullptr, VT(0), VT(0)}, desc, res});
         else
         {
             launch(K_OTHER, [&](){ batches_pos_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, stream_>>>(desc, count, bi.pos_off, pos_base); });
-            Lookup_Batches_Visitor<set_, VT> vis{{T_, nullptr, nullptr, nullptr}, batch_of, desc, pos_base};
-            stream_launch(K_LOOKUP, bi, 0, bi.nsegs, vis);
-            launch(K_OTHER, [&](){ batches_hits_kernel<<<grid_for(N, 8), 256, 0, stream_>>>(desc, batch_of, bi.pos_off, pos_base, N, per_seq); });
+            stream_launch(K_LOOKUP, bi, 0, bi.nsegs, Lookup_Batches_Visitor<set_, VT>{{T_, nullptr, nullptr, nullptr}, desc, pos_base, res});
         }
-        // Per-batch results: the per-sequence counters (keys inserted, k-mers present, positions found, counts)
-        // summed per batch.
-        check(cudaMemsetAsync(res, 0, count * 8, stream_), "memset");
-        launch(K_OTHER, [&](){ batches_sum_kernel<<<grid_for((N + 31) / 32 / 64 + 1, 8), 256, 0, stream_>>>(per_seq, batch_of, N, res); });
         auto* hr = pin_multi_.as<uint64_t>();
         check(cudaMemcpyAsync(hr, res, count * 8, cudaMemcpyDeviceToHost, stream_), "D2H results");
         sync();

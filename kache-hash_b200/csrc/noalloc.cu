@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(32 * stream_warps) noalloc_count_kernel(const 
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if(*s.overflow)
         return;
-    Seq_Reduce_Visitor<set_, uint8_t, 0> vis{T, counts, 0, 0, 0, 0};
+    Seq_Reduce_Visitor<set_, uint8_t, 0> vis{T, counts, 0, 0};
     vis.begin();
 
     const uint64_t nsegs = min(static_cast<uint64_t>(*s.count), noalloc_max_segments);
@@ -91,9 +91,10 @@ __global__ void __launch_bounds__(32 * stream_warps) noalloc_count_kernel(const 
         const uint64_t packed = s.segs[g], q = packed >> 24;
         const uint64_t b0 = off[q], len = off[q + 1] - b0;
         const uint64_t p0 = (packed & 0xFFFFFF) * seg_positions;
-        vis.begin_segment(q, 0);
+        const Seg_Of of{q, 0, 0};
+        vis.begin_segment(of);
         describe_segment<k, l>(bases + b0 + p0, static_cast<uint32_t>(min(len - k + 1 - p0, static_cast<uint64_t>(seg_positions))), ring_all[wid], tab, lane, vis);
-        vis.end_segment(q, lane);
+        vis.end_segment(of, lane);
     }
 }
 
