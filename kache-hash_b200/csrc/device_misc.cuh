@@ -338,12 +338,35 @@ static __global__ void batch_counts_kernel(const uint64_t* off, const uint64_t n
         atomicOr(too_long, 1u);
 }
 
-// The counting and summing of a small device batch's staging in one block of 1024 threads: each thread takes a run
-// of sequences; pos_off[0..n] and seg_off[0..n] get the exclusive sums of positions and segments, and out[0..2] the
-// positions, the segments and the segment length, fitted to the batch (fitted_seg_len, then eight times longer while
-// the longest sequence would have more segments than a list entry indexes). In place of a counting kernel, two scans
-// and their copies; segs_kernel then lists the segments.
-constexpr uint32_t small_stage_max = 4096;  // Sequences of a batch summed by one block (at most 4 per thread).
+// The staging of a small device batch, or of several run as one, in one block of 1024 threads: it counts, fits the segment
+// length (fitted_seg_len, then eight times longer while the longest sequence would have more segments than a list entry
+// indexes), sums and lists the segments, in place of a counting kernel, two scans, a listing kernel and the host reading
+// the counts in between. The launch behind it takes its number of segments from ctr[6]: none if the batch has more
+// segments or positions than the caller made room for, which the host reads with the launch's results.
+constexpr uint32_t small_stage_max = 4096;      // Sequences (at most 4 per thread).
+constexpr uint32_t small_segs_max = 16384;      // Segments listed by the block.
+
+struct Small_Stage
+{
+    // One batch's n + 1 offsets; or (null) several batches, 8 words each as batches_list_kernel takes them, with the arrays
+    // it fills, and each batch's first merged position.
+    const uint64_t* off;
+    const uint64_t* desc;
+    uint64_t count;
+    uint64_t* addr;
+    uint32_t* batch_of;
+    uint64_t* pos_base;
+    bool zero_out0;             // Zeroes each sequence's word of its batch's out0.
+    uint64_t n;
+    int k;
+    uint32_t sms;
+    uint64_t max_segs, max_pos;
+    uint64_t *pos_off, *seg_off;    // n + 1 sums each.
+    Segment* segs;
+    unsigned long long* ctr;    // [0] and the low half of [2] are zeroed; [3..6]: positions, segments, segment length, segments to run.
+    unsigned long long* zero;   // zero_n words zeroed.
+    uint64_t zero_n;
+};
 
 // The inclusive sum of x over the block's threads in order; `warps` is 32 words of shared memory.
 __device__ __forceinline__ unsigned long long block_sum(unsigned long long x, unsigned long long* warps)
@@ -375,44 +398,102 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long x, un
     return x + (wid ? warps[wid - 1] : 0);
 }
 
-static __global__ void __launch_bounds__(1024) stage_small_kernel(const uint64_t* off, const uint64_t n, const int k, const uint32_t sms,
-                                                                 uint64_t* pos_off, uint64_t* seg_off, unsigned long long* out)
+static __global__ void __launch_bounds__(1024) stage_small_kernel(const Small_Stage a)
 {
-    __shared__ unsigned long long wp[32], ws[32], longest;
+    __shared__ unsigned long long wp[32], ws[32], wtop[32];
+    __shared__ uint32_t first_seg[small_stage_max + 1];
     const uint32_t t = threadIdx.x;
-    if(t == 0)
-        longest = 0;
-    const uint64_t per = (n + 1023) / 1024, q0 = min(n, uint64_t(t) * per), q1 = min(n, q0 + per);
-    const auto npos = [&](const uint64_t q) -> uint64_t
-    {
-        const uint64_t len = off[q + 1] - off[q];
-        return len >= uint64_t(k) ? len - k + 1 : 0;
-    };
+    const uint64_t per = (a.n + 1023) / 1024, q0 = min(a.n, uint64_t(t) * per);
+    const uint32_t mine = static_cast<uint32_t>(min(a.n, q0 + per) - q0);
+    uint64_t np[4];
     unsigned long long P = 0, S = 0, top = 0;
-    for(uint64_t q = q0; q < q1; ++q)
-    {
-        const unsigned long long np = npos(q);
-        P += np, top = max(top, np);
-    }
+    uint64_t lo = 0;
+    if(a.desc && mine)
+        for(uint64_t hi = a.count; hi - lo > 1; )   // The last batch whose first merged sequence is at or before q0.
+        {
+            const uint64_t mid = (lo + hi) / 2;
+            if(a.desc[8 * mid + 3] <= q0)
+                lo = mid;
+            else
+                hi = mid;
+        }
+#pragma unroll
+    for(uint32_t i = 0; i < 4; ++i)
+        if(i < mine)
+        {
+            const uint64_t q = q0 + i;
+            uint64_t len;
+            if(a.desc)
+            {
+                while(lo + 1 < a.count && a.desc[8 * (lo + 1) + 3] <= q)
+                    ++lo;
+                const uint64_t* d = a.desc + 8 * lo;
+                const uint64_t j = q - d[3], b0 = reinterpret_cast<const uint64_t*>(d[1])[j];
+                len = reinterpret_cast<const uint64_t*>(d[1])[j + 1] - b0;
+                a.addr[q] = d[0] + b0;
+                a.batch_of[q] = static_cast<uint32_t>(lo);
+                if(a.zero_out0)
+                    reinterpret_cast<uint64_t*>(d[4])[j] = 0;
+            }
+            else
+                len = a.off[q + 1] - a.off[q];
+            np[i] = len >= uint64_t(a.k) ? len - a.k + 1 : 0;
+            P += np[i], top = max(top, static_cast<unsigned long long>(np[i]));
+        }
+    for(uint64_t i = t; i < a.zero_n; i += 1024)
+        a.zero[i] = 0;
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1)
+        top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+    if((t & 31) == 0)
+        wtop[t >> 5] = top;
     unsigned long long bp = block_sum(P, wp) - P;
-    atomicMax(&longest, top);
-    __syncthreads();
-    uint64_t seg_len = fitted_seg_len(wp[31], sms);
+    const uint64_t total = wp[31];
+    unsigned long long longest = 0;
+#pragma unroll
+    for(int i = 0; i < 32; ++i)
+        longest = max(longest, wtop[i]);
+    uint64_t seg_len = fitted_seg_len(total, a.sms);
     while((longest + seg_len - 1) / seg_len > max_seg_index + 1)
         seg_len *= 8;
-    for(uint64_t q = q0; q < q1; ++q)
-        S += (npos(q) + seg_len - 1) / seg_len;
+#pragma unroll
+    for(uint32_t i = 0; i < 4; ++i)
+        if(i < mine)
+            S += (np[i] + seg_len - 1) / seg_len;
     unsigned long long bs = block_sum(S, ws) - S;
-    for(uint64_t q = q0; q < q1; ++q)
-    {
-        const uint64_t np = npos(q);
-        pos_off[q] = bp, seg_off[q] = bs;
-        bp += np, bs += (np + seg_len - 1) / seg_len;
-    }
+    const uint64_t nsegs = ws[31], run = nsegs <= a.max_segs && total <= a.max_pos ? nsegs : 0;
+#pragma unroll
+    for(uint32_t i = 0; i < 4; ++i)
+        if(i < mine)
+        {
+            const uint64_t q = q0 + i;
+            a.pos_off[q] = bp, a.seg_off[q] = bs;
+            if(run)
+                first_seg[q] = static_cast<uint32_t>(bs);
+            if(a.desc && a.desc[8 * uint64_t(a.batch_of[q]) + 3] == q)
+                a.pos_base[a.batch_of[q]] = bp;
+            bp += np[i], bs += (np[i] + seg_len - 1) / seg_len;
+        }
     if(t == 1023)
     {
-        pos_off[n] = wp[31], seg_off[n] = ws[31];
-        out[0] = wp[31], out[1] = ws[31], out[2] = seg_len;
+        a.pos_off[a.n] = total, a.seg_off[a.n] = nsegs;
+        a.ctr[3] = total, a.ctr[4] = nsegs, a.ctr[5] = seg_len, a.ctr[6] = run;
+        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0;
+    }
+    __syncthreads();
+    for(uint32_t i = t; i < run; i += 1024)
+    {
+        uint32_t l = 0, h = static_cast<uint32_t>(a.n);     // The last q with first_seg[q] <= i.
+        while(h - l > 1)
+        {
+            const uint32_t mid = (l + h) / 2;
+            if(first_seg[mid] <= i)
+                l = mid;
+            else
+                h = mid;
+        }
+        const uint64_t p0 = (i - first_seg[l]) * seg_len, first = a.pos_off[l] + p0;
+        a.segs[i] = Segment{(a.desc ? a.addr[l] : a.off[l]) + p0, first, l, static_cast<uint32_t>(min(a.pos_off[l + 1] - first, seg_len)), a.desc ? a.batch_of[l] : 0};
     }
 }
 

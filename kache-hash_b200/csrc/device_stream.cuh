@@ -190,8 +190,11 @@ __device__ __forceinline__ void describe_segment(const uint8_t* const seq, const
 }
 
 template <int k, int l, typename Visitor>
-__global__ void __launch_bounds__(32 * stream_warps, Visitor::min_blocks) stream_kernel(const Dev_Batch batch, const uint64_t seg_b, const uint64_t seg_e, Visitor vis)
+__global__ void __launch_bounds__(32 * stream_warps, Visitor::min_blocks) stream_kernel(const Dev_Batch batch, const uint64_t seg_b, const uint64_t segs_end,
+                                                                                        const unsigned long long* run, Visitor vis)
 {
+    // The segments [seg_b, segs_end), or as many as `run` says, counted by the kernel before.
+    const uint64_t seg_e = run ? static_cast<uint64_t>(*run) : segs_end;
     __shared__ uint32_t ring_all[stream_warps][ring_words];
     __shared__ uint8_t tab[base_table_bytes];
     fill_base_table(tab);

@@ -780,19 +780,48 @@ class Engine final : public kache_table
         return stage_dev(reinterpret_cast<const uint8_t*>(d), reinterpret_cast<const uint64_t*>(d + o_off), n);
     }
 
+    // A small device batch's staging arguments: the offsets of one, or none for the caller to set several.
+    Small_Stage small_stage(const uint64_t* off, const uint64_t n)
+    {
+        dtmp_.ensure(2 * (n + 1) * 8);
+        Small_Stage a{};
+        a.off = off, a.n = n, a.k = k, a.sms = static_cast<uint32_t>(sm_count_);
+        a.pos_off = dtmp_.as<uint64_t>(), a.seg_off = a.pos_off + (n + 1), a.ctr = ctr();
+        return a;
+    }
+
     // stage_dev for a batch of at most small_stage_max sequences: one block counts, fits the segment length and sums, one
     // kernel lists.
     Batch_Info stage_dev_small(const uint8_t* bases, const uint64_t* off, const uint64_t n, const uint64_t* addr, const uint32_t* batch_of)
     {
-        dtmp_.ensure(2 * (n + 1) * 8);
-        uint64_t* pos_off = dtmp_.as<uint64_t>();
-        uint64_t* seg_off = pos_off + (n + 1);
-        unsigned long long* out = ctr() + 3;    // Three words: positions, segments, segment length.
+        const Small_Stage a = small_stage(off, n);
+        launch(K_OTHER, [&](){ stage_small_kernel<<<1, 1024, 0, stream_>>>(a); });
         uint64_t* h = pin_ctr_.as<uint64_t>(32);
-        launch(K_OTHER, [&](){ stage_small_kernel<<<1, 1024, 0, stream_>>>(off, n, k, static_cast<uint32_t>(sm_count_), pos_off, seg_off, out); });
-        check(cudaMemcpyAsync(h, out, 24, cudaMemcpyDeviceToHost, stream_), "D2H");
+        check(cudaMemcpyAsync(h, ctr() + 3, 24, cudaMemcpyDeviceToHost, stream_), "D2H");
         sync();
-        return list_dev(bases, off, addr, batch_of, n, pos_off, seg_off, h[0], h[1], static_cast<uint32_t>(h[2]));
+        small_fits_ = h[1] <= small_segs_max;
+        return list_dev(bases, off, addr, batch_of, n, a.pos_off, a.seg_off, h[0], h[1], static_cast<uint32_t>(h[2]));
+    }
+
+    // Whether to run a batch of n sequences by run_small: the last small batch had no more segments than its block lists.
+    bool small_fits_ = true;
+    bool small(const uint64_t n) const { return n > 0 && n <= small_stage_max && small_fits_; }
+
+    // Stages a small batch and runs the visitor over it with no host read in between (stage_small_kernel); returns the
+    // counters, of which [4] and [6] are equal if the batch ran. The launch's grid fills the GPU, its segments being
+    // unknown here.
+    template <typename Vis> const unsigned long long* run_small(const uint32_t kind, const uint8_t* bases, Small_Stage a, const Vis& vis)
+    {
+        dbatch_.ensure(small_segs_max * sizeof(Segment));
+        a.segs = dbatch_.as<Segment>(), a.max_segs = small_segs_max;
+        launch(K_OTHER, [&](){ stage_small_kernel<<<1, 1024, 0, stream_>>>(a); });
+        launch(kind, [&]()
+        {
+            stream_kernel<k, l, Vis><<<static_cast<unsigned>(sm_count_) * Vis::min_blocks, 32 * stream_warps, 0, stream_>>>(Dev_Batch{bases, a.segs}, 0, 0, ctr() + 6, vis);
+        });
+        const unsigned long long* c = read_ctr(7);
+        small_fits_ = c[4] <= small_segs_max;
+        return c;
     }
 
     // Lists the segments of a batch whose positions and segments are counted.
@@ -873,7 +902,7 @@ class Engine final : public kache_table
 
     template <typename Vis> void segs_launch(const uint32_t kind, const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Vis& vis)
     {
-        launch(kind, [&](){ stream_kernel<k, l, Vis><<<grid_for(se - sb, stream_warps), 32 * stream_warps, 0, stream_>>>(bi.b, sb, se, vis); });
+        launch(kind, [&](){ stream_kernel<k, l, Vis><<<grid_for(se - sb, stream_warps), 32 * stream_warps, 0, stream_>>>(bi.b, sb, se, nullptr, vis); });
     }
 
     // The reference's per-user flush accounting over one call (include/Streaming_Kmer_Hash_Table.hpp:2248-2286,
@@ -1015,12 +1044,7 @@ class Engine final : public kache_table
 
         for(uint64_t sb = 0; sb < nsegs; )
         {
-            if(dretry_dirty_ || dretry_a_.bytes < bits || dretry_b_.bytes < bits)
-            {
-                dretry_a_.ensure(bits), dretry_b_.ensure(bits);
-                check(cudaMemsetAsync(dretry_a_.p, 0, dretry_a_.bytes, stream_), "memset");
-                dretry_dirty_ = false;
-            }
+            clear_retries(bits);
             // A chunk may take the device table to 95 % of its slots, at a quarter above the expected rate (and at
             // least a quarter of the positions); the schedule then resizes it, as the reference would.
             const double slots = static_cast<double>(T_.cap * B);
@@ -1039,36 +1063,95 @@ class Engine final : public kache_table
             Upsert_Visitor<set_, VT, Fn> vis{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per, by_batch};
             stream_launch(K_UPSERT, bi, sb, se, vis);
             const unsigned long long* c = read_ctr(3);
-            uint64_t ins = c[0];
-            while(static_cast<uint32_t>(c[2]))
-            {
-                dretry_dirty_ = true;   // Until the retries end with no bit left set (a failure may come first).
-                grow_overflow();
-                check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
-                check(cudaMemsetAsync(retried, 0, 4, stream_), "memset");
-                check(cudaMemsetAsync(dretry_b_.p, 0, bits, stream_), "memset");
-                Upsert_Visitor<set_, VT, Fn> rv{T_, fn, ctr(), dretry_b_.as<unsigned int>(), dretry_a_.as<unsigned int>(), retried, per, by_batch};
-                stream_launch(K_UPSERT, bi, sb, se, rv);
-                check(cudaMemsetAsync(dretry_a_.p, 0, bits, stream_), "memset");
-                std::swap(dretry_a_.p, dretry_b_.p), std::swap(dretry_a_.bytes, dretry_b_.bytes);
-                c = read_ctr(3);
-                ins += c[0];
-            }
+            const uint64_t ins = c[0] + retry_full(bi, sb, se, fn, per, by_batch, c);
 
             const double chunk_pos = (se - sb) * pos_per_seg;
             novelty = chunk_pos > 0 ? std::max(static_cast<double>(ins) / chunk_pos, 1e-3) : novelty;
-            size_ += ins, total_ins += ins;
-            acct.add(ins);
-            if(cap_ > T_.cap)
-                resize(rebuild_cap(cap_));
-            if(c[1] * 4 > ov_slots_ * 3)
-                grow_overflow();
+            total_ins += ins;
+            inserted(acct, ins, c[1]);
             sb = se;
         }
-        pending_[user] = acct.left();
-        if(bi.total_pos > 0)
-            novelty_ = std::max(static_cast<double>(total_ins) / static_cast<double>(bi.total_pos), 1e-3), novelty_seen_ = true;
+        upsert_done(user, acct, total_ins, bi.total_pos);
         return total_ins;
+    }
+
+    // Re-runs the positions of segments [sb, se) that found the overflow table full (c: the counters as their run left
+    // them), the overflow table doubled each time; returns the keys inserted.
+    template <typename Fn> uint64_t retry_full(const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Fn& fn, unsigned long long* per, const bool by_batch,
+                                               const unsigned long long*& c)
+    {
+        const size_t bits = bi.total_pos / 8 + 8;
+        unsigned int* retried = reinterpret_cast<unsigned int*>(ctr() + 2);
+        uint64_t ins = 0;
+        while(static_cast<uint32_t>(c[2]))
+        {
+            dretry_dirty_ = true;   // Until the retries end with no bit left set (a failure may come first).
+            grow_overflow();
+            check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
+            check(cudaMemsetAsync(retried, 0, 4, stream_), "memset");
+            check(cudaMemsetAsync(dretry_b_.p, 0, bits, stream_), "memset");
+            Upsert_Visitor<set_, VT, Fn> rv{T_, fn, ctr(), dretry_b_.as<unsigned int>(), dretry_a_.as<unsigned int>(), retried, per, by_batch};
+            stream_launch(K_UPSERT, bi, sb, se, rv);
+            check(cudaMemsetAsync(dretry_a_.p, 0, bits, stream_), "memset");
+            std::swap(dretry_a_.p, dretry_b_.p), std::swap(dretry_a_.bytes, dretry_b_.bytes);
+            c = read_ctr(3);
+            ins += c[0];
+        }
+        return ins;
+    }
+
+    // Makes room for `bits` retry bits, all clear.
+    void clear_retries(const size_t bytes)
+    {
+        if(!dretry_dirty_ && dretry_a_.bytes >= bytes && dretry_b_.bytes >= bytes)
+            return;
+        dretry_a_.ensure(bytes), dretry_b_.ensure(bytes);
+        check(cudaMemsetAsync(dretry_a_.p, 0, dretry_a_.bytes, stream_), "memset");
+        dretry_dirty_ = false;
+    }
+
+    // After a launch that inserted `ins` keys: the schedule, and the tables it finds too small.
+    void inserted(Call_Acct& acct, const uint64_t ins, const uint64_t ov_keys)
+    {
+        size_ += ins;
+        acct.add(ins);
+        if(cap_ > T_.cap)
+            resize(rebuild_cap(cap_));
+        if(ov_keys * 4 > ov_slots_ * 3)
+            grow_overflow();
+    }
+
+    void upsert_done(const uint32_t user, const Call_Acct& acct, const uint64_t ins, const uint64_t total_pos)
+    {
+        pending_[user] = acct.left();
+        if(total_pos > 0)
+            novelty_ = std::max(static_cast<double>(ins) / static_cast<double>(total_pos), 1e-3), novelty_seen_ = true;
+    }
+
+    // Upserts a small batch by run_small, if it would fit the device table were every position a new key; returns whether
+    // it did, with the keys inserted in `ins`. Otherwise nothing was done.
+    template <typename Fn> bool upsert_small(const uint32_t user, const uint8_t* bases, Small_Stage a, const Fn& fn, uint64_t& ins, unsigned long long* per = nullptr)
+    {
+        const double room = 0.95 * static_cast<double>(T_.cap * B) - static_cast<double>(size_);
+        constexpr uint64_t most = uint64_t(small_segs_max) * seg_positions;
+        if(room < 1)
+            return false;
+        a.max_pos = static_cast<uint64_t>(std::min(room, static_cast<double>(most)));
+        clear_retries(most / 8 + 8);
+        unsigned int* retried = reinterpret_cast<unsigned int*>(ctr() + 2);
+        const unsigned long long* c = run_small(K_UPSERT, bases, a, Upsert_Visitor<set_, VT, Fn>{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per, per != nullptr});
+        if(c[6] != c[4])
+            return false;
+        Batch_Info bi;
+        bi.b = Dev_Batch{bases, dbatch_.as<Segment>()};
+        bi.n = a.n, bi.total_pos = c[3], bi.nsegs = c[4];
+        ins = c[0];
+        if(static_cast<uint32_t>(c[2]))
+            ins += retry_full(bi, 0, bi.nsegs, fn, per, per != nullptr, c);
+        Call_Acct acct(Sched{approx_sz_, cap_, resize_th_, step_, lf_}, pending_[user]);
+        inserted(acct, ins, c[1]);
+        upsert_done(user, acct, ins, bi.total_pos);
+        return true;
     }
 
     template <typename Fn> uint64_t run_update(const Batch_Info& bi, const Fn& fn)
@@ -1384,9 +1467,10 @@ public:
     uint64_t upsert_dev(uint32_t user, const uint8_t* b, const uint64_t* off, uint64_t n, uint32_t op, uint64_t x, uint64_t init) override
     {
         std::lock_guard<std::mutex> g(work);
-        const auto bi = stage_dev(b, off, n);
-        const uint64_t r = run_upsert(user, bi, op_fn(op, x, init));
-        return r;
+        uint64_t ins;
+        if(small(n) && upsert_small(user, b, small_stage(off, n), op_fn(op, x, init), ins))
+            return ins;
+        return run_upsert(user, stage_dev(b, off, n), op_fn(op, x, init));
     }
 
     uint64_t upsert_oriented_dev(uint32_t user, const uint8_t* b, const uint64_t* off, uint64_t n, uint32_t op, uint64_t xf, uint64_t xr) override
@@ -1396,9 +1480,11 @@ public:
         else
         {
             std::lock_guard<std::mutex> g(work);
-            const auto bi = stage_dev(b, off, n);
-            const uint64_t r = run_upsert(user, bi, Oriented_Op_Fn<VT>{op, static_cast<VT>(xf), static_cast<VT>(xr)});
-            return r;
+            const Oriented_Op_Fn<VT> fn{op, static_cast<VT>(xf), static_cast<VT>(xr)};
+            uint64_t ins;
+            if(small(n) && upsert_small(user, b, small_stage(off, n), fn, ins))
+                return ins;
+            return run_upsert(user, stage_dev(b, off, n), fn);
         }
     }
 
@@ -1409,17 +1495,31 @@ public:
         else
         {
             std::lock_guard<std::mutex> g(work);
-            const auto bi = stage_dev(b, off, n);
-            const uint64_t r = run_update(bi, op_fn(op, x, 0));
-            return r;
+            if(small(n))
+            {
+                Small_Stage a = small_stage(off, n);
+                a.max_pos = ~0ull;
+                const auto* c = run_small(K_UPDATE, b, a, Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), nullptr});
+                if(c[6] == c[4])
+                    return c[0];
+            }
+            return run_update(stage_dev(b, off, n), op_fn(op, x, 0));
         }
     }
 
     void lookup_dev(const uint8_t* b, const uint64_t* off, uint64_t n, uint8_t* found, void* values, uint8_t* fwd) override
     {
         std::lock_guard<std::mutex> g(work);
-        const auto bi = stage_dev(b, off, n);
-        run_lookup(bi, found, set_ ? nullptr : static_cast<VT*>(values), fwd);
+        auto* v = set_ ? nullptr : static_cast<VT*>(values);
+        if(small(n))
+        {
+            Small_Stage a = small_stage(off, n);
+            a.max_pos = ~0ull;
+            const auto* c = run_small(K_LOOKUP, b, a, Lookup_Visitor<set_, VT>{T_, found, v, fwd});
+            if(c[6] == c[4])
+                return;
+        }
+        run_lookup(stage_dev(b, off, n), found, v, fwd);
         sync();
     }
 
@@ -1486,8 +1586,16 @@ public:
     void count_dev(const uint8_t* b, const uint64_t* off, uint64_t n, uint64_t* counts) override
     {
         std::lock_guard<std::mutex> g(work);
-        const auto bi = stage_dev(b, off, n);
-        run_seq_reduce(bi, 0, 0, 0, reinterpret_cast<unsigned long long*>(counts));
+        auto* out = reinterpret_cast<unsigned long long*>(counts);
+        if(small(n))
+        {
+            Small_Stage a = small_stage(off, n);
+            a.max_pos = ~0ull, a.zero = out, a.zero_n = n;
+            const auto* c = run_small(K_REDUCE, b, a, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(0), VT(0)});
+            if(c[6] == c[4])
+                return;
+        }
+        run_seq_reduce(stage_dev(b, off, n), 0, 0, 0, out);
         sync();
     }
 
@@ -1527,6 +1635,43 @@ public:
         auto* res = reinterpret_cast<unsigned long long*>(d + o_res);
         auto* batch_of = reinterpret_cast<uint32_t*>(d + o_bof);
         check(cudaMemcpyAsync(desc, hd, count * 64, cudaMemcpyHostToDevice, stream_), "H2D descriptors");
+        const auto results = [&]()
+        {
+            auto* hr = pin_multi_.as<uint64_t>();
+            check(cudaMemcpyAsync(hr, res, count * 8, cudaMemcpyDeviceToHost, stream_), "D2H results");
+            sync();
+            for(size_t b = 0; b < count; ++b)
+                bs[b].result = hr[b];
+        };
+        const Oriented_Op_Fn<VT> ofn{op, static_cast<VT>(x), static_cast<VT>(y)};
+        if(small(N))
+        {
+            Small_Stage a = small_stage(nullptr, N);
+            a.desc = desc, a.count = count, a.addr = addr, a.batch_of = batch_of, a.pos_base = pos_base;
+            a.zero_out0 = kind == KACHE_B200_RUN_COUNT, a.zero = res, a.zero_n = count, a.max_pos = ~0ull;
+            uint64_t ins = 0;
+            bool ran = false;
+            if(kind == KACHE_B200_RUN_UPSERT)
+                ran = upsert_small(user, nullptr, a, op_fn(op, x, y), ins, res);
+            else if(kind == KACHE_B200_RUN_UPSERT_ORIENTED)
+            {
+                if constexpr(!set_)
+                    ran = upsert_small(user, nullptr, a, ofn, ins, res);
+            }
+            else
+            {
+                const unsigned long long* c = nullptr;
+                if(kind == KACHE_B200_RUN_COUNT)
+                    c = run_small(K_REDUCE, nullptr, a, Count_Batches_Visitor<set_, VT>{{T_, nullptr, VT(0), VT(0)}, desc, res});
+                else if(kind == KACHE_B200_RUN_LOOKUP)
+                    c = run_small(K_LOOKUP, nullptr, a, Lookup_Batches_Visitor<set_, VT>{{T_, nullptr, nullptr, nullptr}, desc, pos_base, res});
+                else if constexpr(!set_)
+                    c = run_small(K_UPDATE, nullptr, a, Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), res});
+                ran = c && c[6] == c[4];
+            }
+            if(ran)
+                return results();
+        }
         launch(K_OTHER, [&](){ batches_list_kernel<<<grid_for((N + 31) / 32, 8), 256, 0, stream_>>>(desc, count, N, lens, addr, batch_of, kind == KACHE_B200_RUN_COUNT); });
         check(cudaMemsetAsync(voff, 0, 8, stream_), "memset");
         size_t tmp = 0;
@@ -1542,7 +1687,7 @@ public:
         else if(kind == KACHE_B200_RUN_UPSERT_ORIENTED)
         {
             if constexpr(!set_)
-                run_upsert(user, bi, Oriented_Op_Fn<VT>{op, static_cast<VT>(x), static_cast<VT>(y)}, res, true);
+                run_upsert(user, bi, ofn, res, true);
         }
         else if(kind == KACHE_B200_RUN_UPDATE)
         {
@@ -1559,11 +1704,7 @@ public:
             launch(K_OTHER, [&](){ batches_pos_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, stream_>>>(desc, count, bi.pos_off, pos_base); });
             stream_launch(K_LOOKUP, bi, 0, bi.nsegs, Lookup_Batches_Visitor<set_, VT>{{T_, nullptr, nullptr, nullptr}, desc, pos_base, res});
         }
-        auto* hr = pin_multi_.as<uint64_t>();
-        check(cudaMemcpyAsync(hr, res, count * 8, cudaMemcpyDeviceToHost, stream_), "D2H results");
-        sync();
-        for(size_t b = 0; b < count; ++b)
-            bs[b].result = hr[b];
+        results();
     }
 
     bool get(const char* kmer, uint64_t& value) override
