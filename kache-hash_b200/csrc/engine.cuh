@@ -351,6 +351,7 @@ class Engine final : public kache_table
     uint64_t pending_[KACHE_MAX_USERS] = {};
     double novelty_ = 0.5;      // Keys inserted per position in the last upsert call.
     bool novelty_seen_ = false; // Whether an upsert call has measured it.
+    uint64_t last_pos_ = 0;     // Positions of the last upsert call.
 
     // Batches.
     Pinned_Buf pin_, pin_ctr_, pin_out_;
@@ -974,11 +975,20 @@ class Engine final : public kache_table
         const uint64_t wide = 2 * target;
         if(wide > max_buckets)
             return target;
+        if(spare_holds(wide))
+            return wide;
         const size_t need = wide * (B + 32 + B * slot_bytes) + ov_slots_for(std::max<uint64_t>(1024, wide)) * 32;
         size_t free_b = 0, total_b = 0;
         check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
         const size_t spare = cs2_.bytes + spill2_.bytes + slots2_.bytes + ov2_.bytes;
         return 2 * need <= free_b + spare ? wide : target;
+    }
+
+    // Whether the spare arrays hold a table of `cap` buckets (but for its overflow table): then a rebuild need not ask the
+    // driver for the free memory, which took up to 2 ms a time.
+    bool spare_holds(const uint64_t cap) const
+    {
+        return cs2_.bytes >= cap * B && spill2_.bytes >= cap * 32 && slots2_.bytes >= cap * B * slot_bytes;
     }
 
     // Grows the device table to `target` buckets ahead of a call's inserts: where keys sit is not observable, so the
@@ -990,9 +1000,10 @@ class Engine final : public kache_table
             return;
         const uint64_t ov_slots = ov_slots_for(std::max<uint64_t>(1024, target));
         const size_t need = target * (B + 32 + B * slot_bytes) + ov_slots * 32;
-        const bool allocated = size_ == 0 && cs_.bytes >= target * B && spill_.bytes >= target * 32 &&
-                               slots_.bytes >= target * B * slot_bytes && ov_.bytes >= ov_slots * 32;
-        if(!allocated)      // The arrays would be allocated: only if they fit in free device memory.
+        const bool allocated = size_ == 0 ? cs_.bytes >= target * B && spill_.bytes >= target * 32 &&
+                                            slots_.bytes >= target * B * slot_bytes && ov_.bytes >= ov_slots * 32
+                                          : spare_holds(target) && ov2_.bytes >= ov_slots * 32;
+        if(!allocated)      // Arrays would be allocated: only if they fit in free device memory.
         {
             size_t free_b = 0, total_b = 0;
             check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
@@ -1015,9 +1026,11 @@ class Engine final : public kache_table
         }
         else
         {
-            check(cudaMemsetAsync(cs_.p, 0, target * B, stream_), "memset");
-            check(cudaMemsetAsync(spill_.p, 0, target * 32, stream_), "memset");
-            check(cudaMemsetAsync(slots_.p, 0, target * B * slot_bytes, stream_), "memset");
+            // The buckets that an empty table has are zero already.
+            const uint64_t have = T_.cap, more = target - have;
+            check(cudaMemsetAsync(cs_.as<char>() + have * B, 0, more * B, stream_), "memset");
+            check(cudaMemsetAsync(spill_.as<char>() + have * 32, 0, more * 32, stream_), "memset");
+            check(cudaMemsetAsync(slots_.as<char>() + have * B * slot_bytes, 0, more * B * slot_bytes, stream_), "memset");
         }
         bind(T_, cs_, spill_, slots_, target);
         ov_slots_ = ov_slots;
@@ -1124,19 +1137,21 @@ class Engine final : public kache_table
     void upsert_done(const uint32_t user, const Call_Acct& acct, const uint64_t ins, const uint64_t total_pos)
     {
         pending_[user] = acct.left();
+        last_pos_ = total_pos;
         if(total_pos > 0)
             novelty_ = std::max(static_cast<double>(ins) / static_cast<double>(total_pos), 1e-3), novelty_seen_ = true;
     }
 
     // Upserts a small batch by run_small, if it would fit the device table were every position a new key; returns whether
-    // it did, with the keys inserted in `ins`. Otherwise nothing was done.
+    // it did, with the keys inserted in `ins`. Otherwise nothing was done. (Not tried if the last upsert would not have
+    // fitted: the batches of a stream are mostly alike.)
     template <typename Fn> bool upsert_small(const uint32_t user, const uint8_t* bases, Small_Stage a, const Fn& fn, uint64_t& ins, unsigned long long* per = nullptr)
     {
         const double room = 0.95 * static_cast<double>(T_.cap * B) - static_cast<double>(size_);
         constexpr uint64_t most = uint64_t(small_segs_max) * seg_positions;
-        if(room < 1)
+        a.max_pos = static_cast<uint64_t>(std::clamp(room, 0.0, static_cast<double>(most)));
+        if(last_pos_ > a.max_pos)
             return false;
-        a.max_pos = static_cast<uint64_t>(std::min(room, static_cast<double>(most)));
         clear_retries(most / 8 + 8);
         unsigned int* retried = reinterpret_cast<unsigned int*>(ctr() + 2);
         const unsigned long long* c = run_small(K_UPSERT, bases, a, Upsert_Visitor<set_, VT, Fn>{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per, per != nullptr});
