@@ -303,17 +303,13 @@ struct Upsert_Visitor
         const uint32_t need_m = __ballot_sync(all, active && r == NONE);
         if(need_m)
         {
-            const uint32_t c = checksum_of(d.key);
-            // The bucket is read again: its checksums would take registers that other warps need.
-            if((need_m >> lane) & 1)
-                r = bucket_probe<set_>(T, at, key_st, c, j);
+            // Of lanes with one key, the first upserts it; the others then update it where it is. (The chain reads the
+            // bucket again: its checksums would take registers that other warps need.)
             const bool need = active && r == NONE;
-            // Of lanes with one key, the first upserts it; the others then update it where it is.
             uint32_t lead = lane;
-            const uint32_t lead_m = __ballot_sync(all, need);
             if(need)
-                lead = __ffs(__match_any_sync(lead_m, key_st)) - 1;
-            warp_claim<set_>(T, key_st, d.h, c, lane, need && lead == lane, at, j, r, ov_i);
+                lead = __ffs(__match_any_sync(need_m, key_st)) - 1;
+            warp_claim<set_>(T, key_st, d.h, checksum_of(d.key), lane, need && lead == lane, at, j, r, ov_i);
             if(__any_sync(all, lead != lane))
             {
                 const uint32_t r_l = __shfl_sync(all, r, lead), at_l = __shfl_sync(all, at, lead), j_l = __shfl_sync(all, j, lead);
@@ -323,17 +319,15 @@ struct Upsert_Visitor
             }
         }
 
+        // A claimed slot is published after its value is written; where the operation commutes, from a zeroed value, it is
+        // published at once and its initial value is then one more update.
         const bool comm = fn.commutes(), main = at != no_bucket;
         unsigned long long* const val = main ? key_word<set_>(T, at, j) + 1 : T.ov + 4 * ov_i + 1;
         if(r == INSERTED)
         {
             if constexpr(!set_)
-            {
-                if(comm)
-                    fn.apply_init(val, d.fwd);
-                else
+                if(!comm)
                     write_val<V>(val, fn.initial(d.fwd)), __threadfence();
-            }
             if(main)
                 *reinterpret_cast<volatile uint8_t*>(cs_of(T, at, j)) = static_cast<uint8_t>(checksum_of(d.key));
             else
@@ -348,16 +342,23 @@ struct Upsert_Visitor
             atomicOr(retry_out + (gpos >> 5), 1u << (gpos & 31));
             *retried = 1;
         }
-        seg_ins += __popc(__ballot_sync(all, r == INSERTED));
+        const uint32_t ins_m = __ballot_sync(all, r == INSERTED);
+        seg_ins += __popc(ins_m);
 
         if constexpr(!set_)
-            if((r == FOUND || r == FOUND_PENDING) && !fn.is_noop())
+        {
+            if(comm)
             {
-                if(r == FOUND_PENDING && !comm &&
-                   !await_published(Landing{val, main ? cs_of(T, at, j) : nullptr, main ? nullptr : val + 1, 0}, T.wait_polls))
+                if(r == INSERTED || ((r == FOUND || r == FOUND_PENDING) && !fn.is_noop()))
+                    fn.apply_or_init(val, d.fwd, r == INSERTED);
+            }
+            else if(r == FOUND || r == FOUND_PENDING)
+            {
+                if(r == FOUND_PENDING && !await_published(Landing{val, main ? cs_of(T, at, j) : nullptr, main ? nullptr : val + 1, 0}, T.wait_polls))
                     atomicOr(T.err, ERR_WAIT);
                 fn.apply(val, d.fwd);
             }
+        }
     }
 
     __device__ __forceinline__ void end(const uint32_t lane) { warp_flush(inserted, ins, lane); }

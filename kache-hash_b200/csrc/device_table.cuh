@@ -155,12 +155,13 @@ struct Op_Fn
         return op == OP_KEEP || op == OP_ADD || op == OP_ADD_WRAP || op == OP_OR || op == OP_MAX;
     }
 
-    __device__ __forceinline__ void apply_init(unsigned long long* w, bool) const
+    // For operations that commute: an occurrence's update, the key's first one giving it its initial value.
+    __device__ __forceinline__ void apply_or_init(unsigned long long* w, bool, const bool first) const
     {
-        if(op == OP_KEEP)
+        if(op != OP_KEEP)
+            Op_Fn<V>{op, first ? init : x, init}.apply(w, true);
+        else if(first)
             write_val<V>(w, init);
-        else
-            Op_Fn<V>{op, init, init}.apply(w, true);
     }
 
     __device__ __forceinline__ void apply(unsigned long long* w, bool) const
@@ -224,7 +225,7 @@ struct Oriented_Op_Fn
     __device__ __forceinline__ V initial(const bool fwd) const { return at(fwd)(V(0)); }
     __device__ __forceinline__ bool is_noop() const { return false; }
     __device__ __forceinline__ bool commutes() const { return op == OP_ADD || op == OP_ADD_WRAP || op == OP_OR || op == OP_MAX; }
-    __device__ __forceinline__ void apply_init(unsigned long long* w, const bool fwd) const { at(fwd).apply(w, fwd); }
+    __device__ __forceinline__ void apply_or_init(unsigned long long* w, const bool fwd, bool) const { at(fwd).apply(w, fwd); }
     __device__ __forceinline__ void apply(unsigned long long* w, const bool fwd) const { at(fwd).apply(w, fwd); }
 };
 
@@ -237,7 +238,7 @@ struct User_Fn
     __device__ __forceinline__ V initial(bool) const { return val; }
     __device__ __forceinline__ bool is_noop() const { return false; }
     __device__ __forceinline__ bool commutes() const { return false; }
-    __device__ __forceinline__ void apply_init(unsigned long long* w, bool) const { write_val<V>(w, val); }
+    __device__ __forceinline__ void apply_or_init(unsigned long long* w, bool, bool) const { cas_update<V>(w, f); }
     __device__ __forceinline__ void apply(unsigned long long* w, bool) const { cas_update<V>(w, f); }
 };
 
@@ -249,7 +250,7 @@ struct User_Oriented_Fn
     __device__ __forceinline__ V initial(const bool fwd) const { return f(V(), fwd); }
     __device__ __forceinline__ bool is_noop() const { return false; }
     __device__ __forceinline__ bool commutes() const { return false; }
-    __device__ __forceinline__ void apply_init(unsigned long long* w, const bool fwd) const { write_val<V>(w, f(V(), fwd)); }
+    __device__ __forceinline__ void apply_or_init(unsigned long long* w, const bool fwd, bool) const { apply(w, fwd); }
     __device__ __forceinline__ void apply(unsigned long long* w, const bool fwd) const
     {
         const F& g = f;
@@ -404,10 +405,10 @@ __device__ __forceinline__ uint32_t upsert_chain(const Dev_Table& T, const uint6
     return r;
 }
 
-// The upsert chain past the first probe, for the lanes of a whole warp that `want` it (no two with the same key). On
-// entry such a lane's `at` is its primary bucket, `j` that bucket's first empty slot as probed (B if full) and `r`
-// NONE; every other lane's `at` is its k-mer's primary bucket, or no_bucket. On return r is as upsert_chain's, with the
-// slot at (at, j), or with at = no_bucket at overflow slot `ov_i`.
+// The upsert chain of the lanes of a whole warp that `want` it (no two with the same key). On entry `at` is a lane's
+// primary bucket (no_bucket in lanes without a k-mer). On return r is as upsert_chain's, with the slot at (at, j), or with
+// at = no_bucket at overflow slot `ov_i`. All stages of the chain go through one loop, with one probe and one swap in it:
+// the kernel's code is large enough that its size costs time (unrolled twice, 40M upserts took 1.28 ms against 1.04).
 //
 // The lanes hold consecutive k-mers, so the new ones come in runs of neighbours that share a minimizer, hence a bucket.
 // A run claims together: its lane of rank i tries slot j + i at once with the others, where lanes trying the same slot
@@ -427,85 +428,81 @@ __device__ __forceinline__ void warp_claim(const Dev_Table& T, const unsigned lo
 {
     constexpr uint32_t all = 0xFFFFFFFFu;
     const uint32_t le = all >> (31 - lane), lt = le >> 1;
-    for(uint32_t stage = 0; ; ++stage)
+    uint32_t stage = 0;         // 0: the primary bucket; 1 and 2: the secondary ones.
+    bool probe = want;
+    for(;;)
     {
-        for(;;)
+        if(probe)
+            r = bucket_probe<set_>(T, at, key_st, c, j);
+        const bool open = want && r == NONE, in = open && j < B;
+        if(!__any_sync(all, open))
+            return;
+        probe = open && !in && stage < 2;
+        if(probe)
         {
-            const bool in = want && r == NONE && j < B;
-            const uint32_t in_m = __ballot_sync(all, in);
-            if(in_m == 0)
-                break;
-            // This lane's run: the lanes from the last change of bucket on, up to the next.
-            const uint32_t left = __shfl_up_sync(all, at, 1);
-            const uint32_t heads = __ballot_sync(all, lane == 0 || at != left);
-            const uint32_t from = all << (31 - __clz(heads & le)), next = heads & ~le;
-            const uint32_t run = next ? from & ((next & (0u - next)) - 1) : from;
-            // Lanes of a run whose probes saw different first empty slots do not claim together: those unlike the
-            // first probe afresh.
-            const uint32_t first = __shfl_sync(all, j, in ? __ffs(in_m & run) - 1 : lane);
-            const bool ok = in && j == first;
-            const uint32_t ok_run = __ballot_sync(all, ok) & run;
-            const uint32_t rank = __popc(ok_run & lt), slot = j + rank;
-            const bool tries = ok && (rank == 0 || slot < B - 1);
-            unsigned long long cur = 0;
-            uint32_t got = slot;
-            if(tries)
+            // A full bucket: a primary one's spill filter is marked before the key goes beyond it.
+            if(stage == 0)
             {
-                cur = atomicCAS(key_word<set_>(T, at, slot), 0ull, key_st);
-                if(cur == 0)
-                    r = INSERTED;
-                else if(cur == key_st)
-                    r = FOUND_PENDING;
+                const uint32_t fp = filter_pos(h);
+                uint32_t* sw = T.spill + uint64_t(at) * 8 + (fp >> 5);
+                const uint32_t bit = 1u << (fp & 31);
+                if(!(__ldcg(sw) & bit))
+                    atomicOr(sw, bit);
             }
-            const uint32_t tried = __popc(__ballot_sync(all, tries) & run);
-            // Where a swap lost, its run's lanes compare their keys with what it showed: every run at once, lane by lane
-            // from its first.
-            const uint32_t lost = __ballot_sync(all, tries && r == NONE);
-            if(lost)
-                for(uint32_t left_m = run & lost; __any_sync(all, left_m); left_m &= left_m - 1)
-                {
-                    const uint32_t s = left_m ? __ffs(left_m) - 1 : lane;
-                    const unsigned long long k_s = __shfl_sync(all, cur, s);
-                    const uint32_t slot_s = __shfl_sync(all, slot, s);
-                    if(ok && left_m && k_s == key_st && (r == NONE || slot_s < got))
-                    {
-                        if(r == INSERTED)
-                            *reinterpret_cast<volatile unsigned long long*>(key_word<set_>(T, at, got)) = hole_key;
-                        r = FOUND_PENDING, got = slot_s;
-                    }
-                }
-            if(ok)
-                j = r == NONE ? j + tried : got;
-            else if(in)
-                r = bucket_probe<set_>(T, at, key_st, c, j);
+            at = stage == 0 ? second_bucket(h, T.cap) : third_bucket(h, T.cap);
+            ++stage;
+        }
+        else if(open && !in)
+        {
+            at = no_bucket;
+            r = overflow_upsert(T, key_st, ov_i);
         }
 
-        const bool full = want && r == NONE;
-        if(!__any_sync(all, full))
-            return;
-        if(full)
+        const uint32_t in_m = __ballot_sync(all, in);
+        if(in_m == 0)
+            continue;
+        // This lane's run: the lanes from the last change of bucket on, up to the next.
+        const uint32_t left = __shfl_up_sync(all, at, 1);
+        const uint32_t heads = __ballot_sync(all, lane == 0 || at != left);
+        const uint32_t from = all << (31 - __clz(heads & le)), next = heads & ~le;
+        const uint32_t run = next ? from & ((next & (0u - next)) - 1) : from;
+        // Lanes of a run whose probes saw different first empty slots do not claim together: those unlike the first
+        // probe afresh.
+        const uint32_t first = __shfl_sync(all, j, in ? __ffs(in_m & run) - 1 : lane);
+        const bool ok = in && j == first;
+        const uint32_t ok_run = __ballot_sync(all, ok) & run;
+        const uint32_t rank = __popc(ok_run & lt), slot = j + rank;
+        const bool tries = ok && (rank == 0 || slot < B - 1);
+        unsigned long long cur = 0;
+        uint32_t got = slot;
+        if(tries)
         {
-            if(stage == 2)
-            {
-                at = no_bucket;
-                r = overflow_upsert(T, key_st, ov_i);
-            }
-            else
-            {
-                if(stage == 0)
-                {
-                    const uint32_t fp = filter_pos(h);
-                    uint32_t* sw = T.spill + uint64_t(at) * 8 + (fp >> 5);
-                    const uint32_t bit = 1u << (fp & 31);
-                    if(!(__ldcg(sw) & bit))
-                        atomicOr(sw, bit);
-                }
-                at = stage == 0 ? second_bucket(h, T.cap) : third_bucket(h, T.cap);
-                r = bucket_probe<set_>(T, at, key_st, c, j);
-            }
+            cur = atomicCAS(key_word<set_>(T, at, slot), 0ull, key_st);
+            if(cur == 0)
+                r = INSERTED;
+            else if(cur == key_st)
+                r = FOUND_PENDING;
         }
-        if(stage == 2)
-            return;
+        const uint32_t tried = __popc(__ballot_sync(all, tries) & run);
+        // Where a swap lost, its run's lanes compare their keys with what it showed: every run at once, lane by lane
+        // from its first.
+        const uint32_t lost = __ballot_sync(all, tries && r == NONE);
+        if(lost)
+            for(uint32_t left_m = run & lost; __any_sync(all, left_m); left_m &= left_m - 1)
+            {
+                const uint32_t s = left_m ? __ffs(left_m) - 1 : lane;
+                const unsigned long long k_s = __shfl_sync(all, cur, s);
+                const uint32_t slot_s = __shfl_sync(all, slot, s);
+                if(ok && left_m && k_s == key_st && (r == NONE || slot_s < got))
+                {
+                    if(r == INSERTED)
+                        *reinterpret_cast<volatile unsigned long long*>(key_word<set_>(T, at, got)) = hole_key;
+                    r = FOUND_PENDING, got = slot_s;
+                }
+            }
+        if(ok)
+            j = r == NONE ? j + tried : got;
+        probe = probe || (in && !ok);
     }
 }
 
