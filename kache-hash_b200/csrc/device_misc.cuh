@@ -324,32 +324,21 @@ __global__ void get_kernel(const Dev_Table T, const uint64_t* keys, const uint64
     out[2 * i + 1] = (v && !set_) ? static_cast<unsigned long long>(read_val<V>(v)) : 0ull;
 }
 
-// Device-side batch preparation, for batches already in HBM: per sequence, its positions and segments.
-static __global__ void batch_counts_kernel(const uint64_t* off, const uint64_t n, const int k, const uint32_t seg_len, uint64_t* npos, uint64_t* nseg, unsigned int* too_long)
-{
-    const uint64_t q = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if(q >= n)
-        return;
-    const uint64_t len = off[q + 1] - off[q];
-    const uint64_t p = len >= uint64_t(k) ? len - k + 1 : 0;
-    npos[q] = p;
-    nseg[q] = (p + seg_len - 1) / seg_len;
-    if(nseg[q] > max_seg_index + 1)
-        atomicOr(too_long, 1u);
-}
+// The staging of a device batch, or of several run as one: its sequences are counted, the counts summed, and its segments
+// listed, with no host read in between. The launch behind it takes its number of segments from ctr[6]: none if the batch
+// has more segments or positions than the caller made room for, which the host reads with the launch's results. Up to
+// small_stage_max sequences take one block (stage_small_kernel), more take two launches (stage_count_kernel,
+// stage_list_kernel). A million sequences take 26 and 30 us; a counting kernel, two scans, a search per segment and the
+// host's read of the counts before it took 45 us of kernels and about 30 of waiting.
+constexpr uint32_t small_stage_max = 4096;      // Sequences of a block (at most 4 per thread).
+constexpr uint32_t small_segs_max = 16384;      // Segments that it lists.
+constexpr uint32_t stage_block = 1024;
 
-// The staging of a small device batch, or of several run as one, in one block of 1024 threads: it counts, fits the segment
-// length (fitted_seg_len, then eight times longer while the longest sequence would have more segments than a list entry
-// indexes), sums and lists the segments, in place of a counting kernel, two scans, a listing kernel and the host reading
-// the counts in between. The launch behind it takes its number of segments from ctr[6]: none if the batch has more
-// segments or positions than the caller made room for, which the host reads with the launch's results.
-constexpr uint32_t small_stage_max = 4096;      // Sequences (at most 4 per thread).
-constexpr uint32_t small_segs_max = 16384;      // Segments listed by the block.
-
-struct Small_Stage
+struct Stage
 {
-    // One batch's n + 1 offsets; or (null) several batches, 8 words each as batches_list_kernel takes them, with the arrays
-    // it fills, and each batch's first merged position.
+    // One batch's n + 1 offsets; or (null) several batches, 8 words each -- bases, offsets, sequences, first merged
+    // sequence, out0, out1, out2, 0 -- in batch order, with, to be filled, the address of each merged sequence's first
+    // base, its batch, and each batch's first merged position.
     const uint64_t* off;
     const uint64_t* desc;
     uint64_t count;
@@ -361,12 +350,46 @@ struct Small_Stage
     int k;
     uint32_t sms;
     uint64_t max_segs, max_pos;
-    uint64_t *pos_off, *seg_off;    // n + 1 sums each.
+    uint64_t *npos, *pos_off, *seg_off;     // Positions of each sequence; n + 1 sums of positions and of segments.
+    unsigned long long* blocks;     // Two words per block of stage_count_kernel: the positions and segments before it.
     Segment* segs;
-    unsigned long long* ctr;    // [0] and the low half of [2] are zeroed; [3..6]: positions, segments, segment length, segments to run.
+    unsigned long long* ctr;    // [0] and the low half of [2] are zeroed; [3..6]: positions, segments, segment length, segments to run; [7]: zero between launches.
     unsigned long long* zero;   // zero_n words zeroed.
     uint64_t zero_n;
 };
+
+// The length of sequence q. Of several batches, `lo` is a batch at or before q's (or, at first, no less than 0 with
+// `seek`), and becomes q's; the sequence's entries are filled.
+__device__ __forceinline__ uint64_t stage_length(const Stage& a, const uint64_t q, uint64_t& lo, const bool seek)
+{
+    if(a.desc == nullptr)
+        return a.off[q + 1] - a.off[q];
+    if(seek)
+        for(uint64_t hi = a.count; hi - lo > 1; )   // The last batch whose first merged sequence is at or before q.
+        {
+            const uint64_t mid = (lo + hi) / 2;
+            if(a.desc[8 * mid + 3] <= q)
+                lo = mid;
+            else
+                hi = mid;
+        }
+    while(lo + 1 < a.count && a.desc[8 * (lo + 1) + 3] <= q)
+        ++lo;
+    const uint64_t* d = a.desc + 8 * lo;
+    const uint64_t j = q - d[3], b0 = reinterpret_cast<const uint64_t*>(d[1])[j];
+    a.addr[q] = d[0] + b0;
+    a.batch_of[q] = static_cast<uint32_t>(lo);
+    if(a.zero_out0)
+        reinterpret_cast<uint64_t*>(d[4])[j] = 0;
+    return reinterpret_cast<const uint64_t*>(d[1])[j + 1] - b0;
+}
+
+// Segment number i of sequence q, which starts at `first` of its np positions.
+__device__ __forceinline__ Segment stage_segment(const Stage& a, const uint64_t q, const uint64_t i, const uint64_t np, const uint64_t first, const uint64_t seg_len)
+{
+    const uint64_t p0 = i * seg_len;
+    return Segment{(a.desc ? a.addr[q] : a.off[q]) + p0, first + p0, q, static_cast<uint32_t>(min(np - p0, seg_len)), a.desc ? a.batch_of[q] : 0};
+}
 
 // The inclusive sum of x over the block's threads in order; `warps` is 32 words of shared memory.
 __device__ __forceinline__ unsigned long long block_sum(unsigned long long x, unsigned long long* warps)
@@ -379,6 +402,7 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long x, un
         if(lane >= static_cast<uint32_t>(o))
             x += a;
     }
+    __syncthreads();    // The words' last use is over.
     if(lane == 31)
         warps[wid] = x;
     __syncthreads();
@@ -398,64 +422,27 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long x, un
     return x + (wid ? warps[wid - 1] : 0);
 }
 
-static __global__ void __launch_bounds__(1024) stage_small_kernel(const Small_Stage a)
+static __global__ void __launch_bounds__(stage_block) stage_small_kernel(const Stage a)
 {
-    __shared__ unsigned long long wp[32], ws[32], wtop[32];
+    __shared__ unsigned long long wp[32], ws[32];
     __shared__ uint32_t first_seg[small_stage_max + 1];
     const uint32_t t = threadIdx.x;
-    const uint64_t per = (a.n + 1023) / 1024, q0 = min(a.n, uint64_t(t) * per);
+    const uint64_t per = (a.n + stage_block - 1) / stage_block, q0 = min(a.n, uint64_t(t) * per);
     const uint32_t mine = static_cast<uint32_t>(min(a.n, q0 + per) - q0);
-    uint64_t np[4];
-    unsigned long long P = 0, S = 0, top = 0;
-    uint64_t lo = 0;
-    if(a.desc && mine)
-        for(uint64_t hi = a.count; hi - lo > 1; )   // The last batch whose first merged sequence is at or before q0.
-        {
-            const uint64_t mid = (lo + hi) / 2;
-            if(a.desc[8 * mid + 3] <= q0)
-                lo = mid;
-            else
-                hi = mid;
-        }
+    uint64_t np[4], lo = 0;
+    unsigned long long P = 0, S = 0;
 #pragma unroll
     for(uint32_t i = 0; i < 4; ++i)
         if(i < mine)
         {
-            const uint64_t q = q0 + i;
-            uint64_t len;
-            if(a.desc)
-            {
-                while(lo + 1 < a.count && a.desc[8 * (lo + 1) + 3] <= q)
-                    ++lo;
-                const uint64_t* d = a.desc + 8 * lo;
-                const uint64_t j = q - d[3], b0 = reinterpret_cast<const uint64_t*>(d[1])[j];
-                len = reinterpret_cast<const uint64_t*>(d[1])[j + 1] - b0;
-                a.addr[q] = d[0] + b0;
-                a.batch_of[q] = static_cast<uint32_t>(lo);
-                if(a.zero_out0)
-                    reinterpret_cast<uint64_t*>(d[4])[j] = 0;
-            }
-            else
-                len = a.off[q + 1] - a.off[q];
+            const uint64_t len = stage_length(a, q0 + i, lo, i == 0);
             np[i] = len >= uint64_t(a.k) ? len - a.k + 1 : 0;
-            P += np[i], top = max(top, static_cast<unsigned long long>(np[i]));
+            P += np[i];
         }
-    for(uint64_t i = t; i < a.zero_n; i += 1024)
+    for(uint64_t i = t; i < a.zero_n; i += stage_block)
         a.zero[i] = 0;
-#pragma unroll
-    for(int o = 16; o > 0; o >>= 1)
-        top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-    if((t & 31) == 0)
-        wtop[t >> 5] = top;
     unsigned long long bp = block_sum(P, wp) - P;
-    const uint64_t total = wp[31];
-    unsigned long long longest = 0;
-#pragma unroll
-    for(int i = 0; i < 32; ++i)
-        longest = max(longest, wtop[i]);
-    uint64_t seg_len = fitted_seg_len(total, a.sms);
-    while((longest + seg_len - 1) / seg_len > max_seg_index + 1)
-        seg_len *= 8;
+    const uint64_t total = wp[31], seg_len = fitted_seg_len(total, a.sms);
 #pragma unroll
     for(uint32_t i = 0; i < 4; ++i)
         if(i < mine)
@@ -474,14 +461,14 @@ static __global__ void __launch_bounds__(1024) stage_small_kernel(const Small_St
                 a.pos_base[a.batch_of[q]] = bp;
             bp += np[i], bs += (np[i] + seg_len - 1) / seg_len;
         }
-    if(t == 1023)
+    if(t == stage_block - 1)
     {
         a.pos_off[a.n] = total, a.seg_off[a.n] = nsegs;
         a.ctr[3] = total, a.ctr[4] = nsegs, a.ctr[5] = seg_len, a.ctr[6] = run;
         a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0;
     }
     __syncthreads();
-    for(uint32_t i = t; i < run; i += 1024)
+    for(uint32_t i = t; i < run; i += stage_block)
     {
         uint32_t l = 0, h = static_cast<uint32_t>(a.n);     // The last q with first_seg[q] <= i.
         while(h - l > 1)
@@ -492,12 +479,76 @@ static __global__ void __launch_bounds__(1024) stage_small_kernel(const Small_St
             else
                 h = mid;
         }
-        const uint64_t p0 = (i - first_seg[l]) * seg_len, first = a.pos_off[l] + p0;
-        a.segs[i] = Segment{(a.desc ? a.addr[l] : a.off[l]) + p0, first, l, static_cast<uint32_t>(min(a.pos_off[l + 1] - first, seg_len)), a.desc ? a.batch_of[l] : 0};
+        const uint64_t first = a.pos_off[l];
+        a.segs[i] = stage_segment(a, l, i - first_seg[l], a.pos_off[l + 1] - first, first, seg_len);
     }
 }
 
-// Lists the segments, one thread per segment: its sequence by binary search in seg_off[0..n] (exclusive sums of
+// Larger batches, first launch: each block counts stage_block sequences, and the block that ends last sums the blocks'
+// counts. (A batch of this many sequences has a warp's segment of seg_positions for each.)
+static __global__ void __launch_bounds__(stage_block) stage_count_kernel(const Stage a)
+{
+    __shared__ unsigned long long wp[32], ws[32];
+    __shared__ bool last;
+    const uint32_t t = threadIdx.x;
+    const uint64_t q = uint64_t(blockIdx.x) * stage_block + t;
+    uint64_t np = 0, lo = 0;
+    if(q < a.n)
+    {
+        const uint64_t len = stage_length(a, q, lo, true);
+        np = len >= uint64_t(a.k) ? len - a.k + 1 : 0;
+        a.npos[q] = np;
+    }
+    for(uint64_t i = q; i < a.zero_n; i += uint64_t(gridDim.x) * stage_block)
+        a.zero[i] = 0;
+    block_sum(np, wp);
+    block_sum((np + seg_positions - 1) / seg_positions, ws);
+    if(t == 0)
+    {
+        __stcg(a.blocks + 2 * blockIdx.x, wp[31]), __stcg(a.blocks + 2 * blockIdx.x + 1, ws[31]);
+        __threadfence();
+        last = atomicAdd(a.ctr + 7, 1ull) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if(!last)
+        return;
+    unsigned long long P = 0, S = 0;
+    for(uint64_t b0 = 0; b0 < gridDim.x; b0 += stage_block)
+    {
+        const uint64_t b = b0 + t;
+        const unsigned long long p = b < gridDim.x ? __ldcg(a.blocks + 2 * b) : 0, s = b < gridDim.x ? __ldcg(a.blocks + 2 * b + 1) : 0;
+        const unsigned long long p1 = block_sum(p, wp), s1 = block_sum(s, ws);
+        if(b < gridDim.x)
+            a.blocks[2 * b] = P + p1 - p, a.blocks[2 * b + 1] = S + s1 - s;
+        P += wp[31], S += ws[31];
+    }
+    if(t == 0)
+    {
+        a.pos_off[a.n] = P, a.seg_off[a.n] = S;
+        a.ctr[3] = P, a.ctr[4] = S, a.ctr[5] = seg_positions, a.ctr[6] = S <= a.max_segs && P <= a.max_pos ? S : 0;
+        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[7] = 0;
+    }
+}
+
+// Second launch: each block sums its own sequences and lists their segments.
+static __global__ void __launch_bounds__(stage_block) stage_list_kernel(const Stage a)
+{
+    __shared__ unsigned long long wp[32], ws[32];
+    const uint64_t q = uint64_t(blockIdx.x) * stage_block + threadIdx.x;
+    const uint64_t np = q < a.n ? a.npos[q] : 0, ns = (np + seg_positions - 1) / seg_positions;
+    const unsigned long long first = a.blocks[2 * blockIdx.x] + block_sum(np, wp) - np, first_seg = a.blocks[2 * blockIdx.x + 1] + block_sum(ns, ws) - ns;
+    if(q >= a.n)
+        return;
+    a.pos_off[q] = first, a.seg_off[q] = first_seg;
+    if(a.desc && a.desc[8 * uint64_t(a.batch_of[q]) + 3] == q)
+        a.pos_base[a.batch_of[q]] = first;
+    if(a.ctr[6])
+        for(uint64_t i = 0; i < ns; ++i)
+            a.segs[first_seg + i] = stage_segment(a, q, i, np, first, seg_positions);
+}
+
+// Lists the segments of a staged batch that had more of them than its listing took, one thread per segment: its sequence by binary search in seg_off[0..n] (exclusive sums of
 // segments per sequence), so that long sequences' many segments are listed in parallel. Sequence q's bases are at offset
 // off[q], or with `addr` at the address addr[q], where it is of batch batch_of[q].
 static __global__ void segs_kernel(const uint64_t* seg_off, const uint64_t* pos_off, const uint64_t* off, const uint64_t* addr, const uint32_t* batch_of, const uint64_t n,
@@ -518,42 +569,6 @@ static __global__ void segs_kernel(const uint64_t* seg_off, const uint64_t* pos_
         const uint64_t p0 = (i - seg_off[lo]) * seg_len, first = pos_off[lo] + p0;
         segs[i] = Segment{(addr ? addr[lo] : off[lo]) + p0, first, lo, static_cast<uint32_t>(min(pos_off[lo + 1] - first, static_cast<uint64_t>(seg_len))), batch_of ? batch_of[lo] : 0};
     }
-}
-
-// Several device batches run as one call. desc holds 8 words per batch -- bases, offsets, sequences, first merged
-// sequence, out0, out1, out2, 0 -- in batch order. For merged sequence q: its batch, its length (the merged offsets are
-// the lengths' sums) and the device address of its first base; with `zero`, its word of the batch's out0 is zeroed.
-static __global__ void batches_list_kernel(const uint64_t* desc, const uint64_t count, const uint64_t N, uint64_t* lens,
-                                           uint64_t* addr, uint32_t* batch_of, const bool zero)
-{
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for(uint64_t q = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < N; q += stride)
-    {
-        uint64_t lo = 0, hi = count;    // The last batch whose first merged sequence is at or before q: never empty.
-        while(hi - lo > 1)
-        {
-            const uint64_t mid = (lo + hi) / 2;
-            if(desc[8 * mid + 3] <= q)
-                lo = mid;
-            else
-                hi = mid;
-        }
-        const uint64_t* off = reinterpret_cast<const uint64_t*>(desc[8 * lo + 1]);
-        const uint64_t j = q - desc[8 * lo + 3], a = off[j];
-        lens[q] = off[j + 1] - a;
-        addr[q] = desc[8 * lo] + a;
-        batch_of[q] = static_cast<uint32_t>(lo);
-        if(zero)
-            reinterpret_cast<uint64_t*>(desc[8 * lo + 4])[j] = 0;
-    }
-}
-
-// The merged position of each batch's first k-mer.
-static __global__ void batches_pos_kernel(const uint64_t* desc, const uint64_t count, const uint64_t* pos_off, uint64_t* pos_base)
-{
-    const uint64_t b = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if(b < count)
-        pos_base[b] = pos_off[desc[8 * b + 3]];
 }
 
 }

@@ -13,8 +13,6 @@
 #include "host_copy.hpp"
 #include "kache_b200.h"
 
-#include <cub/device/device_scan.cuh>
-
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -382,7 +380,7 @@ class Engine final : public kache_table
             check(cudaEventCreateWithFlags(&ev_bases_, cudaEventDisableTiming), "event");
     }
     Pinned_Buf pin_piece_;
-    Dev_Buf dbatch_, dout_, dretry_a_, dretry_b_, dscan_, dtmp_;
+    Dev_Buf dbatch_, dout_, dretry_a_, dretry_b_, dtmp_;
     Dev_Buf dhost_;     // A page-locked host batch's bases and offsets, copied as they lie.
     Dev_Buf dmulti_;    // Several device batches run as one: their descriptors and the merged sequence list.
     Pinned_Buf pin_multi_;
@@ -580,17 +578,6 @@ class Engine final : public kache_table
 
     // ---- Batches ----
 
-    // Positions per segment: 512 (16 rows of a warp), halved down to one row while a batch of `total` positions would
-    // give each SM fewer than 32 warps; eight times longer while the longest sequence, of `longest` positions, would
-    // have more segments than a list entry indexes.
-    uint32_t seg_len_for(const uint64_t longest, const uint64_t total) const
-    {
-        uint64_t s = fitted_seg_len(total, static_cast<uint32_t>(sm_count_));
-        while((longest + s - 1) / s > max_seg_index + 1)
-            s *= 8;
-        return static_cast<uint32_t>(s);
-    }
-
     // Stages a host batch. With `defer_bases` (a lookup in pieces), a batch laid end to end in page-locked memory is
     // listed from its offsets alone and its bases are left for the caller to copy (to bi.b.bases), piece by piece;
     // bi.host_bases is then set.
@@ -691,7 +678,7 @@ class Engine final : public kache_table
         }
         if(n >= host_list_max)
             return stage_gathered(seqs, lens, n, bytes);
-        const uint32_t seg_len = seg_len_for(max_pos, all_pos);
+        const uint32_t seg_len = fitted_seg_len(all_pos, static_cast<uint32_t>(sm_count_));
         uint64_t nsegs = 0;
         for(size_t i = 0; i < n; ++i)
         {
@@ -781,107 +768,84 @@ class Engine final : public kache_table
         return stage_dev(reinterpret_cast<const uint8_t*>(d), reinterpret_cast<const uint64_t*>(d + o_off), n);
     }
 
-    // A small device batch's staging arguments: the offsets of one, or none for the caller to set several.
-    Small_Stage small_stage(const uint64_t* off, const uint64_t n)
+    // A device batch's staging arguments: the offsets of one, or none for the caller to set several.
+    Stage new_stage(const uint64_t* off, const uint64_t n)
     {
-        dtmp_.ensure(2 * (n + 1) * 8);
-        Small_Stage a{};
-        a.off = off, a.n = n, a.k = k, a.sms = static_cast<uint32_t>(sm_count_);
-        a.pos_off = dtmp_.as<uint64_t>(), a.seg_off = a.pos_off + (n + 1), a.ctr = ctr();
+        const uint64_t blocks = (n + stage_block - 1) / stage_block;
+        dtmp_.ensure((3 * (n + 1) + 2 * blocks) * 8);
+        Stage a{};
+        a.off = off, a.n = n, a.k = k, a.sms = static_cast<uint32_t>(sm_count_), a.max_pos = ~0ull;
+        a.npos = dtmp_.as<uint64_t>(), a.pos_off = a.npos + (n + 1), a.seg_off = a.pos_off + (n + 1);
+        a.blocks = reinterpret_cast<unsigned long long*>(a.seg_off + (n + 1)), a.ctr = ctr();
         return a;
     }
 
-    // stage_dev for a batch of at most small_stage_max sequences: one block counts, fits the segment length and sums, one
-    // kernel lists.
-    Batch_Info stage_dev_small(const uint8_t* bases, const uint64_t* off, const uint64_t n, const uint64_t* addr, const uint32_t* batch_of)
+    // Counts and lists a batch's segments on the device.
+    void launch_stage(Stage& a)
     {
-        const Small_Stage a = small_stage(off, n);
-        launch(K_OTHER, [&](){ stage_small_kernel<<<1, 1024, 0, stream_>>>(a); });
-        uint64_t* h = pin_ctr_.as<uint64_t>(32);
-        check(cudaMemcpyAsync(h, ctr() + 3, 24, cudaMemcpyDeviceToHost, stream_), "D2H");
-        sync();
-        small_fits_ = h[1] <= small_segs_max;
-        return list_dev(bases, off, addr, batch_of, n, a.pos_off, a.seg_off, h[0], h[1], static_cast<uint32_t>(h[2]));
+        dbatch_.ensure((a.n <= small_stage_max ? small_segs_max : a.n + a.n / 8 + 1024) * sizeof(Segment));
+        a.segs = dbatch_.as<Segment>();
+        a.max_segs = a.n <= small_stage_max ? small_segs_max : dbatch_.bytes / sizeof(Segment);
+        const unsigned blocks = static_cast<unsigned>((a.n + stage_block - 1) / stage_block);
+        if(a.n <= small_stage_max)
+            launch(K_OTHER, [&](){ stage_small_kernel<<<1, stage_block, 0, stream_>>>(a); });
+        else
+        {
+            launch(K_OTHER, [&](){ stage_count_kernel<<<blocks, stage_block, 0, stream_>>>(a); });
+            launch(K_OTHER, [&](){ stage_list_kernel<<<blocks, stage_block, 0, stream_>>>(a); });
+        }
     }
 
-    // Whether to run a batch of n sequences by run_small: the last small batch had no more segments than its block lists.
+    // Whether the last batch of few sequences had no more segments than its block lists.
     bool small_fits_ = true;
-    bool small(const uint64_t n) const { return n > 0 && n <= small_stage_max && small_fits_; }
 
-    // Stages a small batch and runs the visitor over it with no host read in between (stage_small_kernel); returns the
-    // counters, of which [4] and [6] are equal if the batch ran. The launch's grid fills the GPU, its segments being
-    // unknown here.
-    template <typename Vis> const unsigned long long* run_small(const uint32_t kind, const uint8_t* bases, Small_Stage a, const Vis& vis)
+    // Whether to run a batch of n sequences directly (run_staged) rather than after the host has read its counts.
+    bool direct(const uint64_t n) const { return n > 0 && (n > small_stage_max || small_fits_); }
+
+    // Stages a batch and runs the visitor over it with no host read in between; returns the counters, of which [4] and [6]
+    // are equal if the batch ran. The launch's grid is made for the segments that are likely, as their number is unknown
+    // here.
+    template <typename Vis> const unsigned long long* run_staged(const uint32_t kind, const uint8_t* bases, Stage& a, const Vis& vis)
     {
-        dbatch_.ensure(small_segs_max * sizeof(Segment));
-        a.segs = dbatch_.as<Segment>(), a.max_segs = small_segs_max;
-        launch(K_OTHER, [&](){ stage_small_kernel<<<1, 1024, 0, stream_>>>(a); });
+        launch_stage(a);
         launch(kind, [&]()
         {
-            stream_kernel<k, l, Vis><<<static_cast<unsigned>(sm_count_) * Vis::min_blocks, 32 * stream_warps, 0, stream_>>>(Dev_Batch{bases, a.segs}, 0, 0, ctr() + 6, vis);
+            const int blocks = a.n <= small_stage_max ? sm_count_ * Vis::min_blocks : grid_for(a.n, stream_warps);
+            stream_kernel<k, l, Vis><<<blocks, 32 * stream_warps, 0, stream_>>>(Dev_Batch{bases, a.segs}, 0, 0, ctr() + 6, vis);
         });
         const unsigned long long* c = read_ctr(7);
-        small_fits_ = c[4] <= small_segs_max;
+        if(a.n <= small_stage_max)
+            small_fits_ = c[4] <= small_segs_max;
         return c;
     }
 
-    // Lists the segments of a batch whose positions and segments are counted.
-    Batch_Info list_dev(const uint8_t* bases, const uint64_t* off, const uint64_t* addr, const uint32_t* batch_of, const uint64_t n, const uint64_t* pos_off,
-                        const uint64_t* seg_off, const uint64_t total_pos, const uint64_t nsegs, const uint32_t seg_len)
+    // Prepares a batch already in device memory (or several run as one, their bases' addresses in their segments).
+    Batch_Info stage_dev(const uint8_t* bases, Stage a)
     {
-        dbatch_.ensure((nsegs + 1) * sizeof(Segment));
-        if(nsegs > 0)
-            launch(K_OTHER, [&](){ segs_kernel<<<grid_for((nsegs + 31) / 32, 8), 256, 0, stream_>>>(seg_off, pos_off, off, addr, batch_of, n, nsegs, seg_len, dbatch_.as<Segment>()); });
         Batch_Info bi;
+        bi.n = a.n;
+        if(a.n == 0)
+            return bi;
+        a.max_pos = ~0ull;
+        launch_stage(a);
+        const unsigned long long* c = read_ctr(7);
+        const uint64_t nsegs = c[4], run = c[6];
+        if(a.n <= small_stage_max)
+            small_fits_ = nsegs <= small_segs_max;
+        bi.nsegs = nsegs, bi.total_pos = c[3], bi.off = a.off, bi.pos_off = a.pos_off, bi.seg_off = a.seg_off;
+        if(run != nsegs)
+        {
+            const uint32_t seg_len = static_cast<uint32_t>(c[5]);
+            dbatch_.ensure(nsegs * sizeof(Segment));
+            launch(K_OTHER, [&]()
+            {
+                segs_kernel<<<grid_for((nsegs + 31) / 32, 8), 256, 0, stream_>>>(a.seg_off, a.pos_off, a.off, a.addr, a.batch_of, a.n, nsegs, seg_len, dbatch_.as<Segment>());
+            });
+        }
         bi.b = Dev_Batch{bases, dbatch_.as<Segment>()};
-        bi.n = n, bi.nsegs = nsegs, bi.total_pos = total_pos;
-        bi.off = off, bi.pos_off = pos_off, bi.seg_off = seg_off;
         return bi;
     }
-
-    // Prepares a batch already in device memory: positions and segments computed on the device. With `addr`, sequence q's
-    // bases are at the device address addr[q], of batch batch_of[q], and off only lays the lengths end to end.
-    Batch_Info stage_dev(const uint8_t* bases, const uint64_t* off, const uint64_t n, const uint64_t* addr = nullptr,
-                         const uint32_t* batch_of = nullptr)
-    {
-        if(n > 0 && n <= small_stage_max)
-            return stage_dev_small(bases, off, n, addr, batch_of);
-        const size_t o_npos = 0, o_nseg = o_npos + (n + 1) * 8, o_pos = o_nseg + (n + 1) * 8, o_sego = o_pos + (n + 1) * 8;
-        const size_t head = o_sego + (n + 1) * 8;
-        dtmp_.ensure(head);
-        char* d = dtmp_.as<char>();
-        auto* npos = reinterpret_cast<uint64_t*>(d + o_npos);
-        auto* nseg = reinterpret_cast<uint64_t*>(d + o_nseg);
-        auto* pos_off = reinterpret_cast<uint64_t*>(d + o_pos);
-        auto* seg_off = reinterpret_cast<uint64_t*>(d + o_sego);
-        unsigned int* too_long = reinterpret_cast<unsigned int*>(ctr() + 3);
-        uint64_t* h = pin_ctr_.as<uint64_t>(32);
-        uint32_t seg_len = seg_positions;   // A batch of this many sequences has a warp's segment for each.
-        for(;;)
-        {
-            check(cudaMemsetAsync(too_long, 0, 4, stream_), "memset");
-            if(n > 0)
-                launch(K_OTHER, [&](){ batch_counts_kernel<<<(n + 255) / 256, 256, 0, stream_>>>(off, n, k, seg_len, npos, nseg, too_long); });
-            check(cudaMemsetAsync(pos_off, 0, 8, stream_), "memset");
-            check(cudaMemsetAsync(seg_off, 0, 8, stream_), "memset");
-            size_t tmp = 0;
-            if(n > 0)
-            {
-                check(cub::DeviceScan::InclusiveSum(nullptr, tmp, npos, pos_off + 1, static_cast<int64_t>(n), stream_), "scan");
-                dscan_.ensure(tmp);
-                check(cub::DeviceScan::InclusiveSum(dscan_.p, tmp, npos, pos_off + 1, static_cast<int64_t>(n), stream_), "scan");
-                check(cub::DeviceScan::InclusiveSum(dscan_.p, tmp, nseg, seg_off + 1, static_cast<int64_t>(n), stream_), "scan");
-            }
-            check(cudaMemcpyAsync(h, pos_off + n, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
-            check(cudaMemcpyAsync(h + 1, seg_off + n, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
-            check(cudaMemcpyAsync(h + 2, too_long, 4, cudaMemcpyDeviceToHost, stream_), "D2H");
-            sync();
-            if(static_cast<uint32_t>(h[2]) == 0)
-                break;
-            seg_len *= 8;   // A sequence has more segments than a list entry indexes.
-        }
-        return list_dev(bases, off, addr, batch_of, n, pos_off, seg_off, h[0], h[1], seg_len);
-    }
+    Batch_Info stage_dev(const uint8_t* bases, const uint64_t* off, const uint64_t n) { return stage_dev(bases, new_stage(off, n)); }
 
     // Runs the visitor over segments [sb, se) of a batch, a warp per segment (device_stream.cuh).
     template <typename Vis> void stream_launch(const uint32_t kind, const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Vis& vis)
@@ -1142,19 +1106,20 @@ class Engine final : public kache_table
             novelty_ = std::max(static_cast<double>(ins) / static_cast<double>(total_pos), 1e-3), novelty_seen_ = true;
     }
 
-    // Upserts a small batch by run_small, if it would fit the device table were every position a new key; returns whether
+    // Upserts a batch by run_staged, if it would fit the device table were every position a new key; returns whether
     // it did, with the keys inserted in `ins`. Otherwise nothing was done. (Not tried if the last upsert would not have
     // fitted: the batches of a stream are mostly alike.)
-    template <typename Fn> bool upsert_small(const uint32_t user, const uint8_t* bases, Small_Stage a, const Fn& fn, uint64_t& ins, unsigned long long* per = nullptr)
+    template <typename Fn> bool upsert_direct(const uint32_t user, const uint8_t* bases, Stage& a, const Fn& fn, uint64_t& ins, unsigned long long* per = nullptr)
     {
         const double room = 0.95 * static_cast<double>(T_.cap * B) - static_cast<double>(size_);
         constexpr uint64_t most = uint64_t(small_segs_max) * seg_positions;
         a.max_pos = static_cast<uint64_t>(std::clamp(room, 0.0, static_cast<double>(most)));
-        if(last_pos_ > a.max_pos)
-            return false;
+        if(!direct(a.n) || a.n > a.max_pos || last_pos_ > a.max_pos ||
+           predicted_cap(user, static_cast<uint64_t>(novelty_ * static_cast<double>(last_pos_))) > T_.cap)
+            return false;   // The last one also where the table is to grow ahead of the call (run_upsert).
         clear_retries(most / 8 + 8);
         unsigned int* retried = reinterpret_cast<unsigned int*>(ctr() + 2);
-        const unsigned long long* c = run_small(K_UPSERT, bases, a, Upsert_Visitor<set_, VT, Fn>{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per, per != nullptr});
+        const unsigned long long* c = run_staged(K_UPSERT, bases, a, Upsert_Visitor<set_, VT, Fn>{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per, per != nullptr});
         if(c[6] != c[4])
             return false;
         Batch_Info bi;
@@ -1483,9 +1448,10 @@ public:
     {
         std::lock_guard<std::mutex> g(work);
         uint64_t ins;
-        if(small(n) && upsert_small(user, b, small_stage(off, n), op_fn(op, x, init), ins))
+        Stage a = new_stage(off, n);
+        if(upsert_direct(user, b, a, op_fn(op, x, init), ins))
             return ins;
-        return run_upsert(user, stage_dev(b, off, n), op_fn(op, x, init));
+        return run_upsert(user, stage_dev(b, a), op_fn(op, x, init));
     }
 
     uint64_t upsert_oriented_dev(uint32_t user, const uint8_t* b, const uint64_t* off, uint64_t n, uint32_t op, uint64_t xf, uint64_t xr) override
@@ -1497,9 +1463,10 @@ public:
             std::lock_guard<std::mutex> g(work);
             const Oriented_Op_Fn<VT> fn{op, static_cast<VT>(xf), static_cast<VT>(xr)};
             uint64_t ins;
-            if(small(n) && upsert_small(user, b, small_stage(off, n), fn, ins))
+            Stage a = new_stage(off, n);
+            if(upsert_direct(user, b, a, fn, ins))
                 return ins;
-            return run_upsert(user, stage_dev(b, off, n), fn);
+            return run_upsert(user, stage_dev(b, a), fn);
         }
     }
 
@@ -1510,11 +1477,10 @@ public:
         else
         {
             std::lock_guard<std::mutex> g(work);
-            if(small(n))
+            if(direct(n))
             {
-                Small_Stage a = small_stage(off, n);
-                a.max_pos = ~0ull;
-                const auto* c = run_small(K_UPDATE, b, a, Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), nullptr});
+                Stage a = new_stage(off, n);
+                const auto* c = run_staged(K_UPDATE, b, a, Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), nullptr});
                 if(c[6] == c[4])
                     return c[0];
             }
@@ -1526,11 +1492,10 @@ public:
     {
         std::lock_guard<std::mutex> g(work);
         auto* v = set_ ? nullptr : static_cast<VT*>(values);
-        if(small(n))
+        if(direct(n))
         {
-            Small_Stage a = small_stage(off, n);
-            a.max_pos = ~0ull;
-            const auto* c = run_small(K_LOOKUP, b, a, Lookup_Visitor<set_, VT>{T_, found, v, fwd});
+            Stage a = new_stage(off, n);
+            const auto* c = run_staged(K_LOOKUP, b, a, Lookup_Visitor<set_, VT>{T_, found, v, fwd});
             if(c[6] == c[4])
                 return;
         }
@@ -1602,11 +1567,11 @@ public:
     {
         std::lock_guard<std::mutex> g(work);
         auto* out = reinterpret_cast<unsigned long long*>(counts);
-        if(small(n))
+        if(direct(n))
         {
-            Small_Stage a = small_stage(off, n);
-            a.max_pos = ~0ull, a.zero = out, a.zero_n = n;
-            const auto* c = run_small(K_REDUCE, b, a, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(0), VT(0)});
+            Stage a = new_stage(off, n);
+            a.zero = out, a.zero_n = n;
+            const auto* c = run_staged(K_REDUCE, b, a, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(0), VT(0)});
             if(c[6] == c[4])
                 return;
         }
@@ -1626,10 +1591,9 @@ public:
             bs[b].result = 0, N += bs[b].n;
         if(N == 0 || ((kind == KACHE_B200_RUN_UPSERT_ORIENTED || kind == KACHE_B200_RUN_UPDATE) && set_))
             return;
-        // Descriptors, 8 words per batch; the merged list: offsets (N + 1), addresses (N), lengths (N), per-batch
-        // first positions and results (count each), batch of each sequence (N, 32-bit).
-        const size_t o_desc = 0, o_off = o_desc + count * 64, o_addr = o_off + (N + 1) * 8, o_len = o_addr + N * 8;
-        const size_t o_pb = o_len + N * 8, o_res = o_pb + count * 8, o_bof = o_res + count * 8, total = o_bof + N * 4;
+        // Descriptors, 8 words per batch; the merged list: addresses (N), per-batch first positions and results (count each),
+        // batch of each sequence (N, 32-bit).
+        const size_t o_desc = 0, o_addr = o_desc + count * 64, o_pb = o_addr + N * 8, o_res = o_pb + count * 8, o_bof = o_res + count * 8, total = o_bof + N * 4;
         pin_multi_.ensure(count * 64);
         auto* hd = pin_multi_.as<uint64_t>();
         for(size_t b = 0, s = 0; b < count; s += bs[b].n, ++b)
@@ -1643,9 +1607,7 @@ public:
         dmulti_.ensure(total);
         char* d = dmulti_.as<char>();
         auto* desc = reinterpret_cast<uint64_t*>(d + o_desc);
-        auto* voff = reinterpret_cast<uint64_t*>(d + o_off);
         auto* addr = reinterpret_cast<uint64_t*>(d + o_addr);
-        auto* lens = reinterpret_cast<uint64_t*>(d + o_len);
         auto* pos_base = reinterpret_cast<uint64_t*>(d + o_pb);
         auto* res = reinterpret_cast<unsigned long long*>(d + o_res);
         auto* batch_of = reinterpret_cast<uint32_t*>(d + o_bof);
@@ -1659,44 +1621,36 @@ public:
                 bs[b].result = hr[b];
         };
         const Oriented_Op_Fn<VT> ofn{op, static_cast<VT>(x), static_cast<VT>(y)};
-        if(small(N))
+        Stage a = new_stage(nullptr, N);
+        a.desc = desc, a.count = count, a.addr = addr, a.batch_of = batch_of, a.pos_base = pos_base;
+        a.zero_out0 = kind == KACHE_B200_RUN_COUNT, a.zero = res, a.zero_n = count;
+        if(direct(N))
         {
-            Small_Stage a = small_stage(nullptr, N);
-            a.desc = desc, a.count = count, a.addr = addr, a.batch_of = batch_of, a.pos_base = pos_base;
-            a.zero_out0 = kind == KACHE_B200_RUN_COUNT, a.zero = res, a.zero_n = count, a.max_pos = ~0ull;
             uint64_t ins = 0;
             bool ran = false;
             if(kind == KACHE_B200_RUN_UPSERT)
-                ran = upsert_small(user, nullptr, a, op_fn(op, x, y), ins, res);
+                ran = upsert_direct(user, nullptr, a, op_fn(op, x, y), ins, res);
             else if(kind == KACHE_B200_RUN_UPSERT_ORIENTED)
             {
                 if constexpr(!set_)
-                    ran = upsert_small(user, nullptr, a, ofn, ins, res);
+                    ran = upsert_direct(user, nullptr, a, ofn, ins, res);
             }
             else
             {
                 const unsigned long long* c = nullptr;
                 if(kind == KACHE_B200_RUN_COUNT)
-                    c = run_small(K_REDUCE, nullptr, a, Count_Batches_Visitor<set_, VT>{{T_, nullptr, VT(0), VT(0)}, desc, res});
+                    c = run_staged(K_REDUCE, nullptr, a, Count_Batches_Visitor<set_, VT>{{T_, nullptr, VT(0), VT(0)}, desc, res});
                 else if(kind == KACHE_B200_RUN_LOOKUP)
-                    c = run_small(K_LOOKUP, nullptr, a, Lookup_Batches_Visitor<set_, VT>{{T_, nullptr, nullptr, nullptr}, desc, pos_base, res});
+                    c = run_staged(K_LOOKUP, nullptr, a, Lookup_Batches_Visitor<set_, VT>{{T_, nullptr, nullptr, nullptr}, desc, pos_base, res});
                 else if constexpr(!set_)
-                    c = run_small(K_UPDATE, nullptr, a, Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), res});
+                    c = run_staged(K_UPDATE, nullptr, a, Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), res});
                 ran = c && c[6] == c[4];
             }
             if(ran)
                 return results();
         }
-        launch(K_OTHER, [&](){ batches_list_kernel<<<grid_for((N + 31) / 32, 8), 256, 0, stream_>>>(desc, count, N, lens, addr, batch_of, kind == KACHE_B200_RUN_COUNT); });
-        check(cudaMemsetAsync(voff, 0, 8, stream_), "memset");
-        size_t tmp = 0;
-        check(cub::DeviceScan::InclusiveSum(nullptr, tmp, lens, voff + 1, static_cast<int64_t>(N), stream_), "scan");
-        dscan_.ensure(tmp);
-        check(cub::DeviceScan::InclusiveSum(dscan_.p, tmp, lens, voff + 1, static_cast<int64_t>(N), stream_), "scan");
-
-        const auto bi = stage_dev(nullptr, voff, N, addr, batch_of);
         // Per-batch results, added up by the visitors: keys inserted, k-mers present, positions found or counts.
-        check(cudaMemsetAsync(res, 0, count * 8, stream_), "memset");
+        const auto bi = stage_dev(nullptr, a);
         if(kind == KACHE_B200_RUN_UPSERT)
             run_upsert(user, bi, op_fn(op, x, y), res, true);
         else if(kind == KACHE_B200_RUN_UPSERT_ORIENTED)
@@ -1716,7 +1670,6 @@ public:
             stream_launch(K_REDUCE, bi, 0, bi.nsegs, Count_Batches_Visitor<set_, VT>{{T_, nullptr, VT(0), VT(0)}, desc, res});
         else
         {
-            launch(K_OTHER, [&](){ batches_pos_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, stream_>>>(desc, count, bi.pos_off, pos_base); });
             stream_launch(K_LOOKUP, bi, 0, bi.nsegs, Lookup_Batches_Visitor<set_, VT>{{T_, nullptr, nullptr, nullptr}, desc, pos_base, res});
         }
         results();
