@@ -353,7 +353,7 @@ struct Stage
     uint64_t *npos, *pos_off, *seg_off;     // Positions of each sequence; n + 1 sums of positions and of segments.
     unsigned long long* blocks;     // Two words per block of stage_count_kernel: the positions and segments before it.
     Segment* segs;
-    unsigned long long* ctr;    // [0] and the low half of [2] are zeroed; [3..6]: positions, segments, segment length, segments to run; [7]: zero between launches.
+    unsigned long long* ctr;    // [0] and the low half of [2] are zeroed; [3..6]: positions, segments, segment length, segments to run; [7]: zero between launches; [8] is zeroed.
     unsigned long long* zero;   // zero_n words zeroed.
     uint64_t zero_n;
 };
@@ -465,7 +465,7 @@ static __global__ void __launch_bounds__(stage_block) stage_small_kernel(const S
     {
         a.pos_off[a.n] = total, a.seg_off[a.n] = nsegs;
         a.ctr[3] = total, a.ctr[4] = nsegs, a.ctr[5] = seg_len, a.ctr[6] = run;
-        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0;
+        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[8] = 0;
     }
     __syncthreads();
     for(uint32_t i = t; i < run; i += stage_block)
@@ -527,7 +527,7 @@ static __global__ void __launch_bounds__(stage_block) stage_count_kernel(const S
     {
         a.pos_off[a.n] = P, a.seg_off[a.n] = S;
         a.ctr[3] = P, a.ctr[4] = S, a.ctr[5] = seg_positions, a.ctr[6] = S <= a.max_segs && P <= a.max_pos ? S : 0;
-        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[7] = 0;
+        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[7] = 0, a.ctr[8] = 0;
     }
 }
 

@@ -191,7 +191,7 @@ __device__ __forceinline__ void describe_segment(const uint8_t* const seq, const
 
 template <int k, int l, typename Visitor>
 __global__ void __launch_bounds__(32 * stream_warps, Visitor::min_blocks) stream_kernel(const Dev_Batch batch, const uint64_t seg_b, const uint64_t segs_end,
-                                                                                        const unsigned long long* run, Visitor vis)
+                                                                                        const unsigned long long* run, unsigned long long* taken, Visitor vis)
 {
     // The segments [seg_b, segs_end), or as many as `run` says, counted by the kernel before.
     const uint64_t seg_e = run ? static_cast<uint64_t>(*run) : segs_end;
@@ -200,21 +200,36 @@ __global__ void __launch_bounds__(32 * stream_warps, Visitor::min_blocks) stream
     fill_base_table(tab);
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     vis.begin();
-    const uint64_t warps = uint64_t(gridDim.x) * stream_warps;
+    // After its first segment a warp takes more, a few at a time, from the counter `taken` (zero before the launch); without
+    // one every warp has a fixed share (see Engine::shares).
+    const uint64_t warps = uint64_t(gridDim.x) * stream_warps, nsegs = seg_e > seg_b ? seg_e - seg_b : 0;
+    const uint64_t some = max(uint64_t(1), min(uint64_t(4), nsegs / (warps * 8)));
+    const auto take = [&]() -> uint64_t
+    {
+        unsigned long long g = 0;
+        if(lane == 0)
+            g = atomicAdd(taken, static_cast<unsigned long long>(some));
+        return warps + __shfl_sync(0xFFFFFFFFu, g, 0);
+    };
     // A segment's entry is asked for a segment ahead, a word per lane.
     const auto ask = [&](const uint64_t g) -> uint32_t
     {
-        return g < seg_e && lane < sizeof(Segment) / 4 ? __ldg(reinterpret_cast<const uint32_t*>(batch.segs + g) + lane) : 0u;
+        return g < nsegs && lane < sizeof(Segment) / 4 ? __ldg(reinterpret_cast<const uint32_t*>(batch.segs + seg_b + g) + lane) : 0u;
     };
-    uint64_t g = seg_b + uint64_t(blockIdx.x) * stream_warps + wid;
-    for(uint32_t entry = ask(g); g < seg_e; )
+    uint64_t g = uint64_t(blockIdx.x) * stream_warps + wid, left = 1;
+    for(uint32_t entry = ask(g); g < nsegs; )
     {
         const auto word = [&](const int i) { return __shfl_sync(0xFFFFFFFFu, entry, i); };
         const auto wide = [&](const int i) { return uint64_t(word(i + 1)) << 32 | word(i); };
         const uint64_t base = wide(0);
         const Seg_Of s{wide(4), wide(2), word(7)};
         const uint32_t npos = word(6);
-        g += warps;
+        if(!taken)
+            g += warps;
+        else if(--left)
+            ++g;
+        else
+            g = take(), left = some;
         entry = ask(g);
         vis.begin_segment(s);
         describe_segment<k, l>(batch.bases + base, npos, ring_all[wid], tab, lane, vis);
