@@ -130,7 +130,7 @@ def max_over_ranks(dist, x, device):
 def ncu_traffic(kernel):
     """DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the kernel on this workload, from the
     committed ncu summary under profiles/, or None."""
-    name = {"lookup": "lookup_stream_kernel_config1.md", "upsert": "upsert_lane_kernel_config1.md"}.get(kernel)
+    name = {"lookup": "lookup_stream_kernel_config1.md", "upsert": "upsert_stream_kernel_config1.md"}.get(kernel)
     try:
         with open(os.path.join(os.path.dirname(os.path.abspath(__file__)), "profiles", name)) as f:
             m = re.search(r"\| dram bytes per launch \| (\d+) \|", f.read())
@@ -536,7 +536,7 @@ def sub_config3(dev, stream, device_index):
     A_up = b_in + 32 * rho + 32 * (1 - inserted / P1) + 32 * 1.0
     A_lk = b_in + 3 + 32 * rho + 32 * hit
     peak, peak_kind = load_peaks()
-    kern = {"upsert_oriented": kernel_roofline("lane_kernel<27,16,Upsert_Visitor> (batched)", prof["upsert"][0], prof["upsert"][1],
+    kern = {"upsert_oriented": kernel_roofline("stream_kernel<27,16,Upsert_Visitor> (batched)", prof["upsert"][0], prof["upsert"][1],
                                                A_up * P1 / max(1, prof["upsert"][1]), A_up, peak, peak_kind),
             "lookup": kernel_roofline("stream_kernel<27,16,Lookup_Batches_Visitor> (batched)", prof["lookup"][0], prof["lookup"][1],
                                       A_lk * P1 / max(1, prof["lookup"][1]), A_lk, peak, peak_kind)}
@@ -649,11 +649,11 @@ def sub_config5(dev, stream, device_index, scale=0.05, requests=300):
     A_up = b_in + 32 * rho + 32 * (1 - res["ins"] / max(1, P_kind[0])) + 32 * 1.0
     A_lk = b_in + 5 + 32 * rho + 32 * hit
     A_ct = b_in + 32 * rho + 32 * hit
-    kern = {"upsert": kernel_roofline("lane_kernel<31,22,Upsert_Visitor> (batched)", prof["upsert"][0], prof["upsert"][1],
+    kern = {"upsert": kernel_roofline("stream_kernel<31,22,Upsert_Visitor> (batched)", prof["upsert"][0], prof["upsert"][1],
                                       A_up * P_kind[0] / max(1, prof["upsert"][1]), A_up, peak, peak_kind),
             "lookup": kernel_roofline("stream_kernel<31,22,Lookup_Batches_Visitor> (batched)", prof["lookup"][0], prof["lookup"][1],
                                       A_lk * P_kind[1] / max(1, prof["lookup"][1]), A_lk, peak, peak_kind),
-            "count": kernel_roofline("lane_kernel<31,22,Seq_Reduce_Visitor> (batched)", prof["reduce"][0], prof["reduce"][1],
+            "count": kernel_roofline("stream_kernel<31,22,Seq_Reduce_Visitor> (batched)", prof["reduce"][0], prof["reduce"][1],
                                      A_ct * P_kind[2] / max(1, prof["reduce"][1]), A_ct, peak, peak_kind)}
     dom = max(kern, key=lambda k_: kern[k_]["ms_total"])
     roof = dict(kern[dom])

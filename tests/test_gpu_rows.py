@@ -70,3 +70,78 @@ def test_counts_past_full_buckets(vb):
     assert G.stats().overflow_keys > 0
     assert np.array_equal(G.count(q), O.count(q))
     G.close()
+
+
+def _dev(bases, off):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(bases)).cuda(), torch.from_numpy(off.view(np.int64)).cuda()
+
+
+@pytest.mark.parametrize("n", [1, 2, 1023, 1024, 1025, 4096, 4097, 9001])
+def test_staging_edges(n):
+    """Device batches of as many sequences as its staging's blocks and launches divide by, some empty or shorter than k,
+    alone and as several batches (one of them empty): upserts, lookups, updates and counts against the oracle."""
+    import torch
+    rng = np.random.default_rng(n)
+    lens = rng.choice([0, 5, 30, 31, 32, 62, 63, 100], n)
+    lens[0] = 700
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(lens)
+    b = Batch(np.concatenate([ACGT[rng.integers(0, 4, int(off[-1]))], np.zeros(16, np.uint8)]), off)
+    bases, offs = _dev(b.bases, b.off)
+    G, O = kache.Table(31, 4, 1000), oracle.OracleTable(31, 4, 1000)
+    u, uo = G.register(), O.register()
+    torch.cuda.synchronize()
+    cut = n // 3
+    parts = [(bases.data_ptr(), offs.data_ptr(), cut), (bases.data_ptr(), offs.data_ptr() + 8 * cut, 0), (bases.data_ptr(), offs.data_ptr() + 8 * cut, n - cut)]
+    assert G.upsert_dev(u, bases.data_ptr(), offs.data_ptr(), n, kache.ADD, 1, 1) == O.upsert(uo, b, kache.ADD, 1, 1)
+    assert sum(G.run_dev_batches(kache.RUN_UPSERT, parts, kache.ADD, 2, 2, u)) == O.upsert(uo, b, kache.ADD, 2, 2)
+    assert G.update_dev(bases.data_ptr(), offs.data_ptr(), n, kache.ADD, 1) == O.update(b, kache.ADD, 1)
+    assert G.capacity() == O.capacity()
+    fo, vo, _ = O.lookup(b)
+    P = len(fo)
+    f, v, c = (torch.full((max(m, 1),), 7, dtype=t, device="cuda") for m, t in ((P, torch.uint8), (P, torch.int32), (n, torch.int64)))
+    torch.cuda.synchronize()
+    G.lookup_dev(bases.data_ptr(), offs.data_ptr(), n, f.data_ptr(), v.data_ptr())
+    G.count_dev(bases.data_ptr(), offs.data_ptr(), n, c.data_ptr())
+    assert np.array_equal(f.cpu().numpy()[:P], fo) and np.array_equal(v.cpu().numpy()[:P].view(np.uint32), vo)
+    assert np.array_equal(c.cpu().numpy().view(np.uint64), O.count(b))
+    first = int(b.slice(0, cut).positions(31).sum()) if cut else 0
+    f.fill_(7), c.fill_(7)
+    torch.cuda.synchronize()
+    hits = G.run_dev_batches(kache.RUN_LOOKUP, [parts[0] + (f.data_ptr(),), parts[1] + (f.data_ptr(),), parts[2] + (f.data_ptr() + first,)])
+    sums = G.run_dev_batches(kache.RUN_COUNT, [parts[0] + (c.data_ptr(),), parts[1] + (c.data_ptr(),), parts[2] + (c.data_ptr() + 8 * cut,)])
+    assert np.array_equal(f.cpu().numpy()[:P], fo) and np.array_equal(c.cpu().numpy().view(np.uint64), O.count(b))
+    assert hits == sums == [int((fo[:first] == 1).sum()), 0, int((fo[first:] == 1).sum())]
+    G.close()
+
+
+@pytest.mark.parametrize("n,length", [(150_000, 150), (3, 4_000_000)])
+def test_large_launches_equal_prepared_ones(n, length):
+    """Batches whose warps take segments from a counter, and few sequences of more segments than a block lists: staged
+    lookups and counts equal prepared ones, whose shares are fixed, and the update's total is theirs."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(5)
+    bases = torch.tensor(list(b"ACGT"), dtype=torch.uint8, device="cuda")[torch.randint(0, 4, (n * length + 64,), device="cuda", generator=g)]
+    bases[n * length // 2:n * length] = bases[:n * length - n * length // 2].clone()    # Each half's k-mers again.
+    off = torch.arange(n + 1, dtype=torch.int64, device="cuda") * length
+    half = torch.arange(n // 2 + 1, dtype=torch.int64, device="cuda") * length
+    G = kache.Table(31, 4, 10_000_000)
+    u, P = G.register(), n * (length - 30)
+    f, h = (torch.zeros(P, dtype=torch.uint8, device="cuda") for _ in range(2))
+    v, w = (torch.zeros(P, dtype=torch.int32, device="cuda") for _ in range(2))
+    c, d = (torch.zeros(n, dtype=torch.int64, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    G.upsert_dev(u, bases.data_ptr(), half.data_ptr(), n // 2, kache.ADD, 1, 1)
+    p = G.prepare_dev(off.data_ptr(), n)
+    G.lookup_dev(bases.data_ptr(), off.data_ptr(), n, f.data_ptr(), v.data_ptr())
+    G.lookup_prepared(p, bases.data_ptr(), h.data_ptr(), w.data_ptr())
+    G.count_prepared(p, bases.data_ptr(), d.data_ptr())
+    G.count_dev(bases.data_ptr(), off.data_ptr(), n, c.data_ptr())
+    torch.cuda.synchronize()
+    assert torch.equal(f, h) and torch.equal(v, w) and torch.equal(c, d)
+    present = int((f == 1).sum())
+    assert present == int(c.sum()) == G.update_dev(bases.data_ptr(), off.data_ptr(), n, kache.ADD, 1) and 0 < present
+    assert int(v[f == 1].min()) >= 1
+    G.prepared_free(p)
+    G.close()
