@@ -15,12 +15,12 @@
 //   - non-ACGT characters split sequences (DNA_Utility.hpp:199-224): a window with one is not a k-mer.
 // Every operation runs so, also those without per-position outputs: consecutive k-mers share minimizers, so a row of 32
 // touches about seven buckets where 32 lanes on 32 different reads would touch 32 (a lane per segment, rolling its k-mers,
-// took 9.19 ms for 130M upserts into a 6.7 GB map, rows 3.1 ms; 7.1 against 4.0 ms for 190M updates).
+// took 9.19 ms for 130M upserts into a 6.7 GB map, rows 2.8 ms; 7.1 against 3.6 ms for 190M updates).
 //
-// What bounds it is instructions (about 290 per row in a lookup, the integer pipe two thirds busy) and, next, the latency
+// What bounds it is instructions (327 per row in a lookup of 150 bp reads, issue slots two thirds used), then the latency
 // of three dependent loads; so more resident warps pay even at the price of some spills: six blocks of 256 threads per SM
-// (40 registers) against five, four and three, lookup of 120M positions 1.81 against 1.82, 1.80 (a variant that overlapped
-// two rows) and 2.29 ms, upsert of 40M 1.08 against 1.11, 1.15 and 1.46 ms.
+// (40 registers) against five, four and three, with fixed shares of segments, lookup of 120M positions 1.81 against 1.82,
+// 1.80 (overlapping two rows) and 2.29 ms, upsert of 40M 1.08 against 1.11, 1.15 and 1.46; now 1.73 and 0.94 ms.
 // Sequences are cut into segments of up to `seg_positions` positions; each segment re-reads the k - 1 bases it
 // shares with the next, so segments, like the reference's lanes (include/Streaming_Kmer_Hash_Table.hpp:1751-1781),
 // need no state from one another.
