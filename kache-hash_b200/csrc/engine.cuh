@@ -341,6 +341,7 @@ class Engine final : public kache_table
     Dev_Buf cs2_, spill2_, slots2_, ov2_;   // The previous table's arrays, kept for the next resize to build into.
     Dev_Table T_{};
     uint64_t ov_slots_ = 0;
+    bool blank_ = true;     // Whether the table's buckets are all zero: no upsert has run on them since they were zeroed.
 
     // The reference's sizing state (include/Streaming_Kmer_Hash_Table.hpp:81-86, 224-229).
     const double lf_;
@@ -1020,8 +1021,9 @@ class Engine final : public kache_table
         }
         else
         {
-            // The buckets that an empty table has are zero already.
-            const uint64_t have = T_.cap, more = target - have;
+            // A blank table's buckets are zero already. (A table of no keys need not be blank: an upsert that failed,
+            // for want of memory for the overflow table, may have left some that were never counted.)
+            const uint64_t have = blank_ ? T_.cap : 0, more = target - have;
             check(cudaMemsetAsync(cs_.as<char>() + have * B, 0, more * B, stream_), "memset");
             check(cudaMemsetAsync(spill_.as<char>() + have * 32, 0, more * 32, stream_), "memset");
             check(cudaMemsetAsync(slots_.as<char>() + have * B * slot_bytes, 0, more * B * slot_bytes, stream_), "memset");
@@ -1030,6 +1032,7 @@ class Engine final : public kache_table
         ov_slots_ = ov_slots;
         set_ov(T_, ov_, ov_slots_);
         check(cudaMemsetAsync(ctr() + 1, 0, sizeof(unsigned long long), stream_), "memset");
+        blank_ = true;
     }
 
     // Upserts a staged batch with the value functor `fn`, chunk by chunk (see the top of this file).
@@ -1067,6 +1070,7 @@ class Engine final : public kache_table
 
             check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
             check(cudaMemsetAsync(retried, 0, 4, stream_), "memset");
+            blank_ = false;
             Upsert_Visitor<set_, VT, Fn> vis{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per, by_batch};
             stream_launch(K_UPSERT, bi, sb, se, vis);
             const unsigned long long* c = read_ctr(3);
@@ -1148,6 +1152,7 @@ class Engine final : public kache_table
            predicted_cap(user, static_cast<uint64_t>(novelty_ * static_cast<double>(last_pos_))) > T_.cap)
             return false;   // The last one also where the table is to grow ahead of the call (run_upsert).
         clear_retries(most / 8 + 8);
+        blank_ = false;
         unsigned int* retried = reinterpret_cast<unsigned int*>(ctr() + 2);
         const unsigned long long* c = run_staged(K_UPSERT, bases, a, Upsert_Visitor<set_, VT, Fn>{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per, per != nullptr});
         if(c[6] != c[4])
@@ -1848,6 +1853,7 @@ public:
     {
         std::lock_guard<std::mutex> g(work);
         unsigned long long* d = ctr() + 4;
+        blank_ = false;
         launch(K_OTHER, [&](){ plant_claim_kernel<k, l, set_><<<1, 1, 0, stream_>>>(T_, key_of_encoding(key), d); });
         auto* h = pin_ctr_.as<uint64_t>(0);
         check(cudaMemcpyAsync(h, d, 8, cudaMemcpyDeviceToHost, stream_), "D2H");
@@ -1877,6 +1883,7 @@ public:
             check(cudaMemsetAsync(ov_.p, 0, ov_slots_ * 32, stream_), "memset");
         }
         check(cudaMemsetAsync(ctr(), 0, 72, stream_), "memset");
+        blank_ = true;
         cap_ = cap0_;
         resize_th_ = static_cast<uint64_t>(static_cast<double>(cap_ * B) * lf_);
         step_ = step_for(resize_th_);

@@ -193,3 +193,22 @@ def config1(scale=1.0):
     ins = reads_fixed(g, int(333_333 * scale), 150, seed=11)
     held = reads_fixed(g, int(1_000_000 * scale), 150, seed=2)
     return g, ins, held
+
+
+def one_minimizer(n, seed, k=31, l=22):
+    """n reads, 2k - l bases long each, of random bases around one l-mer, the one of 50,000 with the least placement hash (lmer_hash,
+    csrc/device_common.cuh): their k-mers share it as their minimizer, but for one in hundreds, so that all but 96 of the
+    keys of a table go to its overflow table."""
+    rng = np.random.default_rng(seed)
+    w = rng.integers(0, 4, (50_000, l), dtype=np.uint8)
+    bit = 1 << np.arange(l - 1, -1, -1, dtype=np.uint64)
+    top = np.uint64(0xFFFFFFFF)
+
+    def odd(c):
+        return (((c >> 1) * bit).sum(1) * np.uint64(0x9E3779B2) + ((c & 1) * bit).sum(1) * np.uint64(0x85EBCA76) + np.uint64(0x809CB0CB)) & top
+
+    x = odd(w) * odd((3 - w)[:, ::-1])
+    h = ((x >> np.uint64(32)) * np.uint64(0xC2B2AE3D) + x) & top
+    reads = rng.integers(0, 4, (n, 2 * k - l), dtype=np.uint8)
+    reads[:, k - l:k] = w[np.argmin(h)]
+    return np.concatenate([ASCII[reads].reshape(-1), np.zeros(16, np.uint8)]), np.arange(n + 1, dtype=np.uint64) * np.uint64(2 * k - l)

@@ -98,3 +98,31 @@ def test_plant_rejects_present_and_invalid_kmers():
     assert L.kache_b200_testing_plant_claim(T.h, b"ACGTN" * 7, 10) == kache.KACHE_EINVAL
     assert L.kache_b200_testing_plant_claim(None, b"A" * 31, 10) == kache.KACHE_EINVAL
     T.close()
+
+
+def test_failed_first_upsert_leaves_no_keys_behind():
+    """A table emptied after it had grown; its next upsert, of keys that share a minimizer, fills the overflow table,
+    whose growth fails; the one after, which takes the empty table to a larger capacity again, makes the table the
+    oracle makes of it alone."""
+    L = kache.lib()
+    g = synth.genome(300_000, seed=78)
+    first, last = (Batch(*synth.stretches(x, 500)) for x in (g[:150_000], g[150_000:]))
+    shared = Batch(*synth.one_minimizer(1000, 79))
+    T = kache.Table(31, 8, 1000, capi=False)
+    u = T.register()
+    T.upsert(u, first, kache.ADD, 1, 1)
+    T.clear()
+    r = ctypes.c_uint64()
+    try:
+        L.kache_b200_testing_fail_allocation(0)
+        assert L.kache_b200_upsert(T.h, u, *shared.args(), kache.ADD, 1, 1, ctypes.byref(r)) == kache.KACHE_ENOMEM
+    finally:
+        L.kache_b200_testing_fail_allocation(-1)
+    assert T.stats().overflow_keys > 1000       # It was the overflow table's growth that failed.
+    inserted = T.upsert(u, last, kache.ADD, 1, 1)
+    O = oracle.OracleTable(31, 8, 1000)
+    assert inserted == O.upsert(O.register(), last, kache.ADD, 1, 1)
+    kg, vg = T.dump()
+    ko, vo = O.dump()
+    assert T.size() == O.size() and np.array_equal(kg, ko) and np.array_equal(vg, vo)
+    T.close()
