@@ -331,7 +331,7 @@ __global__ void get_kernel(const Dev_Table T, const uint64_t* keys, const uint64
 // stage_list_kernel). A million sequences take 26 and 30 us; a counting kernel, two scans, a search per segment and the
 // host's read of the counts before it took 45 us of kernels and about 30 of waiting.
 constexpr uint32_t small_stage_max = 4096;      // Sequences of a block (at most 4 per thread).
-constexpr uint32_t small_segs_max = 16384;      // Segments that it lists.
+constexpr uint32_t small_segs_max = 16384;      // Segments that a block lists.
 constexpr uint32_t stage_block = 1024;
 
 struct Stage
@@ -353,7 +353,7 @@ struct Stage
     uint64_t *npos, *pos_off, *seg_off;     // Positions of each sequence; n + 1 sums of positions and of segments.
     unsigned long long* blocks;     // Two words per block of stage_count_kernel: the positions and segments before it.
     Segment* segs;
-    unsigned long long* ctr;    // [0] and the low half of [2] are zeroed; [3..6]: positions, segments, segment length, segments to run; [7]: zero between launches; [8] is zeroed.
+    unsigned long long* ctr;    // [0] and the low half of [2] are zeroed; [3..6]: positions, segments, segment length, segments to run; [7]: zero between launches; [8] is zeroed; [9]: whether the segments fit the list.
     unsigned long long* zero;   // zero_n words zeroed.
     uint64_t zero_n;
 };
@@ -465,7 +465,7 @@ static __global__ void __launch_bounds__(stage_block) stage_small_kernel(const S
     {
         a.pos_off[a.n] = total, a.seg_off[a.n] = nsegs;
         a.ctr[3] = total, a.ctr[4] = nsegs, a.ctr[5] = seg_len, a.ctr[6] = run;
-        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[8] = 0;
+        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[8] = 0, a.ctr[9] = nsegs <= a.max_segs;
     }
     __syncthreads();
     for(uint32_t i = t; i < run; i += stage_block)
@@ -485,10 +485,11 @@ static __global__ void __launch_bounds__(stage_block) stage_small_kernel(const S
 }
 
 // Larger batches, first launch: each block counts stage_block sequences, and the block that ends last sums the blocks'
-// counts. (A batch of this many sequences has a warp's segment of seg_positions for each.)
+// counts. The segments are listed behind it (stage_list_kernel) if they are not many more than the sequences, nor too many
+// of them one block's: otherwise the host, which reads so, lists them by a thread each (segs_kernel).
 static __global__ void __launch_bounds__(stage_block) stage_count_kernel(const Stage a)
 {
-    __shared__ unsigned long long wp[32], ws[32];
+    __shared__ unsigned long long wp[32], ws[32], most;     // `most`: segments of a block.
     __shared__ bool last;
     const uint32_t t = threadIdx.x;
     const uint64_t q = uint64_t(blockIdx.x) * stage_block + t;
@@ -507,7 +508,7 @@ static __global__ void __launch_bounds__(stage_block) stage_count_kernel(const S
     {
         __stcg(a.blocks + 2 * blockIdx.x, wp[31]), __stcg(a.blocks + 2 * blockIdx.x + 1, ws[31]);
         __threadfence();
-        last = atomicAdd(a.ctr + 7, 1ull) == gridDim.x - 1;
+        last = atomicAdd(a.ctr + 7, 1ull) == gridDim.x - 1, most = 0;
         __threadfence();
     }
     __syncthreads();
@@ -519,37 +520,59 @@ static __global__ void __launch_bounds__(stage_block) stage_count_kernel(const S
         const uint64_t b = b0 + t;
         const unsigned long long p = b < gridDim.x ? __ldcg(a.blocks + 2 * b) : 0, s = b < gridDim.x ? __ldcg(a.blocks + 2 * b + 1) : 0;
         const unsigned long long p1 = block_sum(p, wp), s1 = block_sum(s, ws);
+        if(s > small_segs_max)
+            atomicMax(&most, s);
         if(b < gridDim.x)
             a.blocks[2 * b] = P + p1 - p, a.blocks[2 * b + 1] = S + s1 - s;
         P += wp[31], S += ws[31];
     }
+    __syncthreads();
     if(t == 0)
     {
+        const bool fits = S <= a.max_segs && most == 0;
         a.pos_off[a.n] = P, a.seg_off[a.n] = S;
-        a.ctr[3] = P, a.ctr[4] = S, a.ctr[5] = seg_positions, a.ctr[6] = S <= a.max_segs && P <= a.max_pos ? S : 0;
-        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[7] = 0, a.ctr[8] = 0;
+        a.ctr[3] = P, a.ctr[4] = S, a.ctr[5] = seg_positions, a.ctr[6] = fits && P <= a.max_pos ? S : 0;
+        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[7] = 0, a.ctr[8] = 0, a.ctr[9] = fits;
     }
 }
 
-// Second launch: each block sums its own sequences and lists their segments.
+// Second launch: each block sums its own sequences and lists their segments. A thread writes an entry in some 30 ns, so it
+// lists its own sequence if that has up to own_segs; a longer one's are listed by its warp, an entry per lane. (A thread
+// each took 5.9 ms for 5,000 sequences one of which has 90 Mbp, and 1.67 for 200,000 with one of 25 Mbp.)
+constexpr uint32_t own_segs = 32;
+
 static __global__ void __launch_bounds__(stage_block) stage_list_kernel(const Stage a)
 {
     __shared__ unsigned long long wp[32], ws[32];
     const uint64_t q = uint64_t(blockIdx.x) * stage_block + threadIdx.x;
     const uint64_t np = q < a.n ? a.npos[q] : 0, ns = (np + seg_positions - 1) / seg_positions;
     const unsigned long long first = a.blocks[2 * blockIdx.x] + block_sum(np, wp) - np, first_seg = a.blocks[2 * blockIdx.x + 1] + block_sum(ns, ws) - ns;
-    if(q >= a.n)
+    if(q < a.n)
+    {
+        a.pos_off[q] = first, a.seg_off[q] = first_seg;
+        if(a.desc && a.desc[8 * uint64_t(a.batch_of[q]) + 3] == q)
+            a.pos_base[a.batch_of[q]] = first;
+    }
+    if(a.ctr[6] == 0)
         return;
-    a.pos_off[q] = first, a.seg_off[q] = first_seg;
-    if(a.desc && a.desc[8 * uint64_t(a.batch_of[q]) + 3] == q)
-        a.pos_base[a.batch_of[q]] = first;
-    if(a.ctr[6])
+    if(ns <= own_segs)
         for(uint64_t i = 0; i < ns; ++i)
             a.segs[first_seg + i] = stage_segment(a, q, i, np, first, seg_positions);
+    constexpr uint32_t all = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31;
+    for(uint32_t m = __ballot_sync(all, ns > own_segs); m; m &= m - 1)
+    {
+        const int s = __ffs(m) - 1;
+        const uint64_t q_s = q - lane + s, np_s = __shfl_sync(all, np, s), ns_s = __shfl_sync(all, ns, s);
+        const uint64_t first_s = __shfl_sync(all, first, s), at = __shfl_sync(all, first_seg, s);
+        for(uint64_t i = lane; i < ns_s; i += 32)
+            a.segs[at + i] = stage_segment(a, q_s, i, np_s, first_s, seg_positions);
+    }
 }
 
-// Lists the segments of a staged batch that had more of them than its listing took, one thread per segment: its sequence by binary search in seg_off[0..n] (exclusive sums of
-// segments per sequence), so that long sequences' many segments are listed in parallel. Sequence q's bases are at offset
+// Lists the segments of a staged batch that had more of them than its listing took, one thread per segment: its sequence
+// by binary search in seg_off[0..n] (exclusive sums of segments per sequence), so that long sequences' many segments are
+// listed in parallel. Sequence q's bases are at offset
 // off[q], or with `addr` at the address addr[q], where it is of batch batch_of[q].
 static __global__ void segs_kernel(const uint64_t* seg_off, const uint64_t* pos_off, const uint64_t* off, const uint64_t* addr, const uint32_t* batch_of, const uint64_t n,
                                    const uint64_t nsegs, const uint32_t seg_len, Segment* segs)

@@ -393,7 +393,9 @@ class Engine final : public kache_table
     double prof_ms_[K_KINDS] = {};
     uint64_t prof_n_[K_KINDS] = {};
 
-    // Device counters: [0] inserted/present, [1] overflow keys, [2] retry flag + error word, [3..4] scratch.
+    // Device counters: [0] inserted/present, [1] overflow keys, [2] retry flag + error word, [3..6] scratch, or what staging
+    // counted, [7] its blocks done, [8] the work counter, [9] whether the staged segments fitted their list (see Stage::ctr).
+    static constexpr size_t ctr_bytes = 10 * 8;
     unsigned long long* ctr() const { return ctr_.as<unsigned long long>(); }
 
     struct Batch_Info
@@ -809,9 +811,10 @@ class Engine final : public kache_table
     // Counts and lists a batch's segments on the device.
     void launch_stage(Stage& a)
     {
-        dbatch_.ensure((a.n <= small_stage_max ? small_segs_max : a.n + a.n / 8 + 1024) * sizeof(Segment));
+        // The room is the batch's own, whatever the list has had to hold before: a batch is staged alike at each call.
+        a.max_segs = a.n <= small_stage_max ? small_segs_max : a.n + a.n / 8 + 1024;
+        dbatch_.ensure(a.max_segs * sizeof(Segment));
         a.segs = dbatch_.as<Segment>();
-        a.max_segs = a.n <= small_stage_max ? small_segs_max : dbatch_.bytes / sizeof(Segment);
         const unsigned blocks = static_cast<unsigned>((a.n + stage_block - 1) / stage_block);
         if(a.n <= small_stage_max)
             launch(K_OTHER, [&](){ stage_small_kernel<<<1, stage_block, 0, stream_>>>(a); });
@@ -822,11 +825,11 @@ class Engine final : public kache_table
         }
     }
 
-    // Whether the last batch of few sequences had no more segments than its block lists.
-    bool small_fits_ = true;
+    // Whether the segments of the last batch of few sequences, and of the last one of more, fitted the list.
+    bool fits_[2] = {true, true};
 
     // Whether to run a batch of n sequences directly (run_staged) rather than after the host has read its counts.
-    bool direct(const uint64_t n) const { return n > 0 && (n > small_stage_max || small_fits_); }
+    bool direct(const uint64_t n) const { return n > 0 && fits_[n > small_stage_max]; }
 
     // Stages a batch and runs the visitor over it with no host read in between; returns the counters, of which [4] and [6]
     // are equal if the batch ran. The launch's grid is made for the segments that are likely, as their number is unknown
@@ -841,9 +844,8 @@ class Engine final : public kache_table
                 s.blocks = sm_count_ * Vis::min_blocks;
             stream_kernel<k, l, Vis><<<s.blocks, 32 * stream_warps, 0, stream_>>>(Dev_Batch{bases, a.segs}, 0, 0, ctr() + 6, s.taken, vis);
         });
-        const unsigned long long* c = read_ctr(7);
-        if(a.n <= small_stage_max)
-            small_fits_ = c[4] <= small_segs_max;
+        const unsigned long long* c = read_ctr(10);
+        fits_[a.n > small_stage_max] = c[9];
         return c;
     }
 
@@ -856,10 +858,9 @@ class Engine final : public kache_table
             return bi;
         a.max_pos = ~0ull;
         launch_stage(a);
-        const unsigned long long* c = read_ctr(7);
+        const unsigned long long* c = read_ctr(10);
         const uint64_t nsegs = c[4], run = c[6];
-        if(a.n <= small_stage_max)
-            small_fits_ = nsegs <= small_segs_max;
+        fits_[a.n > small_stage_max] = c[9];
         bi.nsegs = nsegs, bi.total_pos = c[3], bi.off = a.off, bi.pos_off = a.pos_off, bi.seg_off = a.seg_off;
         if(run != nsegs)
         {
@@ -1330,9 +1331,9 @@ public:
         check(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, dev), "attribute");
         check(cudaStreamCreateWithFlags(&own_, cudaStreamNonBlocking), "cudaStreamCreate");
         stream_ = own_;
-        pin_ctr_.ensure(64);
-        ctr_.ensure(72);
-        check(cudaMemsetAsync(ctr_.p, 0, 72, stream_), "memset");
+        pin_ctr_.ensure(ctr_bytes);
+        ctr_.ensure(ctr_bytes);
+        check(cudaMemsetAsync(ctr_.p, 0, ctr_bytes, stream_), "memset");
         alloc_table(cs_, spill_, slots_, cap_);
         bind(T_, cs_, spill_, slots_, cap_);
         // The overflow table starts with room for max(1024, capacity / 32) keys (Streaming_Kmer_Hash_Table.hpp:775).
@@ -1882,7 +1883,7 @@ public:
             check(cudaMemsetAsync(slots_.p, 0, cap0_ * B * slot_bytes, stream_), "memset");
             check(cudaMemsetAsync(ov_.p, 0, ov_slots_ * 32, stream_), "memset");
         }
-        check(cudaMemsetAsync(ctr(), 0, 72, stream_), "memset");
+        check(cudaMemsetAsync(ctr(), 0, ctr_bytes, stream_), "memset");
         blank_ = true;
         cap_ = cap0_;
         resize_th_ = static_cast<uint64_t>(static_cast<double>(cap_ * B) * lf_);

@@ -1,0 +1,98 @@
+"""Device batches of thousands of sequences with long ones among them: every call against the oracle, at each size by which
+their segments are listed differently, once and again; and the time that their staging takes."""
+import numpy as np
+import pytest
+
+import kache
+import oracle
+from kache import Batch
+
+pytestmark = pytest.mark.gpu
+
+ACGT = np.frombuffer(b"ACGT", np.uint8)
+
+
+def _batch(lens, seed):
+    rng = np.random.default_rng(seed)
+    off = np.zeros(len(lens) + 1, np.uint64)
+    off[1:] = np.cumsum(lens)
+    bases = ACGT[rng.integers(0, 4, int(off[-1]))]
+    bases[rng.integers(0, len(bases), len(bases) // 5000)] = ord("N")
+    return Batch(np.concatenate([bases, np.zeros(16, np.uint8)]), off)
+
+
+def _on_gpu(b):
+    import torch
+    return torch.from_numpy(b.bases).cuda(), torch.from_numpy(b.off.view(np.int64)).cuda()
+
+
+# A thread lists up to 32 segments of 512 positions; a block's sequences (1,024) may have 16,384; the list has room for
+# n / 8 + 1,024 more than the sequences.
+@pytest.mark.parametrize("n,at,longs", [
+    (4097, 4095, [30 + 32 * 512, 31 + 32 * 512]),               # The last segment that a thread lists, the first of a warp.
+    (5000, 1023, [600_000]),                                    # Listed by a warp.
+    (5000, 0, [1_400_000]),                                       # More than the list has room for.
+    (150_000, 77, [30 + 512 * 15_361]),                         # 16,384 segments of one block with its 1,023 others,
+    (150_000, 77, [31 + 512 * 15_361]),                         # and one more.
+])
+def test_long_sequences_among_many(n, at, longs):
+    import torch
+    lens = np.full(n, 33)
+    lens[::7], lens[::11] = 0, 31
+    if n > 100_000:
+        lens[:1024] = 40        # Each of one segment, so that the long one's make up the block's.
+    lens[at:at + len(longs)] = longs[:n - at]
+    b = _batch(lens, n)
+    bases, off = _on_gpu(b)
+    T, O = kache.Table(31, 4, 1000), oracle.OracleTable(31, 4, 1000)
+    u, uo = T.register(), O.register()
+    P = int(b.positions(31).sum())
+    cut = n // 3
+    first = int(b.slice(0, cut).positions(31).sum())
+    f, v, c = (torch.zeros(m, dtype=t, device="cuda") for m, t in ((P, torch.uint8), (P, torch.int32), (n, torch.int64)))
+    torch.cuda.synchronize()
+    p, q, s = bases.data_ptr(), off.data_ptr(), off.data_ptr() + 8 * cut
+    for _ in range(2):
+        assert T.upsert_dev(u, p, q, n, kache.ADD, 1, 1) == O.upsert(uo, b, kache.ADD, 1, 1)
+        assert sum(T.run_dev_batches(kache.RUN_UPSERT, [(p, q, cut), (p, s, n - cut)], kache.ADD, 1, 1, u)) == O.upsert(uo, b, kache.ADD, 1, 1)
+        assert T.update_dev(p, q, n, kache.ADD, 3) == O.update(b, kache.ADD, 3)
+        fo, vo, _ = O.lookup(b)
+        co = O.count(b)
+        hits = [int((fo[:first] == 1).sum()), int((fo[first:] == 1).sum())]
+        for merged in (False, True):
+            f.fill_(7), v.fill_(7), c.fill_(7)
+            torch.cuda.synchronize()
+            if merged:
+                assert T.run_dev_batches(kache.RUN_LOOKUP, [(p, q, cut, f.data_ptr(), v.data_ptr()), (p, s, n - cut, f.data_ptr() + first, v.data_ptr() + 4 * first)]) == hits
+                assert T.run_dev_batches(kache.RUN_COUNT, [(p, q, cut, c.data_ptr()), (p, s, n - cut, c.data_ptr() + 8 * cut)]) == hits
+            else:
+                T.lookup_dev(p, q, n, f.data_ptr(), v.data_ptr())
+                T.count_dev(p, q, n, c.data_ptr())
+            assert np.array_equal(f.cpu().numpy(), fo) and np.array_equal(v.cpu().numpy().view(np.uint32), vo)
+            assert np.array_equal(c.cpu().numpy().view(np.uint64), co)
+    ko, vo = O.dump()
+    kg, vg = T.dump()
+    assert np.array_equal(kg, ko) and np.array_equal(vg, vo)
+    T.close()
+
+
+@pytest.mark.parametrize("n,length", [(5000, 90_000_000), (200_000, 25_000_000)])
+def test_listing_long_sequences_in_parallel(n, length):
+    """The kernels that stage such a batch take some tens of microseconds, where one thread that writes the long sequence's
+    segments takes 1.6 and 5.9 ms; at the first call and at later ones, whose list has had to hold them."""
+    import torch
+    off = torch.full((n + 1,), 100, dtype=torch.int64, device="cuda").cumsum(0) - 100
+    off[-1] += length - 100
+    bases = torch.full((int(off[-1]) + 16,), ord("A"), dtype=torch.uint8, device="cuda")
+    c = torch.zeros(n, dtype=torch.int64, device="cuda")
+    T = kache.Table(31, 4, 1000)
+    torch.cuda.synchronize()
+    other = []
+    for _ in range(4):
+        T.profile(True)
+        T.count_dev(bases.data_ptr(), off.data_ptr(), n, c.data_ptr())
+        other.append(T.profile_read(5)[0])
+        T.profile(False)
+    print(other)
+    assert max(other) < 1 and int(c.sum()) == 0
+    T.close()
