@@ -96,3 +96,35 @@ def test_listing_long_sequences_in_parallel(n, length):
     print(other)
     assert max(other) < 1 and int(c.sum()) == 0
     T.close()
+
+
+def test_a_warp_per_segment_of_a_middling_batch():
+    """4,100 sequences of 5,125 segments, which the GPU's resident warps can take one each: the lookup staged with them
+    takes no longer than one over the listed segments (1.45 times as long where it is launched for a segment each)."""
+    import torch
+    lens = np.tile([500, 500, 500, 1000], 1025)
+    b = _batch(lens, 3)
+    bases, off = _on_gpu(b)
+    T = kache.Table(31, 8, 100_000_000)      # Larger than the caches.
+    P = int(b.positions(31).sum())
+    f = torch.zeros(P, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    T.upsert_dev(T.register(), bases.data_ptr(), off.data_ptr(), b.n, kache.KEEP, 0, 1)
+    shape = T.prepare_dev(off.data_ptr(), b.n)
+
+    def least(call):
+        ms = []
+        for _ in range(20):
+            T.profile(True)
+            call()
+            torch.cuda.synchronize()
+            ms.append(T.profile_read(2)[0])
+            T.profile(False)
+        return min(ms)
+
+    staged = least(lambda: T.lookup_dev(bases.data_ptr(), off.data_ptr(), b.n, f.data_ptr()))
+    prepared = least(lambda: T.lookup_prepared(shape, bases.data_ptr(), f.data_ptr()))
+    print(staged, prepared)
+    assert 0 < staged < 1.2 * prepared, (staged, prepared)
+    T.prepared_free(shape)
+    T.close()
