@@ -105,6 +105,10 @@ std::atomic<uint64_t>& launches();
 // before one fails as out of memory (0: the next one); -1 when off.
 std::atomic<int64_t>& alloc_fail_countdown();
 
+// Failure injection for tests: while nonnegative, the bytes of device memory that the library's buffers may still take,
+// as if a larger allocation failed for want of them; -1 when off.
+std::atomic<int64_t>& device_memory_left();
+
 // Fails the allocation about to be made if the injected countdown reaches it.
 inline void alloc_gate()
 {
@@ -158,7 +162,11 @@ struct Dev_Buf
     void release()
     {
         if(p)
+        {
             cudaFree(p);
+            if(device_memory_left() >= 0)
+                device_memory_left() += static_cast<int64_t>(bytes);
+        }
         p = nullptr, bytes = 0;
     }
 
@@ -169,12 +177,27 @@ struct Dev_Buf
             return;
         release();
         alloc_gate();
-        check(cudaMalloc(&p, std::max<size_t>(n, 256)), "cudaMalloc");
-        bytes = std::max<size_t>(n, 256);
+        const size_t m = std::max<size_t>(n, 256);
+        const int64_t left = device_memory_left();
+        if(left >= 0 && static_cast<int64_t>(m) > left)
+            throw std::bad_alloc();
+        check(cudaMalloc(&p, m), "cudaMalloc");
+        if(left >= 0)
+            device_memory_left() -= static_cast<int64_t>(m);
+        bytes = m;
     }
 
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
+
+// The device memory free.
+inline size_t free_device_memory()
+{
+    size_t free_b = 0, total_b = 0;
+    check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+    const int64_t left = device_memory_left();
+    return left >= 0 ? std::min(free_b, static_cast<size_t>(left)) : free_b;
+}
 
 struct Pinned_Buf
 {
@@ -977,17 +1000,17 @@ class Engine final : public kache_table
         if(spare_holds(wide))
             return wide;
         const size_t need = wide * (B + 32 + B * slot_bytes) + ov_slots_for(std::max<uint64_t>(1024, wide)) * 32;
-        size_t free_b = 0, total_b = 0;
-        check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
         const size_t spare = cs2_.bytes + spill2_.bytes + slots2_.bytes + ov2_.bytes;
-        return 2 * need <= free_b + spare ? wide : target;
+        return 2 * need <= free_device_memory() + spare ? wide : target;
     }
 
-    // Whether the spare arrays hold a table of `cap` buckets (but for its overflow table): then a rebuild need not ask the
-    // driver for the free memory, which took up to 2 ms a time.
+    // Whether a rebuild at `cap` buckets finds all its arrays made, the overflow table and the marks of moved keys too: then
+    // it need not ask the driver for the free memory, which took up to 2 ms a time.
     bool spare_holds(const uint64_t cap) const
     {
-        return cs2_.bytes >= cap * B && spill2_.bytes >= cap * 32 && slots2_.bytes >= cap * B * slot_bytes;
+        const size_t marks = (T_.cap * B + ov_slots_) / 8 + 8;
+        return cs2_.bytes >= cap * B && spill2_.bytes >= cap * 32 && slots2_.bytes >= cap * B * slot_bytes &&
+               ov2_.bytes >= ov_slots_for(std::max<uint64_t>(1024, cap)) * 32 && dretry_a_.bytes >= marks && dretry_b_.bytes >= marks;
     }
 
     // Grows the device table to `target` buckets ahead of a call's inserts: where keys sit is not observable, so the
@@ -1001,13 +1024,11 @@ class Engine final : public kache_table
         const size_t need = target * (B + 32 + B * slot_bytes) + ov_slots * 32;
         const bool allocated = size_ == 0 ? cs_.bytes >= target * B && spill_.bytes >= target * 32 &&
                                             slots_.bytes >= target * B * slot_bytes && ov_.bytes >= ov_slots * 32
-                                          : spare_holds(target) && ov2_.bytes >= ov_slots * 32;
+                                          : spare_holds(target);
         if(!allocated)      // Arrays would be allocated: only if they fit in free device memory.
         {
-            size_t free_b = 0, total_b = 0;
-            check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
             const size_t held = size_ == 0 ? cs2_.bytes + spill2_.bytes + slots2_.bytes + ov2_.bytes : 0;
-            if(need + (size_t(1) << 30) > free_b + held)
+            if(need + (size_t(1) << 30) > free_device_memory() + held)
                 return;
         }
         if(size_ != 0)

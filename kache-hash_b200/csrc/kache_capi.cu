@@ -26,6 +26,12 @@ std::atomic<int64_t>& alloc_fail_countdown()
     return c;
 }
 
+std::atomic<int64_t>& device_memory_left()
+{
+    static std::atomic<int64_t> c{-1};
+    return c;
+}
+
 // The engine's instantiations, one translation unit per (k, l) (tables_<k>_<l>.cu).
 kache_table* make_table_31_22(uint32_t vb, uint64_t n, double lf, bool pow2);
 kache_table* make_table_27_16(uint32_t vb, uint64_t n, double lf, bool pow2);
@@ -492,6 +498,12 @@ uint64_t kache_b200_kernel_launches(void) noexcept
 int kache_b200_testing_fail_allocation(const int64_t after) noexcept
 {
     kache_b200::alloc_fail_countdown().store(after < 0 ? -1 : after);
+    return KACHE_OK;
+}
+
+int kache_b200_testing_device_memory(const int64_t bytes) noexcept
+{
+    kache_b200::device_memory_left().store(bytes < 0 ? -1 : bytes);
     return KACHE_OK;
 }
 

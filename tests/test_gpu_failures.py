@@ -126,3 +126,39 @@ def test_failed_first_upsert_leaves_no_keys_behind():
     ko, vo = O.dump()
     assert T.size() == O.size() and np.array_equal(kg, ko) and np.array_equal(vg, vo)
     T.close()
+
+
+def test_rebuild_that_failed_midway_takes_the_smaller_table_next():
+    """A rebuild at four times the buckets (one doubling ahead) fails at its overflow table, its other arrays made. With
+    memory then left for the overflow table of twice the buckets but not of four times, the call made again rebuilds at
+    twice, and the table is the oracle's."""
+    L = kache.lib()
+    g = synth.genome(90_060, seed=80)
+    first, more = (Batch(*synth.stretches(x, 500)) for x in (g[:42_600], g[42_600:]))
+    T = kache.Table(31, 8, 40_000, 0.8, True, capi=False)       # 2,048 buckets.
+    u = T.register()
+    T.upsert(u, first, kache.ADD, 1, 1)
+    T.lookup(more)      # The batch's staging is allocated.
+    r = ctypes.c_uint64()
+
+    def upsert():
+        return L.kache_b200_upsert(T.h, u, *more.args(), kache.ADD, 1, 1, ctypes.byref(r))
+
+    try:
+        L.kache_b200_testing_fail_allocation(3)
+        assert upsert() == kache.KACHE_ENOMEM
+        L.kache_b200_testing_fail_allocation(-1)
+        L.kache_b200_testing_device_memory(400_000)     # 8,192 slots of 32 bytes, but not 16,384.
+        assert upsert() == kache.KACHE_OK
+    finally:
+        L.kache_b200_testing_fail_allocation(-1)
+        L.kache_b200_testing_device_memory(-1)
+    O = oracle.OracleTable(31, 8, 40_000, 0.8, True)
+    uo = O.register()
+    O.upsert(uo, first, kache.ADD, 1, 1)
+    assert r.value == O.upsert(uo, more, kache.ADD, 1, 1)
+    assert T.capacity() == O.capacity()
+    kg, vg = T.dump()
+    ko, vo = O.dump()
+    assert T.size() == O.size() and np.array_equal(kg, ko) and np.array_equal(vg, vo)
+    T.close()
