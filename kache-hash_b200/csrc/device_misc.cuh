@@ -570,27 +570,24 @@ static __global__ void __launch_bounds__(stage_block) stage_list_kernel(const St
     }
 }
 
-// Lists the segments of a staged batch that had more of them than its listing took, one thread per segment: its sequence
-// by binary search in seg_off[0..n] (exclusive sums of segments per sequence), so that long sequences' many segments are
-// listed in parallel. Sequence q's bases are at offset
-// off[q], or with `addr` at the address addr[q], where it is of batch batch_of[q].
-static __global__ void segs_kernel(const uint64_t* seg_off, const uint64_t* pos_off, const uint64_t* off, const uint64_t* addr, const uint32_t* batch_of, const uint64_t n,
-                                   const uint64_t nsegs, const uint32_t seg_len, Segment* segs)
+// Lists the segments [sb, se) of a staged batch at `segs`, one thread per segment: its sequence by binary search in
+// seg_off[0..n] (exclusive sums of segments per sequence), so that long sequences' many segments are listed in parallel.
+static __global__ void segs_kernel(const Stage a, const uint64_t sb, const uint64_t se, const uint32_t seg_len, Segment* segs)
 {
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for(uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nsegs; i += stride)
+    for(uint64_t i = sb + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < se; i += stride)
     {
-        uint64_t lo = 0, hi = n;      // The last q with seg_off[q] <= i.
+        uint64_t lo = 0, hi = a.n;      // The last q with seg_off[q] <= i.
         while(hi - lo > 1)
         {
             const uint64_t mid = (lo + hi) / 2;
-            if(seg_off[mid] <= i)
+            if(a.seg_off[mid] <= i)
                 lo = mid;
             else
                 hi = mid;
         }
-        const uint64_t p0 = (i - seg_off[lo]) * seg_len, first = pos_off[lo] + p0;
-        segs[i] = Segment{(addr ? addr[lo] : off[lo]) + p0, first, lo, static_cast<uint32_t>(min(pos_off[lo + 1] - first, static_cast<uint64_t>(seg_len))), batch_of ? batch_of[lo] : 0};
+        const uint64_t first = a.pos_off[lo];
+        segs[i - sb] = stage_segment(a, lo, i - a.seg_off[lo], a.pos_off[lo + 1] - first, first, seg_len);
     }
 }
 

@@ -430,6 +430,11 @@ class Engine final : public kache_table
         // Listed on the device in sequence order: seg_off[q] (device) counts the segments of the sequences before q,
         // so a range of sequences is a range of segments and of output positions. Null where listed otherwise.
         const uint64_t* seg_off = nullptr;
+        // Of a batch listed on the device: how, and the segment length. With list_room, device memory did not take the list
+        // whole: before each launch over list_room segments (at most) these are listed.
+        Stage staged{};
+        uint32_t seg_len = 0;
+        uint64_t list_room = 0;
         // Set where the bases are still in page-locked host memory here, laid end to end (staged with defer_bases).
         const char* host_bases = nullptr;
         // Set where the bases cross in two halves of sequences (ev_in_[0], ev_in_[1]): the table's stream waits for
@@ -831,12 +836,19 @@ class Engine final : public kache_table
         return a;
     }
 
-    // Counts and lists a batch's segments on the device.
+    // Counts and lists a batch's segments on the device (only counts, if there is no memory for the list's usual room).
     void launch_stage(Stage& a)
     {
         // The room is the batch's own, whatever the list has had to hold before: a batch is staged alike at each call.
         a.max_segs = a.n <= small_stage_max ? small_segs_max : a.n + a.n / 8 + 1024;
-        dbatch_.ensure(a.max_segs * sizeof(Segment));
+        try
+        {
+            dbatch_.ensure(a.max_segs * sizeof(Segment));
+        }
+        catch(const std::bad_alloc&)
+        {
+            a.max_segs = 0;
+        }
         a.segs = dbatch_.as<Segment>();
         const unsigned blocks = static_cast<unsigned>((a.n + stage_block - 1) / stage_block);
         if(a.n <= small_stage_max)
@@ -875,6 +887,27 @@ class Engine final : public kache_table
         return c;
     }
 
+    // Makes room for a list of n segments, or where memory does not take it, of a quarter (8 bytes for each of the n); the
+    // segments that there is room for.
+    uint64_t room_for(const uint64_t n)
+    {
+        try
+        {
+            dbatch_.ensure(n * sizeof(Segment));
+            return n;
+        }
+        catch(const std::bad_alloc&)
+        {
+            dbatch_.ensure((n + 3) / 4 * sizeof(Segment));
+            return (n + 3) / 4;
+        }
+    }
+
+    void list_segments(const Batch_Info& bi, const uint64_t sb, const uint64_t se, Segment* const to)
+    {
+        launch(K_OTHER, [&](){ segs_kernel<<<grid_for((se - sb + 31) / 32, 8), 256, 0, stream_>>>(bi.staged, sb, se, bi.seg_len, to); });
+    }
+
     // Prepares a batch already in device memory (or several run as one, their bases' addresses in their segments).
     Batch_Info stage_dev(const uint8_t* bases, Stage a)
     {
@@ -888,14 +921,14 @@ class Engine final : public kache_table
         const uint64_t nsegs = c[4], run = c[6];
         fits_[a.n > small_stage_max] = c[9];
         bi.nsegs = nsegs, bi.total_pos = c[3], bi.off = a.off, bi.pos_off = a.pos_off, bi.seg_off = a.seg_off;
+        bi.staged = a, bi.seg_len = static_cast<uint32_t>(c[5]);
         if(run != nsegs)
         {
-            const uint32_t seg_len = static_cast<uint32_t>(c[5]);
-            dbatch_.ensure(nsegs * sizeof(Segment));
-            launch(K_OTHER, [&]()
-            {
-                segs_kernel<<<grid_for((nsegs + 31) / 32, 8), 256, 0, stream_>>>(a.seg_off, a.pos_off, a.off, a.addr, a.batch_of, a.n, nsegs, seg_len, dbatch_.as<Segment>());
-            });
+            const uint64_t room = room_for(nsegs);
+            if(room < nsegs)
+                bi.list_room = room;
+            else
+                list_segments(bi, 0, nsegs, dbatch_.as<Segment>());
         }
         bi.b = Dev_Batch{bases, dbatch_.as<Segment>()};
         return bi;
@@ -921,6 +954,18 @@ class Engine final : public kache_table
     }
 
     template <typename Vis> void segs_launch(const uint32_t kind, const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Vis& vis)
+    {
+        if(bi.list_room == 0)
+            return rows_launch(kind, bi, sb, se, vis);
+        for(uint64_t b = sb; b < se; b += bi.list_room)
+        {
+            const uint64_t e = std::min(se, b + bi.list_room);
+            list_segments(bi, b, e, dbatch_.as<Segment>());
+            rows_launch(kind, bi, 0, e - b, vis);
+        }
+    }
+
+    template <typename Vis> void rows_launch(const uint32_t kind, const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Vis& vis)
     {
         const Shares s = shares(se - sb, bi.nsegs ? static_cast<double>(bi.total_pos) / static_cast<double>(bi.nsegs) : 0, Vis::min_blocks, bi.fixed_shares);
         if(s.taken)
@@ -1573,9 +1618,17 @@ public:
         try
         {
             p->t = this, p->n = n, p->nsegs = bi.nsegs, p->total_pos = bi.total_pos;
-            p->segs.ensure((bi.nsegs + 1) * sizeof(Segment));
+            try
+            {
+                p->segs.ensure((bi.nsegs + 1) * sizeof(Segment));
+            }
+            catch(const std::bad_alloc&)
+            {
+                dbatch_.release();      // Memory for one list: the handle's.
+                p->segs.ensure((bi.nsegs + 1) * sizeof(Segment));
+            }
             if(bi.nsegs)
-                check(cudaMemcpyAsync(p->segs.p, bi.b.segs, bi.nsegs * sizeof(Segment), cudaMemcpyDeviceToDevice, stream_), "copy");
+                list_segments(bi, 0, bi.nsegs, p->segs.as<Segment>());
             sync();
         }
         catch(...)

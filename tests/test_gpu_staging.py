@@ -128,3 +128,59 @@ def test_a_warp_per_segment_of_a_middling_batch():
     assert 0 < staged < 1.2 * prepared, (staged, prepared)
     T.prepared_free(shape)
     T.close()
+
+
+def test_segment_lists_in_little_memory():
+    """Calls with memory for no more than 24 bytes per sequence and 8 per segment (and, merged, 12 per sequence), where a list
+    takes 32 per segment: its segments are then listed and run a part at a time. A shape prepared with room for one list."""
+    import torch
+    n = 100_000
+    lens = np.full(n, 60)
+    lens[5], lens[n - 3] = 400_000, 20_000
+    b = _batch(lens, 9)
+    bases, off = _on_gpu(b)
+    T, O = kache.Table(31, 4, 5_000_000), oracle.OracleTable(31, 4, 5_000_000)
+    u, uo = T.register(), O.register()
+    P = int(b.positions(31).sum())
+    f, v, c = (torch.zeros(m, dtype=t, device="cuda") for m, t in ((P, torch.uint8), (P, torch.int32), (n, torch.int64)))
+    p, q = bases.data_ptr(), off.data_ptr()
+    cut = n // 3
+    first = int(b.slice(0, cut).positions(31).sum())
+    s = q + 8 * cut
+    torch.cuda.synchronize()
+    few = b.slice(0, 5)
+    assert T.upsert_dev(u, p, q, 5, kache.ADD, 1, 1) == O.upsert(uo, few, kache.ADD, 1, 1)     # The retry marks are made.
+    segs = int(((b.positions(31) + 511) // 512).sum())
+    left = kache.lib().kache_b200_testing_device_memory
+    try:
+        left(24 * n + 12 * segs)
+        assert T.upsert_dev(u, p, q, n, kache.ADD, 1, 1) == O.upsert(uo, b, kache.ADD, 1, 1)
+        assert T.update_dev(p, q, n, kache.ADD, 3) == O.update(b, kache.ADD, 3)
+        T.lookup_dev(p, q, n, f.data_ptr(), v.data_ptr())
+        T.count_dev(p, q, n, c.data_ptr())
+        fo, vo, _ = O.lookup(b)
+        co = O.count(b)
+        assert np.array_equal(f.cpu().numpy(), fo) and np.array_equal(v.cpu().numpy().view(np.uint32), vo)
+        assert np.array_equal(c.cpu().numpy().view(np.uint64), co)
+        left(16 * n)
+        hits = [int((fo[:first] == 1).sum()), int((fo[first:] == 1).sum())]
+        f.fill_(7)
+        torch.cuda.synchronize()
+        assert T.run_dev_batches(kache.RUN_LOOKUP, [(p, q, cut, f.data_ptr(), v.data_ptr()), (p, s, n - cut, f.data_ptr() + first, v.data_ptr() + 4 * first)]) == hits
+        assert np.array_equal(f.cpu().numpy(), fo)
+        assert sum(T.run_dev_batches(kache.RUN_UPSERT, [(p, q, cut), (p, s, n - cut)], kache.ADD, 1, 1, u)) == O.upsert(uo, b, kache.ADD, 1, 1)
+        left(30 * segs)     # With the 8 per segment that the table holds.
+        shape = T.prepare_dev(q, n)
+        f.fill_(7)
+        torch.cuda.synchronize()
+        T.lookup_prepared(shape, p, f.data_ptr(), v.data_ptr())
+        torch.cuda.synchronize()
+        fo, vo, _ = O.lookup(b)
+        assert np.array_equal(f.cpu().numpy(), fo) and np.array_equal(v.cpu().numpy().view(np.uint32), vo)
+        T.prepared_free(shape)
+    finally:
+        left(-1)
+    kg, vg = T.dump()
+    ko, vo = O.dump()
+    assert np.array_equal(kg, ko) and np.array_equal(vg, vo)
+    T.close()
