@@ -145,3 +145,101 @@ def test_large_launches_equal_prepared_ones(n, length):
     assert int(v[f == 1].min()) >= 1
     G.prepared_free(p)
     G.close()
+
+
+@pytest.mark.parametrize("op,x,init", [(kache.ADD_WRAP, 1, 1), (kache.MIN, 3, 9)])
+def test_upserts_by_the_work_counter(op, x, init):
+    """121,000 reads of 121 k-mers, whose warps take segments from a counter, one of an operation that commutes and one
+    that waits for a racing insert; as one batch and as two."""
+    import torch
+    g = synth.genome(1_000_000, seed=85)
+    b = Batch(*synth.reads_fixed(g, 121_000, 151, seed=86))
+    bases, offs = _dev(b.bases, b.off)
+    G, O = kache.Table(31, 4, 30_000_000), oracle.OracleTable(31, 4, 30_000_000)
+    u, uo = G.register(), O.register()
+    torch.cuda.synchronize()
+    p, o, cut = bases.data_ptr(), offs.data_ptr(), 500
+    assert G.upsert_dev(u, p, o, b.n, op, x, init) == O.upsert(uo, b, op, x, init)
+    parts = [(p, o, cut), (p, o + 8 * cut, b.n - cut)]
+    assert G.run_dev_batches(kache.RUN_UPSERT, parts, op, x, init, u) == [0, 0]
+    O.upsert(uo, b, op, x, init)
+    assert sum(G.run_dev_batches(kache.RUN_UPDATE, parts, kache.ADD, 2)) == O.update(b, kache.ADD, 2)
+    kg, vg = G.dump()
+    ko, vo = O.dump()
+    assert G.size() == O.size() and np.array_equal(kg, ko) and np.array_equal(vg, vo)
+    f, _, _ = O.lookup(b)
+    d = torch.zeros(len(f), dtype=torch.uint8, device="cuda")
+    c = torch.zeros(b.n, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    first = 121 * cut
+    hits = G.run_dev_batches(kache.RUN_LOOKUP, [parts[0] + (d.data_ptr(),), parts[1] + (d.data_ptr() + first,)])
+    assert hits == [int((f[:first] == 1).sum()), int((f[first:] == 1).sum())]
+    assert G.run_dev_batches(kache.RUN_COUNT, [parts[0] + (c.data_ptr(),), parts[1] + (c.data_ptr() + 8 * cut,)]) == hits
+    assert np.array_equal(d.cpu().numpy(), f) and np.array_equal(c.cpu().numpy().view(np.uint64), O.count(b))
+    G.close()
+
+
+@pytest.mark.parametrize("vb", [0, 2, 8])
+def test_overflow_grows_behind_a_staged_upsert(vb):
+    """Device upserts of 10,000 keys of one minimizer, of which 96 have room in buckets: the overflow table's 2,048 slots
+    fill up, and the k-mers left over are upserted again in larger ones, from the list that was staged."""
+    import torch
+    b = Batch(*synth.one_minimizer(1000, 87))
+    bases, offs = _dev(b.bases, b.off)
+    G, O = kache.Table(31, vb, 20_000), oracle.OracleTable(31, vb, 20_000)
+    u, uo = G.register(), O.register()
+    torch.cuda.synchronize()
+    p, o = bases.data_ptr(), offs.data_ptr()
+    G.profile(True)
+    ins = G.upsert_dev(u, p, o, b.n, kache.ADD, 1, 1)
+    assert G.profile_read(0)[1] > 2     # The launch, and at least two more after the overflow table's growth.
+    assert ins == O.upsert(uo, b, kache.ADD, 1, 1) and G.stats().overflow_keys > 9000
+    assert sum(G.run_dev_batches(kache.RUN_UPSERT, [(p, o, 300), (p, o + 2400, 700)], kache.ADD, 1, 1, u)) == O.upsert(uo, b, kache.ADD, 1, 1)
+    kg, vg = G.dump()
+    ko, vo = O.dump()
+    assert np.array_equal(kg, ko) and (vb == 0 or np.array_equal(vg, vo))
+    c = torch.zeros(b.n, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    G.count_dev(p, o, b.n, c.data_ptr())
+    assert np.array_equal(c.cpu().numpy().view(np.uint64), O.count(b))
+    G.close()
+
+
+def test_slot_given_up_for_a_lower_claim():
+    """A read's ten new keys of one bucket, the fourth of which has a claim there already that was never published: the keys
+    claim slots side by side, the fourth then finds the earlier claim in the slot that the first one lost, and leaves its
+    own slot as a hole. Nobody sees the hole, and later keys of the bucket go past it."""
+    b = Batch(*synth.one_minimizer(200, 88))
+    one = b.slice(0, 1)
+    kmer = bytes(b.bases[3:34])
+    G, O = kache.Table(31, 4, 20_000), oracle.OracleTable(31, 4, 20_000)
+    u, uo = G.register(), O.register()
+    assert kache.lib().kache_b200_testing_plant_claim(G.h, kmer, 1000) == kache.KACHE_OK
+    O.upsert(uo, one, kache.ADD, 1, 1)
+    assert G.upsert(u, one, kache.ADD, 1, 1) == 9
+    O.upsert(uo, b.slice(1, 200), kache.ADD, 1, 1)
+    assert G.upsert(u, b.slice(1, 200), kache.ADD, 1, 1) == O.size() - 10
+    ko, vo = O.dump()
+    fo, _, _ = O.lookup(b)
+    kg, vg = G.dump()
+    f, v, _ = G.lookup(b)
+    missing = np.setdiff1d(ko, kg)      # The planted k-mer's, which is not published.
+    assert len(missing) == 1 and len(kg) == len(ko) - 1
+    assert np.array_equal(kg, ko[ko != missing]) and np.array_equal(vg, vo[ko != missing])
+    assert fo[3] == 1 and f[3] == 0 and np.array_equal(np.delete(f, 3), np.delete(fo, 3))
+    assert G.size() == len(kg) == G.reduce(kache.REDUCE_KEYS)
+    G.close()
+
+
+@pytest.mark.parametrize("vb", [2, 4])
+def test_histogram_past_a_blocks_bins(vb):
+    """Counts on both sides of the 8,192 that a block holds, and of the largest asked for."""
+    g = synth.genome(5000, seed=89)
+    G, O = kache.Table(31, vb, 10_000), oracle.OracleTable(31, vb, 10_000)
+    u, uo = G.register(), O.register()
+    for i, x in enumerate((1, 8190, 8191, 8192, 8193, 9999, 10_000, 10_001, 65_535)):
+        b = Batch(*synth.stretches(g[500 * i:500 * i + 130 + i], 1000))
+        assert G.upsert(u, b, kache.ASSIGN, x, x) == O.upsert(uo, b, kache.ASSIGN, x, x)
+    for m in (0, 1, 8190, 8191, 8192, 8193, 10_000, 70_000):
+        assert np.array_equal(G.histogram(m), O.histogram(m))
+    G.close()
