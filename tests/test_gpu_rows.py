@@ -243,3 +243,22 @@ def test_histogram_past_a_blocks_bins(vb):
     for m in (0, 1, 8190, 8191, 8192, 8193, 10_000, 70_000):
         assert np.array_equal(G.histogram(m), O.histogram(m))
     G.close()
+
+
+@pytest.mark.parametrize("vb", [1, 2, 4])
+@pytest.mark.parametrize("x", [1, 200, 255])
+def test_wrapping_adds_to_hot_keys(vb, x):
+    """Values of 1, 2 and 4 bytes that wrap around many times, added to from all warps at once; then an operation that
+    compares the whole values."""
+    x = x * 257 if vb == 2 else x
+    b = Batch.of([b"ACGTTGCAAC" * 15] * 3000 + [b"A" * 150] * 1000 + [_rand(np.random.default_rng(i % 50), 150) for i in range(3000)])
+    G, O = kache.Table(31, vb, 20_000), oracle.OracleTable(31, vb, 20_000)
+    u, uo = G.register(), O.register()
+    for _ in range(2):
+        assert G.upsert(u, b, kache.ADD_WRAP, x, 3) == O.upsert(uo, b, kache.ADD_WRAP, x, 3)
+        assert G.update(b, kache.ADD_WRAP, x, capi=False) == O.update(b, kache.ADD_WRAP, x)
+        assert np.array_equal(G.dump()[1], O.dump()[1])
+    assert G.update(b, kache.MAX, 77, capi=False) == O.update(b, kache.MAX, 77)
+    assert G.update(b, kache.ADD, 100) == O.update(b, kache.ADD, 100)
+    assert np.array_equal(G.dump()[1], O.dump()[1])
+    G.close()
