@@ -212,7 +212,8 @@ __device__ __forceinline__ bool slot_value(const Dev_Table& T, const uint64_t s,
     const uint64_t n_main = T.cap * B;
     if(s < n_main)
     {
-        if(*cs_of(T, static_cast<uint32_t>(s / B), s % B) == 0)
+        // A set has no values, so its checksums can be taken in the order they lie in.
+        if((set_ ? T.cs[s] : *cs_of(T, static_cast<uint32_t>(s / B), s % B)) == 0)
             return false;
         if constexpr(!set_)
             raw = T.slots[s * 2 + 1];
