@@ -347,14 +347,15 @@ struct Stage
     uint32_t* batch_of;
     uint64_t* pos_base;
     bool zero_out0;             // Zeroes each sequence's word of its batch's out0.
+    bool group;                 // May make groups (of more than small_stage_max sequences).
     uint64_t n;
     int k;
     uint32_t sms;
     uint64_t max_segs, max_pos;
-    uint64_t *npos, *pos_off, *seg_off;     // Positions of each sequence; n + 1 sums of positions and of segments.
-    unsigned long long* blocks;     // Two words per block of stage_count_kernel: the positions and segments before it.
-    Segment* segs;
-    unsigned long long* ctr;    // [0] and the low half of [2] are zeroed; [3..6]: positions, segments, segment length, segments to run; [7]: zero between launches; [8] is zeroed; [9]: whether the segments fit the list.
+    uint64_t *npos, *pos_off, *seg_off;     // Positions of each sequence, with in_group; n + 1 sums of positions and of segments.
+    unsigned long long* blocks;     // Two words per block of stage_count_kernel: the positions before it, the segments and groups (entries).
+    Segment *segs, *groups;
+    unsigned long long* ctr;    // [0] and the low half of [2] are zeroed; [3..6]: positions, segments, segment length, segments to run; [7]: zero between launches; [8] is zeroed; [9]: whether the segments fit the list; [10], [11]: groups to run, and listed.
     unsigned long long* zero;   // zero_n words zeroed.
     uint64_t zero_n;
 };
@@ -383,6 +384,45 @@ __device__ __forceinline__ uint64_t stage_length(const Stage& a, const uint64_t 
     if(a.zero_out0)
         reinterpret_cast<uint64_t*>(d[4])[j] = 0;
     return reinterpret_cast<const uint64_t*>(d[1])[j + 1] - b0;
+}
+
+constexpr uint64_t in_group = uint64_t(1) << 63;
+
+// Segments and groups are counted together, in 34 bits and 30.
+constexpr int group_shift = 34;
+constexpr uint64_t segs_mask = (uint64_t(1) << group_shift) - 1;
+__device__ __forceinline__ uint64_t entries(const uint64_t q, const uint64_t np, const bool g)
+{
+    return g ? uint64_t(q % group_seqs == 0) << group_shift : (np + seg_positions - 1) / seg_positions;
+}
+
+// Whether the calling lane's sequence q, of batch `lo`, is of a group (device_stream.cuh): groups of short sequences, the first a
+// multiple of group_seqs, are made where that saves instructions, in units of ten: 45 for a row of a group and 1 for 23 of its
+// bases against 31 for a row of a sequence and 13 to start on one. A whole warp, with consecutive sequences.
+__device__ __forceinline__ bool grouped(const Stage& a, const uint64_t q, const uint64_t len, const uint64_t np, const uint64_t lo)
+{
+    constexpr uint32_t all = 0xFFFFFFFFu;
+    if(!a.group)
+        return false;
+    const int leader = static_cast<int>(threadIdx.x & 31 & ~(group_seqs - 1));
+    const uint64_t lo_leader = __shfl_sync(all, lo, leader);    // (All lanes take part: not behind a condition.)
+    const bool ok = q < a.n && len <= group_len && lo == lo_leader;
+    const uint32_t no = (__ballot_sync(all, !ok) >> leader) & ((1u << group_seqs) - 1);
+    // Bases, positions and rows of the sequences by themselves, in 12 bits, 12 and 8.
+    uint32_t x = ok ? static_cast<uint32_t>(len << 20 | np << 8 | (np + 31) / 32) : 0;
+#pragma unroll
+    for(uint32_t o = 1; o < group_seqs; o *= 2)
+        x += __shfl_xor_sync(all, x, o);
+    const uint32_t bases = x >> 20, pos = x >> 8 & 0xFFFu, rows = x & 0xFFu;
+    return no == 0 && pos > 0 && 45 * ((pos + 31) / 32) + bases / 23 + 10 < 31 * rows + 13 * group_seqs;
+}
+
+// The group that starts at sequence q: `pos` positions, from `first` on, the last sequence's np_last among them.
+__device__ __forceinline__ Segment stage_group(const Stage& a, const uint64_t q, const uint64_t pos, const uint64_t first, const uint64_t np_last)
+{
+    const uint64_t* at = (a.desc ? a.addr : a.off) + q;
+    const uint64_t bases = at[group_seqs - 1] - at[0] + (np_last ? np_last + a.k - 1 : 0);
+    return Segment{at[0], first, q, group_word(static_cast<uint32_t>(pos), static_cast<uint32_t>(bases)), a.desc ? a.batch_of[q] : 0};
 }
 
 // Segment number i of sequence q, which starts at `first` of its np positions.
@@ -466,7 +506,7 @@ static __global__ void __launch_bounds__(stage_block) stage_small_kernel(const S
     {
         a.pos_off[a.n] = total, a.seg_off[a.n] = nsegs;
         a.ctr[3] = total, a.ctr[4] = nsegs, a.ctr[5] = seg_len, a.ctr[6] = run;
-        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[8] = 0, a.ctr[9] = nsegs <= a.max_segs;
+        a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[8] = 0, a.ctr[9] = nsegs <= a.max_segs, a.ctr[10] = 0, a.ctr[11] = 0;
     }
     __syncthreads();
     for(uint32_t i = t; i < run; i += stage_block)
@@ -494,17 +534,19 @@ static __global__ void __launch_bounds__(stage_block) stage_count_kernel(const S
     __shared__ bool last;
     const uint32_t t = threadIdx.x;
     const uint64_t q = uint64_t(blockIdx.x) * stage_block + t;
-    uint64_t np = 0, lo = 0;
+    uint64_t np = 0, len = 0, lo = 0;
     if(q < a.n)
     {
-        const uint64_t len = stage_length(a, q, lo, true);
+        len = stage_length(a, q, lo, true);
         np = len >= uint64_t(a.k) ? len - a.k + 1 : 0;
-        a.npos[q] = np;
     }
+    const bool g = grouped(a, q, len, np, lo);
+    if(q < a.n)
+        a.npos[q] = g ? np | in_group : np;
     for(uint64_t i = q; i < a.zero_n; i += uint64_t(gridDim.x) * stage_block)
         a.zero[i] = 0;
     block_sum(np, wp);
-    block_sum((np + seg_positions - 1) / seg_positions, ws);
+    block_sum(entries(q, np, g), ws);
     if(t == 0)
     {
         __stcg(a.blocks + 2 * blockIdx.x, wp[31]), __stcg(a.blocks + 2 * blockIdx.x + 1, ws[31]);
@@ -521,7 +563,7 @@ static __global__ void __launch_bounds__(stage_block) stage_count_kernel(const S
         const uint64_t b = b0 + t;
         const unsigned long long p = b < gridDim.x ? __ldcg(a.blocks + 2 * b) : 0, s = b < gridDim.x ? __ldcg(a.blocks + 2 * b + 1) : 0;
         const unsigned long long p1 = block_sum(p, wp), s1 = block_sum(s, ws);
-        if(s > small_segs_max)
+        if((s & segs_mask) > small_segs_max)
             atomicMax(&most, s);
         if(b < gridDim.x)
             a.blocks[2 * b] = P + p1 - p, a.blocks[2 * b + 1] = S + s1 - s;
@@ -530,14 +572,16 @@ static __global__ void __launch_bounds__(stage_block) stage_count_kernel(const S
     __syncthreads();
     if(t == 0)
     {
-        const bool fits = S <= a.max_segs && most == 0;
-        a.pos_off[a.n] = P, a.seg_off[a.n] = S;
-        a.ctr[3] = P, a.ctr[4] = S, a.ctr[5] = seg_positions, a.ctr[6] = fits && P <= a.max_pos ? S : 0;
+        const uint64_t segs = S & segs_mask, groups = S >> group_shift;
+        const bool fits = segs <= a.max_segs && most == 0, run = fits && P <= a.max_pos;
+        a.pos_off[a.n] = P, a.seg_off[a.n] = segs;
+        a.ctr[3] = P, a.ctr[4] = segs, a.ctr[5] = seg_positions, a.ctr[6] = run ? segs : 0;
         a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[7] = 0, a.ctr[8] = 0, a.ctr[9] = fits;
+        a.ctr[10] = run ? groups : 0, a.ctr[11] = groups;
     }
 }
 
-// Second launch: each block sums its own sequences and lists their segments. A thread writes an entry in some 30 ns, so it
+// Second launch: each block sums its own sequences and lists their segments and groups. A thread writes an entry in some 30 ns, so it
 // lists its own sequence if that has up to own_segs; a longer one's are listed by its warp, an entry per lane. (A thread
 // each took 5.9 ms for 5,000 sequences one of which has 90 Mbp, and 1.67 for 200,000 with one of 25 Mbp.)
 constexpr uint32_t own_segs = 32;
@@ -546,21 +590,33 @@ static __global__ void __launch_bounds__(stage_block) stage_list_kernel(const St
 {
     __shared__ unsigned long long wp[32], ws[32];
     const uint64_t q = uint64_t(blockIdx.x) * stage_block + threadIdx.x;
-    const uint64_t np = q < a.n ? a.npos[q] : 0, ns = (np + seg_positions - 1) / seg_positions;
-    const unsigned long long first = a.blocks[2 * blockIdx.x] + block_sum(np, wp) - np, first_seg = a.blocks[2 * blockIdx.x + 1] + block_sum(ns, ws) - ns;
+    constexpr uint32_t all = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31;
+    uint64_t np = q < a.n ? a.npos[q] : 0;
+    const bool g = np & in_group;
+    np &= ~in_group;
+    const uint64_t x = entries(q, np, g), ns = x & segs_mask;
+    const unsigned long long first = a.blocks[2 * blockIdx.x] + block_sum(np, wp) - np, before = a.blocks[2 * blockIdx.x + 1] + block_sum(x, ws) - x;
+    const uint64_t first_seg = before & segs_mask;
     if(q < a.n)
     {
         a.pos_off[q] = first, a.seg_off[q] = first_seg;
         if(a.desc && a.desc[8 * uint64_t(a.batch_of[q]) + 3] == q)
             a.pos_base[a.batch_of[q]] = first;
     }
+    if(__any_sync(all, g))
+    {
+        // The positions up to the group's end, from its last lane.
+        const int end = static_cast<int>(lane | (group_seqs - 1));
+        const uint64_t to = __shfl_sync(all, first + np, end), np_last = __shfl_sync(all, np, end);
+        if(x >> group_shift)
+            a.groups[before >> group_shift] = stage_group(a, q, to - first, first, np_last);
+    }
     if(a.ctr[6] == 0)
         return;
     if(ns <= own_segs)
         for(uint64_t i = 0; i < ns; ++i)
             a.segs[first_seg + i] = stage_segment(a, q, i, np, first, seg_positions);
-    constexpr uint32_t all = 0xFFFFFFFFu;
-    const uint32_t lane = threadIdx.x & 31;
     for(uint32_t m = __ballot_sync(all, ns > own_segs); m; m &= m - 1)
     {
         const int s = __ffs(m) - 1;

@@ -38,9 +38,17 @@ struct alignas(16) Segment
     uint64_t base;      // Its first base, as an offset from the batch's bases.
     uint64_t pos;       // Its first position, counted over the batch's sequences.
     uint64_t q;         // Its sequence.
-    uint32_t npos;      // Its positions.
+    uint32_t npos;      // Its positions. (Of a group, see below: group_word.)
     uint32_t batch;     // Its batch, of several run as one.
 };
+
+// A group: group_seqs sequences, in order and of one batch, of up to group_len bases each, whose k-mers are a warp's rows of 32
+// together (group_kernel); its entry has its first sequence's q, and base and pos where that starts. Sequences of few k-mers
+// leave most lanes of a row idle by themselves: 2M reads of 33 bases, three 31-mers each, took 1,040 us to count and 1,484 to
+// upsert, in groups 341 and 503.
+constexpr uint32_t group_seqs = 8, group_len = 124;
+
+__device__ __forceinline__ uint32_t group_word(const uint32_t npos, const uint32_t bases) { return bases << 10 | npos; }
 
 // What visitors get of a segment.
 struct Seg_Of
@@ -55,6 +63,10 @@ struct Dev_Batch
 {
     const uint8_t* bases;
     const Segment* segs;
+    // Groups, and for them where each sequence starts, as Segment::base says, and the positions before it.
+    const Segment* groups;
+    const uint64_t* start;
+    const uint64_t* pos_off;
 };
 
 constexpr int stream_warps = 8;
@@ -234,6 +246,98 @@ __global__ void __launch_bounds__(32 * stream_warps, Visitor::min_blocks) stream
         vis.begin_segment(s);
         describe_segment<k, l>(batch.bases + base, npos, ring_all[wid], tab, lane, vis);
         vis.end_segment(s, lane);
+    }
+    vis.end(lane);
+}
+
+// The planes of a group's bases, end to end in `planes`: 32 words each of high and low code bits and of flags.
+__device__ __forceinline__ void pack_group(const uint8_t* const seq, const uint32_t bases, uint32_t* const planes, const uint8_t* const tab, const uint32_t lane)
+{
+#pragma unroll 1
+    for(uint32_t o = 0; o < bases; o += 128)
+    {
+        uint32_t ch[4];
+#pragma unroll
+        for(int i = 0; i < 4; ++i)
+            ch[i] = o + 32 * i + lane < bases ? __ldg(seq + o + 32 * i + lane) : 0u;
+#pragma unroll
+        for(int i = 0; i < 4; ++i)
+        {
+            const Row r = pack_row(ch[i], tab);
+            if(lane == 0)
+                planes[o / 32 + i] = r.hi, planes[32 + o / 32 + i] = r.lo, planes[64 + o / 32 + i] = r.valid;
+        }
+    }
+    __syncwarp();
+}
+
+// The k-mer at position j of a group, whose sequence number i starts at first (in lane i) of its positions and `from` of its
+// bases; its sequence's number goes to `i`. The lanes' k-mers are not all neighbours, so each lane hashes the w l-mers of
+// its own.
+template <int k, int l>
+__device__ __forceinline__ Kmer_Desc group_kmer(const uint32_t j, const uint32_t* const planes, const uint32_t first, const uint32_t from, uint32_t& i)
+{
+    constexpr uint32_t all = 0xFFFFFFFFu, km = (k == 32 ? ~0u : (1u << k) - 1), lm = (1u << l) - 1;
+    i = 0;      // The last one that starts at or before j.
+#pragma unroll
+    for(uint32_t step = group_seqs / 2; step; step /= 2)
+        i += __shfl_sync(all, first, i + step) <= j ? step : 0;
+    const uint32_t b = __shfl_sync(all, from, i) + (j - __shfl_sync(all, first, i));
+    const uint32_t* p = planes + (b >> 5);
+    const uint32_t hi = __funnelshift_r(p[0], p[1], b), lo = __funnelshift_r(p[32], p[33], b);
+    const Planes f{__brev(hi) >> (32 - k), __brev(lo) >> (32 - k)}, r{~hi & km, ~lo & km};
+    const bool gt = planes_greater(f, r);
+    Kmer_Desc d;
+    d.key = gt ? key_of(r) : key_of(f);
+    d.fwd = !gt;
+    d.valid = (__funnelshift_r(p[64], p[65], b) & km) == km;
+    d.h = ~0u;
+#pragma unroll
+    for(int x = 0; x <= k - l; ++x)
+        d.h = min(d.h, lmer_hash(Planes{(f.hi >> (k - l - x)) & lm, (f.lo >> (k - l - x)) & lm}, Planes{(r.hi >> x) & lm, (r.lo >> x) & lm}));
+    return d;
+}
+
+// The kernel over groups [grp_b, grp_end), or as many as `run` says, counted by the kernel before. A row costs some 430
+// instructions, where a segment's costs 330 and its start 120: which sequences make a group is staging's choice (`grouped`).
+// A kernel of its own, behind the one over segments: as a branch of that one it cost the rows of 150 bp reads 4 to 6 %, whose
+// registers are few enough as it is, and with one loop for both kinds of row they took three times as long.
+template <int k, int l, typename Visitor>
+__global__ void __launch_bounds__(32 * stream_warps, Visitor::min_blocks) group_kernel(const Dev_Batch batch, const uint64_t grp_b, const uint64_t grp_end, const unsigned long long* run, Visitor vis)
+{
+    __shared__ uint32_t planes_all[stream_warps][96];
+    __shared__ uint8_t tab[base_table_bytes];
+    fill_base_table(tab);
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr uint32_t all = 0xFFFFFFFFu;
+    uint32_t* const planes = planes_all[wid];
+    vis.begin();
+    const uint64_t grp_e = run ? static_cast<uint64_t>(*run) : grp_end, warps = uint64_t(gridDim.x) * stream_warps;
+    for(uint64_t g = grp_b + uint64_t(blockIdx.x) * stream_warps + wid; g < grp_e; g += warps)
+    {
+        const Segment e = batch.groups[g];
+        const Seg_Of s{e.q, e.pos, e.batch};
+        const uint32_t npos = e.npos & 0x3FFu;
+        // Lane i has where the group's sequence i starts, in its bases and in its positions.
+        uint32_t from = 0, first = ~0u;
+        if(lane < group_seqs)
+            from = static_cast<uint32_t>(batch.start[s.q + lane] - e.base), first = static_cast<uint32_t>(batch.pos_off[s.q + lane] - s.pos);
+        pack_group(batch.bases + e.base, e.npos >> 10, planes, tab, lane);
+        vis.begin_segment(s);
+#pragma unroll 1
+        for(uint32_t o = 0; o < npos; o += 32)
+        {
+            uint32_t i;
+            Kmer_Desc d = group_kmer<k, l>(min(o + lane, npos - 1), planes, first, from, i);
+            d.pos = o + lane;
+            d.in = d.pos < npos;
+            d.valid = d.valid && d.in;
+            vis.visit(d, lane);
+            if constexpr(requires { vis.end_group_row(s, i, lane); })
+                vis.end_group_row(s, i, lane);
+        }
+        vis.end_segment(s, lane);
+        __syncwarp(all);
     }
     vis.end(lane);
 }
@@ -479,7 +583,7 @@ struct Lookup_Batches_Visitor : Lookup_Visitor<set_, V>
 };
 
 // Per-sequence reductions over lookups (capi/Kmer_Table.hpp:134-161): 0 count, 1 masked count, 2 sum. A segment
-// belongs to one sequence, so each warp adds its segment's total once.
+// belongs to one sequence, so each warp adds its segment's total once; of a group's row, each sequence's lanes add theirs.
 template <bool set_, typename V, int mode_>
 struct Seq_Reduce_Visitor
 {
@@ -491,18 +595,43 @@ struct Seq_Reduce_Visitor
 
     __device__ __forceinline__ void begin() {}
     __device__ __forceinline__ void begin_segment(const Seg_Of&) { acc = 0; }
-    __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t)
+    // What the k-mer adds.
+    __device__ __forceinline__ unsigned long long term(const Kmer_Desc& d) const
     {
         const Found<set_, !set_ && mode_ != 0> f(T, d);
         if(!f.hit)
-            return;
+            return 0;
         if constexpr(mode_ == 0)
-            acc += 1;
+            return 1;
         else if constexpr(mode_ == 1)
-            acc += (value_of<V>(f.val) & (d.fwd ? m_fwd : m_rev)) != 0;
+            return (value_of<V>(f.val) & (d.fwd ? m_fwd : m_rev)) != 0;
         else
-            acc += static_cast<unsigned long long>(value_of<V>(f.val));
+            return static_cast<unsigned long long>(value_of<V>(f.val));
     }
+    __device__ __forceinline__ void visit(const Kmer_Desc& d, const uint32_t) { acc += term(d); }
+    // After a group's row, whose lanes are of the group's sequences i in order: adds what each sequence's lanes have to its
+    // word of `counts`. With lanes' terms of 0 and 1, returns how many are 1.
+    __device__ __forceinline__ uint32_t flush_row(unsigned long long* counts, const uint32_t i, const uint32_t lane)
+    {
+        constexpr uint32_t all = 0xFFFFFFFFu;
+        const uint32_t ones = __ballot_sync(all, acc != 0), left = __shfl_up_sync(all, i, 1);
+        const uint32_t heads = __ballot_sync(all, lane == 0 || i != left);
+        if constexpr(mode_ == 2)
+        {
+            if(acc)
+                atomicAdd(counts + i, acc);
+        }
+        else if(heads >> lane & 1)
+        {
+            const uint32_t from = all << lane, next = heads & (from << 1);
+            const uint32_t n = __popc(ones & (next ? from & ((next & (0u - next)) - 1) : from));
+            if(n)
+                atomicAdd(counts + i, static_cast<unsigned long long>(n));
+        }
+        acc = 0;
+        return __popc(ones);
+    }
+    __device__ __forceinline__ void end_group_row(const Seg_Of& s, const uint32_t i, const uint32_t lane) { flush_row(out + s.q, i, lane); }
     __device__ __forceinline__ unsigned long long seg_total() const
     {
         unsigned long long a = acc;
@@ -527,14 +656,23 @@ struct Count_Batches_Visitor : Seq_Reduce_Visitor<set_, V, 0>
     const uint64_t* outs;       // Per batch, 8 words: its first merged sequence at word 3, its counts' address at word 4.
     unsigned long long* per_batch;
 
+    uint32_t grouped = 0;       // Found in the rows of the current group.
+
+    __device__ __forceinline__ void end_group_row(const Seg_Of& s, const uint32_t i, const uint32_t lane)
+    {
+        const uint64_t* o = outs + 8 * uint64_t(s.batch);
+        grouped += this->flush_row(reinterpret_cast<unsigned long long*>(o[4]) + (s.q - o[3]), i, lane);
+    }
     __device__ __forceinline__ void end_segment(const Seg_Of& s, const uint32_t lane)
     {
-        const unsigned long long a = this->seg_total();
-        if(lane == 0 && a)
+        const unsigned long long a = this->seg_total(), n = a + grouped;
+        grouped = 0;
+        if(lane == 0 && n)
         {
             const uint64_t* o = outs + 8 * uint64_t(s.batch);
-            atomicAdd(reinterpret_cast<unsigned long long*>(o[4]) + (s.q - o[3]), a);
-            atomicAdd(per_batch + s.batch, a);
+            if(a)
+                atomicAdd(reinterpret_cast<unsigned long long*>(o[4]) + (s.q - o[3]), a);
+            atomicAdd(per_batch + s.batch, n);
         }
     }
 };

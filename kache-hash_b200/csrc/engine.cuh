@@ -405,6 +405,7 @@ class Engine final : public kache_table
     }
     Pinned_Buf pin_piece_;
     Dev_Buf dbatch_, dout_, dretry_a_, dretry_b_, dtmp_;
+    Dev_Buf dgroups_;   // The groups of the batch in dbatch_.
     Dev_Buf dhost_;     // A page-locked host batch's bases and offsets, copied as they lie.
     Dev_Buf dmulti_;    // Several device batches run as one: their descriptors and the merged sequence list.
     Pinned_Buf pin_multi_;
@@ -417,17 +418,19 @@ class Engine final : public kache_table
     uint64_t prof_n_[K_KINDS] = {};
 
     // Device counters: [0] inserted/present, [1] overflow keys, [2] retry flag + error word, [3..6] scratch, or what staging
-    // counted, [7] its blocks done, [8] the work counter, [9] whether the staged segments fitted their list (see Stage::ctr).
-    static constexpr size_t ctr_bytes = 10 * 8;
+    // counted, [7] its blocks done, [8] the work counter, [9] whether the staged segments fitted their list, [10..11] groups (see Stage::ctr).
+    static constexpr int ctr_words = 12;
+    static constexpr size_t ctr_bytes = ctr_words * 8;
     unsigned long long* ctr() const { return ctr_.as<unsigned long long>(); }
 
     struct Batch_Info
     {
         Dev_Batch b{};
-        uint64_t n = 0, nsegs = 0, total_pos = 0;
+        uint64_t n = 0, nsegs = 0, ngroups = 0, total_pos = 0;
+        uint64_t entries() const { return nsegs + ngroups; }     // Groups are counted on from the segments.
         // Of a batch listed on the device, in sequence order: device arrays of the offsets of the sequences' bases, and of the
-        // positions and segments before each (n + 1 each), so that a range of sequences is a range of bases, of output
-        // positions and of segments. Null where listed otherwise.
+        // positions and segments before each (n + 1 each), so that a range of sequences, if there are no groups, is a range of
+        // bases, of output positions and of segments. Null where listed otherwise.
         const uint64_t *off = nullptr, *pos_off = nullptr, *seg_off = nullptr;
         // Of a batch listed on the device: how, and the segment length. With list_room, device memory did not take the list
         // whole: before each launch over list_room segments (at most) these are listed.
@@ -648,7 +651,7 @@ class Engine final : public kache_table
     }
 
     Batch_Info stage_host(const char* const* seqs, const size_t* lens, const size_t n, const bool defer_bases = false,
-                          const Host_Scan* scanned = nullptr)
+                          const Host_Scan* scanned = nullptr, const bool group = true)
     {
         const Host_Scan hs = scanned ? *scanned : scan_host(seqs, lens, n);
         const uint64_t bytes = hs.bytes, max_pos = hs.max_pos, all_pos = hs.all_pos;
@@ -691,7 +694,7 @@ class Engine final : public kache_table
                     check(cudaMemcpyAsync(d + b_half, base + b_half, bytes - b_half, cudaMemcpyHostToDevice, in_stream_), "H2D batch");
                 check(cudaEventRecord(ev_bases_, in_stream_), "event record");
             }
-            Batch_Info bi = stage_dev(reinterpret_cast<const uint8_t*>(d), reinterpret_cast<const uint64_t*>(d + o_off), n);
+            Batch_Info bi = stage_dev(reinterpret_cast<const uint8_t*>(d), reinterpret_cast<const uint64_t*>(d + o_off), n, group && !halves);
             if(defer_bases)
             {
                 bi.host_bases = base;
@@ -709,7 +712,7 @@ class Engine final : public kache_table
             return bi;
         }
         if(n >= host_list_max)
-            return stage_gathered(seqs, lens, n, bytes);
+            return stage_gathered(seqs, lens, n, bytes, group);
         const uint32_t seg_len = fitted_seg_len(all_pos, static_cast<uint32_t>(sm_count_));
         uint64_t nsegs = 0;
         for(size_t i = 0; i < n; ++i)
@@ -762,7 +765,7 @@ class Engine final : public kache_table
         if(whole && o_bases + bytes > 0)
             check(cudaMemcpyAsync(d, pin_.p, o_bases + bytes, cudaMemcpyHostToDevice, stream_), "H2D batch");
         Batch_Info bi;
-        bi.b = Dev_Batch{reinterpret_cast<const uint8_t*>(d + o_bases), reinterpret_cast<const Segment*>(d)};
+        bi.b = Dev_Batch{reinterpret_cast<const uint8_t*>(d + o_bases), reinterpret_cast<const Segment*>(d), nullptr, nullptr, nullptr};
         bi.n = n, bi.nsegs = nsegs;
         bi.total_pos = p;
         return bi;
@@ -773,7 +776,7 @@ class Engine final : public kache_table
     // million reads on the host (three passes and a counting sort) would take longer than the kernel that follows.
     static constexpr size_t host_list_max = 16384;
 
-    Batch_Info stage_gathered(const char* const* seqs, const size_t* lens, const size_t n, const uint64_t bytes)
+    Batch_Info stage_gathered(const char* const* seqs, const size_t* lens, const size_t n, const uint64_t bytes, const bool group)
     {
         const size_t o_hb = (n + 1) * 8;
         pin_.ensure(o_hb + bytes + 64);
@@ -805,7 +808,7 @@ class Engine final : public kache_table
             i0 = i1;
         }
         check(cudaMemsetAsync(d + bytes, 0, 64, stream_), "memset");
-        return stage_dev(reinterpret_cast<const uint8_t*>(d), reinterpret_cast<const uint64_t*>(d + o_off), n);
+        return stage_dev(reinterpret_cast<const uint8_t*>(d), reinterpret_cast<const uint64_t*>(d + o_off), n, group);
     }
 
     // A launch over nsegs segments: its blocks, and the counter its warps take segments from (null: fixed shares). Rows cost
@@ -831,8 +834,11 @@ class Engine final : public kache_table
         return Shares{grid_for(nsegs, stream_warps), nullptr};
     }
 
+    // Batches of at least so many sequences may be listed in groups of short ones: fewer have a warp for most of theirs.
+    static constexpr uint64_t group_min = 16384;
+
     // A device batch's staging arguments: the offsets of one, or none for the caller to set several.
-    Stage new_stage(const uint64_t* off, const uint64_t n)
+    Stage new_stage(const uint64_t* off, const uint64_t n, const bool group = true)
     {
         const uint64_t blocks = (n + stage_block - 1) / stage_block;
         dtmp_.ensure((3 * (n + 1) + 2 * blocks) * 8);
@@ -840,6 +846,7 @@ class Engine final : public kache_table
         a.off = off, a.n = n, a.k = k, a.sms = static_cast<uint32_t>(sm_count_), a.max_pos = ~0ull;
         a.npos = dtmp_.as<uint64_t>(), a.pos_off = a.npos + (n + 1), a.seg_off = a.pos_off + (n + 1);
         a.blocks = reinterpret_cast<unsigned long long*>(a.seg_off + (n + 1)), a.ctr = ctr();
+        a.group = group && n >= group_min;
         return a;
     }
 
@@ -851,12 +858,15 @@ class Engine final : public kache_table
         try
         {
             dbatch_.ensure(a.max_segs * sizeof(Segment));
+            if(a.group)
+                dgroups_.ensure(a.n / group_seqs * sizeof(Segment));
         }
         catch(const std::bad_alloc&)
         {
-            a.max_segs = 0;
+            a.max_segs = 0, a.group = false;
+            dgroups_.release();
         }
-        a.segs = dbatch_.as<Segment>();
+        a.segs = dbatch_.as<Segment>(), a.groups = dgroups_.as<Segment>();
         const unsigned blocks = static_cast<unsigned>((a.n + stage_block - 1) / stage_block);
         if(a.n <= small_stage_max)
             launch(K_OTHER, [&](){ stage_small_kernel<<<1, stage_block, 0, stream_>>>(a); });
@@ -873,13 +883,22 @@ class Engine final : public kache_table
     // Whether to run a batch of n sequences directly (run_staged) rather than after the host has read its counts.
     bool direct(const uint64_t n) const { return n > 0 && fits_[n > small_stage_max]; }
 
-    // Stages a batch and runs the visitor over it with no host read in between; returns the counters, of which [4] and [6]
-    // are equal if the batch ran. The launch's grid is made for the segments that the batch may have, as their number is
-    // unknown here: above small_stage_max sequences those that the list has room for. (On a grid for one of each sequence, a
-    // quarter of the warps of a lookup of 4,100 reads, one in four of two segments, took two in turn: 80 us against 56.)
+    // Whether the last batch that could have groups had some.
+    bool groups_seen_ = false;
+
+    // Whether a staged batch's segments and groups were run, given the counters behind it.
+    static bool ran(const unsigned long long* c, const Stage& a) { return c[9] && c[3] <= a.max_pos; }
+
+    // Stages a batch and runs the visitor over it with no host read in between; returns the counters (see ran()). The
+    // launch's grid is made for the segments that the batch may have, as their number is unknown here: above small_stage_max
+    // sequences those that the list has room for. (On a grid for one of each sequence, a quarter of the warps of a lookup of
+    // 4,100 reads, one in four of two segments, took two in turn: 80 us against 56.) The launch over groups is made ahead of
+    // the counters if the last such batch had groups, as the batches of a stream are mostly alike, else behind them if the
+    // batch has some.
     template <typename Vis> const unsigned long long* run_staged(const uint32_t kind, const uint8_t* bases, Stage& a, const Vis& vis)
     {
         launch_stage(a);
+        const Dev_Batch b = dev_batch(bases, a);
         launch(kind, [&]()
         {
             Shares s = shares(a.n, 128, Vis::min_blocks, false);
@@ -887,12 +906,30 @@ class Engine final : public kache_table
                 s.blocks = sm_count_ * Vis::min_blocks;
             else if(!s.taken)
                 s.blocks = grid_for(a.max_segs, stream_warps);
-            stream_kernel<k, l, Vis><<<s.blocks, 32 * stream_warps, 0, stream_>>>(Dev_Batch{bases, a.segs}, 0, 0, ctr() + 6, s.taken, vis);
+            stream_kernel<k, l, Vis><<<s.blocks, 32 * stream_warps, 0, stream_>>>(b, 0, 0, ctr() + 6, s.taken, vis);
         });
-        const unsigned long long* c = read_ctr(10);
+        const bool ahead = a.group && groups_seen_;
+        if(ahead)
+            groups_launch(kind, b, 0, a.n / group_seqs, ctr() + 10, vis);
+        const unsigned long long* c = read_ctr(ctr_words);
         fits_[a.n > small_stage_max] = c[9];
+        if(a.group)
+            groups_seen_ = c[11] > 0;
+        if(!ahead && c[10])
+        {
+            groups_launch(kind, b, 0, c[10], nullptr, vis);
+            c = read_ctr(ctr_words);
+        }
         return c;
     }
+
+    // Runs the visitor over groups [gb, ge), or of those over as many as `run` says.
+    template <typename Vis> void groups_launch(const uint32_t kind, const Dev_Batch& b, const uint64_t gb, const uint64_t ge, const unsigned long long* run, const Vis& vis)
+    {
+        launch(kind, [&](){ group_kernel<k, l, Vis><<<grid_for(ge - gb, stream_warps), 32 * stream_warps, 0, stream_>>>(b, gb, ge, run, vis); });
+    }
+
+    static Dev_Batch dev_batch(const uint8_t* bases, const Stage& a) { return Dev_Batch{bases, a.segs, a.groups, a.desc ? a.addr : a.off, a.pos_off}; }
 
     // Makes room for a list of n segments, or where memory does not take it, of a quarter (8 bytes for each of the n); the
     // segments that there is room for.
@@ -924,9 +961,12 @@ class Engine final : public kache_table
             return bi;
         a.max_pos = ~0ull;
         launch_stage(a);
-        const unsigned long long* c = read_ctr(10);
+        const unsigned long long* c = read_ctr(ctr_words);
         const uint64_t nsegs = c[4], run = c[6];
         fits_[a.n > small_stage_max] = c[9];
+        if(a.group)
+            groups_seen_ = c[11] > 0;
+        bi.ngroups = c[11];
         bi.nsegs = nsegs, bi.total_pos = c[3], bi.off = a.off, bi.pos_off = a.pos_off, bi.seg_off = a.seg_off;
         bi.staged = a, bi.seg_len = static_cast<uint32_t>(c[5]);
         if(run != nsegs)
@@ -937,12 +977,13 @@ class Engine final : public kache_table
             else
                 list_segments(bi, 0, nsegs, dbatch_.as<Segment>());
         }
-        bi.b = Dev_Batch{bases, dbatch_.as<Segment>()};
+        a.segs = dbatch_.as<Segment>();
+        bi.b = dev_batch(bases, a);
         return bi;
     }
-    Batch_Info stage_dev(const uint8_t* bases, const uint64_t* off, const uint64_t n) { return stage_dev(bases, new_stage(off, n)); }
+    Batch_Info stage_dev(const uint8_t* bases, const uint64_t* off, const uint64_t n, const bool group = true) { return stage_dev(bases, new_stage(off, n, group)); }
 
-    // Runs the visitor over segments [sb, se) of a batch, a warp per segment (device_stream.cuh).
+    // Runs the visitor over entries [sb, se) of a batch, its segments and then its groups, a warp each (device_stream.cuh).
     template <typename Vis> void stream_launch(const uint32_t kind, const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Vis& vis)
     {
         if(se <= sb)
@@ -957,7 +998,10 @@ class Engine final : public kache_table
             segs_launch(kind, bi, std::max(sb, bi.half_seg), se, vis);
             return;
         }
-        segs_launch(kind, bi, sb, se, vis);
+        if(sb < bi.nsegs)
+            segs_launch(kind, bi, sb, std::min(se, bi.nsegs), vis);
+        if(se > bi.nsegs)
+            groups_launch(kind, bi.b, std::max(sb, bi.nsegs) - bi.nsegs, se - bi.nsegs, nullptr, vis);
     }
 
     template <typename Vis> void segs_launch(const uint32_t kind, const Batch_Info& bi, const uint64_t sb, const uint64_t se, const Vis& vis)
@@ -1115,8 +1159,7 @@ class Engine final : public kache_table
     // Upserts a staged batch with the value functor `fn`, chunk by chunk (see the top of this file).
     template <typename Fn> uint64_t run_upsert(const uint32_t user, const Batch_Info& bi, const Fn& fn, unsigned long long* per = nullptr, const bool by_batch = false)
     {
-        const uint64_t nsegs = bi.nsegs;
-        const double pos_per_seg = nsegs ? static_cast<double>(bi.total_pos) / nsegs : 1.0;
+        const uint64_t entries = bi.entries();
         uint64_t total_ins = 0;
         // Keys inserted per position: as the previous call measured (1/2 before the first), then as the last chunk
         // measured. The device table is first grown to the capacity the schedule would reach at that rate, so that
@@ -1129,9 +1172,12 @@ class Engine final : public kache_table
         const size_t bits = bi.total_pos / 8 + 8;
         unsigned int* retried = reinterpret_cast<unsigned int*>(ctr() + 2);
 
-        for(uint64_t sb = 0; sb < nsegs; )
+        for(uint64_t sb = 0; sb < entries; )
         {
             clear_retries(bits);
+            // Chunks are of segments or of groups, sized as if all positions were in those, unless all fits in one.
+            const uint64_t nsegs = sb < bi.nsegs ? bi.nsegs : entries;
+            const double pos_per_seg = static_cast<double>(bi.total_pos) / static_cast<double>(sb < bi.nsegs ? bi.nsegs : bi.ngroups);
             // A chunk may take the device table to 95 % of its slots, at a quarter above the expected rate (and at
             // least a quarter of the positions); the schedule then resizes it, as the reference would.
             const double slots = static_cast<double>(T_.cap * B);
@@ -1143,6 +1189,8 @@ class Engine final : public kache_table
             if(se + (se - sb) / 2 >= nsegs && static_cast<double>(nsegs - sb) * pos_per_seg * rate <= 1.25 * room)
                 se = nsegs;
             se = std::min(se, nsegs);
+            if(sb == 0 && static_cast<double>(bi.total_pos) * rate <= 1.25 * room)
+                se = entries;
             assume_all_new = false;
 
             check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
@@ -1153,7 +1201,7 @@ class Engine final : public kache_table
             const unsigned long long* c = read_ctr(3);
             const uint64_t ins = c[0] + retry_full(bi, sb, se, fn, per, by_batch, c);
 
-            const double chunk_pos = (se - sb) * pos_per_seg;
+            const double chunk_pos = std::min((se - sb) * pos_per_seg, static_cast<double>(bi.total_pos));
             novelty = chunk_pos > 0 ? std::max(static_cast<double>(ins) / chunk_pos, 1e-3) : novelty;
             total_ins += ins;
             inserted(acct, ins, c[1]);
@@ -1232,14 +1280,14 @@ class Engine final : public kache_table
         blank_ = false;
         unsigned int* retried = reinterpret_cast<unsigned int*>(ctr() + 2);
         const unsigned long long* c = run_staged(K_UPSERT, bases, a, Upsert_Visitor<set_, VT, Fn>{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per, per != nullptr});
-        if(c[6] != c[4])
+        if(!ran(c, a))
             return false;
         Batch_Info bi;
-        bi.b = Dev_Batch{bases, dbatch_.as<Segment>()};
-        bi.n = a.n, bi.total_pos = c[3], bi.nsegs = c[4];
+        bi.b = dev_batch(bases, a);
+        bi.n = a.n, bi.total_pos = c[3], bi.nsegs = c[4], bi.ngroups = c[11];
         ins = c[0];
         if(static_cast<uint32_t>(c[2]))
-            ins += retry_full(bi, 0, bi.nsegs, fn, per, per != nullptr, c);
+            ins += retry_full(bi, 0, bi.entries(), fn, per, per != nullptr, c);
         Call_Acct acct(Sched{approx_sz_, cap_, resize_th_, step_, lf_}, pending_[user]);
         inserted(acct, ins, c[1]);
         upsert_done(user, acct, ins, bi.total_pos);
@@ -1250,25 +1298,25 @@ class Engine final : public kache_table
     {
         check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
         Update_Visitor<VT, Fn> vis{T_, fn, ctr(), nullptr};
-        stream_launch(K_UPDATE, bi, 0, bi.nsegs, vis);
+        stream_launch(K_UPDATE, bi, 0, bi.entries(), vis);
         return read_ctr(3)[0];
     }
 
     void run_lookup(const Batch_Info& bi, uint8_t* found, VT* values, uint8_t* fwd)
     {
         Lookup_Visitor<set_, VT> vis{T_, found, values, fwd};
-        stream_launch(K_LOOKUP, bi, 0, bi.nsegs, vis);
+        stream_launch(K_LOOKUP, bi, 0, bi.entries(), vis);
     }
 
     void run_seq_reduce(const Batch_Info& bi, const int mode, const uint64_t mf, const uint64_t mr, unsigned long long* out)
     {
         check(cudaMemsetAsync(out, 0, bi.n * 8, stream_), "memset");
         if(mode == 0)
-            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(mf), VT(mr)});
+            stream_launch(K_REDUCE, bi, 0, bi.entries(), Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(mf), VT(mr)});
         else if(mode == 1)
-            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 1>{T_, out, VT(mf), VT(mr)});
+            stream_launch(K_REDUCE, bi, 0, bi.entries(), Seq_Reduce_Visitor<set_, VT, 1>{T_, out, VT(mf), VT(mr)});
         else
-            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 2>{T_, out, VT(mf), VT(mr)});
+            stream_launch(K_REDUCE, bi, 0, bi.entries(), Seq_Reduce_Visitor<set_, VT, 2>{T_, out, VT(mf), VT(mr)});
     }
 
     // Whether host memory at p is page-locked (the caller's cudaHostAlloc'd or registered memory): copies then use it
@@ -1462,7 +1510,7 @@ public:
     uint64_t upsert_split(uint32_t user, const char* const* seqs, const size_t* lens, size_t n, uint32_t op, uint64_t x, uint64_t init, uint64_t* per_seq) override
     {
         std::lock_guard<std::mutex> g(work);
-        const auto bi = stage_host(seqs, lens, n);
+        const auto bi = stage_host(seqs, lens, n, false, nullptr, false);      // Of groups, no sequence's keys are counted.
         dout_.ensure(n * 8 + 8);
         check(cudaMemsetAsync(dout_.p, 0, n * 8, stream_), "memset");
         const uint64_t r = run_upsert(user, bi, op_fn(op, x, init), dout_.as<unsigned long long>());
@@ -1507,7 +1555,7 @@ public:
         const bool out_pinned = P_est > 0 && pinned_range(found, P_est) && (!vb_est || pinned_range(values, P_est * vb_est)) &&
                                 (!fwd || pinned_range(fwd, P_est));
         const bool pieces = out_pinned && n >= 2 * out_pieces && P_est >= (uint64_t(1) << 22);
-        const auto bi = stage_host(seqs, lens, n, pieces, &hs);
+        const auto bi = stage_host(seqs, lens, n, pieces, &hs, !pieces);    // (Pieces are ranges of sequences, which groups are not listed among.)
         const uint64_t P = bi.total_pos;
         const size_t vb = (!set_ && values) ? sizeof(VT) : 0;
         const size_t a_found = (P + 15) / 16 * 16, a_val = (P * vb + 15) / 16 * 16;
@@ -1552,7 +1600,7 @@ public:
         auto* dk = dout_.as<uint64_t>();
         auto* dh = dk + P;
         auto* dc = reinterpret_cast<uint8_t*>(dh + P);
-        stream_launch(K_OTHER, bi, 0, bi.nsegs, Describe_Visitor<k, l>{dk, dh, dc, dc + P, dc + 2 * P});
+        stream_launch(K_OTHER, bi, 0, bi.entries(), Describe_Visitor<k, l>{dk, dh, dc, dc + P, dc + 2 * P});
         d2h(key, dk, P * 8), d2h(h, dh, P * 8), d2h(cs, dc, P), d2h(fwd, dc + P, P), d2h(valid, dc + 2 * P, P);
     }
 
@@ -1593,7 +1641,7 @@ public:
             {
                 Stage a = new_stage(off, n);
                 const auto* c = run_staged(K_UPDATE, b, a, Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), nullptr});
-                if(c[6] == c[4])
+                if(ran(c, a))
                     return c[0];
             }
             return run_update(stage_dev(b, off, n), op_fn(op, x, 0));
@@ -1608,7 +1656,7 @@ public:
         {
             Stage a = new_stage(off, n);
             const auto* c = run_staged(K_LOOKUP, b, a, Lookup_Visitor<set_, VT>{T_, found, v, fwd});
-            if(c[6] == c[4])
+            if(ran(c, a))
                 return;
         }
         run_lookup(stage_dev(b, off, n), found, v, fwd);
@@ -1620,7 +1668,7 @@ public:
     kache_prepared* prepare_dev(const uint64_t* off, const uint64_t n) override
     {
         std::lock_guard<std::mutex> g(work);
-        const auto bi = stage_dev(nullptr, off, n);
+        const auto bi = stage_dev(nullptr, off, n, false);     // No groups: the handle holds no offsets.
         auto* p = new kache_prepared;
         try
         {
@@ -1652,7 +1700,7 @@ public:
     {
         std::lock_guard<std::mutex> g(work);
         Batch_Info bi;
-        bi.b = Dev_Batch{b, p.segs.as<Segment>()};
+        bi.b = Dev_Batch{b, p.segs.as<Segment>(), nullptr, nullptr, nullptr};
         bi.n = p.n, bi.nsegs = p.nsegs, bi.total_pos = p.total_pos, bi.fixed_shares = true;
         run_lookup(bi, found, set_ ? nullptr : static_cast<VT*>(values), fwd);
     }
@@ -1663,12 +1711,12 @@ public:
     {
         std::lock_guard<std::mutex> g(work);
         Batch_Info bi;
-        bi.b = Dev_Batch{b, p.segs.as<Segment>()};
+        bi.b = Dev_Batch{b, p.segs.as<Segment>(), nullptr, nullptr, nullptr};
         bi.n = p.n, bi.nsegs = p.nsegs, bi.total_pos = p.total_pos, bi.fixed_shares = true;
         auto* out = reinterpret_cast<unsigned long long*>(counts);
         if(p.n)
             check(cudaMemsetAsync(out, 0, p.n * 8, stream_), "memset");
-        stream_launch(K_REDUCE, bi, 0, bi.nsegs, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(0), VT(0)});
+        stream_launch(K_REDUCE, bi, 0, bi.entries(), Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(0), VT(0)});
     }
 
     // A number that stays the same while the table's device arrays do (a graph captured with a prepared lookup stays
@@ -1692,7 +1740,7 @@ public:
             Stage a = new_stage(off, n);
             a.zero = out, a.zero_n = n;
             const auto* c = run_staged(K_REDUCE, b, a, Seq_Reduce_Visitor<set_, VT, 0>{T_, out, VT(0), VT(0)});
-            if(c[6] == c[4])
+            if(ran(c, a))
                 return;
         }
         run_seq_reduce(stage_dev(b, off, n), 0, 0, 0, out);
@@ -1747,13 +1795,13 @@ public:
         if(direct(N))
         {
             uint64_t ins = 0;
-            bool ran = false;
+            bool done = false;
             if(kind == KACHE_B200_RUN_UPSERT)
-                ran = upsert_direct(user, nullptr, a, op_fn(op, x, y), ins, res);
+                done = upsert_direct(user, nullptr, a, op_fn(op, x, y), ins, res);
             else if(kind == KACHE_B200_RUN_UPSERT_ORIENTED)
             {
                 if constexpr(!set_)
-                    ran = upsert_direct(user, nullptr, a, ofn, ins, res);
+                    done = upsert_direct(user, nullptr, a, ofn, ins, res);
             }
             else
             {
@@ -1764,9 +1812,9 @@ public:
                     c = run_staged(K_LOOKUP, nullptr, a, Lookup_Batches_Visitor<set_, VT>{{T_, nullptr, nullptr, nullptr}, desc, pos_base, res});
                 else if constexpr(!set_)
                     c = run_staged(K_UPDATE, nullptr, a, Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), res});
-                ran = c && c[6] == c[4];
+                done = c && ran(c, a);
             }
-            if(ran)
+            if(done)
                 return results();
         }
         // Per-batch results, added up by the visitors: keys inserted, k-mers present, positions found or counts.
@@ -1783,14 +1831,14 @@ public:
             if constexpr(!set_)
             {
                 check(cudaMemsetAsync(ctr(), 0, 8, stream_), "memset");
-                stream_launch(K_UPDATE, bi, 0, bi.nsegs, Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), res});
+                stream_launch(K_UPDATE, bi, 0, bi.entries(), Update_Visitor<VT, Op_Fn<VT>>{T_, op_fn(op, x, 0), ctr(), res});
             }
         }
         else if(kind == KACHE_B200_RUN_COUNT)
-            stream_launch(K_REDUCE, bi, 0, bi.nsegs, Count_Batches_Visitor<set_, VT>{{T_, nullptr, VT(0), VT(0)}, desc, res});
+            stream_launch(K_REDUCE, bi, 0, bi.entries(), Count_Batches_Visitor<set_, VT>{{T_, nullptr, VT(0), VT(0)}, desc, res});
         else
         {
-            stream_launch(K_LOOKUP, bi, 0, bi.nsegs, Lookup_Batches_Visitor<set_, VT>{{T_, nullptr, nullptr, nullptr}, desc, pos_base, res});
+            stream_launch(K_LOOKUP, bi, 0, bi.entries(), Lookup_Batches_Visitor<set_, VT>{{T_, nullptr, nullptr, nullptr}, desc, pos_base, res});
         }
         results();
     }

@@ -184,3 +184,60 @@ def test_segment_lists_in_little_memory():
     ko, vo = O.dump()
     assert np.array_equal(kg, ko) and np.array_equal(vg, vo)
     T.close()
+
+
+@pytest.mark.parametrize("k,l,vb", [(31, 22, 4), (32, 20, 0), (27, 16, 1)])
+@pytest.mark.parametrize("n,low,high", [(16_384, 25, 40), (16_391, 0, 125), (40_003, 33, 37), (20_000, 120, 127), (16_390, 30, 33)])
+def test_groups_of_short_sequences(k, l, vb, n, low, high):
+    """Short sequences, whose k-mers are a warp's rows together in groups of eight: empty ones and ones shorter than k among
+    them, and, at 124 bases, the longest that a group takes; from the device, as one batch and as several that begin
+    inside a group of eight, and from the host."""
+    import torch
+    rng = np.random.default_rng(n)
+    b = _batch(rng.integers(low, high, n), n + k)
+    bases, off = _on_gpu(b)
+    T, O = kache.Table(k, vb, 1000, 0.8, False, l, capi=False), oracle.OracleTable(k, vb, 1000, 0.8, False)
+    u, uo = T.register(), O.register()
+    p, q = bases.data_ptr(), off.data_ptr()
+    cuts = [0, 3, 3, n // 3 | 1, n - 5, n]
+    first = [int(b.slice(0, c).positions(k).sum()) if c else 0 for c in cuts]
+    P = first[-1]
+    f, w, v, c = (torch.zeros(max(m, 1), dtype=t, device="cuda") for m, t in ((P, torch.uint8), (P, torch.uint8), (P * max(vb, 1), torch.uint8), (n, torch.int64)))
+    vp = v.data_ptr() if vb else None
+    torch.cuda.synchronize()
+
+    def parts(*outs):
+        return [(p, q + 8 * a, e - a) + tuple(o and o + size * (a if seq else x) for o, size, seq in outs) for a, e, x in zip(cuts, cuts[1:], first)]
+
+    for i in range(2):
+        assert T.upsert_dev(u, p, q, n, kache.ADD, 1, 1) == O.upsert(uo, b, kache.ADD, 1, 1)
+        assert sum(T.run_dev_batches(kache.RUN_UPSERT, parts(), kache.ADD, 1, 1, u)) == O.upsert(uo, b, kache.ADD, 1, 1)
+        assert T.upsert(u, b, kache.ADD, 1, 1) == O.upsert(uo, b, kache.ADD, 1, 1)
+        if vb:
+            half = b.slice(0, n // 2)
+            assert T.update_dev(p, q, n // 2, kache.ADD_WRAP, 5) == O.update(half, kache.ADD_WRAP, 5)
+            assert T.upsert_oriented_dev(u, p, q, n, kache.OR, 1, 2) == O.insert_oriented(uo, b, kache.OR, 1, 2)
+        fo, vo, wo = O.lookup(b)
+        co = O.count(b)
+        hits = [int((fo[x:y] == 1).sum()) for x, y in zip(first, first[1:])]
+        for merged in (False, True):
+            f.fill_(7), w.fill_(7), v.fill_(7), c.fill_(7)
+            torch.cuda.synchronize()
+            if merged:
+                assert T.run_dev_batches(kache.RUN_LOOKUP, parts((f.data_ptr(), 1, False), (vp, vb, False), (w.data_ptr(), 1, False))) == hits
+                assert T.run_dev_batches(kache.RUN_COUNT, parts((c.data_ptr(), 8, True))) == hits
+            else:
+                T.lookup_dev(p, q, n, f.data_ptr(), vp, w.data_ptr())
+                T.count_dev(p, q, n, c.data_ptr())
+            assert np.array_equal(f.cpu().numpy()[:P], fo) and np.array_equal(w.cpu().numpy()[:P], wo)
+            assert vb == 0 or np.array_equal(v.cpu().numpy()[:P * vb].view(T.vdt), vo)
+            assert np.array_equal(c.cpu().numpy().view(np.uint64), co)
+        assert np.array_equal(T.count(b), co)
+        if vb:
+            assert np.array_equal(T.count_masked(b, 1, 2), O.count_masked(b, 1, 2)) and np.array_equal(T.sum(b), O.sum(b))
+        fh, vh, wh = T.lookup(b)
+        assert np.array_equal(fh, fo) and np.array_equal(wh, wo) and (vb == 0 or np.array_equal(vh, vo))
+    kg, vg = T.dump()
+    ko, vo = O.dump()
+    assert np.array_equal(kg, ko) and (vb == 0 or np.array_equal(vg, vo))
+    T.close()
