@@ -155,6 +155,8 @@ __device__ __forceinline__ uint8_t base_bits(const uint32_t ch)
 
 // The kernels that describe and probe are bound by their instructions, most of all by the pipe of integer logic, shifts and
 // compares; multiply-adds run beside it, so hashes are multiply-adds as far as they go.
+// Their 32-bit factors are the five primes of xxHash, taken only as numbers of well mixed bits (lmer_hash has two of them off
+// by one, to be even); what is done with them is this library's own.
 
 // The key's 8-bit checksum in the table, 1..255 (0 marks an empty slot).
 __device__ __forceinline__ uint32_t checksum_of(const uint64_t key)

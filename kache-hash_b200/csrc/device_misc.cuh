@@ -19,7 +19,7 @@ __device__ __forceinline__ uint32_t place_key(const Dev_Table& T, const uint64_t
     {
         if constexpr(!set_)
             *L.val = val;
-        publish(L, false);
+        publish(L);
         if(!L.cs)
             atomicAdd(T.ov_count, 1ull);
     }

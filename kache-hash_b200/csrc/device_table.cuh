@@ -11,10 +11,17 @@
 //   ov[ov_cap]           the overflow table: {u64 ~key, u64 value, u64 ready, u64 pad}, linear probing.
 //
 // Concurrency without locks, in place of the reference's bucket spin locks (include/Streaming_Kmer_Hash_Table.hpp:
-// 1125-1212): an insert claims a slot by atomicCAS of its key word from 0, scanning the bucket's slots in order from
-// the first empty checksum, so a bucket's claimed keys always form a prefix and every inserter of a key meets any
-// earlier claim of it. It then writes the value, fences, and publishes the checksum; a racing inserter of the same key
-// that lost the CAS waits (boundedly) for that checksum before applying its update. Every inserter of a key scans the
+// 1125-1212): an insert claims a slot by atomicCAS of its key word from 0. An inserter by itself tries a bucket's slots in
+// order from the first empty checksum on; a run of lanes with one bucket tries neighbouring slots side by side, but as a
+// whole every one from there on (warp_claim). So whoever claims a slot for a key, or meets another's claim of it, has tried
+// all lower slots that were open, and the lowest slot that holds the key is the one that all settle on. A claim that a
+// lower one of its key makes void stays as a hole: checksum 0, a key that no k-mer has. Holes are rare (two warps have to
+// claim one new key in one bucket within the same few hundred nanoseconds) and last until a rebuild leaves them out; one
+// costs its slot and, for each new key of its bucket, a swap that fails, also where the bucket is full. The last slot is
+// never a hole and is claimed only by who has tried all others, so its checksum says that the bucket is full.
+// The claimer then writes the value, fences, and publishes the checksum; a racing inserter of the same key
+// that met the claim waits (boundedly) for that checksum before applying its update. (Where updates commute from a zeroed
+// value nobody fences or waits, see Op_Fn::commutes.) Every inserter of a key scans the
 // same chain -- primary bucket, then secondary p, then q, then the overflow table -- so a key has one copy. A full
 // primary bucket gets its spill-filter bit set before any key of its minimizer goes beyond it, which keeps the
 // reference's lookup rule: absent past a full primary bucket unless its filter marks the minimizer
@@ -73,15 +80,6 @@ __device__ __forceinline__ V read_val(const unsigned long long* w)
         return static_cast<V>(*w);
     else
         return static_cast<V>(*reinterpret_cast<const uint32_t*>(w));
-}
-
-template <typename V>
-__device__ __forceinline__ V read_val_cg(const unsigned long long* w)
-{
-    if constexpr(sizeof(V) == 8)
-        return static_cast<V>(__ldcg(w));
-    else
-        return static_cast<V>(__ldcg(reinterpret_cast<const uint32_t*>(w)));
 }
 
 template <typename V>
@@ -285,7 +283,7 @@ struct Checksums
 {
     uint4 lo, hi;
 
-    __device__ __forceinline__ bool full() const { return (hi.w >> 24) != 0; }  // Keys fill a bucket's slots in order.
+    __device__ __forceinline__ bool full() const { return (hi.w >> 24) != 0; }  // The last slot is claimed after all others.
     // The first slot whose checksum is empty, or B. (The inexact test can flag a byte above an empty one of its word,
     // which is a higher slot.)
     __device__ __forceinline__ uint32_t first_empty() const
@@ -512,11 +510,9 @@ __device__ __forceinline__ void warp_claim(const Dev_Table& T, const unsigned lo
     }
 }
 
-// Publishes a claimed slot after its value is written.
-__device__ __forceinline__ void publish(const Landing& L, const bool fence)
+// Publishes a claimed slot whose value nobody waits for.
+__device__ __forceinline__ void publish(const Landing& L)
 {
-    if(fence)
-        __threadfence();
     if(L.cs)
         *reinterpret_cast<volatile uint8_t*>(L.cs) = static_cast<uint8_t>(L.c);
     else

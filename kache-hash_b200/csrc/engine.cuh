@@ -613,14 +613,11 @@ class Engine final : public kache_table
 
     // ---- Batches ----
 
-    // Stages a host batch. With `defer_bases` (a lookup in pieces), a batch laid end to end in page-locked memory is
-    // listed from its offsets alone and its bases are left for the caller to copy (to bi.b.bases), piece by piece;
-    // bi.host_bases is then set.
-    // A host batch's totals, read once: bases, the longest sequence's and all sequences' positions, and whether the
-    // sequences lie end to end. Large batches are summed over the host pool.
+    // A host batch's totals, read once: bases, positions, and whether the sequences lie end to end. Large batches are
+    // summed over the host pool.
     struct Host_Scan
     {
-        uint64_t bytes = 0, max_pos = 0, all_pos = 0;
+        uint64_t bytes = 0, all_pos = 0;
         bool contiguous = true;
     };
 
@@ -638,7 +635,7 @@ class Engine final : public kache_table
                 {
                     h.bytes += lens[i];
                     const uint64_t np = lens[i] >= size_t(k) ? lens[i] - k + 1 : 0;
-                    h.max_pos = std::max<uint64_t>(h.max_pos, np), h.all_pos += np;
+                    h.all_pos += np;
                     if(i + 1 < n && seqs[i] + lens[i] != seqs[i + 1])
                         h.contiguous = false;
                 }
@@ -646,15 +643,18 @@ class Engine final : public kache_table
         });
         Host_Scan t;
         for(const auto& h : r)
-            t.bytes += h.bytes, t.max_pos = std::max(t.max_pos, h.max_pos), t.all_pos += h.all_pos, t.contiguous &= h.contiguous;
+            t.bytes += h.bytes, t.all_pos += h.all_pos, t.contiguous &= h.contiguous;
         return t;
     }
 
+    // Stages a host batch. With `defer_bases` (a lookup in pieces), a batch laid end to end in page-locked memory is
+    // listed from its offsets alone and its bases are left for the caller to copy (to bi.b.bases), piece by piece;
+    // bi.host_bases is then set.
     Batch_Info stage_host(const char* const* seqs, const size_t* lens, const size_t n, const bool defer_bases = false,
                           const Host_Scan* scanned = nullptr, const bool group = true)
     {
         const Host_Scan hs = scanned ? *scanned : scan_host(seqs, lens, n);
-        const uint64_t bytes = hs.bytes, max_pos = hs.max_pos, all_pos = hs.all_pos;
+        const uint64_t bytes = hs.bytes, all_pos = hs.all_pos;
         const bool contiguous = hs.contiguous;
         // Sequences laid end to end in page-locked memory are copied to the device as they lie, with no gather, and
         // listed in segments there (stage_dev): the host only writes the offsets, in streaming stores (host_copy.hpp).

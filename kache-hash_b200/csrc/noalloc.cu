@@ -2,7 +2,7 @@
 //
 // Some callers cannot call cudaMalloc on the path where they query the table: code running inside a memory pool
 // whose allocator must not be re-entered, or an embedding process that budgets every byte of HBM itself.
-// kache_b200_count_dev allocates the scratch it needs (segment lists, scan buffers) on first use and whenever a batch
+// kache_b200_count_dev allocates the scratch it needs (segment lists, counts of sequences) on first use and whenever a batch
 // outgrows it. This variant does the same counting
 // with its scratch in one fixed array below, which every GPU that loads the library holds until the process exits,
 // and calls no cudaMalloc, cudaFree or allocating library routine.
