@@ -1,10 +1,10 @@
-"""One logical k-mer table over the ranks of a process group, one GPU per rank, partitioned by primary-bucket range.
+"""One logical k-mer table over the ranks of a process group, one GPU per rank, partitioned by minimizer hash.
 
-The partition. A k-mer's primary bucket is ((h & 0xFFFFFFFF) * cap) >> 32 for its minimizer hash h
-(include/Streaming_Kmer_Hash_Table.hpp:1015-1019), monotone in the low 32 bits of h at every capacity. Rank r of N
-owns the k-mers with ((h & 0xFFFFFFFF) * N) >> 32 == r: a contiguous range of the logical table's buckets whatever
-its capacity, and all k-mers of a super-k-mer (consecutive k-mers sharing a minimizer) have one owner. Secondary
-buckets and overflow are the shard's own (placement is not observable).
+The partition. Rank r of N owns the k-mers whose described minimizer hash h (include/Kmer_Lanes.hpp:247-274) has
+((h & 0xFFFFFFFF) * N) >> 32 == r, so all k-mers of a super-k-mer (consecutive k-mers sharing a minimizer) have one
+owner. (In the reference's table these k-mers fill a contiguous range of buckets at every capacity,
+include/Streaming_Kmer_Hash_Table.hpp:1015-1019; where a key sits in a shard is the shard's own: placement is not
+observable.)
 
 One call, on every rank with its own batch:
   1. the batch is described on this rank (canonical keys, minimizer hashes, validity per position);
