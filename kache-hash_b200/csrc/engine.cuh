@@ -1285,7 +1285,7 @@ class Engine final : public kache_table
         if(!direct(a.n) || a.n > a.max_pos || last_pos_ > a.max_pos ||
            predicted_cap(user, static_cast<uint64_t>(novelty_ * static_cast<double>(last_pos_))) > T_.cap)
             return false;   // The last one also where the table is to grow ahead of the call (run_upsert).
-        clear_retries(most / 8 + 8);
+        clear_retries(most / 8);    // 1 MB, and not a byte more: device memory up to that is handed out in 4 us, above in 360.
         blank_ = false;
         unsigned int* retried = reinterpret_cast<unsigned int*>(ctr() + 2);
         const unsigned long long* c = run_staged(K_UPSERT, bases, a, Upsert_Visitor<set_, VT, Fn>{T_, fn, ctr(), dretry_a_.as<unsigned int>(), nullptr, retried, per, per != nullptr});
