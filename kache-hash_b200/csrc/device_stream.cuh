@@ -19,8 +19,10 @@
 //
 // What bounds it is instructions (327 per row in a lookup of 150 bp reads, issue slots two thirds used), then the latency
 // of three dependent loads; so more resident warps pay even at the price of some spills: six blocks of 256 threads per SM
-// (40 registers) against five, four and three, with fixed shares of segments, lookup of 120M positions 1.81 against 1.82,
-// 1.80 (overlapping two rows) and 2.29 ms, upsert of 40M 1.08 against 1.11, 1.15 and 1.46; now 1.73 and 0.94 ms.
+// (40 registers) against five (48, half the spills), with the work counter: an upsert of 40M positions and a lookup of 120M 2.90
+// against 2.98 ms, counts of 1M reads 1.33 against 1.39, 190M updates with a histogram 4.52 against 4.77, 40M lookups of
+// contigs 0.55 against 0.58. (Four and three, with fixed shares of segments, when six took 1.81 and 1.08 ms: lookup 1.80,
+// overlapping two rows, and 2.29 ms, upsert 1.15 and 1.46.)
 // Sequences are cut into segments of up to `seg_positions` positions; each segment re-reads the k - 1 bases it
 // shares with the next, so segments, like the reference's lanes (include/Streaming_Kmer_Hash_Table.hpp:1751-1781),
 // need no state from one another.
