@@ -241,3 +241,27 @@ def test_groups_of_short_sequences(k, l, vb, n, low, high):
     ko, vo = O.dump()
     assert np.array_equal(kg, ko) and (vb == 0 or np.array_equal(vg, vo))
     T.close()
+
+
+def test_short_sequences_in_little_memory():
+    """Short sequences, which might be run in groups, with memory for the sums over them and for a quarter of their segments'
+    list, 24 bytes and 8 for each, and none for groups."""
+    import torch
+    n = 40_000
+    b = _batch(np.full(n, 40), 17)
+    bases, off = _on_gpu(b)
+    T, O = kache.Table(31, 4, 1_000_000), oracle.OracleTable(31, 4, 1_000_000)
+    u, uo = T.register(), O.register()
+    f = torch.zeros(10 * n, dtype=torch.uint8, device="cuda")
+    p, q = bases.data_ptr(), off.data_ptr()
+    torch.cuda.synchronize()
+    assert T.upsert_dev(u, p, q, 5, kache.ADD, 1, 1) == O.upsert(uo, b.slice(0, 5), kache.ADD, 1, 1)     # The retry marks are made.
+    left = kache.lib().kache_b200_testing_device_memory
+    try:
+        left(24 * n + 8 * n + 4096)
+        assert T.upsert_dev(u, p, q, n, kache.ADD, 1, 1) == O.upsert(uo, b, kache.ADD, 1, 1)
+        T.lookup_dev(p, q, n, f.data_ptr())
+    finally:
+        left(-1)
+    assert np.array_equal(f.cpu().numpy(), O.lookup(b)[0])
+    T.close()
