@@ -353,7 +353,7 @@ struct Stage
     uint32_t sms;
     uint64_t max_segs, max_pos;
     uint64_t *npos, *pos_off, *seg_off;     // Positions of each sequence, with in_group; n + 1 sums of positions and of segments.
-    unsigned long long* blocks;     // Two words per block of stage_count_kernel: the positions before it, the segments and groups (entries).
+    unsigned long long* blocks;     // Three words per block of stage_count_kernel: the positions before it, the entries, and the segments were there no groups.
     Segment *segs, *groups;
     unsigned long long* ctr;    // [0] and the low half of [2] are zeroed; [3..6]: positions, segments, segment length, segments to run; [7]: zero between launches; [8] is zeroed; [9]: whether the segments fit the list; [10], [11]: groups to run, and listed.
     unsigned long long* zero;   // zero_n words zeroed.
@@ -396,14 +396,21 @@ __device__ __forceinline__ uint64_t entries(const uint64_t q, const uint64_t np,
     return g ? uint64_t(q % group_seqs == 0) << group_shift : (np + seg_positions - 1) / seg_positions;
 }
 
-// Whether the calling lane's sequence q, of batch `lo`, is of a group (device_stream.cuh): groups of short sequences, the first a
-// multiple of group_seqs, are made where that saves instructions, in units of ten: 45 for a row of a group and 1 for 23 of its
-// bases against 31 for a row of a sequence and 13 to start on one. A whole warp, with consecutive sequences.
-__device__ __forceinline__ bool grouped(const Stage& a, const uint64_t q, const uint64_t len, const uint64_t np, const uint64_t lo)
+// Groups of short sequences (device_stream.cuh), the first a multiple of group_seqs, are made where that saves instructions, in
+// units of ten a warp: 55 for a row of a group (43, but its lanes have several sequences' k-mers and so more buckets: reads of
+// 75 bases at 45 were no faster in groups) and 1 for 23 of its bases against 31 for a row of a sequence and 13 to start on
+// one. And a batch has groups only if they save more than the launch over them takes, at 14 ps a unit with all SMs at work:
+// some 7 us, and up to 50 beside a launch over segments that fills the SMs by itself. (Lookups of 60,000 reads of about 100
+// bases, a few of them in groups, took 149 us with those and 118 without; of 60,000 of 33, 55 with and 69 without.)
+__device__ __forceinline__ bool groups_pay(const uint64_t saved, const uint64_t segs) { return saved >= min(500'000 + 2'000 * segs, uint64_t(4'000'000)); }
+
+// What the group of the calling lane's sequence q, of batch `lo`, saves in those units; 0 if it is not to be one. A whole warp,
+// with consecutive sequences.
+__device__ __forceinline__ uint32_t group_saves(const Stage& a, const uint64_t q, const uint64_t len, const uint64_t np, const uint64_t lo)
 {
     constexpr uint32_t all = 0xFFFFFFFFu;
     if(!a.group)
-        return false;
+        return 0;
     const int leader = static_cast<int>(threadIdx.x & 31 & ~(group_seqs - 1));
     const uint64_t lo_leader = __shfl_sync(all, lo, leader);    // (All lanes take part: not behind a condition.)
     const bool ok = q < a.n && len <= group_len && lo == lo_leader;
@@ -414,7 +421,8 @@ __device__ __forceinline__ bool grouped(const Stage& a, const uint64_t q, const 
     for(uint32_t o = 1; o < group_seqs; o *= 2)
         x += __shfl_xor_sync(all, x, o);
     const uint32_t bases = x >> 20, pos = x >> 8 & 0xFFFu, rows = x & 0xFFu;
-    return no == 0 && pos > 0 && 45 * ((pos + 31) / 32) + bases / 23 + 10 < 31 * rows + 13 * group_seqs;
+    const uint32_t with = 55 * ((pos + 31) / 32) + bases / 23 + 10, without = 31 * rows + 13 * group_seqs;
+    return no == 0 && pos > 0 && with < without ? without - with : 0;
 }
 
 // The group that starts at sequence q: `pos` positions, from `first` on, the last sequence's np_last among them.
@@ -432,24 +440,13 @@ __device__ __forceinline__ Segment stage_segment(const Stage& a, const uint64_t 
     return Segment{(a.desc ? a.addr[q] : a.off[q]) + p0, first + p0, q, static_cast<uint32_t>(min(np - p0, seg_len)), a.desc ? a.batch_of[q] : 0};
 }
 
-// The inclusive sum of x over the block's threads in order; `warps` is 32 words of shared memory.
-__device__ __forceinline__ unsigned long long block_sum(unsigned long long x, unsigned long long* warps)
+// Makes each of x the inclusive sum of its own over the block's threads in order; warps[.][31] is then the block's.
+template <int n_>
+__device__ __forceinline__ void block_sums(unsigned long long (&x)[n_], unsigned long long (*warps)[32])
 {
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for(int o = 1; o < 32; o <<= 1)
+    const auto warp_sum = [&](unsigned long long& a)
     {
-        const unsigned long long a = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if(lane >= static_cast<uint32_t>(o))
-            x += a;
-    }
-    __syncthreads();    // The words' last use is over.
-    if(lane == 31)
-        warps[wid] = x;
-    __syncthreads();
-    if(wid == 0)
-    {
-        unsigned long long a = warps[lane];
 #pragma unroll
         for(int o = 1; o < 32; o <<= 1)
         {
@@ -457,10 +454,43 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long x, un
             if(lane >= static_cast<uint32_t>(o))
                 a += y;
         }
-        warps[lane] = a;
+    };
+    __syncthreads();    // The words' last use is over.
+#pragma unroll
+    for(int i = 0; i < n_; ++i)
+    {
+        warp_sum(x[i]);
+        if(lane == 31)
+            warps[i][wid] = x[i];
     }
     __syncthreads();
-    return x + (wid ? warps[wid - 1] : 0);
+    if(wid < n_)
+    {
+        unsigned long long a = warps[wid][lane];
+        warp_sum(a);
+        warps[wid][lane] = a;
+    }
+    __syncthreads();
+#pragma unroll
+    for(int i = 0; i < n_; ++i)
+        x[i] += wid ? warps[i][wid - 1] : 0;
+}
+
+// The inclusive sum of x over the block's threads in order; `warps` is 32 words of shared memory.
+__device__ __forceinline__ unsigned long long block_sum(const unsigned long long x, unsigned long long* warps)
+{
+    unsigned long long a[1] = {x};
+    block_sums<1>(a, reinterpret_cast<unsigned long long(*)[32]>(warps));
+    return a[0];
+}
+
+// The sum of x over the warp.
+__device__ __forceinline__ unsigned long long warp_total(unsigned long long x)
+{
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1)
+        x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
+    return x;
 }
 
 static __global__ void __launch_bounds__(stage_block) stage_small_kernel(const Stage a)
@@ -530,8 +560,8 @@ static __global__ void __launch_bounds__(stage_block) stage_small_kernel(const S
 // of them one block's: otherwise the host, which reads so, lists them by a thread each (segs_kernel).
 static __global__ void __launch_bounds__(stage_block) stage_count_kernel(const Stage a)
 {
-    __shared__ unsigned long long wp[32], ws[32], most;     // `most`: segments of a block.
-    __shared__ bool last;
+    __shared__ unsigned long long w[3][32];
+    __shared__ bool last, most[2];      // `most`: whether a block has too many segments, without groups and with.
     const uint32_t t = threadIdx.x;
     const uint64_t q = uint64_t(blockIdx.x) * stage_block + t;
     uint64_t np = 0, len = 0, lo = 0;
@@ -540,40 +570,54 @@ static __global__ void __launch_bounds__(stage_block) stage_count_kernel(const S
         len = stage_length(a, q, lo, true);
         np = len >= uint64_t(a.k) ? len - a.k + 1 : 0;
     }
-    const bool g = grouped(a, q, len, np, lo);
+    const uint32_t saves = group_saves(a, q, len, np, lo);
     if(q < a.n)
-        a.npos[q] = g ? np | in_group : np;
+        a.npos[q] = saves ? np | in_group : np;
     for(uint64_t i = q; i < a.zero_n; i += uint64_t(gridDim.x) * stage_block)
         a.zero[i] = 0;
-    block_sum(np, wp);
-    block_sum(entries(q, np, g), ws);
-    if(t == 0)
+    // The block's positions; its entries; the segments without groups, and above them what the groups would save, in sixteens
+    // of its units.
+    unsigned long long p = warp_total(np), x = a.group ? warp_total(entries(q, np, saves != 0)) : 0;
+    unsigned long long y = warp_total(entries(q, np, false) | uint64_t(q % group_seqs ? 0 : saves / 16) << group_shift);
+    if((t & 31) == 0)
+        w[0][t >> 5] = p, w[1][t >> 5] = x, w[2][t >> 5] = y;
+    __syncthreads();
+    if(t < 32)
     {
-        __stcg(a.blocks + 2 * blockIdx.x, wp[31]), __stcg(a.blocks + 2 * blockIdx.x + 1, ws[31]);
-        __threadfence();
-        last = atomicAdd(a.ctr + 7, 1ull) == gridDim.x - 1, most = 0;
-        __threadfence();
+        p = warp_total(w[0][t]), x = warp_total(w[1][t]), y = warp_total(w[2][t]);
+        if(t == 0)
+        {
+            __stcg(a.blocks + 3 * blockIdx.x, p), __stcg(a.blocks + 3 * blockIdx.x + 1, x), __stcg(a.blocks + 3 * blockIdx.x + 2, y);
+            __threadfence();
+            last = atomicAdd(a.ctr + 7, 1ull) == gridDim.x - 1, most[0] = most[1] = false;
+            __threadfence();
+        }
     }
     __syncthreads();
     if(!last)
         return;
-    unsigned long long P = 0, S = 0;
+    unsigned long long P = 0, S = 0, Q = 0;
     for(uint64_t b0 = 0; b0 < gridDim.x; b0 += stage_block)
     {
         const uint64_t b = b0 + t;
-        const unsigned long long p = b < gridDim.x ? __ldcg(a.blocks + 2 * b) : 0, s = b < gridDim.x ? __ldcg(a.blocks + 2 * b + 1) : 0;
-        const unsigned long long p1 = block_sum(p, wp), s1 = block_sum(s, ws);
-        if((s & segs_mask) > small_segs_max)
-            atomicMax(&most, s);
-        if(b < gridDim.x)
-            a.blocks[2 * b] = P + p1 - p, a.blocks[2 * b + 1] = S + s1 - s;
-        P += wp[31], S += ws[31];
+        const bool in = b < gridDim.x;
+        p = in ? __ldcg(a.blocks + 3 * b) : 0, x = in ? __ldcg(a.blocks + 3 * b + 1) : 0, y = in ? __ldcg(a.blocks + 3 * b + 2) : 0;
+        unsigned long long to[3] = {p, x, y};
+        block_sums(to, w);
+        if((y & segs_mask) > small_segs_max)
+            most[0] = true;
+        if((x & segs_mask) > small_segs_max)
+            most[1] = true;
+        if(in)
+            a.blocks[3 * b] = P + to[0] - p, a.blocks[3 * b + 1] = S + to[1] - x, a.blocks[3 * b + 2] = Q + to[2] - y;
+        P += w[0][31], S += w[1][31], Q += w[2][31];
     }
     __syncthreads();
     if(t == 0)
     {
-        const uint64_t segs = S & segs_mask, groups = S >> group_shift;
-        const bool fits = segs <= a.max_segs && most == 0, run = fits && P <= a.max_pos;
+        const bool g = groups_pay((Q >> group_shift) * 16, S & segs_mask);
+        const uint64_t segs = (g ? S : Q) & segs_mask, groups = g ? S >> group_shift : 0;
+        const bool fits = segs <= a.max_segs && !most[g], run = fits && P <= a.max_pos;
         a.pos_off[a.n] = P, a.seg_off[a.n] = segs;
         a.ctr[3] = P, a.ctr[4] = segs, a.ctr[5] = seg_positions, a.ctr[6] = run ? segs : 0;
         a.ctr[0] = 0, *reinterpret_cast<uint32_t*>(a.ctr + 2) = 0, a.ctr[7] = 0, a.ctr[8] = 0, a.ctr[9] = fits;
@@ -588,15 +632,17 @@ constexpr uint32_t own_segs = 32;
 
 static __global__ void __launch_bounds__(stage_block) stage_list_kernel(const Stage a)
 {
-    __shared__ unsigned long long wp[32], ws[32];
+    __shared__ unsigned long long w[2][32];
     const uint64_t q = uint64_t(blockIdx.x) * stage_block + threadIdx.x;
     constexpr uint32_t all = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31;
     uint64_t np = q < a.n ? a.npos[q] : 0;
-    const bool g = np & in_group;
+    const bool groups = a.ctr[11] != 0, g = groups && (np & in_group);
     np &= ~in_group;
     const uint64_t x = entries(q, np, g), ns = x & segs_mask;
-    const unsigned long long first = a.blocks[2 * blockIdx.x] + block_sum(np, wp) - np, before = a.blocks[2 * blockIdx.x + 1] + block_sum(x, ws) - x;
+    unsigned long long to_here[2] = {np, x};
+    block_sums(to_here, w);
+    const unsigned long long first = a.blocks[3 * blockIdx.x] + to_here[0] - np, before = a.blocks[3 * blockIdx.x + (groups ? 1 : 2)] + to_here[1] - x;
     const uint64_t first_seg = before & segs_mask;
     if(q < a.n)
     {

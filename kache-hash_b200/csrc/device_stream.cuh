@@ -301,7 +301,7 @@ __device__ __forceinline__ Kmer_Desc group_kmer(const uint32_t j, const uint32_t
 }
 
 // The kernel over groups [grp_b, grp_end), or as many as `run` says, counted by the kernel before. A row costs some 430
-// instructions, where a segment's costs 330 and its start 120: which sequences make a group is staging's choice (`grouped`).
+// instructions, where a segment's costs 330 and its start 120: which sequences make a group is staging's choice (`group_saves`).
 // A kernel of its own, behind the one over segments: as a branch of that one it cost the rows of 150 bp reads 4 to 6 %, whose
 // registers are few enough as it is, and with one loop for both kinds of row they took three times as long.
 template <int k, int l, typename Visitor>

@@ -841,7 +841,7 @@ class Engine final : public kache_table
     void stage_room(Stage& a)
     {
         const uint64_t blocks = (a.n + stage_block - 1) / stage_block;
-        const uint64_t sums = (3 * (a.n + 1) + 2 * blocks + 1) / 2 * 2 * 8;
+        const uint64_t sums = (3 * (a.n + 1) + 3 * blocks + 1) / 2 * 2 * 8;
         dtmp_.ensure(sums + (a.group ? a.n / group_seqs * sizeof(Segment) : 0));
         a.npos = dtmp_.as<uint64_t>(), a.pos_off = a.npos + (a.n + 1), a.seg_off = a.pos_off + (a.n + 1);
         a.blocks = reinterpret_cast<unsigned long long*>(a.seg_off + (a.n + 1));

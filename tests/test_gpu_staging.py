@@ -265,3 +265,50 @@ def test_short_sequences_in_little_memory():
         left(-1)
     assert np.array_equal(f.cpu().numpy(), O.lookup(b)[0])
     T.close()
+
+
+# Groups are made where they save 500,000 units (groups_pay, device_misc.cuh) and 2,000 for each segment beside them, or
+# 4,000,000. These batches' would save 0, 0, 557,056 with no segments, 552,432 with 170, 1,083,200 with 3, 2,109,024 with 8,846,
+# 5,549,824 with 12,500, and of eight sequences one of which has 124 bases 1,600,000, or, of 125, 0.
+@pytest.mark.parametrize("n,low,high,every,launches", [
+    (17_000, 60, 140, 0, 3), (60_000, 75, 76, 0, 3), (16_384, 33, 34, 0, 4), (16_384, 33, 34, 1000, 3), (40_003, 33, 37, 0, 4), (250_000, 0, 60, 200, 3),
+    (250_000, 31, 46, 200, 4), (80_000, 124, 0, 0, 4), (80_000, 125, 0, 0, 3),
+])
+def test_groups_only_where_they_pay(n, low, high, every, launches):
+    """Lookups and counts of reads of `low` to `high` - 1 bases, one in `every` of 1,100: by how many launches, and against the
+    oracle, as one batch and as two."""
+    import torch
+    lens = np.random.default_rng(n).integers(low, high, n) if high else np.resize([31, 31, 0, 33, 31, 30, 31, low], n)
+    if every:
+        lens[5::every] = 1100
+    b = _batch(lens, n + low)
+    bases, off = _on_gpu(b)
+    T, O = kache.Table(31, 4, 1_000_000), oracle.OracleTable(31, 4, 1_000_000)
+    p, q = bases.data_ptr(), off.data_ptr()
+    torch.cuda.synchronize()
+    u, uo = T.register(), O.register()
+    for s in range(0, n // 2, 5000):        # In batches too small for groups.
+        part = b.slice(s, min(n // 2, s + 5000))
+        assert T.upsert(u, part, kache.ADD, 1, 1) == O.upsert(uo, part, kache.ADD, 1, 1)
+    P = int(b.positions(31).sum())
+    f, v, c = (torch.full((m,), 7, dtype=t, device="cuda") for m, t in ((P, torch.uint8), (P, torch.int32), (n, torch.int64)))
+    torch.cuda.synchronize()
+    before = kache.kernel_launches()
+    T.lookup_dev(p, q, n, f.data_ptr(), v.data_ptr())
+    assert kache.kernel_launches() - before == launches
+    fo, vo, _ = O.lookup(b)
+    co = O.count(b)
+    assert np.array_equal(f.cpu().numpy(), fo) and np.array_equal(v.cpu().numpy().view(np.uint32), vo)
+    T.count_dev(p, q, n, c.data_ptr())
+    assert np.array_equal(c.cpu().numpy().view(np.uint64), co)
+    cut = n // 3 | 1
+    x = int(b.slice(0, cut).positions(31).sum())
+    f.fill_(7)
+    torch.cuda.synchronize()
+    assert T.run_dev_batches(kache.RUN_LOOKUP, [(p, q, cut, f.data_ptr()), (p, q + 8 * cut, n - cut, f.data_ptr() + x)]) == [int((fo[:x] == 1).sum()), int((fo[x:] == 1).sum())]
+    assert np.array_equal(f.cpu().numpy(), fo)
+    assert T.upsert_dev(u, p, q, n, kache.ADD, 1, 1) == O.upsert(uo, b, kache.ADD, 1, 1)
+    kg, vg = T.dump()
+    ko, vo = O.dump()
+    assert np.array_equal(kg, ko) and np.array_equal(vg, vo)
+    T.close()
